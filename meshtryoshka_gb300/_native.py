@@ -110,6 +110,8 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     ),
     "mt_composite_staging_bytes": (c_size_t, [I32, I64]),
     "mt_ssaa_loss": (I32, [P, I32, I32, I32, I32, P, P, c_float, P, P, P]),
+    "mt_finish_images": (I32, [P, I32, P, I32, P, P, P]),
+    "mt_finish_images_backward": (I32, [P, I32, P, I32, P, P, P, P]),
     "mt_intersect": (I32, [P, I64, P, P, P, I32, I32, I32, I32, I32, I32, I32, I32, P, P, P]),
     "mt_interpolate": (I32, [P, P, I32, I32, I32, I32, P, P, P, I64, P, P, P]),
     "mt_interpolate_backward": (I32, [P, P, I32, I32, I32, I32, P, I64, P, P, P, P, P]),

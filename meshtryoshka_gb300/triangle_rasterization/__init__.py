@@ -724,6 +724,63 @@ def intersect_and_composite(vertices, colors, signed_distances, faces, sharpness
 
 
 # ---------------------------------------------------------------------------
+# Background blend, SSAA mean and clip (triangle_rasterization/__init__.py:274-287)
+# ---------------------------------------------------------------------------
+class FinishImages(torch.autograd.Function):
+    """The images of a fused render from its compositing output, in one kernel
+    each way. ``shapes``: (height, width) of every camera's output image;
+    ``stacked``: one [B, 3, h, w] tensor (cameras of one size), else one
+    [3, h, w] tensor per camera, each an allocation of its own."""
+
+    @staticmethod
+    def _pointers(tensors, shapes, stacked):
+        if stacked:
+            (t,) = tensors
+            h, w = shapes[0]
+            found = [None if t is None else t.data_ptr() + 12 * h * w * b for b in range(len(shapes))]
+        else:
+            found = [None if t is None else t.data_ptr() for t in tensors]
+        return (ctypes.c_void_p * len(found))(*found)
+
+    @staticmethod
+    def forward(ctx, raw, background, shapes, ssaa, stacked):
+        with record_function("finish_images_forward"):
+            kw = dict(dtype=torch.float32, device=raw.device)
+            images = ((torch.empty((len(shapes), 3, *shapes[0]), **kw),) if stacked
+                      else tuple(torch.empty((3, h, w), **kw) for h, w in shapes))
+            sizes = (ctypes.c_int32 * (2 * len(shapes)))(*(x for shape in shapes for x in shape))
+            nt.call("mt_finish_images", nt.ptr(raw), len(shapes), sizes, ssaa, nt.ptr(background),
+                    FinishImages._pointers(images, shapes, stacked), nt.stream(raw.device),
+                    launches=(len(shapes) + 63) // 64)
+            ctx.save_for_backward(raw, background)
+            ctx.meta = (shapes, ssaa, stacked, sizes)
+            ctx.set_materialize_grads(False)
+            return images[0] if stacked else images
+
+    @staticmethod
+    def backward(ctx, *grads):
+        with record_function("finish_images_backward"):
+            raw, background = ctx.saved_tensors
+            shapes, ssaa, stacked, sizes = ctx.meta
+            grads = tuple(None if g is None else g.contiguous() for g in grads)
+            grad_raw = torch.empty_like(raw)  # fully written
+            nt.call("mt_finish_images_backward", nt.ptr(raw), len(shapes), sizes, ssaa, nt.ptr(background),
+                    FinishImages._pointers(grads, shapes, stacked), nt.ptr(grad_raw), nt.stream(raw.device),
+                    launches=(len(shapes) + 63) // 64)
+            return grad_raw, None, None, None, None
+
+
+def _finishable(raw: Tensor, background: Tensor) -> bool:
+    """Whether the finishing kernels take this background: a plain float32
+    [3] on the render's device that no gradient or tangent is asked of.
+    Everything else goes through tensor operations."""
+    return (type(background) in (Tensor, torch.nn.Parameter) and background.device == raw.device
+            and background.dtype == torch.float32 and background.shape == (3,) and background.is_contiguous()
+            and not (background.requires_grad and torch.is_grad_enabled())
+            and torch.autograd.forward_ad._current_level < 0)
+
+
+# ---------------------------------------------------------------------------
 # Explicit mode (intersect.py, interpolate.py, composite.py)
 # ---------------------------------------------------------------------------
 class RenderedImages(NamedTuple):
@@ -922,6 +979,8 @@ def render_fused(extrinsics, intrinsics, image_shape, vertices, faces, shell_fac
     images = intersect_and_composite(positions, colors, signed_distances, faces, sharpness, paired.keys,
                                      paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
                                      gradient_mode, paired.count)
+    if b > 0 and isinstance(ssaa, int) and _finishable(images, background):
+        return FinishImages.apply(images, background, ((int(h), int(w)),) * b, max(ssaa, 1), True)
     images = images[:, :3] + images[:, 3:4] * background[:, None, None]
     if ssaa > 1:
         images = _mean_pool(images, ssaa)
@@ -971,6 +1030,8 @@ def render_cameras(extrinsics, intrinsics, image_shapes, vertices, faces, shell_
     raw = intersect_and_composite(positions, colors, signed_distances, faces, sharpness, paired.keys,
                                   paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
                                   gradient_mode, paired.count)
+    if _finishable(raw, background):
+        return list(FinishImages.apply(raw, background, grid.camera_shapes, 1, False))
     bg = background[:, None, None]
     return [(r[:3] + r[3:4] * bg).clip(min=0, max=1) for r in split_cameras(raw, grid)]
 
