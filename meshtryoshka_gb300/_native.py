@@ -125,6 +125,8 @@ _lock = threading.Lock()
 
 def _load():
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -230,7 +232,11 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """Handle of the current stream (asked of the runtime's own table: a
+    torch.cuda.Stream object costs 5 us on a Grace core, and every entry point
+    needs the handle)."""
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:
@@ -291,7 +297,7 @@ _workspaces: dict[tuple[int, int], Workspace] = {}
 
 def workspace(device: torch.device) -> Workspace:
     index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (index, torch.cuda.current_stream(device).cuda_stream)
+    key = (index, torch._C._cuda_getCurrentRawStream(index))
     ws = _workspaces.get(key)
     if ws is None:
         ws = Workspace(device)

@@ -12,7 +12,48 @@ compare the timed form of the step with the oracle stage by stage.
 
 from __future__ import annotations
 
+import functools
 from contextlib import contextmanager
+
+import torch
+from torch.autograd import profiler
+from torch.profiler import record_function
+
+_Fast = getattr(torch._C._profiler, "_RecordFunctionFast", record_function)
+
+
+class annotate:
+    """``record_function(name)``, as a decorator or a context, at the cost of
+    one only while a profiler runs.
+
+    ``record_function`` goes through the operator dispatcher on its way in and
+    out, some 20 us of host time on a Grace core, and a small training step
+    opens 18 of them; otherwise the C++ form is opened, which reaches whatever
+    else observes operators. With the stream handles read directly and one
+    device read less, an eager 64^3 step with one 128^2 camera went from 2.34
+    to 1.45 ms, a 4 x 800^2 render with its gradients from 1.57 to 1.23 ms."""
+
+    def __init__(self, name: str):
+        self.name = name
+
+    def _open(self):
+        return (record_function if profiler._is_profiler_enabled else _Fast)(self.name)
+
+    def __enter__(self):
+        self._context = self._open()
+        return self._context.__enter__()
+
+    def __exit__(self, *exc):
+        return self._context.__exit__(*exc)
+
+    def __call__(self, function):
+        @functools.wraps(function)
+        def annotated(*args, **kwargs):
+            with self._open():
+                return function(*args, **kwargs)
+
+        return annotated
+
 
 _ACTIVE: list[dict] = []
 

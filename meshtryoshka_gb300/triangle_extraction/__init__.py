@@ -20,10 +20,9 @@ from typing import NamedTuple
 import numpy as np
 import torch
 from torch import Tensor
-from torch.profiler import record_function
 
 from .. import _native as nt
-from ..record import note
+from ..record import annotate, note
 
 __all__ = [
     "Voxels",
@@ -97,7 +96,7 @@ def unpack_occupancy(packed_occupancy: Tensor) -> Tensor:
 # ---------------------------------------------------------------------------
 # Scan (triangle_extraction/compute_exclusive_cumsum.py:19-21).
 # ---------------------------------------------------------------------------
-@record_function("compute_exclusive_cumsum")
+@annotate("compute_exclusive_cumsum")
 def compute_exclusive_cumsum(x: Tensor) -> None:
     """In-place exclusive prefix sum of a contiguous int32 CUDA tensor."""
     if x.dtype != torch.int32 or not x.is_contiguous():
@@ -139,7 +138,7 @@ class Voxels(NamedTuple):
         return self.lower_corners.shape[1] - self.upper_corners.shape[1]
 
 
-@record_function("compute_vertex_occupancy")
+@annotate("compute_vertex_occupancy")
 def compute_vertex_occupancy(occupancy: Tensor) -> VertexOccupancyFnResult:
     occupancy = _i32(occupancy, "occupancy")
     device = nt.require_cuda(occupancy)
@@ -155,7 +154,7 @@ def compute_vertex_occupancy(occupancy: Tensor) -> VertexOccupancyFnResult:
     return VertexOccupancyFnResult(vertex_occupancy, vertex_counts)
 
 
-@record_function("count_occupancy")
+@annotate("count_occupancy")
 def count_occupancy(occupancy: Tensor) -> Tensor:
     occupancy = _i32(occupancy, "occupancy")
     device = nt.require_cuda(occupancy)
@@ -165,7 +164,7 @@ def count_occupancy(occupancy: Tensor) -> Tensor:
     return counts
 
 
-@record_function("create_voxels")
+@annotate("create_voxels")
 def create_voxels(
     occupancy: Tensor,
     voxel_offsets: Tensor,
@@ -201,7 +200,7 @@ def create_voxels(
     return Voxels(vertices, neighbors, lower_corners, upper_corners, indices, (i, j, kp * 32))
 
 
-@record_function("extract_voxels")
+@annotate("extract_voxels")
 def extract_voxels(occupancy: Tensor) -> Voxels:
     """Packed occupancy [i, j, kp] -> sparse voxel topology (one host sync)."""
     occupancy = _i32(occupancy, "occupancy")
@@ -224,7 +223,7 @@ def extract_voxels(occupancy: Tensor) -> Voxels:
     )
 
 
-@record_function("dilate_occupancy")
+@annotate("dilate_occupancy")
 def dilate_occupancy(occupancy: Tensor, dilation: int) -> Tensor:
     if dilation == 0:
         return occupancy.clone()
@@ -242,7 +241,7 @@ def dilate_occupancy(occupancy: Tensor, dilation: int) -> Tensor:
 # Coarse-to-fine subdivision (tesseract.py:396-486), occupancy mesh and
 # vertex de-duplication. These run at subdivision steps and in the viewer.
 # ---------------------------------------------------------------------------
-@record_function("write_occupancy")
+@annotate("write_occupancy")
 def write_occupancy(voxel_indices: Tensor, packed_occupancy_shape: tuple[int, ...], min_shell: int,
                     max_shell: int) -> Tensor:
     """Packed occupancy with the bit of every triangle's voxel set
@@ -277,7 +276,7 @@ def _upscale_occupancy(occupancy: Tensor, mask: Tensor | None, target_shape: tup
     return out
 
 
-@record_function("upscale_occupancy")
+@annotate("upscale_occupancy")
 def upscale_occupancy(occupancy: Tensor, target_shape: tuple[int, int, int]) -> Tensor:
     """[i, j, kp] -> [i', j', k'/32] with every extent at least the old one
     (upscale_occupancy.py:24-54)."""
@@ -290,7 +289,7 @@ class UpscaledParameters(NamedTuple):
     occupancy: Tensor  # [i, j, k_packed] int32
 
 
-@record_function("upscale_parameters")
+@annotate("upscale_parameters")
 @torch.no_grad()
 def upscale_parameters(old_signed_distances: Tensor, old_spherical_harmonics: Tensor, old_occupancy: Tensor,
                        occupancy_to_upscale: Tensor, new_resolution: tuple[int, int, int]) -> UpscaledParameters:
@@ -332,7 +331,7 @@ class Mesh(NamedTuple):
     colors: Tensor  # [triangle, 3] float32
 
 
-@record_function("get_occupancy_mesh")
+@annotate("get_occupancy_mesh")
 def get_occupancy_mesh(occupancy: Tensor, colors: Tensor) -> Mesh:
     """Two triangles per face between occupied and free voxels, coloured by
     ``colors[axis, side]`` (get_occupancy_mesh.py:32-80). One host read."""
@@ -420,7 +419,7 @@ def index_vertices(points: Tensor, tol: float = 1e-5) -> Tensor:
 # ---------------------------------------------------------------------------
 # Per-step marching cubes.
 # ---------------------------------------------------------------------------
-@record_function("count_triangle_vertices")
+@annotate("count_triangle_vertices")
 def count_triangle_vertices(signed_distances: Tensor, lower_corners: Tensor, level_sets: Tensor) -> Tensor:
     signed_distances = _f32(signed_distances, "signed_distances")
     lower_corners = _i32(lower_corners, "lower_corners")
@@ -479,7 +478,7 @@ class GridSHColors(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, grid_spherical_harmonics, vertices, extrinsics, sh_degree, deferred):
-        with record_function("grid_sh_colors_forward"):
+        with annotate("grid_sh_colors_forward"):
             gsh = _f32(grid_spherical_harmonics, "grid_spherical_harmonics")
             vertices = _f32(vertices, "vertices")
             extrinsics = _f32(extrinsics, "extrinsics")
@@ -503,7 +502,7 @@ class GridSHColors(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_colors):
-        with record_function("grid_sh_colors_backward"):
+        with annotate("grid_sh_colors_backward"):
             vertices, campos, colors = ctx.saved_tensors
             d = ctx.deferred
             c, g, _ = ctx.gsh_shape
@@ -540,7 +539,7 @@ class CreateTriangleVertices(torch.autograd.Function):
     @staticmethod
     def forward(ctx, grid_vertices, grid_signed_distances, grid_spherical_harmonics, voxel_lower_corners,
                 level_sets, vertex_offsets, num_vertices=None, capacity=None, deferred=None, live_t=False):
-        with record_function("create_triangle_vertices_forward"):
+        with annotate("create_triangle_vertices_forward"):
             grid_vertices = _f32(grid_vertices, "grid_vertices")
             grid_signed_distances = _f32(grid_signed_distances, "grid_signed_distances")
             grid_spherical_harmonics = _f32(grid_spherical_harmonics, "grid_spherical_harmonics")
@@ -605,7 +604,7 @@ class CreateTriangleVertices(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_vertices, grad_signed_distances, grad_spherical_harmonics, grad_types):
-        with record_function("create_triangle_vertices_backward"):
+        with annotate("create_triangle_vertices_backward"):
             grid_signed_distances, lower_corners, level_sets, vertex_offsets = ctx.saved_tensors
             gv_shape, gsh_shape, v = ctx.shapes
             device = grid_signed_distances.device
@@ -690,7 +689,7 @@ class CountTriangleFacesResult(NamedTuple):
     face_counts: Tensor
 
 
-@record_function("count_triangle_faces")
+@annotate("count_triangle_faces")
 def count_triangle_faces(
     signed_distances: Tensor, lower_corners: Tensor, upper_corners: Tensor, level_sets: Tensor
 ) -> CountTriangleFacesResult:
@@ -717,7 +716,7 @@ class CreateTriangleFacesResult(NamedTuple):
     voxel_indices: Tensor | None
 
 
-@record_function("create_triangle_faces")
+@annotate("create_triangle_faces")
 def create_triangle_faces(
     signed_distances: Tensor,
     neighbors: Tensor,
@@ -776,7 +775,7 @@ class SDFRegularizerLosses(NamedTuple):
 class ComputeSDFRegularizers(torch.autograd.Function):
     @staticmethod
     def forward(ctx, grid_signed_distances, voxel_neighbors, voxel_lower_corners, voxel_upper_corners, grid_size):
-        with record_function("compute_sdf_regularizers_forward"):
+        with annotate("compute_sdf_regularizers_forward"):
             sdf = _f32(grid_signed_distances, "grid_signed_distances")
             neighbors = _i32(voxel_neighbors, "voxel_neighbors")
             lower, upper = _i32(voxel_lower_corners, "voxel_lower_corners"), _i32(voxel_upper_corners,
@@ -796,7 +795,7 @@ class ComputeSDFRegularizers(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_pos, grad_neg, grad_curv):
-        with record_function("compute_sdf_regularizers_backward"):
+        with annotate("compute_sdf_regularizers_backward"):
             sdf, neighbors, lower, upper = ctx.saved_tensors
             i, j, k = ctx.grid_size
             _, g = lower.shape
@@ -827,7 +826,7 @@ class TessellationCounts(NamedTuple):
     num_faces: Tensor  # [] int32
 
 
-@record_function("tessellate_voxels")
+@annotate("tessellate_voxels")
 def tessellate_voxels(
     signed_distances: Tensor,
     vertices: Tensor,
@@ -910,10 +909,13 @@ def _tessellate(signed_distances, vertices, spherical_harmonics, neighbors, lowe
                                                               level_sets)
         compute_exclusive_cumsum(face_offsets)
         if capacity is None:
-            # One device->host read for both totals (and the scan status word).
-            totals = torch.stack((vertex_offsets[-1], face_offsets[-1])).cpu()
-            nt.workspace(device).check()
-            num_vertices, num_faces = int(totals[0]), int(totals[1]) // 3
+            # One device->host read for both totals and the scans' status word.
+            ws = nt.workspace(device)
+            num_vertices, total, status = torch.cat(
+                (vertex_offsets[-1:], face_offsets[-1:], ws.buffer[:4].view(torch.int32))).tolist()
+            if status != 0:
+                ws.check()
+            num_faces = total // 3
             counts = None
         else:
             num_vertices, num_faces = capacity

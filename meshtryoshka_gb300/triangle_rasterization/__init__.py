@@ -27,10 +27,9 @@ from typing import Literal, NamedTuple
 
 import torch
 from torch import Tensor
-from torch.profiler import record_function
 
 from .. import _native as nt
-from ..record import note
+from ..record import annotate, note
 
 __all__ = [
     "render",
@@ -257,7 +256,7 @@ class ProjectedVertices(NamedTuple):
     depths: Tensor  # [B, V]
 
 
-@record_function("project_vertices")
+@annotate("project_vertices")
 def project_vertices(vertices: Tensor, extrinsics: Tensor, intrinsics: Tensor) -> ProjectedVertices:
     vertices, extrinsics, intrinsics = _f32(vertices), _f32(extrinsics), _f32(intrinsics)
     device = nt.require_cuda(vertices, extrinsics, intrinsics)
@@ -277,7 +276,7 @@ class TriangleBounds:
     num_tiles_overlapped: Tensor  # [B, F]
 
 
-@record_function("bound_triangles")
+@annotate("bound_triangles")
 def bound_triangles(vertices: Tensor, depths: Tensor, faces: Tensor, grid: TileGrid,
                     near_plane: float, num_faces: Tensor | None = None) -> TriangleBounds:
     """``num_faces`` (optional, not in the reference signature): a device
@@ -313,7 +312,7 @@ class PairedKeys:
         return self.keys.shape[0]
 
 
-@record_function("generate_keys")
+@annotate("generate_keys")
 def generate_keys(depths: Tensor, faces: Tensor, shell_face_boundaries: Tensor, tile_minima: Tensor,
                   tile_maxima: Tensor, num_tiles_overlapped: Tensor, grid: TileGrid,
                   key_defines, capacity: int | None = None) -> PairedKeys:
@@ -347,7 +346,7 @@ def generate_keys(depths: Tensor, faces: Tensor, shell_face_boundaries: Tensor, 
     return PairedKeys(keys, tri, live)
 
 
-@record_function("bound_and_generate_keys")
+@annotate("bound_and_generate_keys")
 def bound_and_generate_keys(vertices: Tensor, depths: Tensor, faces: Tensor, shell_face_boundaries: Tensor,
                             grid: TileGrid, near_plane: float, key_defines, capacity: int,
                             num_faces: Tensor | None = None) -> PairedKeys:
@@ -387,7 +386,7 @@ def _keys(positions, depths, faces, shell_face_boundaries, grid, near_plane, num
                          bounds.num_tiles_overlapped, grid, key_defines)
 
 
-@record_function("sort_keys")
+@annotate("sort_keys")
 def sort_keys(paired_keys: PairedKeys, grid: TileGrid | None = None) -> PairedKeys:
     """Stable sort by signed int64 key (the CUB SortPairs of the reference);
     stream-ordered, so no device synchronisation is needed afterwards."""
@@ -406,7 +405,7 @@ def sort_keys(paired_keys: PairedKeys, grid: TileGrid | None = None) -> PairedKe
     return PairedKeys(out_keys, out_tri, live)
 
 
-@record_function("delineate_tiles")
+@annotate("delineate_tiles")
 def delineate_tiles(sorted_paired_keys: PairedKeys, grid: TileGrid, key_defines, separate_shells: bool,
                     epsilon: float = 1e-8) -> Tensor:
     keys = sorted_paired_keys.keys.contiguous()
@@ -470,7 +469,7 @@ def _camera_positions(extrinsics: Tensor) -> Tensor:
 class EvaluateSphericalHarmonics(torch.autograd.Function):
     @staticmethod
     def forward(ctx, vertices, spherical_harmonics, extrinsics, sh_degree):
-        with record_function("evaluate_spherical_harmonics_forward"):
+        with annotate("evaluate_spherical_harmonics_forward"):
             vertices, sh = _f32(vertices), _f32(spherical_harmonics)
             device = nt.require_cuda(vertices, sh, extrinsics)
             campos = _camera_positions(extrinsics)
@@ -487,7 +486,7 @@ class EvaluateSphericalHarmonics(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_colors):
-        with record_function("evaluate_spherical_harmonics_backward"):
+        with annotate("evaluate_spherical_harmonics_backward"):
             vertices, campos, colors = ctx.saved_tensors
             grad_colors = grad_colors.contiguous()
             device = vertices.device
@@ -567,7 +566,7 @@ class IntersectAndComposite(torch.autograd.Function):
     @staticmethod
     def forward(ctx, vertices, colors, signed_distances, faces, sharpness, sorted_keys, sorted_triangle_indices,
                 tile_boundaries, num_shells, grid, key_defines, gradient_mode=None, num_keys=None):
-        with record_function("intersect_and_composite_forward"):
+        with annotate("intersect_and_composite_forward"):
             xy, colors, sdf, faces = _f32(vertices), _f32(colors), _f32(signed_distances), _i32(faces)
             device = nt.require_cuda(xy, colors, sdf, faces)
             sharp = _sharpness(sharpness, device)
@@ -601,7 +600,7 @@ class IntersectAndComposite(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_out):
-        with record_function("intersect_and_composite_backward"):
+        with annotate("intersect_and_composite_backward"):
             xy, colors, sdf, faces, sharp, keys, tri, bounds, masks, out = ctx.saved_tensors
             num_shells, grid, key_defines, mode, sharp_is_tensor = ctx.meta
             device = xy.device
@@ -640,7 +639,7 @@ class IntersectCompositeLoss(torch.autograd.Function):
     def forward(ctx, vertices, colors, signed_distances, faces, sharpness, sorted_keys, sorted_triangle_indices,
                 tile_boundaries, num_shells, grid, key_defines, target, background, gradient_mode=None,
                 num_keys=None, ssaa=1):
-        with record_function("intersect_composite_loss_forward"):
+        with annotate("intersect_composite_loss_forward"):
             xy, colors, sdf, faces = _f32(vertices), _f32(colors), _f32(signed_distances), _i32(faces)
             target, background = _f32(target), _f32(background)
             device = nt.require_cuda(xy, colors, sdf, faces, target, background)
@@ -688,7 +687,7 @@ class IntersectCompositeLoss(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_loss):
-        with record_function("intersect_composite_loss_backward"):
+        with annotate("intersect_composite_loss_backward"):
             xy, colors, sdf, faces, sharp, keys, tri, bounds, masks, out, target, background = ctx.saved_tensors
             num_shells, grid, key_defines, mode, sharp_is_tensor, scale, ssaa = ctx.meta
             device = xy.device
@@ -744,7 +743,7 @@ class FinishImages(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, raw, background, shapes, ssaa, stacked):
-        with record_function("finish_images_forward"):
+        with annotate("finish_images_forward"):
             kw = dict(dtype=torch.float32, device=raw.device)
             images = ((torch.empty((len(shapes), 3, *shapes[0]), **kw),) if stacked
                       else tuple(torch.empty((3, h, w), **kw) for h, w in shapes))
@@ -759,7 +758,7 @@ class FinishImages(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, *grads):
-        with record_function("finish_images_backward"):
+        with annotate("finish_images_backward"):
             raw, background = ctx.saved_tensors
             shapes, ssaa, stacked, sizes = ctx.meta
             grads = tuple(None if g is None else g.contiguous() for g in grads)
@@ -788,7 +787,7 @@ class RenderedImages(NamedTuple):
     index: Tensor  # [B, S, H, W] (-1 = miss)
 
 
-@record_function("intersect")
+@annotate("intersect")
 def intersect(vertices: Tensor, faces: Tensor, sorted_triangle_indices: Tensor, tile_boundaries: Tensor,
               grid: TileGrid, key_defines) -> RenderedImages:
     xy, faces, tri = _f32(vertices), _i32(faces), _i32(sorted_triangle_indices)
@@ -809,7 +808,7 @@ def intersect(vertices: Tensor, faces: Tensor, sorted_triangle_indices: Tensor, 
 class Interpolate(torch.autograd.Function):
     @staticmethod
     def forward(ctx, uv, index, faces, signed_distances, colors):
-        with record_function("interpolate_forward"):
+        with annotate("interpolate_forward"):
             uv, index, faces = _f32(uv), _i32(index), _i32(faces)
             sdf, colors = _f32(signed_distances), _f32(colors)
             device = nt.require_cuda(uv, index, faces, sdf, colors)
@@ -825,7 +824,7 @@ class Interpolate(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_sdf, grad_colors):
-        with record_function("interpolate_backward"):
+        with annotate("interpolate_backward"):
             uv, index, faces = ctx.saved_tensors
             sdf_shape, colors_shape = ctx.shapes
             device = uv.device
@@ -846,7 +845,7 @@ def interpolate(uv, index, faces, signed_distances, colors):
 class Composite(torch.autograd.Function):
     @staticmethod
     def forward(ctx, signed_distances, colors, mask, sharpness, gradient_mode=None):
-        with record_function("composite_forward"):
+        with annotate("composite_forward"):
             sdf, colors = _f32(signed_distances), _f32(colors)
             device = nt.require_cuda(sdf, colors, mask)
             mask_u8 = mask.contiguous().view(torch.uint8) if mask.dtype == torch.bool else mask.to(torch.uint8)
@@ -863,7 +862,7 @@ class Composite(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_colors, grad_t):
-        with record_function("composite_backward"):
+        with annotate("composite_backward"):
             sdf, colors, mask, sharp, out_colors, out_t = ctx.saved_tensors
             mode, sharp_is_tensor = ctx.meta
             device = sdf.device
@@ -887,7 +886,7 @@ def composite(signed_distances, colors, mask, background, sharpness, gradient_mo
 # ---------------------------------------------------------------------------
 # Render entry points (triangle_rasterization/__init__.py:22-329)
 # ---------------------------------------------------------------------------
-@record_function("rasterize")
+@annotate("rasterize")
 def rasterize(vertices, faces, shell_face_boundaries, extrinsics, intrinsics, image_shape, tile_shape=(16, 16),
               near_plane=0.2, num_camera_bits=6, num_shell_bits=6, num_tile_bits=20) -> RenderedImages:
     h, w = image_shape
@@ -923,7 +922,7 @@ def _mean_pool(images: Tensor, ssaa: int) -> Tensor:
     return images.reshape(b, c, h // ssaa, ssaa, w // ssaa, ssaa).mean(dim=(3, 5))
 
 
-@record_function("render_explicit")
+@annotate("render_explicit")
 def render_explicit(extrinsics, intrinsics, image_shape, vertices, faces, shell_face_boundaries, signed_distances,
                     spherical_harmonics, sh_degree, sharpness, background, tile_shape=(16, 16), near_plane=0.2,
                     num_camera_bits=6, num_shell_bits=6, num_tile_bits=20, ssaa=1, gradient_mode=None) -> Tensor:
@@ -946,7 +945,7 @@ def render_explicit(extrinsics, intrinsics, image_shape, vertices, faces, shell_
     return image
 
 
-@record_function("render_fused")
+@annotate("render_fused")
 def render_fused(extrinsics, intrinsics, image_shape, vertices, faces, shell_face_boundaries, signed_distances,
                  spherical_harmonics, sh_degree, sharpness, background, tile_shape=(16, 16), near_plane=0.2, ssaa=1,
                  num_camera_bits=6, num_shell_bits=6, num_tile_bits=20, gradient_mode=None,
@@ -996,7 +995,7 @@ def split_cameras(raw: Tensor, grid: TileGrid) -> list[Tensor]:
     return views
 
 
-@record_function("render_cameras")
+@annotate("render_cameras")
 def render_cameras(extrinsics, intrinsics, image_shapes, vertices, faces, shell_face_boundaries, signed_distances,
                    spherical_harmonics, sh_degree, sharpness, background, tile_shape=(16, 16), near_plane=0.2,
                    num_camera_bits=6, num_shell_bits=6, num_tile_bits=20, gradient_mode=None,
@@ -1036,7 +1035,7 @@ def render_cameras(extrinsics, intrinsics, image_shapes, vertices, faces, shell_
     return [(r[:3] + r[3:4] * bg).clip(min=0, max=1) for r in split_cameras(raw, grid)]
 
 
-@record_function("render_fused_loss")
+@annotate("render_fused_loss")
 def render_fused_loss(extrinsics, intrinsics, image_shape, vertices, faces, shell_face_boundaries, signed_distances,
                       spherical_harmonics, sh_degree, sharpness, background, target, tile_shape=(16, 16),
                       near_plane=0.2, num_camera_bits=6, num_shell_bits=6, num_tile_bits=20, gradient_mode=None,
