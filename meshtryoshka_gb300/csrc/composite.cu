@@ -311,8 +311,103 @@ __device__ __forceinline__ TriangleBounds3 triangle_bounds(const TriGeom& g) {
                          edge_bound(g.d1223, g.d1323, g.p2x, g.p2y, g.e13x, g.e13y, g.e12x, g.e12y)};
 }
 
+// The columns of a pixel row that a triangle may be accepted at: [xl, xu],
+// inside the accept box, minus what one of the three barycentric numerators
+// provably rejects. edge_excludes applied to a single pixel centre p says
+// that numerator j rejects p when
+//   a qx + b qy + 2E (sx |qx| + sy |qy|) < thr,  q = p - P_j.
+// On a row (qy fixed) this reads g(qx) = a qx + 2E sx |qx| < R with
+// R = thr - b qy - 2E sy |qy|. When |a| > 2E sx, g is monotonic, so the
+// columns that survive form a ray bounded at the root of g(qx) = R (on the
+// side of zero that the sign of R selects), which is widened here by a
+// padding far above the rounding of this computation. Otherwise (an edge
+// within a few ulps of horizontal) g <= 4E sx |qx|, and the edge removes the
+// whole row when that bound stays below R at the farthest of the columns
+// asked about, [bx, bx + width].
+//
+// Branch-free, as a warp's lanes hold edges of every direction: each edge
+// carries its inverses ordered by the sign of R, and bounds that never bind
+// (infinities) for the sides that it does not limit.
+struct RowEdge {
+  float b, sy, px, py;
+  float inv_neg, inv_pos;  // 1 / (a -+ 2E sx) for R <= 0 and for R > 0
+  float flat;              // the bound of a flat edge over the columns asked about; otherwise infinite
+  bool lower, upper;       // limits the columns from the left / from the right
+};
+
+constexpr float kRowError = 0x1p-18f;  // 2E: 2 x 32 u, as in edge_excludes for one point
+
+// 1 / x to an ulp, which the columns' padding covers many times over; x is
+// not subnormal where the result is used (a limiting edge of a triangle whose
+// denominator exceeds 2^-20).
+__device__ __forceinline__ float fast_reciprocal(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+__device__ __forceinline__ RowEdge row_edge(const EdgeBound& e, float bx, float width) {
+  const float slack = kRowError * e.sx;
+  const float inv_lo = fast_reciprocal(e.a - slack), inv_hi = fast_reciprocal(e.a + slack);
+  RowEdge r;
+  r.b = e.b;
+  r.sy = kRowError * e.sy;
+  r.px = e.px;
+  r.py = e.py;
+  r.lower = e.a > slack;   // g increasing: columns at or right of the root survive
+  r.upper = e.a < -slack;  // g decreasing: columns at or left of the root survive
+  r.inv_neg = r.lower ? inv_lo : inv_hi;
+  r.inv_pos = r.lower ? inv_hi : inv_lo;
+  const float qf = fmaxf(fabsf(bx - e.px), fabsf(bx + width - e.px));
+  r.flat = r.lower || r.upper ? __int_as_float(0x7f800000) : 2.02f * slack * qf;
+  return r;
+}
+
+struct RowEdges {
+  RowEdge e[3];
+};
+
+__device__ __forceinline__ RowEdges row_edges(const TriGeom& g, float bx, float width) {
+  const TriangleBounds3 tb = triangle_bounds(g);
+  return RowEdges{{row_edge(tb.v, bx, width), row_edge(tb.w, bx, width), row_edge(tb.u, bx, width)}};
+}
+
+// False when no column of the row survives.
+__device__ __forceinline__ bool row_columns(const RowEdges& q, const CullBox& box, float thr, float y, float& xl,
+                                            float& xu) {
+  const float inf = __int_as_float(0x7f800000);
+  xl = box.x0;
+  xu = box.x1;
+  bool empty = false;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const RowEdge& e = q.e[j];
+    const float qy = y - e.py;
+    const float R = thr - (e.b * qy + e.sy * fabsf(qy));
+    const float x = R * (R <= 0.0f ? e.inv_neg : e.inv_pos);
+    const float root = e.px + x, pad = 0.0625f + 0x1p-16f * (fabsf(e.px) + fabsf(x));
+    xl = fmaxf(xl, e.lower ? root - pad : -inf);
+    xu = fminf(xu, e.upper ? root + pad : inf);
+    empty = empty || e.flat < R;
+  }
+  return !empty;
+}
+
 // The warp blocks of its tile that a key's triangle (corners pa, pb, pc) may
-// cover: bit w = warp w.
+// be accepted in: bit w = warp w.
+//
+// With 8x4 blocks, row by row: the pixel rows of the tile inside the
+// triangle's accept box, each with its surviving columns; a block's bit is
+// set when one of its rows keeps a column of it. So a warp meets only the
+// triangles that can hit one of its pixel centres. A mask by the blocks' edge
+// exclusion alone (the other tile shapes') lets through every triangle that
+// lies near a block: on the 256^3 / 8 shells / 4 x 800^2 step (8x8 tiles,
+// triangles of one to two pixels) two thirds of the (warp, triangle) pairs
+// that were staged had no hit. The rows cost this kernel 24 us there (50 to
+// 74 us, bound by its 59 M warp instructions) and save the forward 46 us (219
+// to 173) and the backward 22 us (220 to 198); a 256^2 view of the same mesh,
+// whose triangles are a fraction of a pixel, goes from 950 to 580 us in the
+// forward.
 __device__ __forceinline__ uint32_t key_mask(const CompositeArgs& a, int warps, int tile, int cols_b, float2 pa,
                                              float2 pb, float2 pc) {
   TriGeom g;
@@ -322,8 +417,26 @@ __device__ __forceinline__ uint32_t key_mask(const CompositeArgs& a, int warps, 
   // Exclusion needs the fast reject, finite coordinates and a
   // well-conditioned triangle: exactly the triangles with a finite box.
   const bool exact_cull = box.x0 > -__int_as_float(0x7f800000);
-  const TriangleBounds3 tb = triangle_bounds(g);
   uint32_t m = 0;
+  if (exact_cull && (a.tile_w & 7) == 0 && (a.tile_h & 3) == 0) {
+    const float bx = (float)(tx * a.tile_w) + 0.5f, by = (float)(ty * a.tile_h) + 0.5f;
+    const int per_row = a.tile_w >> 3;
+    const float last = (float)(a.tile_w - 1);
+    const RowEdges q = row_edges(g, bx, last);
+    const int r0 = max((int)ceilf(fmaxf(box.y0 - by, -1.0f)), 0);
+    const int r1 = min((int)floorf(fminf(box.y1 - by, (float)a.tile_h)), a.tile_h - 1);
+    for (int r = r0; r <= r1; ++r) {
+      float xl, xu;
+      if (!row_columns(q, box, g.thr, by + (float)r, xl, xu)) continue;
+      const int c0 = max((int)ceilf(fmaxf(xl - bx, -1.0f)), 0);
+      const int c1 = (int)floorf(fminf(xu - bx, last));
+      if (c0 > c1) continue;
+      const int b0 = c0 >> 3, b1 = c1 >> 3;  // block columns b0 .. b1
+      m |= ((2u << (b1 - b0)) - 1u) << (b0 + (r >> 2) * per_row);
+    }
+    return m;
+  }
+  const TriangleBounds3 tb = triangle_bounds(g);
   for (int w = 0; w < warps; ++w) {
     float x0, x1, y0, y1;
     warp_block_rect(w, a.tile_w, a.tile_h, tx, ty, x0, x1, y0, y1);
@@ -533,54 +646,18 @@ __device__ __forceinline__ int span_count(uint32_t span) {
 }
 
 // Span of a staged triangle over the 8x4 block whose first pixel centre is
-// (bx, by), row by row: the columns of a row inside the accept box that none
-// of the three barycentric numerators provably rejects. edge_excludes applied
-// to a single pixel centre p says that numerator j rejects p when
-//   a qx + b qy + 2E (sx |qx| + sy |qy|) < thr,  q = p - P_j.
-// On a row (qy fixed) this reads g(qx) = a qx + 2E sx |qx| < R with
-// R = thr - b qy - 2E sy |qy|. When |a| > 2E sx, g is monotonic, so the
-// columns that survive form a ray bounded at the root of g(qx) = R (on the
-// side of zero that the sign of R selects), which is widened here by a
-// padding far above the rounding of this computation. Otherwise (an edge
-// within a few ulps of horizontal) g <= 4E sx |qx|, and the edge removes the
-// whole row when that bound stays below R at the row's farthest column.
-// Triangles without an exact fast reject (open accept box) span every pixel.
+// (bx, by), row by row: the columns that row_columns leaves. Triangles
+// without an exact fast reject (open accept box) span every pixel.
 __device__ __forceinline__ uint32_t edge_span(const TriGeom& g, const CullBox& box, float bx, float by) {
   if (!(box.x0 > -__int_as_float(0x7f800000))) return kFullSpan;
-  constexpr float k2E = 0x1p-18f;  // 2 x 32 u, as in edge_excludes for one point
-  const TriangleBounds3 tb = triangle_bounds(g);
-  const EdgeBound eb[3] = {tb.v, tb.w, tb.u};
-  float slack[3], inv_lo[3], inv_hi[3];  // 2E sx, 1 / (a - 2E sx), 1 / (a + 2E sx)
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    slack[j] = k2E * eb[j].sx;
-    inv_lo[j] = __frcp_rn(eb[j].a - slack[j]);
-    inv_hi[j] = __frcp_rn(eb[j].a + slack[j]);
-  }
+  const RowEdges q = row_edges(g, bx, 7.0f);
   uint32_t span = 0u;
 #pragma unroll 1  // rolled: the unrolled rows cost more in instruction-cache misses than they save
   for (int r = 0; r < 4; ++r) {
     const float y = by + (float)r;
     if (!(y >= box.y0 && y <= box.y1)) continue;
-    float xl = box.x0, xu = box.x1;
-    bool empty = false;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const EdgeBound& e = eb[j];
-      const float qy = y - e.py;
-      const float R = g.thr - (e.b * qy + k2E * e.sy * fabsf(qy));
-      if (e.a > slack[j]) {  // g increasing: columns at or right of the root survive
-        const float q = R * (R <= 0.0f ? inv_lo[j] : inv_hi[j]);
-        xl = fmaxf(xl, e.px + q - (0.0625f + 0x1p-16f * (fabsf(e.px) + fabsf(q))));
-      } else if (e.a < -slack[j]) {  // g decreasing: columns at or left of the root survive
-        const float q = R * (R <= 0.0f ? inv_hi[j] : inv_lo[j]);
-        xu = fminf(xu, e.px + q + (0.0625f + 0x1p-16f * (fabsf(e.px) + fabsf(q))));
-      } else {
-        const float qf = fmaxf(fabsf(bx - e.px), fabsf(bx + 7.0f - e.px));
-        empty = empty || 2.02f * slack[j] * qf < R;
-      }
-    }
-    if (empty) continue;
+    float xl, xu;
+    if (!row_columns(q, box, g.thr, y, xl, xu)) continue;
     const int c0 = max((int)ceilf(fmaxf(xl - bx, -1.0f)), 0);
     const int c1 = min((int)floorf(fminf(xu - bx, 8.0f)), 7);
     if (c0 <= c1) span |= ((uint32_t)c0 | ((uint32_t)(c1 - c0 + 1) << 3)) << (8 * r);

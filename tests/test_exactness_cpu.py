@@ -390,3 +390,45 @@ def test_hit_bit_reservations_fit_the_store_bound():
                     assert r >= walked
                     reserved += r
             assert reserved <= k * warps // 32 + items
+
+
+def _tight_box(g, p):
+    """cull_box with its tighter margin for small triangles."""
+    box = _cull_box(g, p)
+    if box is None:
+        return None
+    ext = max(f32(p[:, 0].max() - p[:, 0].min()), f32(p[:, 1].max() - p[:, 1].min()))
+    m = f32(f32(0.0625) + f32(f32(0.25) * ext))
+    tight = (f32(p[:, 0].min() - m), f32(p[:, 0].max() + m), f32(p[:, 1].min() - m), f32(p[:, 1].max() + m))
+    return (max(box[0], tight[0]), min(box[1], tight[1]), max(box[2], tight[2]), min(box[3], tight[3]))
+
+
+def test_tight_accept_box_holds_every_pixel_that_escapes_the_fast_reject():
+    """Near the conditioning limit (sin^2 of an angle down to 1e-4), from a
+    hundredth of a pixel to several pixels, at coordinates up to 4000."""
+    rng = np.random.default_rng(11)
+    shapes = list(_triangles(rng, 800))
+    for _ in range(2500):
+        c, size = rng.uniform(0, rng.choice([50, 4000]), 2), 10 ** rng.uniform(-2, 1)
+        d = rng.normal(0, 1, 2)
+        d /= np.linalg.norm(d)
+        n = np.array([-d[1], d[0]])
+        thin = 10 ** rng.uniform(-2.2, 0)
+        shapes.append((c + size * np.array([0 * d, d, rng.uniform(0, 1) * d + thin * n])).astype(f32))
+    boxed = near = 0
+    for p in shapes:
+        g = _setup(p[0], p[1], p[2])
+        box = _tight_box(g, p)
+        if box is None:
+            continue
+        boxed += 1
+        lo, hi = np.floor(p.min(0)).astype(int) - 3, np.floor(p.max(0)).astype(int) + 4
+        if (hi - lo).max() > 80:
+            continue
+        px, py = (a.ravel().astype(f32) + f32(0.5) for a in np.meshgrid(np.arange(lo[0], hi[0]), np.arange(lo[1], hi[1])))
+        un, vn, wn = _numerators(g, px, py)
+        escapes = ~((un < g["thr"]) | (vn < g["thr"]) | (wn < g["thr"]))
+        inside = (px >= box[0]) & (px <= box[1]) & (py >= box[2]) & (py <= box[3])
+        assert not (escapes & ~inside).any(), p
+        near += int((inside & ~escapes).any())
+    assert boxed > 2000 and near > 500
