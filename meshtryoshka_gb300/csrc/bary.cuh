@@ -82,8 +82,13 @@ __device__ __forceinline__ void setup_geometry(float p1x, float p1y, float p2x, 
   g.d1223 = d1223;
   g.d1323 = d1323;
   g.dd = dd;
+  // The fast reject's threshold: a numerator below it has a negative quotient.
+  // For dd in (2^-20, inf) a numerator below -dd 2^-100 divides to at most
+  // -2^-100. For dd in (0, 2^-20] any negative numerator will do: dividing by
+  // dd <= 1 cannot round a non-zero quotient to zero. Otherwise (-inf) there is
+  // none.
   const bool fast = dd > 0x1p-20f && dd < __int_as_float(0x7f800000);
-  g.thr = fast ? -__fmul_rn(dd, 0x1p-100f) : __int_as_float(0xff800000);
+  g.thr = fast ? -__fmul_rn(dd, 0x1p-100f) : dd > 0.0f && dd <= 0x1p-20f ? 0.0f : __int_as_float(0xff800000);
 }
 
 // The three barycentric numerators of pixel (px, py)
@@ -160,47 +165,61 @@ namespace mt {
 //
 // A pixel centre p can only be accepted by hit_test if none of the three
 // numerators falls below the fast-reject threshold. For a well-conditioned
-// triangle (every angle's sine^2 >= 1e-4, positive finite denominator above
-// 2^-20, extent below 8192 px) the numerators are affine functions of p whose
+// triangle (every angle's sine^2 >= 1e-4, positive finite denominator, extent
+// below 8192 px) the numerators are affine functions of p whose
 // rounding error is bounded by a few ulps of |coefficients| x |p - p_i|;
 // outside the triangle's bounding box grown by 1 px + 1e-3 x extent, one of
 // them is negative by orders of magnitude more than that error, so
 // hit_test's exact fast reject fires. Such a box is therefore a conservative
 // superset of the accepted pixels, and a warp whose pixel rectangle misses it
 // skips the triangle without changing any decision. Triangles that are not
-// well-conditioned get an infinite box (never culled).
+// well-conditioned get an infinite box.
 //
 // Small triangles get a tighter box: 1/16 px + extent / 4. With L the longest
 // edge, the squared double area D is at least 1e-4 L^2 (L / 2)^2 = 2.5e-5 L^4
 // (the second longest edge is at least L / 2). A pixel centre outside the
 // bounding box by m along an axis has a barycentric weight at or below
-// -m / (2 ext), so a numerator at or below -m D / (2 ext), evaluated with an
-// error of at most 5 u S <= 20 u L^3 d, where d <= sqrt(2) (ext + m) is its
-// distance from the corner. The numerator is below zero for all m with
-// m > 0.096 d, so from m = 0.16 ext on. It matters for triangles of about a
+// -m / (2 ext), so a numerator at or below -m D / (2 ext), known (with the
+// rounding of its coefficients) to 10 u S <= 20 u L^3 d, where
+// d <= sqrt(2) (ext + m) is its distance from the corner. The numerator is
+// below zero for all m with m > 0.096 d, so from m = 0.16 ext on. It matters for triangles of about a
 // pixel, most of a fine mesh's: they reach one to three pixel rows instead of
 // three to five.
 // ---------------------------------------------------------------------------
+//
+// `rows`: the numerators may be bounded over rows and blocks of pixels
+// (composite.cu: edge_excludes, row_columns), which needs the fast reject,
+// finite coordinates and edges whose products stay clear of underflow, but no
+// conditioning. The box does: thin triangles (2 to 3 % of a marching-cubes
+// mesh) have an open box, and are cut down by their rows alone.
 struct CullBox {
   float x0, x1, y0, y1;
+  bool rows;
 };
 
 __device__ __forceinline__ CullBox cull_box(const TriGeom& g, float p1x, float p1y, float p2x, float p2y, float p3x,
                                             float p3y) {
   const float inf = __int_as_float(0x7f800000);
-  CullBox open{-inf, inf, -inf, inf};
+  CullBox open{-inf, inf, -inf, inf, false};
   const float xmin = fminf(fminf(p1x, p2x), p3x), xmax = fmaxf(fmaxf(p1x, p2x), p3x);
   const float ymin = fminf(fminf(p1y, p2y), p3y), ymax = fmaxf(fmaxf(p1y, p2y), p3y);
   const float ext = fmaxf(xmax - xmin, ymax - ymin);
   if (!(ext < 8192.0f) || !(fabsf(xmin) < 1e6f && fabsf(xmax) < 1e6f && fabsf(ymin) < 1e6f && fabsf(ymax) < 1e6f))
     return open;
-  if (!(g.thr > -inf)) return open;  // fast reject unavailable: no culling
   const float e23x = p3x - p2x, e23y = p3y - p2y;
   const float l12 = g.d1212, l13 = g.d1313, l23 = e23x * e23x + e23y * e23y;
+  // Edges of at least 2^-25 px keep the products that bound a numerator over
+  // a block clear of underflow.
+  if (!(g.thr > -inf) || !(fminf(fminf(l12, l13), l23) >= 0x1p-50f)) return open;  // no culling
+  open.rows = true;
   const float worst = fmaxf(fmaxf(l12 * l13, l12 * l23), l13 * l23);
-  if (!(g.dd >= 1e-4f * worst)) return open;
+  // The squared double area: dd, or for small triangles dd less the 1e-8 in
+  // it, held to be known to a percent.
+  const bool small = g.dd <= 0x1p-20f;
+  const float area = small ? g.dd - 1e-8f : g.dd;
+  if (!(area >= 1e-4f * worst) || (small && !(area >= 1e-13f))) return open;
   const float m = fminf(1.0f + 1e-3f * ext, 0.0625f + 0.25f * ext);
-  return CullBox{xmin - m, xmax + m, ymin - m, ymax + m};
+  return CullBox{xmin - m, xmax + m, ymin - m, ymax + m, true};
 }
 
 __device__ __forceinline__ bool box_overlaps(const CullBox& b, float rx0, float rx1, float ry0, float ry1) {

@@ -52,6 +52,7 @@ namespace mt {
 namespace {
 
 constexpr int kBatch = 32;   // triangles gathered per warp batch
+constexpr int kScan = 8;     // groups of 32 masks loaded side by side
 constexpr int kQueue = 64;   // queued key offsets per warp
 constexpr int kRing = 64;    // gradient slots per warp (two batches)
 constexpr int kSavedFwd = 2;  // hits per pixel per batch whose samples the test phase keeps (forward)
@@ -323,7 +324,9 @@ __device__ __forceinline__ TriangleBounds3 triangle_bounds(const TriGeom& g) {
 // padding far above the rounding of this computation. Otherwise (an edge
 // within a few ulps of horizontal) g <= 4E sx |qx|, and the edge removes the
 // whole row when that bound stays below R at the farthest of the columns
-// asked about, [bx, bx + width].
+// asked about, [bx, bx + width]. (2^-100 keeps the reciprocal's operand normal;
+// where R times it overflows, the infinities say what the numbers would, and a
+// NaN limits nothing.)
 //
 // Branch-free, as a warp's lanes hold edges of every direction: each edge
 // carries its inverses ordered by the sign of R, and bounds that never bind
@@ -337,9 +340,8 @@ struct RowEdge {
 
 constexpr float kRowError = 0x1p-18f;  // 2E: 2 x 32 u, as in edge_excludes for one point
 
-// 1 / x to an ulp, which the columns' padding covers many times over; x is
-// not subnormal where the result is used (a limiting edge of a triangle whose
-// denominator exceeds 2^-20).
+// 1 / x to an ulp, which the columns' padding covers many times over, for a
+// normal x (a limiting edge's: above 2^-100).
 __device__ __forceinline__ float fast_reciprocal(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -354,12 +356,12 @@ __device__ __forceinline__ RowEdge row_edge(const EdgeBound& e, float bx, float 
   r.sy = kRowError * e.sy;
   r.px = e.px;
   r.py = e.py;
-  r.lower = e.a > slack;   // g increasing: columns at or right of the root survive
-  r.upper = e.a < -slack;  // g decreasing: columns at or left of the root survive
+  r.lower = e.a - slack > 0x1p-100f;   // g increasing: columns at or right of the root survive
+  r.upper = e.a + slack < -0x1p-100f;  // g decreasing: columns at or left of the root survive
   r.inv_neg = r.lower ? inv_lo : inv_hi;
   r.inv_pos = r.lower ? inv_hi : inv_lo;
   const float qf = fmaxf(fabsf(bx - e.px), fabsf(bx + width - e.px));
-  r.flat = r.lower || r.upper ? __int_as_float(0x7f800000) : 2.02f * slack * qf;
+  r.flat = r.lower || r.upper ? __int_as_float(0x7f800000) : (2.02f * slack + 0x1p-98f) * qf;
   return r;
 }
 
@@ -399,7 +401,9 @@ __device__ __forceinline__ bool row_columns(const RowEdges& q, const CullBox& bo
 // With 8x4 blocks, row by row: the pixel rows of the tile inside the
 // triangle's accept box, each with its surviving columns; a block's bit is
 // set when one of its rows keeps a column of it. So a warp meets only the
-// triangles that can hit one of its pixel centres. A mask by the blocks' edge
+// triangles that can hit one of its pixel centres. Triangles with an open box
+// (thin ones) would walk every row of the tile: they go by the blocks' edge
+// exclusion, a test per block, and leave the rows to the forward's spans. A mask by the blocks' edge
 // exclusion alone (the other tile shapes') lets through every triangle that
 // lies near a block: on the 256^3 / 8 shells / 4 x 800^2 step (8x8 tiles,
 // triangles of one to two pixels) two thirds of the (warp, triangle) pairs
@@ -414,11 +418,9 @@ __device__ __forceinline__ uint32_t key_mask(const CompositeArgs& a, int warps, 
   setup_geometry(pa.x, pa.y, pb.x, pb.y, pc.x, pc.y, g);
   const CullBox box = cull_box(g, pa.x, pa.y, pb.x, pb.y, pc.x, pc.y);
   const int tx = tile % cols_b, ty = tile / cols_b;
-  // Exclusion needs the fast reject, finite coordinates and a
-  // well-conditioned triangle: exactly the triangles with a finite box.
-  const bool exact_cull = box.x0 > -__int_as_float(0x7f800000);
+  const bool boxed = box.x0 > -__int_as_float(0x7f800000);
   uint32_t m = 0;
-  if (exact_cull && (a.tile_w & 7) == 0 && (a.tile_h & 3) == 0) {
+  if (boxed && (a.tile_w & 7) == 0 && (a.tile_h & 3) == 0) {
     const float bx = (float)(tx * a.tile_w) + 0.5f, by = (float)(ty * a.tile_h) + 0.5f;
     const int per_row = a.tile_w >> 3;
     const float last = (float)(a.tile_w - 1);
@@ -441,7 +443,7 @@ __device__ __forceinline__ uint32_t key_mask(const CompositeArgs& a, int warps, 
     float x0, x1, y0, y1;
     warp_block_rect(w, a.tile_w, a.tile_h, tx, ty, x0, x1, y0, y1);
     if (!box_overlaps(box, x0, x1, y0, y1)) continue;
-    if (exact_cull && (edge_excludes(tb.v, g.thr, x0, x1, y0, y1) || edge_excludes(tb.w, g.thr, x0, x1, y0, y1) ||
+    if (box.rows && (edge_excludes(tb.v, g.thr, x0, x1, y0, y1) || edge_excludes(tb.w, g.thr, x0, x1, y0, y1) ||
                        edge_excludes(tb.u, g.thr, x0, x1, y0, y1)))
       continue;
     m |= 1u << w;
@@ -566,31 +568,60 @@ __device__ __forceinline__ int3 gather(const CompositeArgs& a, int cam, int64_t 
   return make_int3(ia, ib, ic);
 }
 
-// Fills the warp's queue with offsets (relative to `start`) of keys whose
-// mask has this warp's bit, until 32 are queued or the list ends. Returns the
-// number queued; `next` advances through the list 32 keys at a time.
-__device__ __forceinline__ int refill(const uint32_t* __restrict__ masks, int64_t start, int64_t end, int64_t& next,
-                                      int queued, int* queue, int warp, int lane) {
-  const uint32_t lt = lanemask_lt();
-  while (queued < kBatch && next < end) {
-    const int64_t k = next + lane;
-    const bool keep = k < end && ((__ldg(masks + k) >> warp) & 1u);
-    const uint32_t sel = __ballot_sync(0xffffffffu, keep);
-    if (keep) queue[queued + __popc(sel & lt)] = (int)(k - start);
-    queued += __popc(sel);
-    next += 32;
-  }
-  __syncwarp();
-  return queued;
+// The walk of a tile's key list by one warp: a queue of the keys whose mask
+// has the warp's bit. The masks of kScan x 32 keys are loaded side by side: a
+// scan costs one load's latency, and few of a long list's keys concern one
+// warp (in a 256^2 view of a 256^3 mesh a tile has up to 17,000 keys, 7 % of
+// them this warp's). With one group of 32 at a time the forward took 584 us
+// there, with eight 499 us; short lists are indifferent (a step at 4 x 800^2,
+// 8x8 tiles: 173 and 172 us).
+struct KeyWalk {
+  const uint32_t* masks;  // of the list's first key
+  int size, next;         // the list's keys, and the first one not yet scanned
+  int head, queued;       // the queue's entries: [head, head + queued)
+};
+
+__device__ __forceinline__ KeyWalk begin_walk(const uint32_t* __restrict__ masks, int64_t start, int64_t end) {
+  return KeyWalk{masks + start, (int)(end - start), 0, 0, 0};
 }
 
-// Drops the first `nb` queue entries.
-__device__ __forceinline__ void pop(int* queue, int queued, int nb, int lane) {
-  const int rest = queued - nb;  // <= 31
-  const int v = lane < rest ? queue[nb + lane] : 0;
-  __syncwarp();
-  if (lane < rest) queue[lane] = v;
-  __syncwarp();
+// Queues keys until 32 are there or the list ends (at most 63: masks loaded
+// past the 32nd are loaded again by the next call); returns the size of the
+// next batch.
+__device__ __forceinline__ int refill(KeyWalk& k, int* queue, int warp, int lane) {
+  if (k.queued < kBatch && k.next < k.size) {
+    const uint32_t lt = lanemask_lt();
+    const int kept = lane < k.queued ? queue[k.head + lane] : 0;
+    __syncwarp();
+    if (lane < k.queued) queue[lane] = kept;
+    k.head = 0;
+    do {
+      uint32_t m[kScan];
+#pragma unroll
+      for (int j = 0; j < kScan; ++j) {
+        const int i = k.next + 32 * j + lane;
+        m[j] = i < k.size ? __ldg(k.masks + i) : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < kScan; ++j) {
+        if (k.queued < kBatch) {
+          const bool keep = (m[j] >> warp) & 1u;
+          const uint32_t sel = __ballot_sync(0xffffffffu, keep);
+          if (keep) queue[k.queued + __popc(sel & lt)] = k.next + lane;
+          k.queued += __popc(sel);
+          k.next += 32;
+        }
+      }
+    } while (k.queued < kBatch && k.next < k.size);
+    __syncwarp();
+  }
+  return min(k.queued, kBatch);
+}
+
+// Takes the first `nb` entries off the queue.
+__device__ __forceinline__ void pop(KeyWalk& k, int nb) {
+  k.head += nb;
+  k.queued -= nb;
 }
 
 // Test phase of a batch: bit i = triangle i of the batch passes the exact
@@ -646,10 +677,14 @@ __device__ __forceinline__ int span_count(uint32_t span) {
 }
 
 // Span of a staged triangle over the 8x4 block whose first pixel centre is
-// (bx, by), row by row: the columns that row_columns leaves. Triangles
-// without an exact fast reject (open accept box) span every pixel.
+// (bx, by), row by row: the columns that row_columns leaves. Triangles whose
+// numerators cannot be bounded span every pixel. (Before, thin and very small
+// triangles did too, 3 % of a mesh's but in every warp of their tiles: in a
+// 256^2 view of a 256^3 mesh their 32 pairs each were most of the test phase,
+// 20,000 cycles a batch. Forward: 499 to 133 us there, 172 to 151 us in the
+// 256^3 step at 4 x 800^2, 1.52 to 1.43 ms in the 512^3 step.)
 __device__ __forceinline__ uint32_t edge_span(const TriGeom& g, const CullBox& box, float bx, float by) {
-  if (!(box.x0 > -__int_as_float(0x7f800000))) return kFullSpan;
+  if (!box.rows) return kFullSpan;
   const RowEdges q = row_edges(g, bx, 7.0f);
   uint32_t span = 0u;
 #pragma unroll 1  // rolled: the unrolled rows cost more in instruction-cache misses than they save
@@ -1038,8 +1073,7 @@ __device__ __forceinline__ float forward_item(const CompositeArgs& a, const uint
 
   const int64_t start = keyless ? 0 : a.bounds[2 * ((int64_t)px.cam * T + px.tile)];
   const int64_t end = keyless ? 0 : a.bounds[2 * ((int64_t)px.cam * T + px.tile) + 1];
-  int64_t next = start;
-  int queued = 0;
+  KeyWalk walk = begin_walk(masks, start, end);
   int batch = 0;
   const int64_t hit_base =
       hs.batches && !keyless
@@ -1052,10 +1086,9 @@ __device__ __forceinline__ float forward_item(const CompositeArgs& a, const uint
   // Each batch's triangles are located (sorted key -> face -> vertex ids)
   // one batch ahead, while the previous batch is tested and composited, so
   // that staging a batch waits on one level of dependent loads only.
-  queued = refill(masks, start, end, next, queued, ws.queue, px.wt, lane);
-  int nb = min(queued, kBatch);
+  int nb = refill(walk, ws.queue, px.wt, lane);
   TriRef ref{0, 0, 0, 0};
-  if (lane < nb) ref = locate(a, start + ws.queue[lane]);
+  if (lane < nb) ref = locate(a, start + ws.queue[walk.head + lane]);
   while (__any_sync(0xffffffffu, active)) {
     if (nb == 0) break;
     uint32_t span = 0u;
@@ -1069,11 +1102,9 @@ __device__ __forceinline__ float forward_item(const CompositeArgs& a, const uint
         span = kFullSpan;
       }
     }
-    pop(ws.queue, queued, nb, lane);
-    queued -= nb;
-    queued = refill(masks, start, end, next, queued, ws.queue, px.wt, lane);
-    const int nb_next = min(queued, kBatch);
-    if (lane < nb_next) ref = locate(a, start + ws.queue[lane]);
+    pop(walk, nb);
+    const int nb_next = refill(walk, ws.queue, px.wt, lane);
+    if (lane < nb_next) ref = locate(a, start + ws.queue[walk.head + lane]);
     uint32_t hits = span_batch_hits(ws, span, blocked, bx, by, px.fx, px.fy, last_shell, active, s, lane);
     if (hit_base >= 0 && hit_base + batch < hs.capacity) __stcs(hs.batches + (hit_base + batch) * 32 + lane, hits);
     ++batch;
@@ -1275,8 +1306,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
 
   const int64_t start = a.bounds[2 * ((int64_t)cam * T + px.tile)];
   const int64_t end = a.bounds[2 * ((int64_t)cam * T + px.tile) + 1];
-  int64_t next = start;
-  int queued = 0;
+  KeyWalk walk = begin_walk(masks, start, end);
   int batch = 0;
   const int64_t hit_base = hs.batches ? (int64_t)hs.item_base[item] : -1;
   // Staged form: the next batch is formed one step ahead and its vertex
@@ -1286,15 +1316,14 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
   uint32_t hits_next = 0, needed_next = 0;
   int3 vid_next = make_int3(0, 0, 0);
   auto form_next = [&](int b) {
-    queued = refill(masks, start, end, next, queued, ws.queue, px.wt, lane);
-    nb_next = min(queued, kBatch);
+    nb_next = refill(walk, ws.queue, px.wt, lane);
     if (nb_next == 0) return;
     stored_next = hit_base >= 0 && hit_base + b < hs.capacity;
     hits_next = stored_next ? __ldcs(hs.batches + (hit_base + b) * 32 + lane) : 0u;
     needed_next = stored_next ? __reduce_or_sync(0xffffffffu, hits_next) : 0xffffffffu;
     const bool mine = lane < nb_next && ((needed_next >> lane) & 1u);
     if (mine) {
-      const int64_t k = start + ws.queue[lane];
+      const int64_t k = start + ws.queue[walk.head + lane];
       const int32_t f = __ldg(a.tri + k);
       const uint64_t key = __ldg(reinterpret_cast<const unsigned long long*>(a.keys) + k);
       vid_next = make_int3(__ldg(a.faces + 3 * (int64_t)f), __ldg(a.faces + 3 * (int64_t)f + 1),
@@ -1313,8 +1342,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
         bulk_copy_to_shared(&ws.stage[lane][2], r + vid_next.z, sizeof(VertexRecord), &ws.bar);
       }
     }
-    pop(ws.queue, queued, nb_next, lane);
-    queued -= nb_next;
+    pop(walk, nb_next);
   };
   if constexpr (kStaged) form_next(0);
   while (__any_sync(0xffffffffu, active)) {
@@ -1346,8 +1374,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
       __syncwarp();
       form_next(batch + 1);  // the next batch's copies overlap this batch's compositing
     } else {
-      queued = refill(masks, start, end, next, queued, ws.queue, px.wt, lane);
-      nb = min(queued, kBatch);
+      nb = refill(walk, ws.queue, px.wt, lane);
       if (nb == 0) break;
       // The half being overwritten held batch - 2: flush it first.
       if (batch >= 2) flush_half(a, gr, cam, ws, half, lane);
@@ -1359,9 +1386,9 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
       hits = stored ? __ldcs(hs.batches + (hit_base + batch) * 32 + lane) : 0u;
       const uint32_t needed = stored ? __reduce_or_sync(0xffffffffu, hits) : 0xffffffffu;
       if (lane < nb && ((needed >> lane) & 1u))
-        ws.vids[half * kBatch + lane] = gather(a, cam, start + ws.queue[lane], ws.geo, ws.attr, lane);
-      pop(ws.queue, queued, nb, lane);
-      queued -= nb;
+        ws.vids[half * kBatch + lane] = gather(a, cam, start + ws.queue[walk.head + lane], ws.geo, ws.attr, lane);
+      __syncwarp();
+      pop(walk, nb);
     }
     if (!stored && active) hits = batch_hits(ws.geo, nb, px.fx, px.fy, last_shell, ws.saved, lane);
     if (active) {

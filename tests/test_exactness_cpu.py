@@ -432,3 +432,76 @@ def test_tight_accept_box_holds_every_pixel_that_escapes_the_fast_reject():
         assert not (escapes & ~inside).any(), p
         near += int((inside & ~escapes).any())
     assert boxed > 2000 and near > 500
+
+
+def _rows_allowed(g, p):
+    """Whether cull_box lets the numerators be bounded over rows and blocks."""
+    ext = max(f32(p[:, 0].max() - p[:, 0].min()), f32(p[:, 1].max() - p[:, 1].min()))
+    return bool(ext < 8192 and np.abs(p).max() < 1e6 and g["thr"] > -INF
+                and min(g["d1212"], g["d1313"], _dot2(*(f32(p[2] - p[1])), *(f32(p[2] - p[1])))) >= f32(2.0 ** -50))
+
+
+def _with_small_threshold(g):
+    """setup_geometry's threshold for denominators up to 2^-20 (dd holds the stored one)."""
+    if f32(0) < g["dd"] <= f32(2.0 ** -20):
+        g = dict(g, thr=f32(0))
+    return g
+
+
+def test_negative_numerators_of_small_triangles_have_negative_quotients():
+    rng = np.random.default_rng(21)
+    dd = np.concatenate((2.0 ** rng.uniform(-149, -20, 200000), [2.0 ** -149, 2.0 ** -20])).astype(f32)
+    un = -np.concatenate((2.0 ** rng.uniform(-149, 60, 200000), [2.0 ** -149, 2.0 ** -149])).astype(f32)
+    with np.errstate(over="ignore"):
+        quotient = (un / dd).astype(f32)
+    assert (un < 0).all() and (dd > 0).all() and (quotient < 0).all()
+
+
+def test_thin_and_tiny_triangles_keep_every_accepted_pixel():
+    """Rows and blocks of triangles of any conditioning and size: pixels that
+    the test accepts (its divisions included) lie in the rows' columns, and in
+    blocks that the edge exclusion leaves."""
+    rng = np.random.default_rng(17)
+    shapes = []
+    for _ in range(3000):
+        c, size = rng.uniform(0, rng.choice([40, 3000]), 2), 10 ** rng.uniform(-4, 1.2)
+        d = rng.normal(0, 1, 2)
+        d /= np.linalg.norm(d)
+        n = np.array([-d[1], d[0]])
+        thin = 10 ** rng.uniform(-7, 0)
+        if rng.random() < 0.4:  # through a pixel centre
+            c = np.floor(c) + 0.5 - rng.uniform(0, 1) * size * d
+        p = (c + size * np.array([0 * d, d, rng.uniform(-0.2, 1.2) * d + thin * n])).astype(f32)
+        shapes.append(p[rng.permutation(3)])
+    lx, ly = np.meshgrid(np.arange(8), np.arange(4))
+    accepted = thin_seen = small_seen = removed = 0
+    for p in shapes:
+        g = _with_small_threshold(_setup(p[0], p[1], p[2]))
+        if not _rows_allowed(g, p):
+            continue
+        box = (-INF, INF, -INF, INF)  # an open box: the rows alone
+        thin_seen += _cull_box(g, p) is None and g["dd"] > f32(2.0 ** -20)
+        small_seen += g["dd"] <= f32(2.0 ** -20)
+        lo, hi = np.floor(p.min(0)).astype(int) - 9, np.floor(p.max(0)).astype(int) + 9
+        for bx in range(lo[0] - lo[0] % 8, hi[0] + 1, 8):
+            for by in range(lo[1] - lo[1] % 4, hi[1] + 1, 4):
+                px, py = (bx + lx + 0.5).astype(f32).ravel(), (by + ly + 0.5).astype(f32).ravel()
+                un, vn, wn = _numerators(g, px, py)
+                with np.errstate(over="ignore"):
+                    u, v, w = ((x / g["dd"]).astype(f32) for x in (un, vn, wn))
+                total = ((u + v).astype(f32) + w).astype(f32)
+                ok = np.ones(32, bool)
+                for x in (u, v, w):
+                    ok &= (x >= 0) & (x <= 1)
+                ok &= (total >= f32(0.999)) & (total <= f32(1.001))
+                escapes = ~((un < g["thr"]) | (vn < g["thr"]) | (wn < g["thr"]))
+                assert not (ok & ~escapes).any(), p  # the fast reject only rejects
+                rows = _edge_span(g, box, f32(bx + 0.5), f32(by + 0.5))
+                covered = np.array([rows[k // 8] is not None and rows[k // 8][0] <= k % 8 <= rows[k // 8][1]
+                                    for k in range(32)])
+                assert not (escapes & ~covered).any(), (p, bx, by, rows)
+                if _block_excluded(g, f32(bx + 0.5), f32(bx + 7.5), f32(by + 0.5), f32(by + 3.5)):
+                    assert not escapes.any(), (p, bx, by)
+                accepted += int(ok.sum())
+                removed += int((~covered).sum())
+    assert accepted > 100 and thin_seen > 200 and small_seen > 200 and removed > 100000
