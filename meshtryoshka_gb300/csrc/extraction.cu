@@ -7,10 +7,10 @@
 // count_triangle_faces.slang and create_triangle_faces.slang.
 //
 // Layout choices: every per-word kernel indexes the packed k axis fastest so
-// a warp reads consecutive words; create_voxels runs one warp per packed word
-// with lane = bit, turning the reference's serial 32-bit walk into warp-ballot
-// stream compaction (popcount of the lanes below); all [*, G] / [*, Nv] tables
-// are read one row at a time so every row read is coalesced.
+// a warp reads consecutive words; create_voxels deals the vertices of 32 words
+// out to a warp's lanes, where the reference walks a word's bits in a loop; all
+// [*, G] / [*, Nv] tables are read one row at a time so every row read is
+// coalesced.
 //
 // For the captured training step the per-vertex SH rows can be skipped: the
 // grid-SH colour kernels evaluate vertex colours straight from the grid
@@ -19,6 +19,7 @@
 // the grid through the per-grid-vertex contribution list, with the same bits
 // as the row path.
 
+#include "lookback.cuh"  // warp_inclusive_sum
 #include "mc_tables.h"
 #include "mt_common.cuh"
 #include "sh.cuh"
@@ -39,10 +40,8 @@ __global__ void vertex_occupancy_kernel(const int32_t* __restrict__ occ, int I, 
   const int64_t total = (int64_t)(I + 1) * (J + 1) * (KP + 1);
   for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < total;
        w += (int64_t)gridDim.x * blockDim.x) {
-    const int kp = (int)(w % (KP + 1));
-    const int64_t ij = w / (KP + 1);
-    const int j = (int)(ij % (J + 1));
-    const int i = (int)(ij / (J + 1));
+    int i, j, kp;
+    word_position(w, J + 1, KP + 1, i, j, kp);
     uint32_t result = 0;
 #pragma unroll
     for (int di = 0; di < 2; ++di) {
@@ -68,10 +67,8 @@ __global__ void count_occupancy_kernel(const int32_t* __restrict__ occ, int I, i
   const int64_t total = (int64_t)(I + 1) * (J + 1) * (KP + 1);
   for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < total;
        w += (int64_t)gridDim.x * blockDim.x) {
-    const int kp = (int)(w % (KP + 1));
-    const int64_t ij = w / (KP + 1);
-    const int j = (int)(ij % (J + 1));
-    const int i = (int)(ij / (J + 1));
+    int i, j, kp;
+    word_position(w, J + 1, KP + 1, i, j, kp);
     int c = 0;
     if (i < I && j < J && kp < KP) c = __popc((uint32_t)occ[((int64_t)i * J + j) * KP + kp]);
     counts[w] = c;
@@ -80,7 +77,21 @@ __global__ void count_occupancy_kernel(const int32_t* __restrict__ occ, int I, i
 }
 
 // ---------------------------------------------------------------------------
-// create_voxels.slang:3-276, one warp per vertex-grid word, lane = bit.
+// create_voxels.slang:3-276.
+//
+// A warp takes 32 consecutive words of the vertex grid. Each lane reads its
+// own word, and where that holds a vertex the occupancy words and offsets of
+// the four rows (i, j), (i, j + 1), (i + 1, j), (i + 1, j + 1), into the
+// warp's shared memory; then the span's vertices are dealt out 32 at a time
+// (lane r takes the r-th one). Offsets are exclusive scans in word order, so
+// consecutive lanes write consecutive entries of every table.
+//
+// Bound by its writes (12 B a vertex, 16 B a lower corner, 48 B a voxel). A
+// warp to each word, lane = bit, waited out the loads of one word after
+// another, 460 words to a warp at 512^3 and nine in ten of them empty, and
+// ran with the few lanes of the bits that a word has: 766 us at 512^3 (the
+// large benchmark scene's band; extract_voxels 967 us). With this the call
+// takes 310 us.
 // ---------------------------------------------------------------------------
 struct VoxelGrid {
   const int32_t* occ;   // [I, J, KP]
@@ -90,37 +101,40 @@ struct VoxelGrid {
   int I, J, KP;
   int64_t Nv;
 
-  __device__ __forceinline__ int64_t vw(int i, int j, int kp) const {
-    return ((int64_t)i * (J + 1) + j) * (KP + 1) + kp;
-  }
   // Voxel occupancy word; 0 outside the voxel grid.
   __device__ __forceinline__ uint32_t vx(int i, int j, int kp) const {
     if (i >= I || j >= J || kp >= KP) return 0u;
-    return (uint32_t)occ[((int64_t)i * J + j) * KP + kp];
+    return (uint32_t)__ldg(occ + ((int64_t)i * J + j) * KP + kp);
   }
+};
+
+constexpr int kVoxelWarps = 8;  // warps per CTA: 21 KB of shared memory
+
+// A span's words: the four rows' vertex and voxel occupancy and offsets, what
+// bit 31 needs of the next words, and the word's position.
+struct SpanWords {
+  uint32_t vo[4][32], vx[4][32];
+  int32_t voff[4][32], xoff[4][32];
+  uint32_t last[32];  // bit 0: the vertex after bit 31 exists; bits 1..7: bit 31's x, y, z, xy, yz, xz, xyz neighbours are subvoxels
+  int32_t i[32], j[32], kp[32];
 };
 
 // Per-neighbour-word state at a given bit: the reference's local_* arrays.
 struct WordState {
   int32_t vidx, xidx, sidx;  // indices of the entry at this bit (-64 when out of range)
-  uint32_t vo, vx, so;       // vertex / voxel / subvoxel occupancy words
+  uint32_t vo, so;           // vertex / subvoxel occupancy words
 };
 
-__device__ __forceinline__ WordState word_state(const VoxelGrid& g, int i, int j, int kp, uint32_t below) {
+__device__ __forceinline__ WordState word_state(const SpanWords& q, int row, int word, bool outside, uint32_t below,
+                                                int32_t Nv) {
   WordState s;
-  if (i > g.I || j > g.J) {
-    s.vidx = s.xidx = s.sidx = -64;
-    s.vo = s.vx = s.so = 0u;
-    return s;
-  }
-  const int64_t w = g.vw(i, j, kp);
-  s.vo = (uint32_t)g.vocc[w];
-  s.vx = g.vx(i, j, kp);
-  s.so = s.vo & ~s.vx;
-  const int32_t xo = g.xoff[w], vo = g.voff[w];
-  s.vidx = vo + __popc(s.vo & below);
-  s.xidx = xo + __popc(s.vx & below);
-  s.sidx = (int32_t)g.Nv + (vo - xo) + __popc(s.so & below);
+  s.vo = q.vo[row][word];
+  const uint32_t vx = q.vx[row][word];
+  s.so = s.vo & ~vx;
+  const int32_t xo = q.xoff[row][word], vo = q.voff[row][word];
+  s.vidx = outside ? -64 : vo + __popc(s.vo & below);
+  s.xidx = outside ? -64 : xo + __popc(vx & below);
+  s.sidx = outside ? -64 : Nv + (vo - xo) + __popc(s.so & below);
   return s;
 }
 
@@ -129,66 +143,98 @@ __device__ __forceinline__ int32_t pick_diag(bool diag_sub, bool side_sub, const
   return diag_sub ? (side_sub ? s.sidx + 1 : s.sidx) : (side_sub ? s.xidx : s.xidx + 1);
 }
 
-__global__ void create_voxels_kernel(VoxelGrid g, float* __restrict__ vertices, int32_t* __restrict__ neighbors,
-                                     int32_t* __restrict__ lower, int32_t* __restrict__ upper,
-                                     int32_t* __restrict__ indices, int64_t G) {
+// The neighbour test of bit 31 (create_voxels.slang:211-275).
+__device__ __forceinline__ uint32_t last_bit_flags(const VoxelGrid& g, int i, int j, int kp, int64_t w) {
+  const bool cx = kp < g.KP - 1, cy = j < g.J - 1, cz = i < g.I - 1;
+  const uint32_t top = 1u << 31;
+  uint32_t m = kp < g.KP && (__ldg(g.vocc + w + 1) & 1) ? 1u : 0u;
+  m |= (cx ? (g.vx(i, j, kp + 1) & 1u) == 0u : true) ? 2u : 0u;
+  m |= (cy ? (g.vx(i, j + 1, kp) & top) == 0u : true) ? 4u : 0u;
+  m |= (cz ? (g.vx(i + 1, j, kp) & top) == 0u : true) ? 8u : 0u;
+  m |= (cx && cy ? (g.vx(i, j + 1, kp + 1) & 1u) == 0u : true) ? 16u : 0u;
+  m |= (cy && cz ? (g.vx(i + 1, j + 1, kp) & top) == 0u : true) ? 32u : 0u;
+  m |= (cx && cz ? (g.vx(i + 1, j, kp + 1) & 1u) == 0u : true) ? 64u : 0u;
+  m |= (cx && cy && cz ? (g.vx(i + 1, j + 1, kp + 1) & 1u) == 0u : true) ? 128u : 0u;
+  return m;
+}
+
+__global__ void __launch_bounds__(32 * kVoxelWarps)
+    create_voxels_kernel(VoxelGrid g, float* __restrict__ vertices, int32_t* __restrict__ neighbors,
+                         int32_t* __restrict__ lower, int32_t* __restrict__ upper, int32_t* __restrict__ indices,
+                         int64_t G) {
+  __shared__ SpanWords spans[kVoxelWarps];
+  SpanWords& q = spans[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const int64_t warps_total = (int64_t)(g.I + 1) * (g.J + 1) * (g.KP + 1);
-  const int64_t warp_global = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t warp_stride = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const uint32_t below = (1u << lane) - 1u;
-  const uint32_t bit = 1u << lane;
+  const int J1 = g.J + 1, KP1 = g.KP + 1;
+  const int64_t total = (int64_t)(g.I + 1) * J1 * KP1;
+  const int64_t mine = (blockIdx.x * (int64_t)kVoxelWarps + (threadIdx.x >> 5)) * 32 + lane;
+  const uint32_t my_chunk = mine < total ? (uint32_t)__ldg(g.vocc + mine) : 0u;
+  const int my_count = __popc(my_chunk);
+  const int incl = warp_inclusive_sum(my_count);
+  const int span = __shfl_sync(0xffffffffu, incl, 31);
+  if (span == 0) return;  // the whole warp
+  if (my_chunk != 0u) {
+    int i, j, kp;
+    word_position(mine, J1, KP1, i, j, kp);
+#pragma unroll
+    for (int row = 0; row < 4; ++row) {
+      const int ri = i + (row >> 1), rj = j + (row & 1);
+      const bool inside = ri <= g.I && rj <= g.J;
+      const int64_t w = mine + (row >> 1) * ((int64_t)J1 * KP1) + (row & 1) * KP1;
+      q.vo[row][lane] = row == 0 ? my_chunk : inside ? (uint32_t)__ldg(g.vocc + w) : 0u;
+      q.vx[row][lane] = g.vx(ri, rj, kp);
+      q.voff[row][lane] = inside ? __ldg(g.voff + w) : 0;
+      q.xoff[row][lane] = inside ? __ldg(g.xoff + w) : 0;
+    }
+    q.last[lane] = (my_chunk >> 31) ? last_bit_flags(g, i, j, kp, mine) : 0u;
+    q.i[lane] = i;
+    q.j[lane] = j;
+    q.kp[lane] = kp;
+  }
+  __syncwarp();
+
   const int64_t Nv = g.Nv;
   const float inv_i = 1.0f / (float)g.I;
   const float inv_j = 1.0f / (float)g.J;
   const float inv_k = 1.0f / (float)(32 * g.KP);
   const int32_t k_max = 32 * g.KP;
-
-  for (int64_t w = warp_global; w < warps_total; w += warp_stride) {
-    const int kp = (int)(w % (g.KP + 1));
-    const int64_t ij = w / (g.KP + 1);
-    const int j = (int)(ij % (g.J + 1));
-    const int i = (int)(ij / (g.J + 1));
-    const uint32_t vo00 = (uint32_t)g.vocc[w];
-    if (vo00 == 0u) continue;  // warp-uniform
-    const int k = 32 * kp + lane;
-
-    const WordState s00 = word_state(g, i, j, kp, below);
-    const WordState s01 = word_state(g, i, j + 1, kp, below);
-    const WordState s10 = word_state(g, i + 1, j, kp, below);
-    const WordState s11 = word_state(g, i + 1, j + 1, kp, below);
+  for (int start = 0; start < span; start += 32) {
+    const int r = start + lane;
+    int before;
+    const int word = dealt_word(incl, my_count, r, before);
+    if (r >= span) continue;
+    const uint32_t chunk = q.vo[0][word];
+    const int pos = select_bit(chunk, r - before);
+    const uint32_t bit = 1u << pos, below = bit - 1u;
+    const int i = q.i[word], j = q.j[word], kp = q.kp[word];
+    const int k = 32 * kp + pos;
+    const bool no_j = j >= g.J, no_i = i >= g.I;
+    const WordState s00 = word_state(q, 0, word, false, below, (int32_t)Nv);
+    const WordState s01 = word_state(q, 1, word, no_j, below, (int32_t)Nv);
+    const WordState s10 = word_state(q, 2, word, no_i, below, (int32_t)Nv);
 
     // Vertices (create_voxels.slang:37-53).
-    if (vo00 & bit) {
-      float* v = vertices + (int64_t)s00.vidx * 3;
-      v[0] = (float)k * inv_k;
-      v[1] = (float)j * inv_j;
-      v[2] = (float)i * inv_i;
-    }
-
-    const bool is_voxel = (s00.vx & bit) != 0u;
-    const bool is_sub = (s00.so & bit) != 0u;
-    if (!is_voxel && !is_sub) continue;
+    float* v = vertices + (int64_t)s00.vidx * 3;
+    v[0] = (float)k * inv_k;
+    v[1] = (float)j * inv_j;
+    v[2] = (float)i * inv_i;
 
     // Lower corners (create_voxels.slang:108-127, last bit fixed up at :201-206).
+    const bool is_voxel = (s00.so & bit) == 0u;
     const int32_t chosen = is_voxel ? s00.xidx : s00.sidx;
-    bool x_valid;
-    if (lane < 31) {
-      x_valid = is_voxel || ((s00.vo >> (lane + 1)) & 1u);
-    } else {
-      x_valid = is_voxel || (kp < g.KP && (g.vocc[g.vw(i, j, kp + 1)] & 1));
-    }
+    const uint32_t last = q.last[word];
+    const bool x_valid = is_voxel || (pos < 31 ? ((chunk >> pos) >> 1) & 1u : last & 1u);
     const bool y_valid = is_voxel || (s01.vo & bit);
     const bool z_valid = is_voxel || (s10.vo & bit);
     lower[chosen] = s00.vidx;
     lower[G + chosen] = x_valid ? s00.vidx + 1 : -64;
     lower[2 * G + chosen] = y_valid ? s01.vidx : -64;
     lower[3 * G + chosen] = z_valid ? s10.vidx : -64;
-
     if (!is_voxel) continue;
-    const int32_t vi = s00.xidx;
 
     // Upper corners and linear index (create_voxels.slang:129-136).
+    const WordState s11 = word_state(q, 3, word, no_i || no_j, below, (int32_t)Nv);
+    const int32_t vi = s00.xidx;
     upper[vi] = s11.vidx + 1;
     upper[Nv + vi] = s11.vidx;
     upper[2 * Nv + vi] = s10.vidx + 1;
@@ -197,7 +243,7 @@ __global__ void create_voxels_kernel(VoxelGrid g, float* __restrict__ vertices, 
 
     // Neighbours (create_voxels.slang:138-193 for bits 0..30, :211-275 for bit 31).
     bool x_sub, y_sub, z_sub, xy_sub, yz_sub, xz_sub, xyz_sub;
-    if (lane < 31) {
+    if (pos < 31) {
       const uint32_t nb = bit << 1;
       x_sub = (s00.so & nb) != 0u;
       y_sub = (s01.so & bit) != 0u;
@@ -207,15 +253,13 @@ __global__ void create_voxels_kernel(VoxelGrid g, float* __restrict__ vertices, 
       xz_sub = (s10.so & nb) != 0u;
       xyz_sub = (s11.so & nb) != 0u;
     } else {
-      const bool cx = kp < g.KP - 1, cy = j < g.J - 1, cz = i < g.I - 1;
-      const uint32_t top = 1u << 31;
-      x_sub = cx ? ((g.vx(i, j, kp + 1) & 1u) == 0u) : true;
-      y_sub = cy ? ((g.vx(i, j + 1, kp) & top) == 0u) : true;
-      z_sub = cz ? ((g.vx(i + 1, j, kp) & top) == 0u) : true;
-      xy_sub = (cx && cy) ? ((g.vx(i, j + 1, kp + 1) & 1u) == 0u) : true;
-      yz_sub = (cy && cz) ? ((g.vx(i + 1, j + 1, kp) & top) == 0u) : true;
-      xz_sub = (cx && cz) ? ((g.vx(i + 1, j, kp + 1) & 1u) == 0u) : true;
-      xyz_sub = (cx && cy && cz) ? ((g.vx(i + 1, j + 1, kp + 1) & 1u) == 0u) : true;
+      x_sub = last & 2u;
+      y_sub = last & 4u;
+      z_sub = last & 8u;
+      xy_sub = last & 16u;
+      yz_sub = last & 32u;
+      xz_sub = last & 64u;
+      xyz_sub = last & 128u;
     }
     neighbors[vi] = x_sub ? s00.sidx : s00.xidx + 1;
     neighbors[Nv + vi] = y_sub ? s01.sidx : s01.xidx;
@@ -235,10 +279,8 @@ __global__ void dilate_kernel(const int32_t* __restrict__ occ, int I, int J, int
   const int64_t total = (int64_t)I * J * KP;
   for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < total;
        w += (int64_t)gridDim.x * blockDim.x) {
-    const int kp = (int)(w % KP);
-    const int64_t ij = w / KP;
-    const int j = (int)(ij % J);
-    const int i = (int)(ij / J);
+    int i, j, kp;
+    word_position(w, J, KP, i, j, kp);
     uint32_t prev = 0, cur = 0, next = 0;
     const int i0 = max(i - d, 0), i1 = min(i + d, I - 1);
     const int j0 = max(j - d, 0), j1 = min(j + d, J - 1);
@@ -1469,9 +1511,8 @@ int mt_create_voxels(const int32_t* occupancy, const int32_t* voxel_offsets, con
   MT_REQUIRE((int64_t)32 * KP * J * I < ((int64_t)1 << 31));
   VoxelGrid g{occupancy, voxel_offsets, vertex_occupancy, vertex_offsets, I, J, KP, num_voxels};
   const int64_t words = (int64_t)(I + 1) * (J + 1) * (KP + 1);
-  const int threads = 256;
-  const int64_t want = (words * 32 + threads - 1) / threads;
-  const unsigned blocks = (unsigned)(want < (int64_t)kSmCount * 16 ? want : (int64_t)kSmCount * 16);
+  const int threads = 32 * kVoxelWarps;  // a lane to a word; the words are below 2^29
+  const unsigned blocks = (unsigned)((words + threads - 1) / threads);
   create_voxels_kernel<<<blocks, threads, 0, as_stream(stream)>>>(g, vertices, neighbors, lower_corners,
                                                                   upper_corners, indices, num_vertices);
   MT_CHECK_LAUNCH();

@@ -50,6 +50,53 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   return m;
 }
 
+// Position of the n-th (0-based) set bit of x (n < popc(x)).
+__device__ __forceinline__ int select_bit(uint32_t x, int n) {
+  int pos = 0;
+#pragma unroll
+  for (int width = 16; width > 0; width >>= 1) {
+    const int c = __popc(x & ((1u << width) - 1u));
+    if (n >= c) {
+      n -= c;
+      x >>= width;
+      pos += width;
+    }
+  }
+  return pos;
+}
+
+// Position (i, j, kp) of word w of a packed grid with rows of J words x KP:
+// in 32 bits where w allows (64-bit divisions by a variable take some 100
+// instructions each, and made the per-word kernels wait on them).
+__device__ __forceinline__ void word_position(int64_t w, int J, int KP, int& i, int& j, int& kp) {
+  if (((uint64_t)w >> 32) == 0) {
+    const uint32_t x = (uint32_t)w, ij = x / (uint32_t)KP;
+    kp = (int)(x - ij * (uint32_t)KP);
+    i = (int)(ij / (uint32_t)J);
+    j = (int)(ij - (uint32_t)i * (uint32_t)J);
+  } else {
+    const int64_t ij = w / KP;
+    kp = (int)(w - ij * KP);
+    i = (int)(ij / J);
+    j = (int)(ij - (int64_t)i * J);
+  }
+}
+
+// Deals the set bits of a warp's 32 words out to its lanes: the word that
+// holds the r-th bit of the span, from every lane's inclusive running count
+// (the smallest word whose count is above r; any word for an r past the
+// span), and the bits before that word. All lanes of the warp call it.
+__device__ __forceinline__ int dealt_word(int inclusive, int count, int r, int& before) {
+  int word = 0;
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1) {
+    const int v = __shfl_sync(0xffffffffu, inclusive, word + step - 1);
+    if (v <= r) word += step;
+  }
+  before = __shfl_sync(0xffffffffu, inclusive - count, word);
+  return word;
+}
+
 // Record the first device-side error code in a status word (0 = ok).
 __device__ __forceinline__ void set_device_error(int* status, int code) {
   if (status != nullptr) atomicCAS(status, 0, code);

@@ -153,21 +153,6 @@ __device__ __forceinline__ void upscale_planes(const OldGrid& g, int c0, const i
   }
 }
 
-// Position of the n-th (0-based) set bit of x (n < popc(x)).
-__device__ __forceinline__ int select_bit(uint32_t x, int n) {
-  int pos = 0;
-#pragma unroll
-  for (int width = 16; width > 0; width >>= 1) {
-    const int c = __popc(x & ((1u << width) - 1u));
-    if (n >= c) {
-      n -= c;
-      x >>= width;
-      pos += width;
-    }
-  }
-  return pos;
-}
-
 // A warp reads 32 consecutive new vertex-occupancy words (one coalesced
 // load) and deals their vertices out 32 at a time: lane r takes the r-th
 // vertex of the span, whose word is found by a shuffle search over the
