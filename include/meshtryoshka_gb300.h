@@ -185,6 +185,20 @@ MT_API int mt_upscale_parameters(
     float* new_signed_distances, float* new_spherical_harmonics,
     mt_stream_t stream);
 
+/* The same, of parameters that each vertex has from its canonical duplicate
+ * (tesseract.py:432-440): vertex v's values are row canonical[v] (checked by
+ * the caller) of old_signed_distances and of [C, sh_rows, 3]
+ * old_spherical_harmonics; canonical NULL: row v. */
+MT_API int mt_upscale_canonical_parameters(
+    const int32_t* old_vertex_occupancy, const int32_t* old_vertex_offsets,
+    const float* old_signed_distances, const float* old_spherical_harmonics,
+    const int32_t* canonical, int64_t sh_rows, int32_t C, int64_t Vold,
+    int32_t I1, int32_t J1, int32_t KP1,
+    const int32_t* new_vertex_occupancy, const int32_t* new_vertex_offsets,
+    int32_t I1n, int32_t J1n, int32_t KP1n, int64_t Vnew,
+    float* new_signed_distances, float* new_spherical_harmonics,
+    mt_stream_t stream);
+
 /* get_occupancy_mesh.slang:1-54 count_triangles: counts[(I+1)(J+1)(KP+1)+1]
  * int32, 2 x boundary faces owned per entry (last entry set to 0, ready for
  * an exclusive scan). */

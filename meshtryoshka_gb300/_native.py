@@ -46,6 +46,10 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_write_occupancy": (I32, [P, I64, P, I64, P]),
     "mt_upscale_occupancy": (I32, [P, P, I32, I32, I32, I32, I32, I32, P, P]),
     "mt_upscale_parameters": (I32, [P, P, P, P, I32, I64, I32, I32, I32, P, P, I32, I32, I32, I64, P, P, P]),
+    "mt_upscale_canonical_parameters": (
+        I32,
+        [P, P, P, P, P, I64, I32, I64, I32, I32, I32, P, P, I32, I32, I32, I64, P, P, P],
+    ),
     "mt_count_occupancy_mesh_triangles": (I32, [P, I32, I32, I32, P, P]),
     "mt_create_occupancy_mesh_triangles": (I32, [P, I32, I32, I32, P, I64, P, P, P, P]),
     "mt_quantize_points": (I32, [P, I64, c_float, P, P, P]),

@@ -274,24 +274,36 @@ __global__ void __launch_bounds__(32 * kVoxelWarps)
 // ---------------------------------------------------------------------------
 // dilate_occupancy.slang:9-94 (box dilation, 0 < d < 32).
 // ---------------------------------------------------------------------------
+//
+// A warp reads 32 consecutive words and writes the inner 30: each lane ORs its
+// word over the box's rows, and takes the words before and after from the
+// lanes beside it. Reading all three words per lane made 3 (2 d + 1)^2 loads
+// a word: 52 us at 256^3, d = 4; now 22 us.
+constexpr int kDilateWords = 30;
+
 __global__ void dilate_kernel(const int32_t* __restrict__ occ, int I, int J, int KP, int d,
                               int32_t* __restrict__ out) {
   const int64_t total = (int64_t)I * J * KP;
-  for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < total;
-       w += (int64_t)gridDim.x * blockDim.x) {
-    int i, j, kp;
-    word_position(w, J, KP, i, j, kp);
-    uint32_t prev = 0, cur = 0, next = 0;
-    const int i0 = max(i - d, 0), i1 = min(i + d, I - 1);
-    const int j0 = max(j - d, 0), j1 = min(j + d, J - 1);
-    for (int ii = i0; ii <= i1; ++ii) {
-      for (int jj = j0; jj <= j1; ++jj) {
-        const int32_t* row = occ + ((int64_t)ii * J + jj) * KP;
-        cur |= (uint32_t)row[kp];
-        if (kp > 0) prev |= (uint32_t)row[kp - 1];
-        if (kp < KP - 1) next |= (uint32_t)row[kp + 1];
+  const int lane = threadIdx.x & 31;
+  const int64_t first_warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t base = first_warp * kDilateWords; base < total; base += warps * kDilateWords) {
+    const int64_t w = base + lane - 1;
+    const bool there = w >= 0 && w < total;
+    int i = 0, j = 0, kp = 0;
+    uint32_t cur = 0;
+    if (there) {
+      word_position(w, J, KP, i, j, kp);
+      const int i0 = max(i - d, 0), i1 = min(i + d, I - 1);
+      const int j0 = max(j - d, 0), j1 = min(j + d, J - 1);
+      for (int ii = i0; ii <= i1; ++ii) {
+        const int32_t* row = occ + ((int64_t)ii * J + j0) * KP + kp;
+#pragma unroll 4
+        for (int jj = j0; jj <= j1; ++jj, row += KP) cur |= (uint32_t)__ldg(row);
       }
     }
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, cur, 1), next = __shfl_down_sync(0xffffffffu, cur, 1);
+    if (!there || lane == 0 || lane > kDilateWords) continue;
     uint32_t result = cur;
     // Bits that spill in from the previous word (dilate_occupancy.slang:41-44).
     if (kp > 0) {
@@ -1526,7 +1538,8 @@ int mt_dilate_occupancy(const int32_t* occupancy, int32_t I, int32_t J, int32_t 
   const int64_t total = (int64_t)I * J * KP;
   if (total == 0) return MT_OK;
   MT_REQUIRE(occupancy && out && occupancy != out);
-  dilate_kernel<<<grid_stride_blocks(total, 256), 256, 0, as_stream(stream)>>>(occupancy, I, J, KP, dilation, out);
+  const int64_t lanes = (total + kDilateWords - 1) / kDilateWords * 32;
+  dilate_kernel<<<grid_stride_blocks(lanes, 256), 256, 0, as_stream(stream)>>>(occupancy, I, J, KP, dilation, out);
   MT_CHECK_LAUNCH();
   return MT_OK;
 }

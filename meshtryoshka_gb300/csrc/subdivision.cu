@@ -11,6 +11,7 @@
 // Floating-point results follow the reference source's operations in order
 // (this unit is compiled without multiply-add contraction).
 
+#include "lookback.cuh"  // warp_inclusive_sum
 #include "mt_common.cuh"
 
 namespace mt {
@@ -41,7 +42,10 @@ __global__ void write_occupancy_kernel(const int32_t* __restrict__ voxel_indices
 // (di, dj) sides, and since the new grid is at least as fine as the old one,
 // the 32 bits x 2 sides of a new word map to old k in [ks_lo, ks_lo + 32]:
 // at most two old words per row. So a word needs 8 loads (the reference
-// samples 256), OR-ed across the four rows before the per-bit selection.
+// samples 256), OR-ed across the four rows; the new bits follow from the runs
+// of set old bits, of which a surface's band has one or two in a word.
+// (Stepping both sides' old k along the 32 bits took every warp with a word of
+// the band some 400 instructions: 78 us from 256^3 to 512^3; now 43 us.)
 // ---------------------------------------------------------------------------
 __global__ void upscale_occupancy_kernel(const int32_t* __restrict__ occ, const int32_t* __restrict__ mask,
                                          uint32_t I, uint32_t J, uint32_t KP, uint32_t I2, uint32_t J2,
@@ -49,7 +53,9 @@ __global__ void upscale_occupancy_kernel(const int32_t* __restrict__ occ, const 
   const int64_t total = (int64_t)I2 * J2 * KP2;
   const uint32_t K = KP << 5, K2 = KP2 << 5;
   for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < total; w += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t kp = (uint32_t)(w % KP2), j = (uint32_t)((w / KP2) % J2), i = (uint32_t)(w / ((int64_t)KP2 * J2));
+    int i_, j_, kp_;
+    word_position(w, (int)J2, (int)KP2, i_, j_, kp_);
+    const uint32_t i = (uint32_t)i_, j = (uint32_t)j_, kp = (uint32_t)kp_;
     const uint32_t k_base = kp << 5;
     const uint32_t lo = ((k_base * K) / K2) >> 5;
     const bool has_hi = lo + 1 < KP;
@@ -72,24 +78,18 @@ __global__ void upscale_occupancy_kernel(const int32_t* __restrict__ occ, const 
       }
     }
     uint32_t result = 0;
-    if (a | b) {
-      // The old k of both sides, k0 = (k K) / K2 and k1 = ((k + 1) K - 1) / K2,
-      // stepped along the word: each bit adds K to both numerators, and since
-      // K <= K2 a quotient grows by at most one per step.
-      const uint32_t n0 = k_base * K, n1 = k_base * K + K - 1;
-      uint32_t k0 = n0 / K2, r0 = n0 - k0 * K2;
-      uint32_t k1 = n1 / K2, r1 = n1 - k1 * K2;
-#pragma unroll 8
-      for (uint32_t bit = 0; bit < 32; ++bit) {
-        const uint32_t w0 = (k0 >> 5) == lo ? a : b;
-        const uint32_t w1 = (k1 >> 5) == lo ? a : b;
-        const uint32_t v = ((w0 >> (k0 & 31)) | (w1 >> (k1 & 31))) & 1u;
-        result |= v << bit;
-        r0 += K;
-        if (r0 >= K2) r0 -= K2, ++k0;
-        r1 += K;
-        if (r1 >= K2) r1 -= K2, ++k1;
-      }
+    // A run of old voxels [first, last] covers the new k with k1 >= first and
+    // k0 <= last, where k0 = (k K) / K2 and k1 = ((k + 1) K - 1) / K2 are the
+    // old k of its two sides: k from (first K2) / K to ((last + 1) K2 - 1) / K.
+    for (uint64_t window = (uint64_t)b << 32 | a; window;) {
+      const int at = __ffsll((long long)window) - 1;
+      const int length = __ffsll((long long)~(window >> at)) - 1;  // -1: all 64 bits
+      const int past = length < 0 ? 64 : at + length;
+      window = past < 64 ? window >> past << past : 0ull;
+      const uint32_t first = ((lo << 5) + at) * K2 / K, last = (((lo << 5) + past) * K2 - 1) / K;
+      if (last < k_base || first > k_base + 31) continue;
+      const uint32_t f = max(first, k_base) - k_base, l = min(last, k_base + 31) - k_base;
+      result |= (0xffffffffu >> (31 - (l - f))) << f;
     }
     out[w] = (int32_t)result;
   }
@@ -105,134 +105,217 @@ struct OldGrid {
   const int32_t* occ;      // old vertex occupancy
   const int32_t* offsets;  // old per-word vertex offsets
   const float* sdf;
-  const float* sh;  // [C, Vold, 3]
-  int64_t Vold;
+  const float* sh;  // [C, sh_rows, 3]
+  int64_t Vold, sh_rows;
+  const int32_t* canonical;  // [Vold]: the row of sdf and sh that holds a vertex's values (NULL: its own)
   int I1, J1, KP1;  // old vertex occupancy dims
 };
 
-// The old vertex at (i, j, k), or -1 when outside the grid or unoccupied
-// (read_vertex, upscale_parameters.slang:9-53; k is never negative here).
-__device__ __forceinline__ int64_t old_vertex(const OldGrid& g, int i, int j, int k) {
-  if (i < 0 || j < 0 || k < 0) return -1;
-  const int kp = k / 32;
-  if (i >= g.I1 || j >= g.J1 || kp >= g.KP1) return -1;
-  const int bit = k % 32;
-  const int64_t word = ((int64_t)i * g.J1 + j) * g.KP1 + kp;
-  const uint32_t chunk = (uint32_t)__ldg(g.occ + word);
-  if ((chunk & (1u << bit)) == 0) return -1;
-  return (int64_t)__ldg(g.offsets + word) + __popc(chunk & ((1u << bit) - 1u));
+// The float `bytes` past a plane's start: 32 bits where a plane's bytes allow,
+// so that a load adds one register to the plane's address.
+template <typename Offset>
+__device__ __forceinline__ float plane_load(const float* __restrict__ plane, Offset bytes) {
+  return __ldg(reinterpret_cast<const float*>(reinterpret_cast<const char*>(plane) + bytes));
 }
 
-// SH planes [c0, c0 + N) of one new vertex: per plane and channel, the sum
-// over the present corners in corner order, times the normaliser. The N
-// planes are independent sums, interleaved for memory-level parallelism.
-template <int N>
-__device__ __forceinline__ void upscale_planes(const OldGrid& g, int c0, const int64_t (&ids)[8],
-                                               const float (&wts)[8], float mult, int64_t Vnew, int64_t vi,
-                                               float* __restrict__ new_sh) {
-  float acc[N][3];
+// N planes of the flat channel that a lane holds: per plane, the sum over the
+// present corners in corner order, times the normaliser. All 8 N loads are
+// issued side by side (a branch around each corner's made them wait for one
+// another). An absent corner reads a present one's row with weight zero: a
+// zero added to a sum that starts at +0 changes nothing, as long as the row is
+// finite. A sum that is not is formed again from the present corners alone.
+template <int N, typename Offset>
+__device__ __forceinline__ void upscale_planes(const float* __restrict__ src, int64_t src_plane, float* __restrict__ dst,
+                                               int64_t dst_plane, uint32_t present, const Offset (&at)[8],
+                                               const float (&wts)[8], float mult) {
+  float x[N][8];
 #pragma unroll
-  for (int n = 0; n < N; ++n) acc[n][0] = acc[n][1] = acc[n][2] = 0.0f;
+  for (int n = 0; n < N; ++n)
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    if (ids[q] < 0) continue;
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-      const float* src = g.sh + ((int64_t)(c0 + n) * g.Vold + ids[q]) * 3;
-      acc[n][0] += wts[q] * __ldg(src + 0);
-      acc[n][1] += wts[q] * __ldg(src + 1);
-      acc[n][2] += wts[q] * __ldg(src + 2);
-    }
-  }
+    for (int q = 0; q < 8; ++q) x[n][q] = plane_load(src + n * src_plane, at[q]);
+  float acc[N];
+  bool finite = true;
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    float* dst = new_sh + ((int64_t)(c0 + n) * Vnew + vi) * 3;
-    dst[0] = acc[n][0] * mult;
-    dst[1] = acc[n][1] * mult;
-    dst[2] = acc[n][2] * mult;
+    acc[n] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[n] += wts[q] * x[n][q];
+    finite = finite && fabsf(acc[n]) < __int_as_float(0x7f800000);
+  }
+  if (!finite) {
+#pragma unroll 1
+    for (int n = 0; n < N; ++n) {
+      float sum = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if ((present >> q) & 1u) sum += wts[q] * plane_load(src + n * src_plane, at[q]);
+      dst[n * dst_plane] = sum * mult;
+    }
+    return;
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) dst[n * dst_plane] = acc[n] * mult;
+}
+
+// What the lanes of a warp share about the 32 vertices that they deal with.
+struct DealtVertices {
+  int32_t id[8][32];  // row of each corner's values, -1 = absent
+  float wt[8][32], mult[32];
+};
+constexpr int kUpscaleWarps = 8, kUpscaleThreads = 32 * kUpscaleWarps;
+
+// The vertices of the old grid's row (i, j) at k and k + 1, -1 where absent
+// (read_vertex, upscale_parameters.slang:9-53; no index is negative here).
+__device__ __forceinline__ void old_vertex_pair(const OldGrid& g, int i, int j, int k, int32_t& v0, int32_t& v1) {
+  v0 = v1 = -1;
+  const int kp = k >> 5, bit = k & 31;
+  if ((unsigned)i >= (unsigned)g.I1 || (unsigned)j >= (unsigned)g.J1 || kp >= g.KP1) return;
+  const int64_t word = ((int64_t)i * g.J1 + j) * g.KP1 + kp;
+  const uint32_t chunk = (uint32_t)__ldg(g.occ + word);
+  const uint32_t here = chunk >> bit;
+  const int32_t base = __ldg(g.offsets + word);
+  const int32_t at = base + __popc(chunk & ((1u << bit) - 1u));  // of the first vertex at or after bit
+  if (here & 1u) v0 = at;
+  if (bit < 31) {
+    if (here & 2u) v1 = at + (int32_t)(here & 1u);
+  } else if (kp + 1 < g.KP1 && ((uint32_t)__ldg(g.occ + word + 1) & 1u)) {
+    v1 = __ldg(g.offsets + word + 1);
   }
 }
 
-// A warp reads 32 consecutive new vertex-occupancy words (one coalesced
-// load) and deals their vertices out 32 at a time: lane r takes the r-th
-// vertex of the span, whose word is found by a shuffle search over the
-// warp's running bit counts and whose bit by a popcount select. Offsets are
-// an exclusive scan in word order, so that vertex is offset[first word] + r:
-// every lane is busy and every [C, V, 3] row the warp stores is contiguous.
-__global__ void __launch_bounds__(256)
+// A CTA takes 256 consecutive words of the new vertex grid, one to a thread,
+// and deals their vertices out to its warps 32 at a time: lane r of a batch
+// takes the batch's r-th vertex, whose word is found in the running bit counts
+// and whose bit by a popcount select. Offsets are an exclusive scan in word
+// order, so that vertex is offset[first word] + r: every lane is busy and every
+// [C, V, 3] row that a warp stores is contiguous.
+//
+// The SH sums go by the row's floats, not by vertices: a lane takes floats
+// lane, lane + 32 and lane + 64 of the 96 that 32 vertices have in a plane
+// (vertex and channel stay the same from plane to plane), so that a warp's
+// load or store covers 128 consecutive bytes of new vertices. With a lane to
+// a vertex every load and store strode over 12 B, and a branch around every
+// corner made four loads wait for the next four: 687 us from 256^3 to 512^3
+// (424 k to 2.93 M vertices, C = 16), and 119 us more for the copy of the
+// canonical rows; now 465 us. Bound by its instructions (8 loads, two
+// operations each, per output float).
+template <typename Offset>
+__global__ void __launch_bounds__(kUpscaleThreads, 3)
     upscale_parameters_kernel(OldGrid g, int C, const int32_t* __restrict__ new_occ,
                               const int32_t* __restrict__ new_offsets, int I1n, int J1n, int KP1n, int64_t Vnew,
                               float* __restrict__ new_sdf, float* __restrict__ new_sh) {
+  __shared__ DealtVertices dealt[kUpscaleWarps];
+  __shared__ uint32_t chunks[kUpscaleThreads];
+  __shared__ int ends[kUpscaleThreads];  // inclusive running bit counts
+  __shared__ int warp_counts[kUpscaleWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  DealtVertices& sh = dealt[warp];
   const int64_t total = (int64_t)I1n * J1n * KP1n;
-  const int lane = threadIdx.x & 31;
-  const int64_t first_warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t base = blockIdx.x * (int64_t)kUpscaleThreads, mine = base + threadIdx.x;
+  const uint32_t my_chunk = mine < total ? (uint32_t)__ldg(new_occ + mine) : 0u;
+  const int incl = warp_inclusive_sum(__popc(my_chunk));
+  if (lane == 31) warp_counts[warp] = incl;
+  chunks[threadIdx.x] = my_chunk;
+  __syncthreads();
+  int before_warp = 0, span = 0;
+#pragma unroll
+  for (int w = 0; w < kUpscaleWarps; ++w) {
+    before_warp += w < warp ? warp_counts[w] : 0;
+    span += warp_counts[w];
+  }
+  if (span == 0) return;  // the whole CTA
+  ends[threadIdx.x] = before_warp + incl;
+  __syncthreads();
   // New grid position scale (upscale_parameters.slang:141-160).
-  const int i_max = I1n - 1, j_max = J1n - 1, kp_max = KP1n - 1;
-  const float inv_i_max = 1.0f / (float)i_max;
-  const float inv_j_max = 1.0f / (float)j_max;
-  const float inv_k_max = 1.0f / (float)(32 * kp_max);
+  const float inv_i_max = 1.0f / (float)(I1n - 1);
+  const float inv_j_max = 1.0f / (float)(J1n - 1);
+  const float inv_k_max = 1.0f / (float)(32 * (KP1n - 1));
   // Old grid scale (sample_trilinear, :63-65).
   const float sx = (float)((g.KP1 - 1) * 32), sy = (float)(g.J1 - 1), sz = (float)(g.I1 - 1);
-  for (int64_t base = first_warp * 32; base < total; base += warps * 32) {
-    const int64_t mine = base + lane;
-    const uint32_t my_chunk = mine < total ? (uint32_t)__ldg(new_occ + mine) : 0u;
-    const int my_count = __popc(my_chunk);
-    int incl = my_count;  // inclusive scan of the bit counts over the warp
+  const int64_t src_plane = 3 * g.sh_rows, dst_plane = 3 * Vnew;
+  const int64_t first_vertex = __ldg(new_offsets + base);
+  for (int start = 32 * warp; start < span; start += kUpscaleThreads) {
+    const int r = start + lane;
+    const int64_t vi = first_vertex + r;
+    if (r < span && vi >= 0 && vi < Vnew) {
+      int src = 0;  // the smallest word with ends[src] > r
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const int span = __shfl_sync(0xffffffffu, incl, 31);
-    if (span == 0) continue;
-    const int64_t first_vertex = __ldg(new_offsets + base);
-    for (int start = 0; start < span; start += 32) {
-      const int r = start + lane;
-      // Smallest word index src with incl[src] > r.
-      int src = 0;
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, incl, src + step - 1);
-        if (v <= r) src += step;
-      }
-      const uint32_t chunk = __shfl_sync(0xffffffffu, my_chunk, src);
-      const int before = __shfl_sync(0xffffffffu, incl - my_count, src);
-      if (r >= span) continue;
-      const int64_t vi = first_vertex + r;
-      if (vi < 0 || vi >= Vnew) continue;
-      const int bit = select_bit(chunk, r - before);
-      const int64_t w = base + src;
-      const int kp = (int)(w % KP1n), j = (int)((w / KP1n) % J1n), i = (int)(w / ((int64_t)KP1n * J1n));
+      for (int step = kUpscaleThreads / 2; step > 0; step >>= 1)
+        if (ends[src + step - 1] <= r) src += step;
+      const int bit = select_bit(chunks[src], r - (src ? ends[src - 1] : 0));
+      int i, j, kp;
+      word_position(base + src, J1n, KP1n, i, j, kp);
       const int k = 32 * kp + bit;
       const float x = (float)k * inv_k_max, y = (float)j * inv_j_max, z = (float)i * inv_i_max;
       const float xu = x * sx, yu = y * sy, zu = z * sz;
       const int oi = (int)zu, oj = (int)yu, ok = (int)xu;
-      const float ti = fmodf(zu, 1.0f), tj = fmodf(yu, 1.0f), tk = fmodf(xu, 1.0f);
-      // Per-corner vertex (-1 = absent) and weight, indexed statically so
-      // that both stay in registers.
-      int64_t ids[8];
-      float wts[8];
+      // fmod(x, 1) of x >= 0, which the difference gives exactly.
+      const float ti = zu - truncf(zu), tj = yu - truncf(yu), tk = xu - truncf(xu);
+      int32_t ids[8];
+#pragma unroll
+      for (int q = 0; q < 8; q += 2) old_vertex_pair(g, oi + (q >> 2), oj + ((q >> 1) & 1), ok, ids[q], ids[q + 1]);
+      float value[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (ids[q] >= g.Vold) ids[q] = -1;
+        if (ids[q] >= 0 && g.canonical) ids[q] = __ldg(g.canonical + ids[q]);
+        value[q] = ids[q] >= 0 ? __ldg(g.sdf + ids[q]) : 0.0f;
+        sh.id[q][lane] = ids[q];
+      }
       float den = 0.0f, d = 0.0f;
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
-        int64_t ov = old_vertex(g, oi + di, oj + dj, ok + dk);
-        if (ov >= g.Vold) ov = -1;
-        const float wgt = (di == 0 ? 1.0f - ti : ti) * (dj == 0 ? 1.0f - tj : tj) * (dk == 0 ? 1.0f - tk : tk);
-        ids[q] = ov;
-        wts[q] = wgt;
-        if (ov >= 0) {
-          d += wgt * __ldg(g.sdf + ov);
+        const float wgt =
+            ((q >> 2) == 0 ? 1.0f - ti : ti) * (((q >> 1) & 1) == 0 ? 1.0f - tj : tj) * ((q & 1) == 0 ? 1.0f - tk : tk);
+        sh.wt[q][lane] = wgt;
+        if (ids[q] >= 0) {
+          d += wgt * value[q];
           den += wgt;
         }
       }
       const float mult = 1.0f / den;
+      sh.mult[lane] = mult;
       new_sdf[vi] = d * mult;
-      int c = 0;
-      for (; c + 4 <= C; c += 4) upscale_planes<4>(g, c, ids, wts, mult, Vnew, vi, new_sh);
-      for (; c < C; ++c) upscale_planes<1>(g, c, ids, wts, mult, Vnew, vi, new_sh);
     }
+    __syncwarp();
+    const int count = min(32, span - start);
+#pragma unroll 1
+    for (int f = lane; f < 3 * count; f += 32) {
+      const int v = f / 3, ch = f - 3 * v;
+      const int64_t row = first_vertex + start + v;
+      if (row < 0 || row >= Vnew) continue;
+      Offset at[8];
+      float wts[8];
+      uint32_t present = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int32_t id = sh.id[q][v];
+        present |= (id >= 0 ? 1u : 0u) << q;
+        at[q] = (Offset)12 * (Offset)id + (Offset)(4 * ch);
+        wts[q] = sh.wt[q][v];
+      }
+      const float mult = sh.mult[v];
+      float* dst = new_sh + 3 * row + ch;
+      if (present == 0u) {
+        for (int c = 0; c < C; ++c) dst[c * dst_plane] = 0.0f * mult;
+        continue;
+      }
+      const Offset any = (Offset)12 * (Offset)sh.id[__ffs(present) - 1][v] + (Offset)(4 * ch);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (!((present >> q) & 1u)) {
+          at[q] = any;
+          wts[q] = 0.0f;
+        }
+      int c = 0;
+#pragma unroll 1
+      for (; c + 4 <= C; c += 4, dst += 4 * dst_plane)
+        upscale_planes<4>(g.sh + c * src_plane, src_plane, dst, dst_plane, present, at, wts, mult);
+#pragma unroll 1
+      for (; c < C; ++c, dst += dst_plane)
+        upscale_planes<1>(g.sh + c * src_plane, src_plane, dst, dst_plane, present, at, wts, mult);
+    }
+    __syncwarp();  // the next 32 vertices overwrite the shared ones
   }
 }
 
@@ -445,25 +528,47 @@ int mt_upscale_occupancy(const int32_t* occupancy, const int32_t* mask, int32_t 
   return MT_OK;
 }
 
-int mt_upscale_parameters(const int32_t* old_vertex_occupancy, const int32_t* old_vertex_offsets,
-                          const float* old_signed_distances, const float* old_spherical_harmonics, int32_t C,
-                          int64_t Vold, int32_t I1, int32_t J1, int32_t KP1, const int32_t* new_vertex_occupancy,
-                          const int32_t* new_vertex_offsets, int32_t I1n, int32_t J1n, int32_t KP1n, int64_t Vnew,
-                          float* new_signed_distances, float* new_spherical_harmonics, mt_stream_t stream) {
+int mt_upscale_canonical_parameters(const int32_t* old_vertex_occupancy, const int32_t* old_vertex_offsets,
+                                    const float* old_signed_distances, const float* old_spherical_harmonics,
+                                    const int32_t* canonical, int64_t sh_rows, int32_t C, int64_t Vold, int32_t I1,
+                                    int32_t J1, int32_t KP1, const int32_t* new_vertex_occupancy,
+                                    const int32_t* new_vertex_offsets, int32_t I1n, int32_t J1n, int32_t KP1n,
+                                    int64_t Vnew, float* new_signed_distances, float* new_spherical_harmonics,
+                                    mt_stream_t stream) {
   MT_REQUIRE(C >= 1 && Vold >= 0 && Vnew >= 0 && I1 >= 2 && J1 >= 2 && KP1 >= 2 && I1n >= 2 && J1n >= 2 &&
              KP1n >= 2);
   if (Vnew == 0) return MT_OK;
   MT_REQUIRE(old_vertex_occupancy && old_vertex_offsets && new_vertex_occupancy && new_vertex_offsets &&
              new_signed_distances && new_spherical_harmonics);
   MT_REQUIRE(Vold == 0 || (old_signed_distances && old_spherical_harmonics));
-  OldGrid g{old_vertex_occupancy, old_vertex_offsets, old_signed_distances, old_spherical_harmonics, Vold, I1, J1,
-            KP1};
+  MT_REQUIRE(sh_rows >= 0 && (canonical || sh_rows >= Vold));
+  OldGrid g{old_vertex_occupancy, old_vertex_offsets, old_signed_distances, old_spherical_harmonics, Vold, sh_rows,
+            canonical, I1, J1, KP1};
   const int64_t total = (int64_t)I1n * J1n * KP1n;
-  upscale_parameters_kernel<<<grid_stride_blocks(total, 256), 256, 0, as_stream(stream)>>>(
-      g, C, new_vertex_occupancy, new_vertex_offsets, I1n, J1n, KP1n, Vnew, new_signed_distances,
-      new_spherical_harmonics);
+  const int64_t blocks64 = (total + kUpscaleThreads - 1) / kUpscaleThreads;  // a thread to a word
+  MT_REQUIRE(blocks64 < ((int64_t)1 << 31));
+  const unsigned blocks = (unsigned)blocks64;
+  if (12 * sh_rows < ((int64_t)1 << 32))
+    upscale_parameters_kernel<uint32_t><<<blocks, kUpscaleThreads, 0, as_stream(stream)>>>(
+        g, C, new_vertex_occupancy, new_vertex_offsets, I1n, J1n, KP1n, Vnew, new_signed_distances,
+        new_spherical_harmonics);
+  else
+    upscale_parameters_kernel<int64_t><<<blocks, kUpscaleThreads, 0, as_stream(stream)>>>(
+        g, C, new_vertex_occupancy, new_vertex_offsets, I1n, J1n, KP1n, Vnew, new_signed_distances,
+        new_spherical_harmonics);
   MT_CHECK_LAUNCH();
   return MT_OK;
+}
+
+int mt_upscale_parameters(const int32_t* old_vertex_occupancy, const int32_t* old_vertex_offsets,
+                          const float* old_signed_distances, const float* old_spherical_harmonics, int32_t C,
+                          int64_t Vold, int32_t I1, int32_t J1, int32_t KP1, const int32_t* new_vertex_occupancy,
+                          const int32_t* new_vertex_offsets, int32_t I1n, int32_t J1n, int32_t KP1n, int64_t Vnew,
+                          float* new_signed_distances, float* new_spherical_harmonics, mt_stream_t stream) {
+  return mt_upscale_canonical_parameters(old_vertex_occupancy, old_vertex_offsets, old_signed_distances,
+                                         old_spherical_harmonics, nullptr, Vold, C, Vold, I1, J1, KP1,
+                                         new_vertex_occupancy, new_vertex_offsets, I1n, J1n, KP1n, Vnew,
+                                         new_signed_distances, new_spherical_harmonics, stream);
 }
 
 int mt_count_occupancy_mesh_triangles(const int32_t* occupancy, int32_t I, int32_t J, int32_t KP, int32_t* counts,

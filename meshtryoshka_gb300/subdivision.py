@@ -34,11 +34,10 @@ def subdivide(voxels: te.Voxels, signed_distances: Tensor, spherical_harmonics: 
     [V] and ``spherical_harmonics`` [C, V, 3] its vertex parameters, and
     ``triangle_voxel_indices`` the voxel of every triangle of the current
     mesh (``Triangles.voxel_indices``)."""
-    canonical = te.index_vertices(voxels.vertices, tol).long()
-    signed_distances = signed_distances[canonical]
-    spherical_harmonics = spherical_harmonics[:, canonical, :]
+    canonical = te.index_vertices(voxels.vertices, tol)
     to_upscale = te.write_occupancy(triangle_voxel_indices, tuple(occupancy.shape), 0, 1)
     if disable_sparsity:
         to_upscale = torch.full_like(to_upscale, -1)
     to_upscale = te.dilate_occupancy(to_upscale, dilation)
-    return te.upscale_parameters(signed_distances, spherical_harmonics, occupancy, to_upscale, new_resolution)
+    return te._upscale_parameters(signed_distances, spherical_harmonics, occupancy, to_upscale, new_resolution,
+                                  canonical)

@@ -296,12 +296,27 @@ def upscale_parameters(old_signed_distances: Tensor, old_spherical_harmonics: Te
     """Upscaled occupancy of ``old_occupancy & occupancy_to_upscale`` and the
     old vertices' parameters resampled trilinearly onto its vertices
     (upscale_parameters.py:35-99). One host read (the new vertex count)."""
+    return _upscale_parameters(old_signed_distances, old_spherical_harmonics, old_occupancy, occupancy_to_upscale,
+                               new_resolution, None)
+
+
+def _upscale_parameters(old_signed_distances, old_spherical_harmonics, old_occupancy, occupancy_to_upscale,
+                        new_resolution, canonical: Tensor | None) -> UpscaledParameters:
+    """upscale_parameters; with ``canonical`` (int32 [vertex], from
+    index_vertices) of the parameters that each vertex has from its canonical
+    duplicate, read in place instead of copied first."""
     old_signed_distances = _f32(old_signed_distances, "old_signed_distances")
     old_spherical_harmonics = _f32(old_spherical_harmonics, "old_spherical_harmonics")
     old_occupancy = _i32(old_occupancy, "old_occupancy")
     device = nt.require_cuda(old_signed_distances, old_spherical_harmonics, old_occupancy)
     num_sh, num_old, _ = old_spherical_harmonics.shape
-    if old_signed_distances.shape[0] != num_old:
+    sh_rows = num_old
+    if canonical is not None:
+        # A canonical duplicate's index is below the vertex count.
+        num_old = canonical.shape[0]
+        if min(sh_rows, old_signed_distances.shape[0]) < num_old:
+            raise IndexError("old_signed_distances and old_spherical_harmonics have fewer rows than vertices")
+    elif old_signed_distances.shape[0] != num_old:
         raise ValueError("old_signed_distances and old_spherical_harmonics disagree on the vertex count")
 
     # The AND of upscale_parameters.py:49 is applied to every word the
@@ -319,8 +334,9 @@ def upscale_parameters(old_signed_distances: Tensor, old_spherical_harmonics: Te
     if num_vertices > 0:
         i1, j1, k1 = old_vertex_occupancy.shape
         i1n, j1n, k1n = new_vertex_occupancy.shape
-        nt.call("mt_upscale_parameters", old_vertex_occupancy.data_ptr(), old_vertex_offsets.data_ptr(),
-                nt.ptr(old_signed_distances), nt.ptr(old_spherical_harmonics), num_sh, num_old, i1, j1, k1,
+        nt.call("mt_upscale_canonical_parameters", old_vertex_occupancy.data_ptr(), old_vertex_offsets.data_ptr(),
+                nt.ptr(old_signed_distances), nt.ptr(old_spherical_harmonics), nt.ptr(canonical), sh_rows, num_sh,
+                num_old, i1, j1, k1,
                 new_vertex_occupancy.data_ptr(), new_vertex_offsets.data_ptr(), i1n, j1n, k1n, num_vertices,
                 new_signed_distances.data_ptr(), new_spherical_harmonics.data_ptr(), nt.stream(device))
     return UpscaledParameters(new_signed_distances, new_spherical_harmonics, new_occupancy)

@@ -1,0 +1,45 @@
+"""Subdivision reads each vertex's parameters from its canonical duplicate in
+place: bit for bit what copying them first gives, also where rows of more
+vertices follow, in every coefficient count and with spans of words that hold
+few and many vertices."""
+
+import numpy as np
+import pytest
+import torch
+
+from meshtryoshka_gb300 import subdivision
+from meshtryoshka_gb300 import triangle_extraction as te
+
+from . import semantics
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("c", [1, 4, 5, 9, 16])
+@pytest.mark.parametrize("density,tol,more", [(0.01, 1e-6, 0), (0.2, 0.08, 0), (1.0, 0.08, 7)])
+def test_canonical_rows_in_place(cuda_device, c, density, tol, more):
+    rng = np.random.default_rng(c)
+    occ = semantics.pack(rng.random((9, 14, 64)) < density)
+    occ = torch.from_numpy(np.ascontiguousarray(occ)).to(cuda_device)
+    vox = te.extract_voxels(occ)
+    v, nv = vox.num_vertices, vox.num_voxels
+    sdf = torch.from_numpy(rng.normal(size=v + more).astype(np.float32)).to(cuda_device)
+    sh = torch.from_numpy(rng.normal(size=(c, v + more, 3)).astype(np.float32)).to(cuda_device)
+    marked = vox.indices[:: max(1, nv // 20)]
+    target = (13, 14, 96)
+    got = subdivision.subdivide(vox, sdf, sh, occ, marked, target, dilation=2, tol=tol)
+    canonical = te.index_vertices(vox.vertices, tol).long()
+    assert (tol < 1e-3) or (canonical != torch.arange(v, device=cuda_device)).any()
+    mask = te.dilate_occupancy(te.write_occupancy(marked, tuple(occ.shape), 0, 1), 2)
+    want = te.upscale_parameters(sdf[canonical], sh[:, canonical], occ, mask, target)
+    assert got.signed_distances.numel() > 0
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+def test_too_few_rows_are_refused(cuda_device):
+    occ = torch.from_numpy(semantics.pack(np.ones((3, 4, 32), bool))).to(cuda_device)
+    vox = te.extract_voxels(occ)
+    sh = torch.zeros((1, vox.num_vertices, 3), device=cuda_device)
+    with pytest.raises(IndexError):
+        subdivision.subdivide(vox, sh.new_zeros(vox.num_vertices - 1), sh, occ, vox.indices, (6, 8, 64))
