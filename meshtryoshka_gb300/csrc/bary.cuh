@@ -175,16 +175,19 @@ namespace mt {
 // skips the triangle without changing any decision. Triangles that are not
 // well-conditioned get an infinite box.
 //
-// Small triangles get a tighter box: 1/16 px + extent / 4. With L the longest
-// edge, the squared double area D is at least 1e-4 L^2 (L / 2)^2 = 2.5e-5 L^4
+// Small triangles get a tighter box: 1/16 px + extent / (40000 r), r the squared
+// double area over the largest product of two edges' squares (at least 1e-4).
+// With L the longest edge, the squared double area D is at least r L^2 (L / 2)^2
 // (the second longest edge is at least L / 2). A pixel centre outside the
 // bounding box by m along an axis has a barycentric weight at or below
 // -m / (2 ext), so a numerator at or below -m D / (2 ext), known (with the
 // rounding of its coefficients) to 10 u S <= 20 u L^3 d, where
 // d <= sqrt(2) (ext + m) is its distance from the corner. The numerator is
-// below zero for all m with m > 0.096 d, so from m = 0.16 ext on. It matters for triangles of about a
-// pixel, most of a fine mesh's: they reach one to three pixel rows instead of
-// three to five.
+// below zero for all m with m > k d, k = 160 u / r = 9.6e-6 / r (0.096 at
+// r = 1e-4), so from m = 1.6 k ext = ext / (65000 r) on. It matters for
+// triangles of about a pixel, most of a fine mesh's: they reach one to three
+// pixel rows instead of three to five. (With ext / 4 for all of them the masks
+// of the 256^3 step took 75 us, now 68.)
 // ---------------------------------------------------------------------------
 //
 // `rows`: the numerators may be bounded over rows and blocks of pixels
@@ -218,7 +221,7 @@ __device__ __forceinline__ CullBox cull_box(const TriGeom& g, float p1x, float p
   const bool small = g.dd <= 0x1p-20f;
   const float area = small ? g.dd - 1e-8f : g.dd;
   if (!(area >= 1e-4f * worst) || (small && !(area >= 1e-13f))) return open;
-  const float m = fminf(1.0f + 1e-3f * ext, 0.0625f + 0.25f * ext);
+  const float m = fminf(1.0f + 1e-3f * ext, 0.0625f + __fdividef(2.5e-5f * worst, area) * ext);
   return CullBox{xmin - m, xmax + m, ymin - m, ymax + m, true};
 }
 
