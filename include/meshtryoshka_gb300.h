@@ -760,6 +760,33 @@ MT_API int mt_composite_backward(const float* signed_distances, const float* col
                                  float* grad_sharpness, int32_t exact_adjoint,
                                  mt_stream_t stream);
 
+/* interpolate.slang + composite.slang of every shell of a pixel in one pass
+ * (no [B,S,H,W] samples): uv [B,S,H,W,2] (8-byte aligned) and index [B,S,H,W]
+ * (-1 = miss) as mt_intersect gives them. out_colors [B,H,W,3] and
+ * out_transmittances [B,H,W] (both, or both NULL); with background [3],
+ * image [B,H,W,3] = out_colors + background * out_transmittance. */
+MT_API int mt_shade_shells(const float* uv, const int32_t* index, int32_t B,
+                           int32_t S, int32_t H, int32_t W, const int32_t* faces,
+                           const float* signed_distances, const float* colors,
+                           int64_t V, const float* sharpness,
+                           const float* background, float* out_colors,
+                           float* out_transmittances, float* image,
+                           mt_stream_t stream);
+
+/* Its adjoint; accumulates (+=) into grad_signed_distances [V], grad_colors
+ * [B,V,3], grad_sharpness [1]. grad_out [B,H,W,3] (NULL: zero) is the image's
+ * gradient when a background is given, else out_colors'; exact_adjoint as in
+ * mt_composite_backward. */
+MT_API int mt_shade_shells_backward(
+    const float* uv, const int32_t* index, int32_t B, int32_t S, int32_t H,
+    int32_t W, const int32_t* faces, const float* signed_distances,
+    const float* colors, int64_t V, const float* sharpness,
+    const float* background, const float* out_colors,
+    const float* out_transmittances, const float* grad_out,
+    const float* grad_out_transmittances, float* grad_signed_distances,
+    float* grad_colors, float* grad_sharpness, int32_t exact_adjoint,
+    mt_stream_t stream);
+
 #ifdef __cplusplus
 }  /* extern "C" */
 #endif

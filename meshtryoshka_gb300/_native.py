@@ -121,6 +121,11 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_interpolate_backward": (I32, [P, P, I32, I32, I32, I32, P, I64, P, P, P, P, P]),
     "mt_composite": (I32, [P, P, P, I64, I32, P, P, P, P]),
     "mt_composite_backward": (I32, [P, P, P, I64, I32, P, P, P, P, P, P, P, P, I32, P]),
+    "mt_shade_shells": (I32, [P, P, I32, I32, I32, I32, P, P, P, I64, P, P, P, P, P, P]),
+    "mt_shade_shells_backward": (
+        I32,
+        [P, P, I32, I32, I32, I32, P, P, P, I64, P, P, P, P, P, P, P, P, P, I32, P],
+    ),
 }
 
 _lib = None

@@ -883,6 +883,51 @@ def composite(signed_distances, colors, mask, background, sharpness, gradient_mo
     return out_colors + background * out_t[:, None]
 
 
+class ShadeShells(torch.autograd.Function):
+    """``interpolate`` and ``composite`` of an explicit render in one kernel
+    each way, without the per-shell samples: ([P, 3] colours, [P]
+    transmittances) of its P pixels, or with ``background`` the [P, 3] image
+    colours + background * transmittance. Same values and gradients."""
+
+    @staticmethod
+    def forward(ctx, uv, index, faces, signed_distances, colors, sharpness, background, gradient_mode):
+        with annotate("shade_shells_forward"):
+            uv, index, faces = _f32(uv), _i32(index), _i32(faces)
+            sdf, colors = _f32(signed_distances), _f32(colors)
+            device = nt.require_cuda(uv, index, faces, sdf, colors)
+            sharp = _sharpness(sharpness, device)
+            b, s, h, w = index.shape
+            kw = dict(dtype=torch.float32, device=device)
+            out_colors = out_t = image = None
+            if background is not None:
+                image = torch.empty((b * h * w, 3), **kw)
+            if background is None or any(ctx.needs_input_grad):
+                out_colors, out_t = torch.empty((b * h * w, 3), **kw), torch.empty((b * h * w,), **kw)
+            nt.call("mt_shade_shells", nt.ptr(uv), nt.ptr(index), b, s, h, w, nt.ptr(faces), nt.ptr(sdf),
+                    nt.ptr(colors), sdf.shape[0], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
+                    nt.ptr(out_t), nt.ptr(image), nt.stream(device))
+            ctx.save_for_backward(uv, index, faces, sdf, colors, sharp, background, out_colors, out_t)
+            ctx.meta = (gradient_mode or _GRADIENT_MODE, torch.is_tensor(sharpness))
+            ctx.set_materialize_grads(False)
+            return image if background is not None else (out_colors, out_t)
+
+    @staticmethod
+    def backward(ctx, grad_out, grad_t=None):
+        with annotate("shade_shells_backward"):
+            uv, index, faces, sdf, colors, sharp, background, out_colors, out_t = ctx.saved_tensors
+            mode, sharp_is_tensor = ctx.meta
+            device = sdf.device
+            b, s, h, w = index.shape
+            gsdf, gcol, gsharp = torch.zeros_like(sdf), torch.zeros_like(colors), torch.zeros_like(sharp)
+            go = grad_out.contiguous() if grad_out is not None else None
+            gt = grad_t.contiguous() if grad_t is not None else None
+            nt.call("mt_shade_shells_backward", nt.ptr(uv), nt.ptr(index), b, s, h, w, nt.ptr(faces), nt.ptr(sdf),
+                    nt.ptr(colors), sdf.shape[0], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
+                    nt.ptr(out_t), nt.ptr(go), nt.ptr(gt), nt.ptr(gsdf), nt.ptr(gcol), nt.ptr(gsharp),
+                    int(mode == "exact"), nt.stream(device))
+            return None, None, None, gsdf, gcol, gsharp if sharp_is_tensor else None, None, None
+
+
 # ---------------------------------------------------------------------------
 # Render entry points (triangle_rasterization/__init__.py:22-329)
 # ---------------------------------------------------------------------------
@@ -932,13 +977,12 @@ def render_explicit(extrinsics, intrinsics, image_shape, vertices, faces, shell_
                           tile_shape=tile_shape, near_plane=near_plane, num_camera_bits=num_camera_bits,
                           num_shell_bits=num_shell_bits, num_tile_bits=num_tile_bits)
     colors = evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
-    sdf, colors = interpolate(uv, index, faces, signed_distances, colors)
-    mask = index != -1
-    b, s, h, w = sdf.shape
-    sdf = sdf.permute(0, 2, 3, 1).reshape(b * h * w, s).contiguous()
-    colors = colors.permute(0, 2, 3, 1, 4).reshape(b * h * w, s, 3).contiguous()
-    mask = mask.permute(0, 2, 3, 1).reshape(b * h * w, s).contiguous()
-    image = composite(sdf, colors, mask, background, sharpness, gradient_mode)
+    b, s, h, w = index.shape
+    if _finishable(index, background):
+        image = ShadeShells.apply(uv, index, faces, signed_distances, colors, sharpness, background, gradient_mode)
+    else:
+        image, out_t = ShadeShells.apply(uv, index, faces, signed_distances, colors, sharpness, None, gradient_mode)
+        image = image + background * out_t[:, None]
     image = image.reshape(b, h, w, 3).permute(0, 3, 1, 2)
     if ssaa > 1:
         image = _mean_pool(image, ssaa)
