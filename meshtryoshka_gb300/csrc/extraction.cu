@@ -441,20 +441,91 @@ __global__ void create_vertices_kernel(const float* __restrict__ gv, const float
 
 // Rows have stride V (the buffer's capacity); only the first `count`
 // vertices (device value, clamped to V; all V when count is NULL) are real.
-__global__ void interpolate_vertex_sh_kernel(const float* __restrict__ gsh, int C, int64_t G,
-                                             const int32_t* __restrict__ sources, int64_t V,
-                                             const int32_t* __restrict__ count, float* __restrict__ out_sh) {
-  const int64_t n = count ? min((int64_t)max(*count, 0), V) : V;
-  const int64_t total = (int64_t)C * n;
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = o / n, vi = o - k * n;
-    const int32_t i0 = __ldg(sources + vi), i1 = __ldg(sources + V + vi);
-    const float t = __int_as_float(__ldg(sources + 2 * V + vi));
-    const float* p0 = gsh + (k * G + i0) * 3;
-    const float* p1 = gsh + (k * G + i1) * 3;
-    float* q = out_sh + (k * V + vi) * 3;
+//
+// A CTA takes kRowTile consecutive grid entries, whose vertices are one run for
+// each shell; its warps deal with 32 vertices of a run at a time, all planes,
+// so the grid's rows come from memory once for all shells (in vertex order,
+// shell after shell, they did for each: 3.7 GB instead of 1.25 at 352^3). A
+// lane takes floats lane, lane + 32 and lane + 64 of the 96 that 32 vertices
+// have in a plane (vertex and channel stay the same from plane to plane), so
+// that a load or store covers 128 consecutive bytes. With a thread to a
+// (plane, vertex) the sources were read again for every plane, as many bytes
+// as the rows written, and every access strode over 12 B. 512^3, 8 shells,
+// C = 16 (9.3 M vertices): 1240 us, now 765 (tiles of 512: 834; 768: 983).
+constexpr int kRowTile = 256;
+constexpr int kRowPlanes = 4;  // planes whose loads are issued side by side
+
+template <typename Offset>
+__device__ __forceinline__ const float* at_bytes(const float* p, Offset bytes) {
+  return reinterpret_cast<const float*>(reinterpret_cast<const char*>(p) + bytes);
+}
+
+// Up to 32 consecutive vertices from v0, all planes.
+template <typename Offset>
+__device__ __forceinline__ void interpolate_rows(const float* __restrict__ gsh, int C, int64_t grid_plane,
+                                                 const int32_t* __restrict__ sources, int64_t V, int64_t v0, int many,
+                                                 int lane, float* __restrict__ out_sh) {
+  const int64_t v = v0 + min(lane, many - 1);
+  const int32_t i0 = __ldg(sources + v), i1 = __ldg(sources + V + v), tb = __ldg(sources + 2 * V + v);
+  const int floats = 3 * many;
+  const int64_t row_plane = 3 * V;
+  Offset a0[3], a1[3];
+  float t[3];
 #pragma unroll
-    for (int ch = 0; ch < 3; ++ch) q[ch] = lerp_ref(__ldg(p0 + ch), __ldg(p1 + ch), t);
+  for (int p = 0; p < 3; ++p) {
+    const int f = 32 * p + lane, q = f / 3, ch = f - 3 * q;
+    a0[p] = (Offset)12 * (Offset)__shfl_sync(0xffffffffu, i0, q) + (Offset)(4 * ch);
+    a1[p] = (Offset)12 * (Offset)__shfl_sync(0xffffffffu, i1, q) + (Offset)(4 * ch);
+    t[p] = __int_as_float(__shfl_sync(0xffffffffu, tb, q));
+  }
+  for (int k0 = 0; k0 < C; k0 += kRowPlanes) {
+    float x0[kRowPlanes][3], x1[kRowPlanes][3];
+#pragma unroll
+    for (int j = 0; j < kRowPlanes; ++j) {
+      if (k0 + j < C) {
+        const float* plane = gsh + (k0 + j) * grid_plane;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          if (32 * p < floats) {
+            x0[j][p] = __ldg(at_bytes(plane, a0[p]));
+            x1[j][p] = __ldg(at_bytes(plane, a1[p]));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kRowPlanes; ++j) {
+      if (k0 + j < C) {
+        float* dst = out_sh + (k0 + j) * row_plane + 3 * v0 + lane;
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+          if (32 * p + lane < floats) __stcs(dst + 32 * p, lerp_ref(x0[j][p], x1[j][p], t[p]));
+      }
+    }
+  }
+}
+
+template <typename Offset>
+__global__ void __launch_bounds__(256, 4)
+    interpolate_vertex_sh_kernel(const float* __restrict__ gsh, int C, int64_t G,
+                                 const int32_t* __restrict__ sources, int64_t V, const int32_t* __restrict__ count,
+                                 const int32_t* __restrict__ voff, int S, float* __restrict__ out_sh) {
+  const int64_t n = count ? min((int64_t)max(*count, 0), V) : V;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t e0 = blockIdx.x * (int64_t)kRowTile, e1 = min(e0 + kRowTile, G);
+  int turn = 0;  // batches so far, dealt to the warps in turn
+  for (int s0 = 0; s0 < S; s0 += 32) {
+    const int64_t row = (int64_t)(s0 + lane) * G;
+    const int32_t first = s0 + lane < S ? __ldg(voff + row + e0) : 0;
+    const int32_t last = s0 + lane < S ? __ldg(voff + row + e1) : 0;
+    for (int j = 0; j < min(32, S - s0); ++j) {
+      const int64_t b = __shfl_sync(0xffffffffu, first, j), e = min((int64_t)__shfl_sync(0xffffffffu, last, j), n);
+      const int batches = (int)((max(e - b, (int64_t)0) + 31) >> 5);
+      for (int i = (warp - turn) & 7; i < batches; i += 8)
+        interpolate_rows<Offset>(gsh, C, 3 * G, sources, V, b + 32 * i, (int)min((int64_t)32, e - b - 32 * i), lane,
+                                 out_sh);
+      turn += batches;
+    }
   }
 }
 
@@ -676,106 +747,74 @@ __global__ void create_vertices_backward_kernel(const float* __restrict__ gsdf, 
 // ---------------------------------------------------------------------------
 // The same backward as a contribution list and a gather (S <= 21 shells).
 //
-// Pass 1 (count) and pass 2 (fill), one thread per grid vertex x, enumerate
-// x's contributions exactly as create_vertices_backward_kernel does; pass 2
-// writes the signed distance and position gradients and lists every
-// contribution (vertex | origin flag << 31, t) at x's offset in a CSR list of
-// at most 2V entries. Pass 3, one thread per (SH row k, grid vertex x), sums
-// the row-k gradient over x's list in list order (the same sums, so the same
-// bits) and writes it: consecutive threads write consecutive grid vertices
-// of one row, and low register use keeps the SMs full.
+// entry_list_kernel (below) lists every contribution (vertex | origin flag
+// << 31, t) of a grid vertex x, in the order in which
+// create_vertices_backward_kernel enumerates them, at x's offset in a CSR list
+// of at most 2V entries; vertex_grads_from_list_kernel and
+// vertex_sh_gather_kernel sum the gradients over x's list in list order (the
+// same sums, so the same bits).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ GatherChunk gather_entries(const float* __restrict__ gsdf,
-                                                      const int32_t* __restrict__ lower, int64_t G,
-                                                      const float* __restrict__ level_sets, int S,
-                                                      const int32_t* __restrict__ inverse, int64_t x) {
-  GatherChunk q;
-  q.e = __ldg(inverse + x);
-  Corners4 own{};
-  if (q.e >= 0) own = load_corners(gsdf, lower, G, q.e);
-  q.d0 = own.d0;
+template <int kRows, int kAhead>
+__device__ __forceinline__ void gather_sh_rows(const float* __restrict__ dsh, int64_t row_plane, int32_t begin,
+                                               int32_t end, int ch, const int2* __restrict__ list,
+                                               float* __restrict__ dst, int64_t grid_plane) {
+  float acc[kRows];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    q.d1[a] = own.d[a];
-    q.h[a] = __ldg(inverse + (int64_t)(a + 1) * G + x);
-  }
-  q.own = q.e >= 0 ? crossing_bits(own, level_sets, 0, S) : 0ull;
+  for (int k = 0; k < kRows; ++k) acc[k] = 0.f;
+  if (dsh) {
+    for (int32_t p = begin; p < end; p += kAhead) {
+      int2 e[kAhead];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    q.nb[a] = 0ull;
-    if (q.h[a] >= 0) {
-      const Corners4 nb = load_corners(gsdf, lower, G, q.h[a]);
-      q.nd0[a] = nb.d0;
-      q.nd1[a] = nb.d[a];
-      q.nb[a] = crossing_bits(nb, level_sets, 0, S);
-    }
-  }
-  return q;
-}
-
-template <bool kFill>
-__global__ void vertex_grad_list_kernel(const float* __restrict__ gsdf, const int32_t* __restrict__ lower, int64_t G,
-                                        const float* __restrict__ level_sets, int S,
-                                        const int32_t* __restrict__ voff, const int32_t* __restrict__ inverse,
-                                        int64_t V, int32_t* __restrict__ counts, int2* __restrict__ list,
-                                        const float* __restrict__ dv, const float* __restrict__ dsdf,
-                                        float* __restrict__ gdv, float* __restrict__ gdsdf) {
-  for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < G; x += (int64_t)gridDim.x * blockDim.x) {
-    const GatherChunk q = gather_entries(gsdf, lower, G, level_sets, S, inverse, x);
-    if (!kFill) {
-      int n = 0;
-      for_each_contribution(q, level_sets, 0, voff, G, V, [&](int64_t, float, bool) { ++n; });
-      counts[x] = n;
-    } else {
-      int64_t pos = counts[x];  // scanned: x's first list entry
-      float d = 0.f, p[3] = {0.f, 0.f, 0.f};
-      for_each_contribution(q, level_sets, 0, voff, G, V, [&](int64_t vi, float t, bool origin) {
-        list[pos++] = make_int2((int)vi | (origin ? (int)0x80000000 : 0), __float_as_int(t));
-        if (dsdf) d += weighted(__ldg(dsdf + vi), t, origin);
-        if (dv) {
+      for (int j = 0; j < kAhead; ++j) e[j] = __ldg(list + min(p + j, end - 1));
+      float x[kAhead][kRows];
 #pragma unroll
-          for (int ch = 0; ch < 3; ++ch) p[ch] += weighted(__ldg(dv + 3 * vi + ch), t, origin);
+      for (int j = 0; j < kAhead; ++j)
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+          x[j][k] = __ldg(dsh + 3 * (int64_t)(e[j].x & 0x7fffffff) + ch + k * row_plane);
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        if (p + j < end) {
+#pragma unroll
+          for (int k = 0; k < kRows; ++k) acc[k] += weighted(x[j][k], __int_as_float(e[j].y), e[j].x < 0);
         }
-      });
-      if (gdsdf) gdsdf[x] = d;
-      if (gdv) {
+      }
+    }
+  }
 #pragma unroll
-        for (int ch = 0; ch < 3; ++ch) gdv[3 * x + ch] = p[ch];
-      }
-    }
-  }
-  if (!kFill && blockIdx.x == 0 && threadIdx.x == 0) counts[G] = 0;
+  for (int k = 0; k < kRows; ++k) __stcs(dst + k * grid_plane, acc[k]);
 }
 
-__global__ void vertex_sh_gather_kernel(const float* __restrict__ dsh, int C, int64_t V, int64_t G,
-                                        const int32_t* __restrict__ offsets, const int2* __restrict__ list,
-                                        float* __restrict__ gdsh) {
-  const int64_t total = (int64_t)C * G;
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = o / G, x = o - k * G;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    if (dsh) {
-      const int32_t end = __ldg(offsets + x + 1);
-      for (int32_t p = __ldg(offsets + x); p < end; ++p) {
-        const int2 e = __ldg(list + p);
-        const int64_t vi = e.x & 0x7fffffff;
-        const bool origin = e.x < 0;
-        const float t = __int_as_float(e.y);
-        const float* src = dsh + (k * V + vi) * 3;
-        a0 += weighted(__ldg(src + 0), t, origin);
-        a1 += weighted(__ldg(src + 1), t, origin);
-        a2 += weighted(__ldg(src + 2), t, origin);
-      }
-    }
-    float* dst = gdsh + (k * G + x) * 3;
-    dst[0] = a0;
-    dst[1] = a1;
-    dst[2] = a2;
-  }
+// A thread to a float (grid vertex, channel) of the grid's rows: neighbouring
+// threads read and write neighbouring floats, four rows at a time with four
+// list entries ahead. Bound by the L1's line look-ups, one for each (list
+// entry, row), as a list's vertices lie apart: a thread to a (row, grid
+// vertex) made three of them and read the list again for every row; 16 rows at
+// a time (one reading of the list) lose the lines that neighbouring lists
+// share. 512^3, 8 shells, C = 16: 1178 us before, 1047 to 1111 with this (16 rows, one
+// entry: 1553 us; 8 and 4: 1205).
+constexpr int kGatherThreads = 192, kGatherRows = 4, kGatherAhead = 4;
+
+__global__ void __launch_bounds__(kGatherThreads)
+    vertex_sh_gather_kernel(const float* __restrict__ dsh, int C, int64_t V, int64_t G,
+                            const int32_t* __restrict__ offsets, const int2* __restrict__ list,
+                            float* __restrict__ gdsh) {
+  const int64_t row_plane = 3 * V, grid_plane = 3 * G;
+  const int64_t o = blockIdx.x * (int64_t)kGatherThreads + threadIdx.x;
+  if (o >= grid_plane) return;
+  const int64_t x = o / 3;
+  const int ch = (int)(o - 3 * x);
+  const int32_t begin = __ldg(offsets + x), end = __ldg(offsets + x + 1);
+  int k = 0;
+  for (; k + kGatherRows <= C; k += kGatherRows)
+    gather_sh_rows<kGatherRows, kGatherAhead>(dsh ? dsh + k * row_plane : nullptr, row_plane, begin, end, ch, list,
+                                              gdsh + k * grid_plane + o, grid_plane);
+  for (; k < C; ++k)
+    gather_sh_rows<1, kGatherAhead>(dsh ? dsh + k * row_plane : nullptr, row_plane, begin, end, ch, list,
+                                    gdsh + k * grid_plane + o, grid_plane);
 }
 
-// The signed-distance and position gradients of the list (pass 2's sums,
-// in list order, so the same bits), for a list built ahead of the backward.
+// The signed-distance and position gradients of the list.
 __global__ void vertex_grads_from_list_kernel(const int32_t* __restrict__ offsets, const int2* __restrict__ list,
                                               int64_t G, const float* __restrict__ dv, const float* __restrict__ dsdf,
                                               float* __restrict__ gdv, float* __restrict__ gdsdf) {
@@ -802,7 +841,7 @@ __global__ void vertex_grads_from_list_kernel(const int32_t* __restrict__ offset
 }
 
 // ---------------------------------------------------------------------------
-// The same contribution list built per grid entry (mt_build_vertex_grad_list).
+// The contribution list, built per grid entry (mt_build_vertex_grad_list).
 //
 // Grid vertex x's list is four segments: the vertices of the entry whose
 // origin x is, then the axis-0, axis-1 and axis-2 vertices of the entries
@@ -813,7 +852,8 @@ __global__ void vertex_grads_from_list_kernel(const int32_t* __restrict__ offset
 // Pass 1 adds each owned segment's length to x's count and stores it in byte
 // r of x's segment word; pass 2 writes the segment at x's scanned offset plus
 // the lengths of x's earlier segments. Each entry loads its own corners once
-// (the per-vertex passes load four entries' corners per grid vertex).
+// (a pass per grid vertex loads four entries' corners for each: 318 + 411 us
+// at 512^3, 8 shells; this 205 + 290).
 // Counts and segment words start at zero (cleared by invert_corners_kernel).
 // ---------------------------------------------------------------------------
 template <bool kFill>
@@ -1157,8 +1197,8 @@ __global__ void grid_sh_gather_kernel(const int32_t* __restrict__ offsets, const
   }
 }
 
-size_t vertex_grad_bytes(int64_t G, int64_t V, int32_t** counts, int2** list, void** scan_ws, size_t* scan_bytes,
-                         char* base) {
+size_t vertex_grad_bytes(int64_t G, int64_t V, int32_t** counts, int2** list, uint32_t** segments, void** scan_ws,
+                         size_t* scan_bytes, char* base) {
   size_t off = 256;  // the workspace status word
   auto take = [&](size_t bytes) {
     char* q = base ? base + off : nullptr;
@@ -1167,10 +1207,12 @@ size_t vertex_grad_bytes(int64_t G, int64_t V, int32_t** counts, int2** list, vo
   };
   char* c = take((size_t)(G + 1) * sizeof(int32_t));
   char* l = take((size_t)2 * (V > 0 ? V : 0) * sizeof(int2));
+  char* seg = take((size_t)G * sizeof(uint32_t));
   const size_t sb = mt_scan_workspace_bytes(G + 1);
   char* sw = take(sb);
   if (counts) *counts = reinterpret_cast<int32_t*>(c);
   if (list) *list = reinterpret_cast<int2*>(l);
+  if (segments) *segments = reinterpret_cast<uint32_t*>(seg);
   if (scan_ws) *scan_ws = sw;
   if (scan_bytes) *scan_bytes = sb;
   return off;
@@ -1588,15 +1630,21 @@ int mt_create_triangle_vertices(const float* grid_vertices, const float* grid_si
   MT_CHECK_LAUNCH();
   if (spherical_harmonics == nullptr) return MT_OK;  // rows left to mt_grid_sh_colors
   MT_REQUIRE(grid_spherical_harmonics);
-  interpolate_vertex_sh_kernel<<<grid_stride_blocks((int64_t)C * V, 256), 256, 0, as_stream(stream)>>>(
-      grid_spherical_harmonics, C, G, vertex_sources, V, num_vertices, spherical_harmonics);
+  const int64_t blocks = (G + kRowTile - 1) / kRowTile;
+  MT_REQUIRE(blocks < ((int64_t)1 << 31));
+  if (12 * G < ((int64_t)1 << 32))
+    interpolate_vertex_sh_kernel<uint32_t><<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
+        grid_spherical_harmonics, C, G, vertex_sources, V, num_vertices, vertex_offsets, S, spherical_harmonics);
+  else
+    interpolate_vertex_sh_kernel<int64_t><<<(unsigned)blocks, 256, 0, as_stream(stream)>>>(
+        grid_spherical_harmonics, C, G, vertex_sources, V, num_vertices, vertex_offsets, S, spherical_harmonics);
   MT_CHECK_LAUNCH();
   return MT_OK;
 }
 
 size_t mt_create_triangle_vertices_backward_workspace_bytes(int64_t G, int64_t V) {
   if (G < 0 || V < 0) return 0;
-  return vertex_grad_bytes(G, V, nullptr, nullptr, nullptr, nullptr, nullptr);
+  return vertex_grad_bytes(G, V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
 }
 
 int mt_create_triangle_vertices_backward(const float* grid_signed_distances, int32_t C, const int32_t* lower_corners,
@@ -1614,14 +1662,21 @@ int mt_create_triangle_vertices_backward(const float* grid_signed_distances, int
   MT_REQUIRE(grad_vertices == nullptr || grad_grid_vertices != nullptr);
   cudaStream_t st = as_stream(stream);
   if (cudaMemsetAsync(corner_inverse, 0xff, (size_t)G * 4 * sizeof(int32_t), st) != cudaSuccess) return MT_ERR_CUDA;
-  invert_corners_kernel<<<grid_stride_blocks(G, 256), 256, 0, st>>>(lower_corners, G, corner_inverse);
-  MT_CHECK_LAUNCH();
   // With no level sets or no vertices, the gather writes zeros everywhere.
   const float* gv = V > 0 ? grad_vertices : nullptr;
   const float* gd = V > 0 ? grad_signed_distances : nullptr;
   const float* gs = V > 0 ? grad_spherical_harmonics : nullptr;
   const bool listed = S <= kShellsPerChunk && V < (int64_t)0x7fffffff && workspace &&
-                      workspace_bytes >= vertex_grad_bytes(G, V, nullptr, nullptr, nullptr, nullptr, nullptr);
+                      workspace_bytes >= mt_create_triangle_vertices_backward_workspace_bytes(G, V);
+  int32_t* counts = nullptr;
+  int2* list = nullptr;
+  uint32_t* segments = nullptr;
+  void* scan_ws = nullptr;
+  size_t scan_bytes = 0;
+  if (listed) vertex_grad_bytes(G, V, &counts, &list, &segments, &scan_ws, &scan_bytes, static_cast<char*>(workspace));
+  invert_corners_kernel<<<grid_stride_blocks(G, 256), 256, 0, st>>>(lower_corners, G, corner_inverse, counts,
+                                                                    segments);
+  MT_CHECK_LAUNCH();
   if (!listed) {
     create_vertices_backward_kernel<<<grid_stride_blocks(G, 128), 128, 0, st>>>(
         grid_signed_distances, C, lower_corners, G, level_sets, S, vertex_offsets, corner_inverse, gv, gd, gs, V,
@@ -1629,23 +1684,24 @@ int mt_create_triangle_vertices_backward(const float* grid_signed_distances, int
     MT_CHECK_LAUNCH();
     return MT_OK;
   }
-  int32_t* counts = nullptr;
-  int2* list = nullptr;
-  void* scan_ws = nullptr;
-  size_t scan_bytes = 0;
-  vertex_grad_bytes(G, V, &counts, &list, &scan_ws, &scan_bytes, static_cast<char*>(workspace));
-  vertex_grad_list_kernel<false><<<grid_stride_blocks(G, 128), 128, 0, st>>>(
-      grid_signed_distances, lower_corners, G, level_sets, S, vertex_offsets, corner_inverse, V, counts, nullptr,
-      nullptr, nullptr, nullptr, nullptr);
+  entry_list_kernel<false><<<grid_stride_blocks(G, 256), 256, 0, st>>>(grid_signed_distances, lower_corners, G,
+                                                                       level_sets, S, vertex_offsets, corner_inverse,
+                                                                       V, counts, segments, nullptr);
   MT_CHECK_LAUNCH();
   const int rc = mt_exclusive_scan_i32(counts, G + 1, scan_ws, scan_bytes, stream);
   if (rc != MT_OK) return rc;
-  vertex_grad_list_kernel<true><<<grid_stride_blocks(G, 128), 128, 0, st>>>(
-      grid_signed_distances, lower_corners, G, level_sets, S, vertex_offsets, corner_inverse, V, counts, list, gv,
-      gd, grad_grid_vertices, grad_grid_signed_distances);
+  entry_list_kernel<true><<<grid_stride_blocks(G, 256), 256, 0, st>>>(grid_signed_distances, lower_corners, G,
+                                                                      level_sets, S, vertex_offsets, corner_inverse,
+                                                                      V, counts, segments, list);
   MT_CHECK_LAUNCH();
-  vertex_sh_gather_kernel<<<grid_stride_blocks((int64_t)C * G, 256), 256, 0, st>>>(gs, C, V, G, counts, list,
-                                                                                 grad_grid_spherical_harmonics);
+  vertex_grads_from_list_kernel<<<grid_stride_blocks(G, 256), 256, 0, st>>>(counts, list, G, gv, gd,
+                                                                            grad_grid_vertices,
+                                                                            grad_grid_signed_distances);
+  MT_CHECK_LAUNCH();
+  const int64_t blocks = (3 * G + kGatherThreads - 1) / kGatherThreads;
+  MT_REQUIRE(blocks < ((int64_t)1 << 31));
+  vertex_sh_gather_kernel<<<(unsigned)blocks, kGatherThreads, 0, st>>>(gs, C, V, G, counts, list,
+                                                                       grad_grid_spherical_harmonics);
   MT_CHECK_LAUNCH();
   return MT_OK;
 }
