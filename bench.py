@@ -457,7 +457,7 @@ def run_ours(args, rank, world, local):
     bytes_by_stage = pipeline.step_bytes(stats)
     # Library entry point -> the step_bytes stages its kernels cover.
     stages_of = {
-        "mt_intersect_and_composite_backward": ("composite_bwd",),
+        "mt_intersect_and_composite_packed_backward": ("composite_bwd",),
         "mt_intersect_and_composite_forward": ("composite_fwd", "warp_masks"),
         "mt_sort_keys_by_tile": ("tile_sort",),
         "mt_bound_and_generate_keys": ("keys",),

@@ -374,6 +374,17 @@ MT_API int mt_grid_sh_colors_backward(const int32_t* list_offsets, const int32_t
                                       const int32_t* num_vertices, void* workspace,
                                       size_t workspace_bytes, mt_stream_t stream);
 
+/* The same from packed_gradients [B,V,4] (16-byte aligned; the fourth float is
+ * not used). */
+MT_API int mt_grid_sh_colors_packed_backward(const int32_t* list_offsets, const int32_t* list,
+                                      int64_t G, int64_t V, const float* vertices,
+                                      int32_t C, int32_t sh_degree,
+                                      const float* camera_positions, int32_t B,
+                                      const float* out_colors, const float* packed_gradients,
+                                      float* grad_grid_spherical_harmonics,
+                                      const int32_t* num_vertices, void* workspace,
+                                      size_t workspace_bytes, mt_stream_t stream);
+
 /* triangle_extraction/compute_sdf_regularizers.slang:18-128 (forward) and its
  * automatic derivative (backward). Per voxel: eikonal_loss_pos / _neg [Nv]
  * (squared excess / deficit of the trilinear SDF's gradient norm at the
@@ -495,6 +506,13 @@ MT_API int mt_evaluate_spherical_harmonics_backward(
     const float* vertices, int64_t V, int32_t C, int32_t sh_degree,
     const float* camera_positions, int32_t B, const float* out_colors,
     const float* grad_colors, float* grad_spherical_harmonics, mt_stream_t stream);
+
+/* The same from packed_gradients [B,V,4] (16-byte aligned; the fourth float is
+ * not used). */
+MT_API int mt_evaluate_spherical_harmonics_packed_backward(
+    const float* vertices, int64_t V, int32_t C, int32_t sh_degree,
+    const float* camera_positions, int32_t B, const float* out_colors,
+    const float* packed_gradients, float* grad_spherical_harmonics, mt_stream_t stream);
 
 /* triangle_rasterization/bound_triangles.slang:144-192.
  * out_min / out_max [B,F,2] (row, col) tile bounds [min, max); out_count
@@ -664,6 +682,30 @@ MT_API int mt_intersect_and_composite_backward(
     void* staging, size_t staging_bytes, const int32_t* tile_order, size_t tile_order_bytes,
     int32_t cta_threads, mt_stream_t stream);
 
+/* The same into packed_gradients [B,V,4] (+=, 16-byte aligned): a (camera,
+ * vertex)'s colour gradient and the camera's part of its signed distance's,
+ * one 16-byte reduction per hit and vertex where the separate tensors take
+ * four of 4 bytes. */
+MT_API int mt_intersect_and_composite_packed_backward(
+    const float* xy, const float* colors, const float* signed_distances, int64_t V,
+    const int32_t* faces, const float* sharpness, const int64_t* sorted_keys,
+    const int32_t* sorted_triangles, int64_t K, const int64_t* tile_boundaries,
+    int32_t B, int32_t num_shells, int32_t rows, int32_t cols, int32_t tile_h,
+    int32_t tile_w, int32_t H, int32_t W, const int32_t* layout,
+    const int64_t* cameras, int64_t camera_tiles, const uint32_t* warp_masks,
+    uint64_t* work_counter, const float* out, const float* grad_out,
+    const float* target, const float* background, float loss_scale,
+    const float* grad_loss, int32_t ssaa, float* packed_gradients,
+    float* grad_sharpness, int32_t exact_adjoint, const void* hit_bits, size_t hit_bits_bytes,
+    void* staging, size_t staging_bytes, const int32_t* tile_order, size_t tile_order_bytes,
+    int32_t cta_threads, mt_stream_t stream);
+
+/* packed_gradients [B,V,4] to grad_colors [B,V,3] (unless NULL) and
+ * grad_signed_distances [V], the sum over the cameras (unless NULL). */
+MT_API int mt_unpack_gradients(const float* packed_gradients, int32_t B, int64_t V,
+                               float* grad_colors, float* grad_signed_distances,
+                               mt_stream_t stream);
+
 /* Bytes of the optional tile order of the compositing kernels (not in the
  * reference, whose CTAs take tiles in grid order): int32 bucket counts and
  * cursors, then one global tile index per tile (camera_tiles of them). With
@@ -773,8 +815,8 @@ MT_API int mt_shade_shells(const float* uv, const int32_t* index, int32_t B,
                            float* out_transmittances, float* image,
                            mt_stream_t stream);
 
-/* Its adjoint; accumulates (+=) into grad_signed_distances [V], grad_colors
- * [B,V,3], grad_sharpness [1]. grad_out [B,H,W,3] (NULL: zero) is the image's
+/* Its adjoint; accumulates (+=) into packed_gradients [B,V,4] (16-byte aligned;
+ * see mt_unpack_gradients), grad_sharpness [1]. grad_out [B,H,W,3] (NULL: zero) is the image's
  * gradient when a background is given, else out_colors'; exact_adjoint as in
  * mt_composite_backward. */
 MT_API int mt_shade_shells_backward(
@@ -783,9 +825,8 @@ MT_API int mt_shade_shells_backward(
     const float* colors, int64_t V, const float* sharpness,
     const float* background, const float* out_colors,
     const float* out_transmittances, const float* grad_out,
-    const float* grad_out_transmittances, float* grad_signed_distances,
-    float* grad_colors, float* grad_sharpness, int32_t exact_adjoint,
-    mt_stream_t stream);
+    const float* grad_out_transmittances, float* packed_gradients,
+    float* grad_sharpness, int32_t exact_adjoint, mt_stream_t stream);
 
 #ifdef __cplusplus
 }  /* extern "C" */

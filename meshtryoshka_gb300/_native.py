@@ -82,6 +82,7 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_grid_sh_colors": (I32, [P, I32, I64, P, I64, P, P, I32, P, I32, P, P]),
     "mt_grid_sh_colors_backward_workspace_bytes": (c_size_t, [I64]),
     "mt_grid_sh_colors_backward": (I32, [P, P, I64, I64, P, I32, I32, P, I32, P, P, P, P, P, c_size_t, P]),
+    "mt_grid_sh_colors_packed_backward": (I32, [P, P, I64, I64, P, I32, I32, P, I32, P, P, P, P, P, c_size_t, P]),
     "mt_capacity_overflow": (I32, [P, I64, P, I64, P, I64, P, P]),
     "mt_sort_pairs_workspace_bytes": (c_size_t, [I64]),
     "mt_sort_pairs_i64_i32": (I32, [P, P, P, P, I64, P, I32, I32, P, c_size_t, P]),
@@ -89,6 +90,7 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_project_vertices": (I32, [P, I64, P, P, I32, P, P, P]),
     "mt_evaluate_spherical_harmonics": (I32, [P, I64, P, I32, I32, P, I32, P, P]),
     "mt_evaluate_spherical_harmonics_backward": (I32, [P, I64, I32, I32, P, I32, P, P, P, P]),
+    "mt_evaluate_spherical_harmonics_packed_backward": (I32, [P, I64, I32, I32, P, I32, P, P, P, P]),
     "mt_bound_triangles": (I32, [P, P, I64, P, I64, P, I32, I32, I32, I32, I32, P, c_float, P, P, P, P]),
     "mt_generate_keys": (I32, [P, I64, P, I64, P, I32, P, P, P, I32, I32, P, P, I64, P, P, P]),
     "mt_bound_and_generate_keys_workspace_bytes": (c_size_t, [I64]),
@@ -112,6 +114,12 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
         [P, P, P, I64, P, P, P, P, I64, P, I32, I32, I32, I32, I32, I32, I32, I32, P, P, I64, P, P, P, P, P, P,
          c_float, P, I32, P, P, P, I32, P, c_size_t, P, c_size_t, P, c_size_t, I32, P],
     ),
+    "mt_intersect_and_composite_packed_backward": (
+        I32,
+        [P, P, P, I64, P, P, P, P, I64, P, I32, I32, I32, I32, I32, I32, I32, I32, P, P, I64, P, P, P, P, P, P,
+         c_float, P, I32, P, P, I32, P, c_size_t, P, c_size_t, P, c_size_t, I32, P],
+    ),
+    "mt_unpack_gradients": (I32, [P, I32, I64, P, P, P]),
     "mt_composite_staging_bytes": (c_size_t, [I32, I64]),
     "mt_ssaa_loss": (I32, [P, I32, I32, I32, I32, P, P, c_float, P, P, P]),
     "mt_finish_images": (I32, [P, I32, P, I32, P, P, P]),
@@ -124,7 +132,7 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_shade_shells": (I32, [P, P, I32, I32, I32, I32, P, P, P, I64, P, P, P, P, P, P]),
     "mt_shade_shells_backward": (
         I32,
-        [P, P, I32, I32, I32, I32, P, P, P, I64, P, P, P, P, P, P, P, P, P, I32, P],
+        [P, P, I32, I32, I32, I32, P, P, P, I64, P, P, P, P, P, P, P, P, I32, P],
     ),
 }
 
@@ -172,6 +180,7 @@ KERNELS_PER_CALL = {
     "mt_bound_and_generate_keys": 3,  # rectangles + chunk counts, chunk scan, keys
     "mt_build_vertex_grad_list": 4,  # corner inverse, count, scan, fill
     "mt_grid_sh_colors_backward": 2,  # per-vertex SH gradients, per-grid-vertex sums
+    "mt_grid_sh_colors_packed_backward": 2,
 }
 
 
@@ -229,6 +238,17 @@ def call(name: str, *args, launches: int | None = None) -> None:
     if status != 0:
         msg = lib.mt_status_string(status).decode()
         raise RuntimeError(f"{name} failed: {msg} (status {status})")
+
+
+def colour_gradient_rows(grad: torch.Tensor) -> tuple[torch.Tensor, bool]:
+    """A [B, V, 3] colour gradient as the SH adjoints read it: in place when it
+    is the colours of packed [B, V, 4] rows (True), else contiguous (False)."""
+    b, v, _ = grad.shape
+    if (grad.numel() > 0 and not grad.is_contiguous() and grad.dtype == torch.float32 and v > 1
+            and grad.stride()[1:] == (4, 1) and (b == 1 or grad.stride(0) == 4 * v) and grad.data_ptr() % 16 == 0
+            and grad.storage_offset() + 4 * b * v <= grad.untyped_storage().nbytes() // 4):
+        return grad, True
+    return grad.contiguous(), False
 
 
 def ptr(t: torch.Tensor | None) -> int | None:

@@ -30,10 +30,9 @@
 // store's capacity lasts; the backward re-walks the same way, reads those
 // bits instead of testing again (gathering only the triangles some pixel
 // hits), re-solves each hit's barycentrics and applies the suffix trick of
-// the reference. Batches past the capacity are tested again. Per-triangle gradient sums live in a per-warp ring
-// of 64 shared-memory slots (the current and the previous batch); a slot is
-// flushed to global memory with one atomic per non-zero scalar when its batch
-// retires, and gradients for older triangles go to global memory directly.
+// the reference. Batches past the capacity are tested again. A hit's gradient
+// goes to its triangle's three vertices in global memory: colour and signed
+// distance of a (camera, vertex) side by side, one 16-byte reduction each.
 // Two routings:
 //   reference (exact_adjoint = 0): the deferred gradient of the previous
 //     (outer) hit is scattered to the previous triangle's vertices with the
@@ -54,7 +53,6 @@ namespace {
 constexpr int kBatch = 32;   // triangles gathered per warp batch
 constexpr int kScan = 8;     // groups of 32 masks loaded side by side
 constexpr int kQueue = 64;   // queued key offsets per warp
-constexpr int kRing = 64;    // gradient slots per warp (two batches)
 constexpr int kSavedFwd = 2;  // hits per pixel per batch whose samples the test phase keeps (forward)
 constexpr int kSavedBwd = 3;  // same, backward (its shared memory is tighter)
 // Hit-bit store (bytes): [0, 8) batch allocator, [8, 8 + 4 items) first
@@ -143,6 +141,7 @@ struct CompositeGrads {
   const float* grad_out;  // [B, 4, H, W]
   float* grad_colors;     // [B, V, 3]
   float* grad_sdf;        // [V]
+  float4* packed;         // [B, V] (r, g, b, signed distance) in place of the two, or NULL
   float* grad_sharpness;  // [1]
   int exact;
 };
@@ -216,8 +215,7 @@ struct WarpBackward {
   TriGeom geo[kBatch];
   TriAttr attr[kBatch];
   SavedHits<kSavedBwd> saved;
-  int3 vids[kRing];
-  float gslot[kRing][13];  // 12 used; stride 13 keeps lanes on distinct banks
+  int3 vids[kBatch];  // the triangles' vertices
   int queue[kQueue];
 };
 
@@ -1184,52 +1182,31 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps)
   }
 }
 
-__device__ __forceinline__ void scatter_global(const CompositeArgs& a, const CompositeGrads& gr, int cam, int3 vid,
-                                               float u, float v, float w, const float (&drgb)[3], float dsdf) {
-  float* gc = gr.grad_colors + (int64_t)cam * a.V * 3;
+// Adds a hit's gradient to its triangle's vertices. (Sums per triangle in
+// shared memory, flushed when its batch retired, cost more than they saved:
+// shared-memory float additions are loops of compare-and-swap, and a triangle
+// of a fine mesh has two to four hits in a warp. Five million hits: 60 to 80 us
+// as 16-byte reductions, 40 to 170 us in shared memory and 150 to 200 us as
+// scalar ones. Backward kernel of the 256^3 step: 195 us with the sums, now
+// 118; of the 512^3 step 2.20 ms, now 1.06.)
+__device__ __forceinline__ void scatter(const CompositeArgs& a, const CompositeGrads& gr, int cam, int3 vid, float u,
+                                        float v, float w, const float (&drgb)[3], float dsdf) {
+  if (drgb[0] == 0.f && drgb[1] == 0.f && drgb[2] == 0.f && dsdf == 0.f) return;
   const int id[3] = {vid.x, vid.y, vid.z};
   const float wt[3] = {u, v, w};
+  if (gr.packed) {
+    float4* rows = gr.packed + (int64_t)cam * a.V;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) red_add(rows + id[q], wt[q] * drgb[0], wt[q] * drgb[1], wt[q] * drgb[2], wt[q] * dsdf);
+    return;
+  }
+  float* gc = gr.grad_colors + (int64_t)cam * a.V * 3;
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) atomicAdd(gc + 3 * (int64_t)id[q] + c, wt[q] * drgb[c]);
     atomicAdd(gr.grad_sdf + id[q], wt[q] * dsdf);
   }
-}
-
-__device__ __forceinline__ void scatter_slot(float* slot, float u, float v, float w, const float (&drgb)[3],
-                                             float dsdf) {
-  const float wt[3] = {u, v, w};
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) atomicAdd(slot + 4 * q + c, wt[q] * drgb[c]);
-    atomicAdd(slot + 4 * q + 3, wt[q] * dsdf);
-  }
-}
-
-// Flushes and clears the 32 ring slots of batch parity `half` (lane i owns
-// slot half * 32 + i).
-__device__ __forceinline__ void flush_half(const CompositeArgs& a, const CompositeGrads& gr, int cam, WarpBackward& ws,
-                                           int half, int lane) {
-  const int slot = half * kBatch + lane;
-  float* g = ws.gslot[slot];
-  const int3 vid = ws.vids[slot];
-  const int id[3] = {vid.x, vid.y, vid.z};
-  float* gc = gr.grad_colors + (int64_t)cam * a.V * 3;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float x = g[4 * q + c];
-      if (x != 0.f) atomicAdd(gc + 3 * (int64_t)id[q] + c, x);
-      g[4 * q + c] = 0.f;
-    }
-    const float y = g[4 * q + 3];
-    if (y != 0.f) atomicAdd(gr.grad_sdf + id[q], y);
-    g[4 * q + 3] = 0.f;
-  }
-  __syncwarp();
 }
 
 // Returns false when a staged wait gave up (the warp then stops).
@@ -1285,11 +1262,6 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
       dL_T = gr.grad_out[o + 3 * px.plane];
     }
   }
-  for (int i = lane; i < kRing * 13; i += 32) (&ws.gslot[0][0])[i] = 0.f;
-  ws.vids[lane] = make_int3(0, 0, 0);
-  ws.vids[kBatch + lane] = make_int3(0, 0, 0);
-  __syncwarp();
-
   float acc[3] = {0.f, 0.f, 0.f};
   float T_ = 1.0f;
   bool active = px.in_image;
@@ -1300,7 +1272,6 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
   float d_sharp = 0.f;
   float dp_rgb[3] = {0.f, 0.f, 0.f};
   float dp_sdf = 0.f;
-  int prev_batch = -2, prev_slot = 0;  // ring slot of the previous hit (valid while its batch is live)
   int3 prev_vid = make_int3(0, 0, 0);
   float pu = 0.f, pv = 0.f, pw = 0.f;
 
@@ -1349,7 +1320,6 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
     int nb;
     bool stored;
     uint32_t hits;
-    const int half = batch & 1;
     if constexpr (kStaged) {
       nb = nb_next;
       if (nb == 0) break;
@@ -1361,7 +1331,6 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
         return false;
       }
       ++phase;
-      if (batch >= 2) flush_half(a, gr, cam, ws, half, lane);
       if (lane < nb && ((needed >> lane) & 1u)) {
         const VertexRecord ra = ws.stage[lane][0], rb = ws.stage[lane][1], rc = ws.stage[lane][2];
         TriGeom g;
@@ -1369,15 +1338,13 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
         g.shell = shell_next;
         ws.geo[lane] = g;
         ws.attr[lane] = TriAttr{{ra.r, ra.g, ra.b}, {rb.r, rb.g, rb.b}, {rc.r, rc.g, rc.b}, ra.sdf, rb.sdf, rc.sdf};
-        ws.vids[half * kBatch + lane] = vid_next;
+        ws.vids[lane] = vid_next;
       }
       __syncwarp();
       form_next(batch + 1);  // the next batch's copies overlap this batch's compositing
     } else {
       nb = refill(walk, ws.queue, px.wt, lane);
       if (nb == 0) break;
-      // The half being overwritten held batch - 2: flush it first.
-      if (batch >= 2) flush_half(a, gr, cam, ws, half, lane);
       // The forward's hit bits for this batch when it stored them (the same
       // walk, so the same bits); otherwise the test phase runs again. With
       // stored bits only the triangles that some pixel of the warp hits are
@@ -1386,7 +1353,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
       hits = stored ? __ldcs(hs.batches + (hit_base + batch) * 32 + lane) : 0u;
       const uint32_t needed = stored ? __reduce_or_sync(0xffffffffu, hits) : 0xffffffffu;
       if (lane < nb && ((needed >> lane) & 1u))
-        ws.vids[half * kBatch + lane] = gather(a, cam, start + ws.queue[walk.head + lane], ws.geo, ws.attr, lane);
+        ws.vids[lane] = gather(a, cam, start + ws.queue[walk.head + lane], ws.geo, ws.attr, lane);
       __syncwarp();
       pop(walk, nb);
     }
@@ -1442,17 +1409,12 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
         if (last_shell != -1) {
           dp_sdf += d_oc * ko * s;
           const float su = gr.exact ? pu : u, sv = gr.exact ? pv : v, sw = gr.exact ? pw : w;
-          if (prev_batch >= batch - 1)
-            scatter_slot(ws.gslot[prev_slot], su, sv, sw, dp_rgb, dp_sdf);
-          else
-            scatter_global(a, gr, cam, prev_vid, su, sv, sw, dp_rgb, dp_sdf);
+          scatter(a, gr, cam, prev_vid, su, sv, sw, dp_rgb, dp_sdf);
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) dp_rgb[c] = d_color[c];
         dp_sdf = d_ic * ki * s;
-        prev_batch = batch;
-        prev_slot = half * kBatch + i;
-        prev_vid = ws.vids[prev_slot];
+        prev_vid = ws.vids[i];
         pu = u;
         pv = v;
         pw = w;
@@ -1483,15 +1445,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
     }
   }
   // The last hit's deferred gradient, with its own weights.
-  if (px.in_image && last_shell != -1) {
-    if (prev_batch >= batch - 2)
-      scatter_slot(ws.gslot[prev_slot], pu, pv, pw, dp_rgb, dp_sdf);
-    else
-      scatter_global(a, gr, cam, prev_vid, pu, pv, pw, dp_rgb, dp_sdf);
-  }
-  __syncwarp();
-  flush_half(a, gr, cam, ws, 0, lane);
-  flush_half(a, gr, cam, ws, 1, lane);
+  if (px.in_image && last_shell != -1) scatter(a, gr, cam, prev_vid, pu, pv, pw, dp_rgb, dp_sdf);
 
   // Sharpness gradient: one atomic per warp.
   float x = px.in_image ? d_sharp : 0.f;
@@ -1528,6 +1482,27 @@ __global__ void __launch_bounds__(32 * kWarps, kStaged ? 1 : (24 / kWarps > 0 ? 
   for (int64_t u = next_item(counter, lane); u < *(volatile int64_t*)&s_keyed; u = next_item(counter, lane)) {
     const int64_t item = ordered_item(a, order, u);
     if (!backward_item<kStaged>(a, masks, gr, ws, pixel_of(a, item), lane, item, hs, st, phase)) return;
+  }
+}
+
+// Packed gradients to their tensors: grad_colors [B, V, 3] (unless NULL), and
+// grad_sdf [V] (unless NULL), the sum over the cameras.
+__global__ void unpack_gradients_kernel(const float4* __restrict__ packed, int B, int64_t V,
+                                        float* __restrict__ grad_colors, float* __restrict__ grad_sdf) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
+    float sdf = 0.0f;
+#pragma unroll 4
+    for (int b = 0; b < B; ++b) {
+      const int64_t o = (int64_t)b * V + v;
+      const float4 g = __ldg(packed + o);
+      sdf += g.w;
+      if (grad_colors) {
+        grad_colors[3 * o] = g.x;
+        grad_colors[3 * o + 1] = g.y;
+        grad_colors[3 * o + 2] = g.z;
+      }
+    }
+    if (grad_sdf) grad_sdf[v] = sdf;
   }
 }
 
@@ -1955,20 +1930,20 @@ int mt_intersect_and_composite_forward(const float* xy, const float* colors, con
   }
 }
 
-int mt_intersect_and_composite_backward(const float* xy, const float* colors, const float* signed_distances,
-                                        int64_t V, const int32_t* faces, const float* sharpness,
-                                        const int64_t* sorted_keys, const int32_t* sorted_triangles, int64_t K,
-                                        const int64_t* tile_boundaries, int32_t B, int32_t num_shells,
-                                        int32_t rows, int32_t cols, int32_t tile_h, int32_t tile_w, int32_t H,
-                                        int32_t W, const int32_t* layout, const int64_t* cameras,
-                                        int64_t camera_tiles, const uint32_t* warp_masks, uint64_t* work_counter,
-                                        const float* out, const float* grad_out, const float* target,
-                                        const float* background, float loss_scale, const float* grad_loss,
-                                        int32_t ssaa, float* grad_colors, float* grad_signed_distances,
-                                        float* grad_sharpness,
-                                        int32_t exact_adjoint, const void* hit_bits, size_t hit_bits_bytes,
-                                        void* staging, size_t staging_bytes, const int32_t* tile_order,
-                                        size_t tile_order_bytes, int32_t cta_threads, mt_stream_t stream) {
+static int composite_backward(const float* xy, const float* colors, const float* signed_distances,
+                              int64_t V, const int32_t* faces, const float* sharpness,
+                              const int64_t* sorted_keys, const int32_t* sorted_triangles, int64_t K,
+                              const int64_t* tile_boundaries, int32_t B, int32_t num_shells,
+                              int32_t rows, int32_t cols, int32_t tile_h, int32_t tile_w, int32_t H,
+                              int32_t W, const int32_t* layout, const int64_t* cameras,
+                              int64_t camera_tiles, const uint32_t* warp_masks, uint64_t* work_counter,
+                              const float* out, const float* grad_out, const float* target,
+                              const float* background, float loss_scale, const float* grad_loss,
+                              int32_t ssaa, float* grad_colors, float* grad_signed_distances,
+                              float* packed, float* grad_sharpness,
+                              int32_t exact_adjoint, const void* hit_bits, size_t hit_bits_bytes,
+                              void* staging, size_t staging_bytes, const int32_t* tile_order,
+                              size_t tile_order_bytes, int32_t cta_threads, mt_stream_t stream) {
   MT_REQUIRE(layout != nullptr && K >= 0 && camera_tiles >= 0);
   CompositeArgs a = make_args(xy, colors, signed_distances, V, faces, sharpness, sorted_keys, sorted_triangles,
                               tile_boundaries, B, num_shells, rows, cols, tile_h, tile_w, H, W, layout, out,
@@ -1983,9 +1958,11 @@ int mt_intersect_and_composite_backward(const float* xy, const float* colors, co
   if (a.total_tiles == 0 || H == 0 || W == 0) return MT_OK;
   MT_REQUIRE(xy && colors && signed_distances && faces && sharpness && tile_boundaries && out);
   MT_REQUIRE(target ? (background && grad_loss) : grad_out != nullptr);
-  MT_REQUIRE(grad_colors && grad_signed_distances && grad_sharpness && work_counter);
+  MT_REQUIRE(((grad_colors && grad_signed_distances) || packed) && grad_sharpness && work_counter);
+  MT_REQUIRE((reinterpret_cast<uintptr_t>(packed) & 15) == 0);
   MT_REQUIRE(K == 0 || (sorted_keys && sorted_triangles && warp_masks));
-  CompositeGrads gr{grad_loss, grad_out, grad_colors, grad_signed_distances, grad_sharpness, exact_adjoint ? 1 : 0};
+  CompositeGrads gr{grad_loss, grad_out, grad_colors, grad_signed_distances, reinterpret_cast<float4*>(packed),
+                    grad_sharpness, exact_adjoint ? 1 : 0};
   HitStore hs;
   rc = make_hit_store(a, const_cast<void*>(hit_bits), hit_bits_bytes, hs);
   if (rc != MT_OK) return rc;
@@ -2028,6 +2005,63 @@ int mt_intersect_and_composite_backward(const float* xy, const float* colors, co
   if (warps == 4) return launch(std::false_type{}, std::integral_constant<int, 4>{});
   if (warps == 16) return launch(std::false_type{}, std::integral_constant<int, 16>{});
   return launch(std::false_type{}, std::integral_constant<int, 8>{});
+}
+
+int mt_intersect_and_composite_backward(const float* xy, const float* colors, const float* signed_distances,
+                                        int64_t V, const int32_t* faces, const float* sharpness,
+                                        const int64_t* sorted_keys, const int32_t* sorted_triangles, int64_t K,
+                                        const int64_t* tile_boundaries, int32_t B, int32_t num_shells,
+                                        int32_t rows, int32_t cols, int32_t tile_h, int32_t tile_w, int32_t H,
+                                        int32_t W, const int32_t* layout, const int64_t* cameras,
+                                        int64_t camera_tiles, const uint32_t* warp_masks, uint64_t* work_counter,
+                                        const float* out, const float* grad_out, const float* target,
+                                        const float* background, float loss_scale, const float* grad_loss,
+                                        int32_t ssaa, float* grad_colors, float* grad_signed_distances,
+                                        float* grad_sharpness,
+                                        int32_t exact_adjoint, const void* hit_bits, size_t hit_bits_bytes,
+                                        void* staging, size_t staging_bytes, const int32_t* tile_order,
+                                        size_t tile_order_bytes, int32_t cta_threads, mt_stream_t stream) {
+  return composite_backward(xy, colors, signed_distances, V, faces, sharpness, sorted_keys, sorted_triangles, K,
+                            tile_boundaries, B, num_shells, rows, cols, tile_h, tile_w, H,
+                            W, layout, cameras, camera_tiles, warp_masks, work_counter, out,
+                            grad_out, target, background, loss_scale, grad_loss, ssaa,
+                            grad_colors, grad_signed_distances, nullptr, grad_sharpness,
+                            exact_adjoint, hit_bits, hit_bits_bytes, staging, staging_bytes,
+                            tile_order, tile_order_bytes, cta_threads, stream);
+}
+
+int mt_intersect_and_composite_packed_backward(const float* xy, const float* colors, const float* signed_distances,
+                                               int64_t V, const int32_t* faces, const float* sharpness,
+                                               const int64_t* sorted_keys, const int32_t* sorted_triangles, int64_t K,
+                                               const int64_t* tile_boundaries, int32_t B, int32_t num_shells,
+                                               int32_t rows, int32_t cols, int32_t tile_h, int32_t tile_w, int32_t H,
+                                               int32_t W, const int32_t* layout, const int64_t* cameras,
+                                               int64_t camera_tiles, const uint32_t* warp_masks, uint64_t* work_counter,
+                                               const float* out, const float* grad_out, const float* target,
+                                               const float* background, float loss_scale, const float* grad_loss,
+                                               int32_t ssaa, float* packed_gradients, float* grad_sharpness,
+                                               int32_t exact_adjoint, const void* hit_bits, size_t hit_bits_bytes,
+                                               void* staging, size_t staging_bytes, const int32_t* tile_order,
+                                               size_t tile_order_bytes, int32_t cta_threads, mt_stream_t stream) {
+  return composite_backward(xy, colors, signed_distances, V, faces, sharpness, sorted_keys, sorted_triangles, K,
+                            tile_boundaries, B, num_shells, rows, cols, tile_h, tile_w, H,
+                            W, layout, cameras, camera_tiles, warp_masks, work_counter, out,
+                            grad_out, target, background, loss_scale, grad_loss, ssaa,
+                            nullptr, nullptr, packed_gradients, grad_sharpness,
+                            exact_adjoint, hit_bits, hit_bits_bytes, staging, staging_bytes,
+                            tile_order, tile_order_bytes, cta_threads, stream);
+}
+
+int mt_unpack_gradients(const float* packed_gradients, int32_t B, int64_t V, float* grad_colors,
+                        float* grad_signed_distances, mt_stream_t stream) {
+  MT_REQUIRE(B >= 0 && V >= 0);
+  if (V == 0 || B == 0) return MT_OK;
+  MT_REQUIRE(packed_gradients && (grad_colors || grad_signed_distances));
+  MT_REQUIRE((reinterpret_cast<uintptr_t>(packed_gradients) & 15) == 0);
+  unpack_gradients_kernel<<<grid_stride_blocks(V, 256), 256, 0, as_stream(stream)>>>(
+      reinterpret_cast<const float4*>(packed_gradients), B, V, grad_colors, grad_signed_distances);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
 }
 
 int mt_finish_images(const float* raw, int32_t B, const int32_t* shapes, int32_t ssaa, const float* background,

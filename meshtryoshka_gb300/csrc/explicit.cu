@@ -438,23 +438,20 @@ __global__ void __launch_bounds__(kShadeThreads)
 // The sample gradients of one hit, onto its face's vertices
 // (interpolate_backward_kernel).
 __device__ __forceinline__ void scatter_hit(const ShellHit& h, const float (&d_rgb)[3], float d_sdf,
-                                            float* __restrict__ grad_colors, float* __restrict__ grad_sdf) {
+                                            float4* __restrict__ rows) {
   if (d_sdf == 0.f && d_rgb[0] == 0.f && d_rgb[1] == 0.f && d_rgb[2] == 0.f) return;
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    if (d_sdf != 0.f) atomicAdd(grad_sdf + h.id[q], h.wt[q] * d_sdf);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) atomicAdd(grad_colors + 3 * (int64_t)h.id[q] + c, h.wt[q] * d_rgb[c]);
-  }
+  for (int q = 0; q < 3; ++q)
+    red_add(rows + h.id[q], h.wt[q] * d_rgb[0], h.wt[q] * d_rgb[1], h.wt[q] * d_rgb[2], h.wt[q] * d_sdf);
 }
 
 // grad_out: d loss / d image when the background is blended in, else
-// d loss / d out_colors (NULL: zero); grad_T: d loss / d out_T (NULL: zero).
+// d loss / d out_colors (NULL: zero); grad_T: d loss / d out_T (NULL: zero);
+// packed: [B, V] (r, g, b, signed distance) gradients.
 __global__ void __launch_bounds__(kShadeThreads)
     shade_shells_backward_kernel(ShellArgs a, const float* __restrict__ out_colors, const float* __restrict__ out_T,
                                  const float* __restrict__ grad_out, const float* __restrict__ grad_T,
-                                 float* __restrict__ grad_sdf, float* __restrict__ grad_colors,
-                                 float* __restrict__ grad_sharpness, int exact) {
+                                 float4* __restrict__ packed, float* __restrict__ grad_sharpness, int exact) {
   const float s = *a.sharpness;
   const int64_t P = a.B * a.HW;
   float bg[3] = {0.f, 0.f, 0.f};
@@ -468,7 +465,7 @@ __global__ void __launch_bounds__(kShadeThreads)
     const int64_t b = p / a.HW;
     const int64_t first = b * a.S * a.HW + (p - b * a.HW);
     const float* col = a.colors + b * a.V * 3;
-    float* gcol = grad_colors + b * a.V * 3;
+    float4* rows = packed + b * a.V;
     float dL[3] = {0.f, 0.f, 0.f}, final_rgb[3];
     float dLT = grad_T ? __ldg(grad_T + p) : 0.f;
 #pragma unroll
@@ -519,7 +516,7 @@ __global__ void __launch_bounds__(kShadeThreads)
       d_sharp += d_ic * ki * h.sdf + d_oc * ko * outer_sdf;
       if (prev_shell >= 0) {
         d_partial += d_oc * ko * s;
-        scatter_hit(prev, prev_d, exact || prev_shell == l - 1 ? d_partial : 0.f, gcol, grad_sdf);
+        scatter_hit(prev, prev_d, exact || prev_shell == l - 1 ? d_partial : 0.f, rows);
       }
       prev = h;
 #pragma unroll
@@ -532,7 +529,7 @@ __global__ void __launch_bounds__(kShadeThreads)
       prev_shell = l;
     }
     if (prev_shell >= 0)
-      scatter_hit(prev, prev_d, exact || prev_shell == a.S - 1 ? d_partial : 0.f, gcol, grad_sdf);
+      scatter_hit(prev, prev_d, exact || prev_shell == a.S - 1 ? d_partial : 0.f, rows);
   }
   block_sum_to(d_sharp, grad_sharpness);
 }
@@ -652,18 +649,18 @@ int mt_shade_shells_backward(const float* uv, const int32_t* index, int32_t B, i
                              const int32_t* faces, const float* signed_distances, const float* colors, int64_t V,
                              const float* sharpness, const float* background, const float* out_colors,
                              const float* out_transmittances, const float* grad_out,
-                             const float* grad_out_transmittances, float* grad_signed_distances, float* grad_colors,
-                             float* grad_sharpness, int32_t exact_adjoint, mt_stream_t stream) {
+                             const float* grad_out_transmittances, float* packed_gradients, float* grad_sharpness,
+                             int32_t exact_adjoint, mt_stream_t stream) {
   MT_REQUIRE(B >= 0 && S >= 1 && H >= 0 && W >= 0 && V >= 0);
   const int64_t P = (int64_t)B * H * W;
   if (P == 0) return MT_OK;
   MT_REQUIRE(uv && index && faces && signed_distances && colors && sharpness && out_colors && out_transmittances);
-  MT_REQUIRE(grad_signed_distances && grad_colors && grad_sharpness);
+  MT_REQUIRE(packed_gradients && grad_sharpness && (reinterpret_cast<uintptr_t>(packed_gradients) & 15) == 0);
   MT_REQUIRE((reinterpret_cast<uintptr_t>(uv) & 7) == 0);
   const ShellArgs a{uv, index, faces, signed_distances, colors, V, (int64_t)H * W, B, S, sharpness, background};
   shade_shells_backward_kernel<<<grid_stride_blocks(P, kShadeThreads, 64), kShadeThreads, 0, as_stream(stream)>>>(
-      a, out_colors, out_transmittances, grad_out, grad_out_transmittances, grad_signed_distances, grad_colors,
-      grad_sharpness, exact_adjoint ? 1 : 0);
+      a, out_colors, out_transmittances, grad_out, grad_out_transmittances,
+      reinterpret_cast<float4*>(packed_gradients), grad_sharpness, exact_adjoint ? 1 : 0);
   MT_CHECK_LAUNCH();
   return MT_OK;
 }

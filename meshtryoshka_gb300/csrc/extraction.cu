@@ -988,6 +988,7 @@ constexpr int kShThreads = 128;
 constexpr int kShX = 64;
 constexpr int kShStride = 49;  // 48 values per entry; odd stride spreads rows over banks
 
+template <bool kPacked>
 __device__ __forceinline__ void entry_sh_gradient(int2 e, int64_t V, const float* __restrict__ verts, int n_coeff,
                                                   const float* __restrict__ campos, int B,
                                                   const float* __restrict__ colors,
@@ -1001,18 +1002,16 @@ __device__ __forceinline__ void entry_sh_gradient(int2 e, int64_t V, const float
   for (int k = 0; k < 16; ++k) d[k][0] = d[k][1] = d[k][2] = 0.f;
 #pragma unroll 2
   for (int b = 0; b < B; ++b) {
-    const int64_t ob = ((int64_t)b * V + vi) * 3;
-    float col[3], dcol[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      col[c] = __ldg(colors + ob + c);
-      dcol[c] = __ldg(dcolors + ob + c);
-    }
+    const int64_t o = (int64_t)b * V + vi;
     float g[3];
+    colour_gradient<kPacked>(dcolors, o, g);
+    // Most (camera, vertex) pairs of a large scene are unseen: their colours
+    // are not read.
+    if (g[0] == 0.0f && g[1] == 0.0f && g[2] == 0.0f) continue;
     bool any = false;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      g[c] = col[c] > 0.0f ? dcol[c] : 0.0f;
+      g[c] = __ldg(colors + 3 * o + c) > 0.0f ? g[c] : 0.0f;
       any |= g[c] != 0.0f;
     }
     if (!any) continue;
@@ -1035,6 +1034,7 @@ __device__ __forceinline__ void entry_sh_gradient(int2 e, int64_t V, const float
   }
 }
 
+template <bool kPacked>
 __global__ void __launch_bounds__(kShThreads)
     grid_sh_colors_backward_kernel(const int32_t* __restrict__ offsets, const int2* __restrict__ list, int64_t G,
                                    int64_t V, const float* __restrict__ verts, int C, int n_coeff,
@@ -1052,8 +1052,8 @@ __global__ void __launch_bounds__(kShThreads)
     for (int kk = 0; kk < 8; ++kk) acc[kk][0] = acc[kk][1] = acc[kk][2] = 0.f;
     for (int32_t base = e_begin; base < e_end; base += kShThreads) {
       if (base + tid < e_end)
-        entry_sh_gradient(__ldg(list + base + tid), V, verts, n_coeff, campos, B, colors, dcolors,
-                          s_grad + tid * kShStride);
+        entry_sh_gradient<kPacked>(__ldg(list + base + tid), V, verts, n_coeff, campos, B, colors, dcolors,
+                                   s_grad + tid * kShStride);
       __syncthreads();
       const int32_t lo = max(my_begin, base), hi = min(my_end, base + kShThreads);
       for (int32_t q = lo; q < hi; ++q) {
@@ -1088,6 +1088,7 @@ __global__ void __launch_bounds__(kShThreads)
 // kernel, with each vertex's gradient formed once instead of once per entry.
 constexpr int kShGradThreads = 128;
 
+template <bool kPacked>
 __global__ void __launch_bounds__(kShGradThreads)
     vertex_sh_grad_kernel(const float* __restrict__ verts, int64_t V, const int32_t* __restrict__ count,
                           int n_coeff, const float* __restrict__ campos, int B, const float* __restrict__ colors,
@@ -1112,12 +1113,13 @@ __global__ void __launch_bounds__(kShGradThreads)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const bool in = b0 + j < B;
-          const int64_t ob = ((int64_t)(b0 + j) * V + v) * 3;
+          const int64_t o = (int64_t)(b0 + j) * V + v;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            col[j][c] = in ? __ldg(colors + ob + c) : 0.0f;
-            dcol[j][c] = in ? __ldg(dcolors + ob + c) : 0.0f;
+            col[j][c] = in ? __ldg(colors + 3 * o + c) : 0.0f;
+            dcol[j][c] = 0.0f;
           }
+          if (in) colour_gradient<kPacked>(dcolors, o, dcol[j]);
         }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
@@ -1527,6 +1529,44 @@ __global__ void capacity_overflow_kernel(const int32_t* __restrict__ nv, int64_t
 
 using namespace mt;
 
+template <bool kPacked>
+static int grid_sh_backward(const int32_t* list_offsets, const int32_t* list, int64_t G, int64_t V,
+                               const float* vertices, int32_t C, int32_t sh_degree, const float* camera_positions,
+                               int32_t B, const float* out_colors, const float* grad_colors,
+                               float* grad_grid_spherical_harmonics, const int32_t* num_vertices, void* workspace,
+                               size_t workspace_bytes, mt_stream_t stream) {
+  MT_REQUIRE(G >= 0 && V >= 0 && B >= 0 && sh_degree >= 0 && sh_degree <= 3);
+  const int n = (sh_degree + 1) * (sh_degree + 1);
+  MT_REQUIRE(C >= n);
+  if (G == 0) return MT_OK;
+  MT_REQUIRE(list_offsets && grad_grid_spherical_harmonics);
+  // No cameras or vertices: every list sum is empty and the rows are zeros.
+  const int Bn = V > 0 ? B : 0;
+  MT_REQUIRE(Bn == 0 || (list && vertices && camera_positions && out_colors && grad_colors));
+  MT_REQUIRE(!kPacked || (reinterpret_cast<uintptr_t>(grad_colors) & 15) == 0);
+  cudaStream_t st = as_stream(stream);
+  if (C > 16 && cudaMemsetAsync(grad_grid_spherical_harmonics + (size_t)16 * G * 3, 0,
+                                (size_t)(C - 16) * G * 3 * sizeof(float), st) != cudaSuccess)
+    return MT_ERR_CUDA;  // rows past degree 3's sixteen are zeros
+  if (workspace && workspace_bytes >= mt_grid_sh_colors_backward_workspace_bytes(V) && Bn > 0) {
+    float4* dsh = reinterpret_cast<float4*>(static_cast<char*>(workspace) + 256);
+    MT_REQUIRE((reinterpret_cast<uintptr_t>(dsh) & 15) == 0);
+    vertex_sh_grad_kernel<kPacked><<<grid_stride_blocks(V, kShGradThreads), kShGradThreads, 0, st>>>(vertices, V, num_vertices, n, camera_positions,
+                                                                      Bn, out_colors, grad_colors, dsh);
+    MT_CHECK_LAUNCH();
+    grid_sh_gather_kernel<<<grid_stride_blocks(2 * G, 256), 256, 0, st>>>(
+        list_offsets, reinterpret_cast<const int2*>(list), G, dsh, C, n, grad_grid_spherical_harmonics);
+    MT_CHECK_LAUNCH();
+    return MT_OK;
+  }
+  const int64_t xblocks = (G + kShX - 1) / kShX;
+  grid_sh_colors_backward_kernel<kPacked><<<(unsigned)min(xblocks, (int64_t)152 * 32), kShThreads, 0, st>>>(
+      list_offsets, reinterpret_cast<const int2*>(list), G, V, vertices, C, n, camera_positions, Bn, out_colors,
+      grad_colors, grad_grid_spherical_harmonics);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
+}
+
 extern "C" {
 
 int mt_compute_vertex_occupancy(const int32_t* occupancy, int32_t I, int32_t J, int32_t KP, int32_t* vertex_occupancy,
@@ -1869,35 +1909,19 @@ int mt_grid_sh_colors_backward(const int32_t* list_offsets, const int32_t* list,
                                int32_t B, const float* out_colors, const float* grad_colors,
                                float* grad_grid_spherical_harmonics, const int32_t* num_vertices, void* workspace,
                                size_t workspace_bytes, mt_stream_t stream) {
-  MT_REQUIRE(G >= 0 && V >= 0 && B >= 0 && sh_degree >= 0 && sh_degree <= 3);
-  const int n = (sh_degree + 1) * (sh_degree + 1);
-  MT_REQUIRE(C >= n);
-  if (G == 0) return MT_OK;
-  MT_REQUIRE(list_offsets && grad_grid_spherical_harmonics);
-  // No cameras or vertices: every list sum is empty and the rows are zeros.
-  const int Bn = V > 0 ? B : 0;
-  MT_REQUIRE(Bn == 0 || (list && vertices && camera_positions && out_colors && grad_colors));
-  cudaStream_t st = as_stream(stream);
-  if (C > 16 && cudaMemsetAsync(grad_grid_spherical_harmonics + (size_t)16 * G * 3, 0,
-                                (size_t)(C - 16) * G * 3 * sizeof(float), st) != cudaSuccess)
-    return MT_ERR_CUDA;  // rows past degree 3's sixteen are zeros
-  if (workspace && workspace_bytes >= mt_grid_sh_colors_backward_workspace_bytes(V) && Bn > 0) {
-    float4* dsh = reinterpret_cast<float4*>(static_cast<char*>(workspace) + 256);
-    MT_REQUIRE((reinterpret_cast<uintptr_t>(dsh) & 15) == 0);
-    vertex_sh_grad_kernel<<<grid_stride_blocks(V, kShGradThreads), kShGradThreads, 0, st>>>(vertices, V, num_vertices, n, camera_positions,
-                                                                      Bn, out_colors, grad_colors, dsh);
-    MT_CHECK_LAUNCH();
-    grid_sh_gather_kernel<<<grid_stride_blocks(2 * G, 256), 256, 0, st>>>(
-        list_offsets, reinterpret_cast<const int2*>(list), G, dsh, C, n, grad_grid_spherical_harmonics);
-    MT_CHECK_LAUNCH();
-    return MT_OK;
-  }
-  const int64_t xblocks = (G + kShX - 1) / kShX;
-  grid_sh_colors_backward_kernel<<<(unsigned)min(xblocks, (int64_t)152 * 32), kShThreads, 0, st>>>(
-      list_offsets, reinterpret_cast<const int2*>(list), G, V, vertices, C, n, camera_positions, Bn, out_colors,
-      grad_colors, grad_grid_spherical_harmonics);
-  MT_CHECK_LAUNCH();
-  return MT_OK;
+  return grid_sh_backward<false>(list_offsets, list, G, V, vertices, C, sh_degree, camera_positions, B, out_colors,
+                                 grad_colors, grad_grid_spherical_harmonics, num_vertices, workspace,
+                                 workspace_bytes, stream);
+}
+
+int mt_grid_sh_colors_packed_backward(const int32_t* list_offsets, const int32_t* list, int64_t G, int64_t V,
+                                      const float* vertices, int32_t C, int32_t sh_degree, const float* camera_positions,
+                                      int32_t B, const float* out_colors, const float* packed_gradients,
+                                      float* grad_grid_spherical_harmonics, const int32_t* num_vertices, void* workspace,
+                                      size_t workspace_bytes, mt_stream_t stream) {
+  return grid_sh_backward<true>(list_offsets, list, G, V, vertices, C, sh_degree, camera_positions, B, out_colors,
+                                packed_gradients, grad_grid_spherical_harmonics, num_vertices, workspace,
+                                workspace_bytes, stream);
 }
 
 }  // extern "C"

@@ -97,6 +97,11 @@ __device__ __forceinline__ int dealt_word(int inclusive, int count, int r, int& 
   return word;
 }
 
+// One 16-byte reduction (each component is its own relaxed addition).
+__device__ __forceinline__ void red_add(float4* p, float x, float y, float z, float w) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+
 // Record the first device-side error code in a status word (0 = ok).
 __device__ __forceinline__ void set_device_error(int* status, int code) {
   if (status != nullptr) atomicCAS(status, 0, code);

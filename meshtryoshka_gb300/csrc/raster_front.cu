@@ -111,6 +111,7 @@ __global__ void sh_forward_kernel(const float* __restrict__ verts, int64_t V, co
 // d sh_k = sum_b basis_k(dir_b) * d rgb_b * [rgb_b + 0.5 > 0]; the mask is
 // read from the forward output (out > 0 exactly when the pre-clamp value is).
 // Every row of the output is written (rows k >= n_coeff get zeros).
+template <bool kPacked>
 __global__ void sh_backward_kernel(const float* __restrict__ verts, int64_t V, int n_coeff, int C,
                                    const float* __restrict__ campos, int B, const float* __restrict__ colors,
                                    const float* __restrict__ dcolors, float* __restrict__ dsh) {
@@ -118,12 +119,13 @@ __global__ void sh_backward_kernel(const float* __restrict__ verts, int64_t V, i
     float acc[16][3];
     for (int k = 0; k < 16; ++k) acc[k][0] = acc[k][1] = acc[k][2] = 0.f;
     for (int b = 0; b < B; ++b) {
-      const int64_t o = ((int64_t)b * V + v) * 3;
+      const int64_t o = (int64_t)b * V + v;
       float g[3];
+      colour_gradient<kPacked>(dcolors, o, g);
       bool any = false;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        g[c] = colors[o + c] > 0.0f ? dcolors[o + c] : 0.0f;
+        g[c] = colors[3 * o + c] > 0.0f ? g[c] : 0.0f;
         any |= g[c] != 0.0f;
       }
       if (!any) continue;
@@ -586,6 +588,28 @@ inline bool layout_ok(const KeyLayout& L) {
 
 using namespace mt;
 
+template <bool kPacked>
+static int sh_backward(const float* vertices, int64_t V, int32_t C, int32_t sh_degree,
+                                             const float* camera_positions, int32_t B, const float* out_colors,
+                                             const float* grad_colors, float* grad_spherical_harmonics,
+                                             mt_stream_t stream) {
+  MT_REQUIRE(V >= 0 && B >= 0 && sh_degree >= 0 && sh_degree <= 3);
+  const int n = (sh_degree + 1) * (sh_degree + 1);
+  MT_REQUIRE(C >= n);
+  if (V == 0) return MT_OK;
+  MT_REQUIRE(grad_spherical_harmonics);
+  if (B == 0) {
+    const size_t bytes = (size_t)C * (size_t)V * 3 * sizeof(float);
+    return cudaMemsetAsync(grad_spherical_harmonics, 0, bytes, as_stream(stream)) == cudaSuccess ? MT_OK : MT_ERR_CUDA;
+  }
+  MT_REQUIRE(vertices && camera_positions && out_colors && grad_colors);
+  MT_REQUIRE(!kPacked || (reinterpret_cast<uintptr_t>(grad_colors) & 15) == 0);
+  sh_backward_kernel<kPacked><<<grid_stride_blocks(V, 128), 128, 0, as_stream(stream)>>>(
+      vertices, V, n, C, camera_positions, B, out_colors, grad_colors, grad_spherical_harmonics);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
+}
+
 extern "C" {
 
 int mt_camera_positions(const float* extrinsics, int32_t B, float* out, mt_stream_t stream) {
@@ -626,20 +650,14 @@ int mt_evaluate_spherical_harmonics_backward(const float* vertices, int64_t V, i
                                              const float* camera_positions, int32_t B, const float* out_colors,
                                              const float* grad_colors, float* grad_spherical_harmonics,
                                              mt_stream_t stream) {
-  MT_REQUIRE(V >= 0 && B >= 0 && sh_degree >= 0 && sh_degree <= 3);
-  const int n = (sh_degree + 1) * (sh_degree + 1);
-  MT_REQUIRE(C >= n);
-  if (V == 0) return MT_OK;
-  MT_REQUIRE(grad_spherical_harmonics);
-  if (B == 0) {
-    const size_t bytes = (size_t)C * (size_t)V * 3 * sizeof(float);
-    return cudaMemsetAsync(grad_spherical_harmonics, 0, bytes, as_stream(stream)) == cudaSuccess ? MT_OK : MT_ERR_CUDA;
-  }
-  MT_REQUIRE(vertices && camera_positions && out_colors && grad_colors);
-  sh_backward_kernel<<<grid_stride_blocks(V, 128), 128, 0, as_stream(stream)>>>(
-      vertices, V, n, C, camera_positions, B, out_colors, grad_colors, grad_spherical_harmonics);
-  MT_CHECK_LAUNCH();
-  return MT_OK;
+  return sh_backward<false>(vertices, V, C, sh_degree, camera_positions, B, out_colors, grad_colors, grad_spherical_harmonics, stream);
+}
+
+int mt_evaluate_spherical_harmonics_packed_backward(const float* vertices, int64_t V, int32_t C, int32_t sh_degree,
+                                             const float* camera_positions, int32_t B, const float* out_colors,
+                                             const float* packed_gradients, float* grad_spherical_harmonics,
+                                             mt_stream_t stream) {
+  return sh_backward<true>(vertices, V, C, sh_degree, camera_positions, B, out_colors, packed_gradients, grad_spherical_harmonics, stream);
 }
 
 int mt_bound_triangles(const float* xy, const float* depth, int64_t V, const int32_t* faces, int64_t F,

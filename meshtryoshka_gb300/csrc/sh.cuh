@@ -58,6 +58,21 @@ __device__ __forceinline__ void view_dir(const float* __restrict__ verts, int64_
   view_dir_at(verts[3 * v], verts[3 * v + 1], verts[3 * v + 2], cam, x, y, z);
 }
 
+// The gradient of a (camera, vertex)'s colour: row o of [B, V, 3], or of packed
+// (r, g, b, signed distance) rows of [B, V, 4], whose 16 bytes come as one load.
+template <bool kPacked>
+__device__ __forceinline__ void colour_gradient(const float* __restrict__ rows, int64_t o, float (&g)[3]) {
+  if constexpr (kPacked) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(rows) + o);
+    g[0] = x.x;
+    g[1] = x.y;
+    g[2] = x.z;
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) g[c] = __ldg(rows + 3 * o + c);
+  }
+}
+
 // Colours of vertex v for every camera from its coefficients (in
 // registers): rgb_b = max(sum_k basis_k(dir_b) coef_k + 0.5, 0), terms added
 // in k order. out: [B, V, 3].

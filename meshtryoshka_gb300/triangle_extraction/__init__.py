@@ -530,9 +530,10 @@ class GridSHColors(torch.autograd.Function):
                 ws_ptr, ws_bytes = nt.workspace(device).get(need)
             else:
                 ws_ptr, ws_bytes = None, 0  # the one-pass form: no scratch
-            nt.call("mt_grid_sh_colors_backward", nt.ptr(d.list_offsets), nt.ptr(d.contributions), g, v,
-                    nt.ptr(vertices), c, ctx.sh_degree, nt.ptr(campos), campos.shape[0], nt.ptr(colors),
-                    nt.ptr(grad_colors.contiguous()), nt.ptr(grad_gsh), nt.ptr(d.num_vertices), ws_ptr, ws_bytes,
+            rows, packed = nt.colour_gradient_rows(grad_colors)
+            nt.call("mt_grid_sh_colors_packed_backward" if packed else "mt_grid_sh_colors_backward",
+                    nt.ptr(d.list_offsets), nt.ptr(d.contributions), g, v, nt.ptr(vertices), c, ctx.sh_degree,
+                    nt.ptr(campos), campos.shape[0], nt.ptr(colors), rows.data_ptr() or None, nt.ptr(grad_gsh), nt.ptr(d.num_vertices), ws_ptr, ws_bytes,
                     nt.stream(device))
             return grad_gsh, None, None, None, None
 

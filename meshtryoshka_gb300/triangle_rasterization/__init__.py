@@ -466,6 +466,27 @@ def _camera_positions(extrinsics: Tensor) -> Tensor:
     return out
 
 
+class _PackedGradients:
+    """The compositing adjoints' [B, V, 4] gradients (colour, and the camera's
+    part of the signed distance's), to be filled by a kernel."""
+
+    def __init__(self, b: int, v: int, device):
+        self.rows = torch.zeros((b, v, 4), dtype=torch.float32, device=device)
+
+    def split(self, in_place: bool) -> tuple[Tensor, Tensor]:
+        """(colour gradient [B, V, 3], signed-distance gradient [V]); the first
+        is a view of the rows with ``in_place``."""
+        b, v, _ = self.rows.shape
+        kw = dict(dtype=torch.float32, device=self.rows.device)
+        if b == 0 or v == 0:
+            return torch.zeros((b, v, 3), **kw), torch.zeros((v,), **kw)
+        sdf = torch.empty((v,), **kw)
+        colors = None if in_place else torch.empty((b, v, 3), **kw)
+        nt.call("mt_unpack_gradients", self.rows.data_ptr(), b, v, nt.ptr(colors), sdf.data_ptr(),
+                nt.stream(self.rows.device))
+        return self.rows[..., :3] if in_place else colors, sdf
+
+
 class EvaluateSphericalHarmonics(torch.autograd.Function):
     @staticmethod
     def forward(ctx, vertices, spherical_harmonics, extrinsics, sh_degree):
@@ -488,12 +509,13 @@ class EvaluateSphericalHarmonics(torch.autograd.Function):
     def backward(ctx, grad_colors):
         with annotate("evaluate_spherical_harmonics_backward"):
             vertices, campos, colors = ctx.saved_tensors
-            grad_colors = grad_colors.contiguous()
             device = vertices.device
             grad_sh = torch.empty(ctx.sh_shape, dtype=torch.float32, device=device)  # fully written
-            nt.call("mt_evaluate_spherical_harmonics_backward", nt.ptr(vertices), vertices.shape[0],
+            rows, packed = nt.colour_gradient_rows(grad_colors)
+            nt.call("mt_evaluate_spherical_harmonics_packed_backward" if packed
+                    else "mt_evaluate_spherical_harmonics_backward", nt.ptr(vertices), vertices.shape[0],
                     ctx.sh_shape[0], ctx.sh_degree, nt.ptr(campos), campos.shape[0], nt.ptr(colors),
-                    nt.ptr(grad_colors), nt.ptr(grad_sh), nt.stream(device))
+                    rows.data_ptr() or None, nt.ptr(grad_sh), nt.stream(device))
             return None, grad_sh, None, None
 
 
@@ -565,7 +587,10 @@ def _hit_bits(ctx, grid: TileGrid, num_keys: int, device) -> Tensor | None:
 class IntersectAndComposite(torch.autograd.Function):
     @staticmethod
     def forward(ctx, vertices, colors, signed_distances, faces, sharpness, sorted_keys, sorted_triangle_indices,
-                tile_boundaries, num_shells, grid, key_defines, gradient_mode=None, num_keys=None):
+                tile_boundaries, num_shells, grid, key_defines, gradient_mode=None, num_keys=None,
+                packed_colour_gradient=False):
+        # packed_colour_gradient: the colours come from the SH evaluation,
+        # whose adjoint reads packed gradient rows in place.
         with annotate("intersect_and_composite_forward"):
             xy, colors, sdf, faces = _f32(vertices), _f32(colors), _f32(signed_distances), _i32(faces)
             device = nt.require_cuda(xy, colors, sdf, faces)
@@ -595,34 +620,34 @@ class IntersectAndComposite(torch.autograd.Function):
             ctx.order = order
             ctx.save_for_backward(xy, colors, sdf, faces, sharp, keys, tri, bounds, masks, out)
             ctx.meta = (int(num_shells), grid, key_defines, gradient_mode or _GRADIENT_MODE,
-                        torch.is_tensor(sharpness))
+                        torch.is_tensor(sharpness), packed_colour_gradient)
             return out
 
     @staticmethod
     def backward(ctx, grad_out):
         with annotate("intersect_and_composite_backward"):
             xy, colors, sdf, faces, sharp, keys, tri, bounds, masks, out = ctx.saved_tensors
-            num_shells, grid, key_defines, mode, sharp_is_tensor = ctx.meta
+            num_shells, grid, key_defines, mode, sharp_is_tensor, packed_colour_gradient = ctx.meta
             device = xy.device
             grad_out = grad_out.contiguous()
-            grad_colors = torch.zeros_like(colors)
-            grad_sdf = torch.zeros_like(sdf)
             grad_sharp = torch.zeros_like(sharp)
             b, v, _ = xy.shape
+            packed = _PackedGradients(b, v, device)
             h, w = grid.image_shape
             rows, cols = grid.grid_shape
             counter = torch.empty((1,), dtype=torch.int64, device=device)
             staging = _staging(b, v, device)
-            nt.call("mt_intersect_and_composite_backward", nt.ptr(xy), nt.ptr(colors), nt.ptr(sdf), v,
+            nt.call("mt_intersect_and_composite_packed_backward", nt.ptr(xy), nt.ptr(colors), nt.ptr(sdf), v,
                     nt.ptr(faces), nt.ptr(sharp), nt.ptr(keys), nt.ptr(tri), keys.numel(), nt.ptr(bounds), b,
                     num_shells, rows, cols, grid.tile_shape[0], grid.tile_shape[1], h, w, _layout(key_defines),
                     nt.ptr(_camera_table(grid, device)), grid.camera_tiles, nt.ptr(masks), nt.ptr(counter),
-                    nt.ptr(out), nt.ptr(grad_out), None, None, 0.0, None, 1, nt.ptr(grad_colors), nt.ptr(grad_sdf),
-                    nt.ptr(grad_sharp), int(mode == "exact"), nt.ptr(ctx.hits), _numel(ctx.hits),
+                    nt.ptr(out), nt.ptr(grad_out), None, None, 0.0, None, 1, nt.ptr(packed.rows), nt.ptr(grad_sharp),
+                    int(mode == "exact"), nt.ptr(ctx.hits), _numel(ctx.hits),
                     nt.ptr(staging), _numel(staging), nt.ptr(ctx.order), _numel(ctx.order), grid.cta_threads,
                     nt.stream(device))
+            grad_colors, grad_sdf = packed.split(packed_colour_gradient)
             return (None, grad_colors, grad_sdf, None, grad_sharp if sharp_is_tensor else None, None, None, None,
-                    None, None, None, None, None)
+                    None, None, None, None, None, None)
 
 
 class IntersectCompositeLoss(torch.autograd.Function):
@@ -638,7 +663,7 @@ class IntersectCompositeLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, vertices, colors, signed_distances, faces, sharpness, sorted_keys, sorted_triangle_indices,
                 tile_boundaries, num_shells, grid, key_defines, target, background, gradient_mode=None,
-                num_keys=None, ssaa=1):
+                num_keys=None, ssaa=1, packed_colour_gradient=False):
         with annotate("intersect_composite_loss_forward"):
             xy, colors, sdf, faces = _f32(vertices), _f32(colors), _f32(signed_distances), _i32(faces)
             target, background = _f32(target), _f32(background)
@@ -682,34 +707,34 @@ class IntersectCompositeLoss(torch.autograd.Function):
             ctx.order = order
             ctx.save_for_backward(xy, colors, sdf, faces, sharp, keys, tri, bounds, masks, out, factor, background)
             ctx.meta = (int(num_shells), grid, key_defines, gradient_mode or _GRADIENT_MODE,
-                        torch.is_tensor(sharpness), scale, ssaa)
+                        torch.is_tensor(sharpness), scale, ssaa, packed_colour_gradient)
             return loss
 
     @staticmethod
     def backward(ctx, grad_loss):
         with annotate("intersect_composite_loss_backward"):
             xy, colors, sdf, faces, sharp, keys, tri, bounds, masks, out, target, background = ctx.saved_tensors
-            num_shells, grid, key_defines, mode, sharp_is_tensor, scale, ssaa = ctx.meta
+            num_shells, grid, key_defines, mode, sharp_is_tensor, scale, ssaa, packed_colour_gradient = ctx.meta
             device = xy.device
             grad_loss = grad_loss.to(torch.float32).contiguous()
-            grad_colors = torch.zeros_like(colors)
-            grad_sdf = torch.zeros_like(sdf)
             grad_sharp = torch.zeros_like(sharp)
             b, v, _ = xy.shape
+            packed = _PackedGradients(b, v, device)
             h, w = grid.image_shape
             rows, cols = grid.grid_shape
             counter = torch.empty((1,), dtype=torch.int64, device=device)
             staging = _staging(b, v, device)
-            nt.call("mt_intersect_and_composite_backward", nt.ptr(xy), nt.ptr(colors), nt.ptr(sdf), v,
+            nt.call("mt_intersect_and_composite_packed_backward", nt.ptr(xy), nt.ptr(colors), nt.ptr(sdf), v,
                     nt.ptr(faces), nt.ptr(sharp), nt.ptr(keys), nt.ptr(tri), keys.numel(), nt.ptr(bounds), b,
                     num_shells, rows, cols, grid.tile_shape[0], grid.tile_shape[1], h, w, _layout(key_defines),
                     nt.ptr(_camera_table(grid, device)), grid.camera_tiles, nt.ptr(masks), nt.ptr(counter),
                     nt.ptr(out), None, nt.ptr(target), nt.ptr(background), scale, grad_loss.data_ptr(), ssaa,
-                    nt.ptr(grad_colors), nt.ptr(grad_sdf), nt.ptr(grad_sharp), int(mode == "exact"),
+                    nt.ptr(packed.rows), nt.ptr(grad_sharp), int(mode == "exact"),
                     nt.ptr(ctx.hits), _numel(ctx.hits), nt.ptr(staging), _numel(staging), nt.ptr(ctx.order),
                     _numel(ctx.order), grid.cta_threads, nt.stream(device))
+            grad_colors, grad_sdf = packed.split(packed_colour_gradient)
             return (None, grad_colors, grad_sdf, None, grad_sharp if sharp_is_tensor else None, None, None, None,
-                    None, None, None, None, None, None, None, None)
+                    None, None, None, None, None, None, None, None, None)
 
 
 def intersect_and_composite(vertices, colors, signed_distances, faces, sharpness, sorted_keys,
@@ -890,7 +915,8 @@ class ShadeShells(torch.autograd.Function):
     colours + background * transmittance. Same values and gradients."""
 
     @staticmethod
-    def forward(ctx, uv, index, faces, signed_distances, colors, sharpness, background, gradient_mode):
+    def forward(ctx, uv, index, faces, signed_distances, colors, sharpness, background, gradient_mode,
+                packed_colour_gradient=False):
         with annotate("shade_shells_forward"):
             uv, index, faces = _f32(uv), _i32(index), _i32(faces)
             sdf, colors = _f32(signed_distances), _f32(colors)
@@ -907,7 +933,7 @@ class ShadeShells(torch.autograd.Function):
                     nt.ptr(colors), sdf.shape[0], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
                     nt.ptr(out_t), nt.ptr(image), nt.stream(device))
             ctx.save_for_backward(uv, index, faces, sdf, colors, sharp, background, out_colors, out_t)
-            ctx.meta = (gradient_mode or _GRADIENT_MODE, torch.is_tensor(sharpness))
+            ctx.meta = (gradient_mode or _GRADIENT_MODE, torch.is_tensor(sharpness), packed_colour_gradient)
             ctx.set_materialize_grads(False)
             return image if background is not None else (out_colors, out_t)
 
@@ -915,17 +941,19 @@ class ShadeShells(torch.autograd.Function):
     def backward(ctx, grad_out, grad_t=None):
         with annotate("shade_shells_backward"):
             uv, index, faces, sdf, colors, sharp, background, out_colors, out_t = ctx.saved_tensors
-            mode, sharp_is_tensor = ctx.meta
+            mode, sharp_is_tensor, packed_colour_gradient = ctx.meta
             device = sdf.device
             b, s, h, w = index.shape
-            gsdf, gcol, gsharp = torch.zeros_like(sdf), torch.zeros_like(colors), torch.zeros_like(sharp)
+            gsharp = torch.zeros_like(sharp)
+            packed = _PackedGradients(b, sdf.shape[0], device)
             go = grad_out.contiguous() if grad_out is not None else None
             gt = grad_t.contiguous() if grad_t is not None else None
             nt.call("mt_shade_shells_backward", nt.ptr(uv), nt.ptr(index), b, s, h, w, nt.ptr(faces), nt.ptr(sdf),
                     nt.ptr(colors), sdf.shape[0], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
-                    nt.ptr(out_t), nt.ptr(go), nt.ptr(gt), nt.ptr(gsdf), nt.ptr(gcol), nt.ptr(gsharp),
+                    nt.ptr(out_t), nt.ptr(go), nt.ptr(gt), nt.ptr(packed.rows), nt.ptr(gsharp),
                     int(mode == "exact"), nt.stream(device))
-            return None, None, None, gsdf, gcol, gsharp if sharp_is_tensor else None, None, None
+            gcol, gsdf = packed.split(packed_colour_gradient)
+            return None, None, None, gsdf, gcol, gsharp if sharp_is_tensor else None, None, None, None
 
 
 # ---------------------------------------------------------------------------
@@ -979,9 +1007,11 @@ def render_explicit(extrinsics, intrinsics, image_shape, vertices, faces, shell_
     colors = evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
     b, s, h, w = index.shape
     if _finishable(index, background):
-        image = ShadeShells.apply(uv, index, faces, signed_distances, colors, sharpness, background, gradient_mode)
+        image = ShadeShells.apply(uv, index, faces, signed_distances, colors, sharpness, background, gradient_mode,
+                                  True)
     else:
-        image, out_t = ShadeShells.apply(uv, index, faces, signed_distances, colors, sharpness, None, gradient_mode)
+        image, out_t = ShadeShells.apply(uv, index, faces, signed_distances, colors, sharpness, None, gradient_mode,
+                                         True)
         image = image + background * out_t[:, None]
     image = image.reshape(b, h, w, 3).permute(0, 3, 1, 2)
     if ssaa > 1:
@@ -1019,9 +1049,9 @@ def render_fused(extrinsics, intrinsics, image_shape, vertices, faces, shell_fac
     paired, tile_boundaries = _sort_and_delineate(paired, grid, key_defines, False)
     colors = evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
     t = tile_boundaries.shape[2]
-    images = intersect_and_composite(positions, colors, signed_distances, faces, sharpness, paired.keys,
-                                     paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
-                                     gradient_mode, paired.count)
+    images = IntersectAndComposite.apply(positions, colors, signed_distances, faces, sharpness, paired.keys,
+                                         paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid,
+                                         key_defines, gradient_mode, paired.count, True)
     if b > 0 and isinstance(ssaa, int) and _finishable(images, background):
         return FinishImages.apply(images, background, ((int(h), int(w)),) * b, max(ssaa, 1), True)
     images = images[:, :3] + images[:, 3:4] * background[:, None, None]
@@ -1070,9 +1100,9 @@ def render_cameras(extrinsics, intrinsics, image_shapes, vertices, faces, shell_
     paired, tile_boundaries = _sort_and_delineate(paired, grid, key_defines, False)
     colors = evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
     t = tile_boundaries.shape[2]
-    raw = intersect_and_composite(positions, colors, signed_distances, faces, sharpness, paired.keys,
-                                  paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
-                                  gradient_mode, paired.count)
+    raw = IntersectAndComposite.apply(positions, colors, signed_distances, faces, sharpness, paired.keys,
+                                      paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
+                                      gradient_mode, paired.count, True)
     if _finishable(raw, background):
         return list(FinishImages.apply(raw, background, grid.camera_shapes, 1, False))
     bg = background[:, None, None]
@@ -1122,7 +1152,7 @@ def render_fused_loss(extrinsics, intrinsics, image_shape, vertices, faces, shel
     t = tile_boundaries.shape[2]
     return IntersectCompositeLoss.apply(positions, colors, signed_distances, faces, sharpness, paired.keys,
                                         paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
-                                        target, background, gradient_mode, paired.count, ssaa)
+                                        target, background, gradient_mode, paired.count, ssaa, True)
 
 
 def render(extrinsics, intrinsics, image_shape, vertices, faces, shell_face_boundaries, signed_distances,

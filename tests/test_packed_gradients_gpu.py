@@ -1,0 +1,94 @@
+"""The compositing adjoint's packed gradients (colour and signed distance of a
+(camera, vertex) in 16 bytes) equal the separate ones, through every entry
+point's path: unpacked for callers of the stage, read in place by the SH
+adjoints. Within 1e-5 of the largest gradient: the order of atomic sums."""
+
+import numpy as np
+import pytest
+import torch
+
+from meshtryoshka_gb300 import _native as nt
+from meshtryoshka_gb300 import triangle_rasterization as tr
+from tests.scenes import make_scene
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(got, want):
+    assert float((got - want).abs().max()) <= 1e-5 * max(float(want.abs().max()), 1e-30)
+
+
+@pytest.mark.parametrize("b,v", [(1, 1), (1, 2), (3, 257), (5, 1000)])
+def test_unpacking_and_rows_in_place(cuda_device, b, v):
+    rows = torch.randn((b, v, 4), device=cuda_device)
+    packed = tr._PackedGradients(b, v, cuda_device)
+    packed.rows.copy_(rows)
+    colors, sdf = packed.split(False)
+    assert torch.equal(colors, rows[..., :3]) and colors.is_contiguous()
+    _close(sdf, rows[..., 3].sum(0))
+    view, _ = packed.split(True)
+    found, in_place = nt.colour_gradient_rows(view)
+    assert in_place == (v > 1) and torch.equal(found, rows[..., :3])
+    # Other strides of the same shape are copied.
+    for other in (rows[..., 1:], torch.randn((v, b, 4), device=cuda_device).transpose(0, 1)[..., :3],
+                  torch.randn((b, 2 * v, 4), device=cuda_device)[:, ::2, :3]):
+        found, in_place = nt.colour_gradient_rows(other)
+        assert torch.equal(found, other) and (not in_place or other.stride()[1:] == (4, 1))
+
+
+@pytest.mark.parametrize("mode", ["reference", "exact"])
+@pytest.mark.parametrize("tile", [(16, 16, 128), (8, 8, 256), (12, 20, 512)])
+def test_stage_and_render_gradients(cuda_device, mode, tile):
+    sc = make_scene(sh_degree=2, levels=(0.03, 0.0, -0.03))
+    d = cuda_device
+
+    def t(a):
+        return torch.from_numpy(np.ascontiguousarray(a)).to(d)
+
+    vertices, faces, sfb = t(sc.vertices), t(sc.faces), t(sc.face_boundaries)
+    ext, intr = t(sc.extrinsics), t(sc.intrinsics)
+    sdf, sh = t(sc.sdf).requires_grad_(True), t(sc.sh).requires_grad_(True)
+    b, s = ext.shape[0], sfb.shape[0]
+    grid = tr.TileGrid(tile, tuple(sc.image_shape), b, s)
+    kd = tr.create_key_defines(("camera", 6), ("tile", 20), ("depth", 32), ("shell", 6))
+    xy, depths = tr.project_vertices(vertices, ext, intr)
+    bounds = tr.bound_triangles(xy, depths, faces, grid, 0.2)
+    keys = tr.sort_keys(tr.generate_keys(depths, faces, sfb, bounds.tile_minima, bounds.tile_maxima,
+                                         bounds.num_tiles_overlapped, grid, kd))
+    ranges = tr.delineate_tiles(keys, grid, kd, False).view(b, -1, 2)
+    colors = tr.evaluate_spherical_harmonics(vertices, sh, ext, sc.sh_degree).detach().requires_grad_(True)
+    raw = tr.intersect_and_composite(xy, colors, sdf, faces, float(sc.sharpness), keys.keys, keys.triangle_indices,
+                                     ranges, s, grid, kd, mode)
+    g = torch.randn(raw.shape, device=d)
+    got_colors, got_sdf = torch.autograd.grad(raw, (colors, sdf), g)
+    assert got_colors.is_contiguous()
+    # The separate gradients of the same kernel.
+    want_colors, want_sdf = torch.zeros_like(colors), torch.zeros_like(sdf)
+    sharp, gsharp = torch.tensor(float(sc.sharpness), device=d), torch.zeros((), device=d)
+    masks = torch.empty_like(keys.triangle_indices)
+    counter = torch.empty(1, dtype=torch.int64, device=d)
+    out = torch.empty_like(raw)
+    h, w = grid.image_shape
+    rows, cols = grid.grid_shape
+    c, f = colors.detach(), sdf.detach()
+    head = (nt.ptr(xy), nt.ptr(c), nt.ptr(f), xy.shape[1], nt.ptr(faces), nt.ptr(sharp), nt.ptr(keys.keys),
+            nt.ptr(keys.triangle_indices), keys.num_keys)
+    shape = (nt.ptr(ranges), b, s, rows, cols, *grid.tile_shape, h, w, tr._layout(kd), None, grid.camera_tiles)
+    nt.call("mt_intersect_and_composite_forward", *head, None, *shape, nt.ptr(masks), nt.ptr(counter), nt.ptr(out), None,
+            None, 0.0, None, None, 0, None, 0, grid.cta_threads, nt.stream(d))
+    nt.call("mt_intersect_and_composite_backward", *head, *shape, nt.ptr(masks), nt.ptr(counter), nt.ptr(out),
+            nt.ptr(g), None, None, 0.0, None, 1, nt.ptr(want_colors), nt.ptr(want_sdf), nt.ptr(gsharp),
+            int(mode == "exact"), None, 0, None, 0, None, 0, grid.cta_threads, nt.stream(d))
+    _close(got_colors, want_colors)
+    _close(got_sdf, want_sdf)
+    # A render's SH gradient (rows read in place) against the stages' one.
+    background = torch.zeros(3, device=d)
+    image = tr.render_fused(ext, intr, sc.image_shape, vertices, faces, sfb, sdf, sh, sc.sh_degree,
+                            float(sc.sharpness), background, tile_shape=tile, gradient_mode=mode)
+    gi = torch.randn(image.shape, device=d)
+    got = torch.autograd.grad(image, (sdf, sh), gi)
+    chained = tr.intersect_and_composite(xy, tr.evaluate_spherical_harmonics(vertices, sh, ext, sc.sh_degree), sdf, faces,
+                                         float(sc.sharpness), keys.keys, keys.triangle_indices, ranges, s, grid, kd, mode)
+    want = torch.autograd.grad((chained[:, :3] + chained[:, 3:] * background[:, None, None]).clip(0, 1), (sdf, sh), gi)
+    for a, x in zip(got, want):
+        _close(a, x)
