@@ -1576,156 +1576,252 @@ __global__ void ssaa_loss_kernel(const float* __restrict__ raw, int B, int H, in
 // cameras of different sizes every camera's slice sent back a zero-filled
 // gradient of all cameras' pixels, added to the others'. Forward and backward
 // of 32 cameras of 200-1600 px per side took 23.3 ms so and take 10.2 ms with
-// this; a 1080 x 1920 view with 2 x 2 samples 1.34 ms and 1.11 ms.
+// this at first; a 1080 x 1920 view with 2 x 2 samples 1.34 ms and 1.11 ms.
 //
-// A CTA row (blockIdx.y) per camera, whose destination comes by value in the
-// launch's parameters: the images stay separate allocations, and a captured
-// graph holds everything that it reads. Four pixels to a thread where a plane
-// and its addresses allow 16-byte words.
+// A CTA takes kFinishChunk pixels of one camera (found among the running block
+// counts), so cameras of any sizes share the launch evenly; with a row of CTAs
+// per camera the largest ones finished late. Cameras' destinations come by
+// value in the launch's parameters: the images stay separate allocations, and
+// a captured graph holds everything that it reads. Without SSAA, four pixels to
+// a thread as 16-byte words where a plane and its addresses allow, else eight
+// apart by the CTA's width; with 2 x 2 samples, pairs of samples as 8-byte
+// words. 32 cameras of 200-1600 px: 446 and 846 us with a row of CTAs per
+// camera, now 121 and 185; 1080 x 1920 with 2 x 2 samples: 57 us, now 23.
 // ---------------------------------------------------------------------------
-constexpr int kFinishCameras = 64;  // cameras per launch (1.5 KB of the 4 KB of parameters)
+constexpr int kFinishCameras = 64;  // cameras per launch (1.8 KB of the 4 KB of parameters)
 constexpr int kFinishThreads = 256;
 
 struct FinishBatch {
   float* image[kFinishCameras];  // [3, h, w]; in the adjoint its gradient, or NULL for zeros
   int64_t raw[kFinishCameras];   // first element of the camera's [4, h f, w f]
   int h[kFinishCameras], w[kFinishCameras];
+  int first[kFinishCameras + 1];  // the camera's first CTA
+  int count;
 };
+
+// Output pixels per CTA. kF: the SSAA factor, 0 for any above 2.
+template <int kF>
+constexpr int finish_chunk() {
+  return (kF == 1 ? 8 : 2) * kFinishThreads;
+}
 
 // clip to [0, 1] that lets NaN through, as torch.clip does.
 __device__ __forceinline__ float clip01(float x) { return x < 0.0f ? 0.0f : (x > 1.0f ? 1.0f : x); }
 
 __device__ __forceinline__ float blend_one(float rgb, float T, float bg) { return __fadd_rn(rgb, __fmul_rn(T, bg)); }
 
-// The blended value of channel c at output pixel (y, x), averaged over its
-// sub-pixels. src: the camera's [4, h f, w f].
-__device__ __forceinline__ float blended_mean(const float* __restrict__ src, int64_t plane, int W, int f, int y,
-                                              int x, int c, float bg) {
-  float acc = 0.0f;
-  for (int dy = 0; dy < f; ++dy) {
-    const int64_t row = ((int64_t)y * f + dy) * W + (int64_t)x * f;
-    for (int dx = 0; dx < f; ++dx)
-      acc = __fadd_rn(acc, blend_one(__ldg(src + c * plane + row + dx), __ldg(src + 3 * plane + row + dx), bg));
+// The blended value of output pixel (y, x), averaged over its sub-pixels. src:
+// the camera's [4, h f, w f].
+template <int kF>
+__device__ __forceinline__ void blended_mean(const float* __restrict__ src, int64_t plane, int W, int f, int y, int x,
+                                             const float (&bg)[3], float (&mean)[3]) {
+  float acc[3] = {0.0f, 0.0f, 0.0f};
+  if constexpr (kF == 2) {
+    const float2* s2 = reinterpret_cast<const float2*>(src + (int64_t)(2 * y) * W + 2 * x);
+    const int64_t plane2 = plane >> 1, row2 = W >> 1;
+    float2 t[2], v[3][2];
+#pragma unroll
+    for (int dy = 0; dy < 2; ++dy) {
+      t[dy] = __ldg(s2 + 3 * plane2 + dy * row2);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[c][dy] = __ldg(s2 + c * plane2 + dy * row2);
+    }
+#pragma unroll
+    for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        acc[c] = __fadd_rn(__fadd_rn(acc[c], blend_one(v[c][dy].x, t[dy].x, bg[c])), blend_one(v[c][dy].y, t[dy].y, bg[c]));
+  } else {
+    for (int dy = 0; dy < f; ++dy) {
+      const int64_t row = ((int64_t)y * f + dy) * W + (int64_t)x * f;
+      for (int dx = 0; dx < f; ++dx) {
+        const float t = __ldg(src + 3 * plane + row + dx);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] = __fadd_rn(acc[c], blend_one(__ldg(src + c * plane + row + dx), t, bg[c]));
+      }
+    }
   }
-  return __fmul_rn(acc, 1.0f / (float)(f * f));
+#pragma unroll
+  for (int c = 0; c < 3; ++c) mean[c] = __fmul_rn(acc[c], 1.0f / (float)(f * f));
 }
 
 __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// The camera of a CTA: the last one whose first CTA is at or before it (cameras
+// without pixels have none).
+__device__ __forceinline__ int finish_camera(const FinishBatch& batch, int block) {
+  int lo = 0, hi = batch.count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (batch.first[mid] <= block) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+template <int kF>
 __global__ void __launch_bounds__(kFinishThreads)
     finish_images_kernel(const float* __restrict__ raw, const __grid_constant__ FinishBatch batch, int f,
                          const float* __restrict__ background) {
-  const int cam = blockIdx.y;
-  const int h = batch.h[cam], w = batch.w[cam];
-  const int64_t n = (int64_t)h * w;
+  const int cam = finish_camera(batch, blockIdx.x);
+  const int w = batch.w[cam];
+  const int64_t n = (int64_t)batch.h[cam] * w;
   const float* src = raw + batch.raw[cam];
   float* dst = batch.image[cam];
   const float bg[3] = {__ldg(background), __ldg(background + 1), __ldg(background + 2)};
-  const int64_t first = blockIdx.x * (int64_t)kFinishThreads + threadIdx.x, step = (int64_t)gridDim.x * kFinishThreads;
-  if (f == 1 && (n & 3) == 0 && aligned16(src) && aligned16(dst)) {
-    const float4* s4 = reinterpret_cast<const float4*>(src);
-    float4* d4 = reinterpret_cast<float4*>(dst);
-    const int64_t n4 = n >> 2;
-    for (int64_t i = first; i < n4; i += step) {
-      const float4 t = __ldg(s4 + 3 * n4 + i);
-      float4 x[3];
+  const int64_t begin = (int64_t)(blockIdx.x - batch.first[cam]) * finish_chunk<kF>();
+  const int64_t end = min(begin + finish_chunk<kF>(), n);
+  if constexpr (kF == 1) {
+    if ((n & 3) == 0 && aligned16(src) && aligned16(dst)) {
+      const float4* s4 = reinterpret_cast<const float4*>(src);
+      float4* d4 = reinterpret_cast<float4*>(dst);
+      const int64_t n4 = n >> 2;
+#pragma unroll 2
+      for (int64_t i = (begin >> 2) + threadIdx.x; i < (end >> 2); i += kFinishThreads) {
+        const float4 t = __ldg(s4 + 3 * n4 + i);
+        float4 x[3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = __ldg(s4 + c * n4 + i);
+        for (int c = 0; c < 3; ++c) x[c] = __ldg(s4 + c * n4 + i);
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
-        d4[c * n4 + i] = make_float4(clip01(blend_one(x[c].x, t.x, bg[c])), clip01(blend_one(x[c].y, t.y, bg[c])),
-                                     clip01(blend_one(x[c].z, t.z, bg[c])), clip01(blend_one(x[c].w, t.w, bg[c])));
+        for (int c = 0; c < 3; ++c)
+          d4[c * n4 + i] = make_float4(clip01(blend_one(x[c].x, t.x, bg[c])), clip01(blend_one(x[c].y, t.y, bg[c])),
+                                       clip01(blend_one(x[c].z, t.z, bg[c])), clip01(blend_one(x[c].w, t.w, bg[c])));
+      }
+      return;
     }
-    return;
-  }
-  const int W = w * f;
-  const int64_t plane = n * f * f;
-  for (int64_t i = first; i < n; i += step) {
-    const int y = (int)(i / w), x = (int)(i - (int64_t)y * w);
+#pragma unroll 4
+    for (int64_t i = begin + threadIdx.x; i < end; i += kFinishThreads) {
+      const float t = __ldg(src + 3 * n + i);
+      float x[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-      dst[c * n + i] = clip01(f == 1 ? blend_one(__ldg(src + c * n + i), __ldg(src + 3 * n + i), bg[c])
-                                     : blended_mean(src, plane, W, f, y, x, c, bg[c]));
+      for (int c = 0; c < 3; ++c) x[c] = __ldg(src + c * n + i);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) dst[c * n + i] = clip01(blend_one(x[c], t, bg[c]));
+    }
+  } else {
+    for (int64_t i = begin + threadIdx.x; i < end; i += kFinishThreads) {
+      const int y = (int)(i / w), x = (int)(i - (int64_t)y * w);
+      float mean[3];
+      blended_mean<kF>(src, n * f * f, w * f, f, y, x, bg, mean);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) dst[c * n + i] = clip01(mean[c]);
+    }
   }
 }
 
 // d / d (rgb, T): the clip passes the gradient where the value lies inside
 // [0, 1] (ends included), each sub-pixel gets 1 / f^2 of it.
+template <int kF>
 __global__ void __launch_bounds__(kFinishThreads)
     finish_images_backward_kernel(const float* __restrict__ raw, const __grid_constant__ FinishBatch batch, int f,
                                   const float* __restrict__ background, float* __restrict__ grad_raw) {
-  const int cam = blockIdx.y;
-  const int h = batch.h[cam], w = batch.w[cam];
-  const int64_t n = (int64_t)h * w;
+  const int cam = finish_camera(batch, blockIdx.x);
+  const int w = batch.w[cam];
+  const int64_t n = (int64_t)batch.h[cam] * w;
   const float* src = raw + batch.raw[cam];
   float* dst = grad_raw + batch.raw[cam];
   const float* grad = batch.image[cam];
   const float bg[3] = {__ldg(background), __ldg(background + 1), __ldg(background + 2)};
-  const int64_t first = blockIdx.x * (int64_t)kFinishThreads + threadIdx.x, step = (int64_t)gridDim.x * kFinishThreads;
+  const int64_t begin = (int64_t)(blockIdx.x - batch.first[cam]) * finish_chunk<kF>();
+  const int64_t end = min(begin + finish_chunk<kF>(), n);
   auto passed = [](float value, float g) { return value >= 0.0f && value <= 1.0f ? g : 0.0f; };
-  if (f == 1 && (n & 3) == 0 && aligned16(src) && aligned16(dst) && aligned16(grad)) {
-    const float4* s4 = reinterpret_cast<const float4*>(src);
-    const float4* g4 = reinterpret_cast<const float4*>(grad);
-    float4* d4 = reinterpret_cast<float4*>(dst);
-    const int64_t n4 = n >> 2;
-    for (int64_t i = first; i < n4; i += step) {
-      float4 d_t = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (kF == 1) {
+    if ((n & 3) == 0 && aligned16(src) && aligned16(dst) && aligned16(grad)) {
+      const float4* s4 = reinterpret_cast<const float4*>(src);
+      const float4* g4 = reinterpret_cast<const float4*>(grad);
+      float4* d4 = reinterpret_cast<float4*>(dst);
+      const int64_t n4 = n >> 2;
+      for (int64_t i = (begin >> 2) + threadIdx.x; i < (end >> 2); i += kFinishThreads) {
+        float4 d_t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (grad) {
+          const float4 t = __ldg(s4 + 3 * n4 + i);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const float4 x = __ldg(s4 + c * n4 + i), g = __ldg(g4 + c * n4 + i);
+            const float4 d =
+                make_float4(passed(blend_one(x.x, t.x, bg[c]), g.x), passed(blend_one(x.y, t.y, bg[c]), g.y),
+                            passed(blend_one(x.z, t.z, bg[c]), g.z), passed(blend_one(x.w, t.w, bg[c]), g.w));
+            d4[c * n4 + i] = d;
+            d_t.x = __fadd_rn(d_t.x, __fmul_rn(d.x, bg[c]));
+            d_t.y = __fadd_rn(d_t.y, __fmul_rn(d.y, bg[c]));
+            d_t.z = __fadd_rn(d_t.z, __fmul_rn(d.z, bg[c]));
+            d_t.w = __fadd_rn(d_t.w, __fmul_rn(d.w, bg[c]));
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) d4[c * n4 + i] = d_t;
+        }
+        d4[3 * n4 + i] = d_t;
+      }
+      return;
+    }
+#pragma unroll 4
+    for (int64_t i = begin + threadIdx.x; i < end; i += kFinishThreads) {
+      float d[3] = {0.f, 0.f, 0.f}, d_t = 0.f;
       if (grad) {
-        const float4 t = __ldg(s4 + 3 * n4 + i);
+        const float t = __ldg(src + 3 * n + i);
+        float x[3], g[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const float4 x = __ldg(s4 + c * n4 + i), g = __ldg(g4 + c * n4 + i);
-          const float4 d = make_float4(passed(blend_one(x.x, t.x, bg[c]), g.x), passed(blend_one(x.y, t.y, bg[c]), g.y),
-                                       passed(blend_one(x.z, t.z, bg[c]), g.z), passed(blend_one(x.w, t.w, bg[c]), g.w));
-          d4[c * n4 + i] = d;
-          d_t.x = __fadd_rn(d_t.x, __fmul_rn(d.x, bg[c]));
-          d_t.y = __fadd_rn(d_t.y, __fmul_rn(d.y, bg[c]));
-          d_t.z = __fadd_rn(d_t.z, __fmul_rn(d.z, bg[c]));
-          d_t.w = __fadd_rn(d_t.w, __fmul_rn(d.w, bg[c]));
+          x[c] = __ldg(src + c * n + i);
+          g[c] = __ldg(grad + c * n + i);
         }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          d[c] = passed(blend_one(x[c], t, bg[c]), g[c]);
+          d_t = __fadd_rn(d_t, __fmul_rn(d[c], bg[c]));
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) dst[c * n + i] = d[c];
+      dst[3 * n + i] = d_t;
+    }
+  } else {
+    const int W = w * f;
+    const int64_t plane = n * f * f;
+    const float share = (float)(f * f);
+    for (int64_t i = begin + threadIdx.x; i < end; i += kFinishThreads) {
+      const int y = (int)(i / w), x = (int)(i - (int64_t)y * w);
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      if (grad) {
+        float mean[3];
+        blended_mean<kF>(src, plane, W, f, y, x, bg, mean);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          d[c] = __fdiv_rn(passed(mean[c], __ldg(grad + c * n + i)), share);
+          d[3] = __fadd_rn(d[3], __fmul_rn(d[c], bg[c]));
+        }
+      }
+      if constexpr (kF == 2) {
+#pragma unroll
+        for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<float2*>(dst + c * plane + (int64_t)(2 * y + dy) * W + 2 * x) = make_float2(d[c], d[c]);
       } else {
+        for (int dy = 0; dy < f; ++dy) {
+          const int64_t row = ((int64_t)y * f + dy) * W + (int64_t)x * f;
+          for (int dx = 0; dx < f; ++dx)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) d4[c * n4 + i] = d_t;
-      }
-      d4[3 * n4 + i] = d_t;
-    }
-    return;
-  }
-  const int W = w * f;
-  const int64_t plane = n * f * f;
-  const float share = (float)(f * f);
-  for (int64_t i = first; i < n; i += step) {
-    const int y = (int)(i / w), x = (int)(i - (int64_t)y * w);
-    float d[3] = {0.f, 0.f, 0.f}, d_t = 0.f;
-    if (grad) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float value = f == 1 ? blend_one(__ldg(src + c * n + i), __ldg(src + 3 * n + i), bg[c])
-                                   : blended_mean(src, plane, W, f, y, x, c, bg[c]);
-        d[c] = __fdiv_rn(passed(value, __ldg(grad + c * n + i)), share);
-        d_t = __fadd_rn(d_t, __fmul_rn(d[c], bg[c]));
-      }
-    }
-    for (int dy = 0; dy < f; ++dy) {
-      const int64_t row = ((int64_t)y * f + dy) * W + (int64_t)x * f;
-      for (int dx = 0; dx < f; ++dx) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) dst[c * plane + row + dx] = d[c];
-        dst[3 * plane + row + dx] = d_t;
+            for (int c = 0; c < 4; ++c) dst[c * plane + row + dx] = d[c];
+        }
       }
     }
   }
 }
 
-// Calls launch(batch, grid) for every kFinishCameras cameras; `images` and
-// `shapes` (h, w per camera, of the output images) are host arrays.
+// Calls launch(kF, batch, CTAs) for every kFinishCameras cameras; `images` and
+// `shapes` (h, w per camera, of the output images) are host arrays. `even`: the
+// compositing output (and its gradient) lies at an 8-byte boundary, which the
+// 2 x 2 form's pairs of samples need (their other offsets are even).
 template <typename F>
-int for_finish_batches(int32_t B, float* const* images, const int32_t* shapes, int32_t f, F&& launch) {
+int for_finish_batches(int32_t B, float* const* images, const int32_t* shapes, int32_t f, bool even, F&& launch) {
+  const int kind = f == 1 ? 1 : f == 2 && even ? 2 : 0;
+  const int64_t chunk = kind == 1 ? finish_chunk<1>() : finish_chunk<0>();
   int64_t raw = 0;
   for (int32_t b0 = 0; b0 < B; b0 += kFinishCameras) {
     const int count = (int)(B - b0 < kFinishCameras ? B - b0 : kFinishCameras);
     FinishBatch batch{};
-    int64_t most = 0;
+    int64_t blocks = 0;
     for (int k = 0; k < count; ++k) {
       const int64_t h = shapes[2 * (b0 + k)], w = shapes[2 * (b0 + k) + 1];
       MT_REQUIRE(h >= 0 && w >= 0 && h * f < ((int64_t)1 << 31) && w * f < ((int64_t)1 << 31));
@@ -1733,14 +1829,17 @@ int for_finish_batches(int32_t B, float* const* images, const int32_t* shapes, i
       batch.raw[k] = raw;
       batch.h[k] = (int)h;
       batch.w[k] = (int)w;
+      batch.first[k] = (int)blocks;
       raw += 4 * h * f * w * f;
-      if (h * w > most) most = h * w;
+      blocks += (h * w + chunk - 1) / chunk;
+      MT_REQUIRE(blocks < ((int64_t)1 << 31));
     }
-    if (most == 0) continue;
-    // Four pixels to a thread, and at most 8 CTAs per SM over the cameras.
-    const int64_t need = (most + 4 * kFinishThreads - 1) / (4 * kFinishThreads);
-    const int64_t cap = ((int64_t)kSmCount * 8 + count - 1) / count;
-    launch(batch, dim3((unsigned)(need < cap ? need : cap), (unsigned)count));
+    if (blocks == 0) continue;
+    batch.first[count] = (int)blocks;
+    batch.count = count;
+    if (kind == 1) launch(std::integral_constant<int, 1>{}, batch, (unsigned)blocks);
+    else if (kind == 2) launch(std::integral_constant<int, 2>{}, batch, (unsigned)blocks);
+    else launch(std::integral_constant<int, 0>{}, batch, (unsigned)blocks);
     MT_CHECK_LAUNCH();
   }
   return MT_OK;
@@ -2069,8 +2168,10 @@ int mt_finish_images(const float* raw, int32_t B, const int32_t* shapes, int32_t
   MT_REQUIRE(B >= 0 && ssaa >= 1);
   if (B == 0) return MT_OK;
   MT_REQUIRE(raw && shapes && background && images);
-  return for_finish_batches(B, images, shapes, ssaa, [&](const FinishBatch& batch, dim3 grid) {
-    finish_images_kernel<<<grid, kFinishThreads, 0, as_stream(stream)>>>(raw, batch, ssaa, background);
+  const bool even = (reinterpret_cast<uintptr_t>(raw) & 7) == 0;
+  return for_finish_batches(B, images, shapes, ssaa, even, [&](auto kind, const FinishBatch& batch, unsigned ctas) {
+    finish_images_kernel<decltype(kind)::value><<<ctas, kFinishThreads, 0, as_stream(stream)>>>(raw, batch, ssaa,
+                                                                                            background);
   });
 }
 
@@ -2080,11 +2181,12 @@ int mt_finish_images_backward(const float* raw, int32_t B, const int32_t* shapes
   MT_REQUIRE(B >= 0 && ssaa >= 1);
   if (B == 0) return MT_OK;
   MT_REQUIRE(raw && shapes && background && grad_images && grad_raw);
-  return for_finish_batches(B, const_cast<float* const*>(grad_images), shapes, ssaa,
-                            [&](const FinishBatch& batch, dim3 grid) {
-                              finish_images_backward_kernel<<<grid, kFinishThreads, 0, as_stream(stream)>>>(
-                                  raw, batch, ssaa, background, grad_raw);
-                            });
+  const bool even = ((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(grad_raw)) & 7) == 0;
+  float* const* grads = const_cast<float* const*>(grad_images);
+  return for_finish_batches(B, grads, shapes, ssaa, even, [&](auto kind, const FinishBatch& batch, unsigned ctas) {
+    finish_images_backward_kernel<decltype(kind)::value><<<ctas, kFinishThreads, 0, as_stream(stream)>>>(
+        raw, batch, ssaa, background, grad_raw);
+  });
 }
 
 int mt_ssaa_loss(const float* raw, int32_t B, int32_t H, int32_t W, int32_t ssaa, const float* background,

@@ -33,8 +33,9 @@ def _operations(raw, background, shapes, ssaa, clip=True):
 
 
 @pytest.mark.parametrize("ssaa", [1, 2, 3])
-@pytest.mark.parametrize("shapes", [[(1, 1)], [(4, 6), (5, 7), (33, 1)], [(20, 24)] * 3, [(3, 5)] * 66],
-                         ids=["one", "uneven", "alike", "two-launches"])
+@pytest.mark.parametrize("shapes", [[(1, 1)], [(4, 6), (5, 7), (33, 1)], [(20, 24)] * 3, [(3, 5)] * 66,
+                                    [(70, 61), (1, 1), (64, 64), (129, 100), (16, 128)]],
+                         ids=["one", "uneven", "alike", "two-launches", "several-blocks"])
 def test_matches_tensor_operations(cuda_device, shapes, ssaa):
     background = torch.tensor(BACKGROUND, device=cuda_device)
     raw = _raw(shapes, ssaa, cuda_device).requires_grad_(True)
