@@ -13,10 +13,11 @@
 //   4. sort each bin's composites: the original index breaks ties, so the
 //      order is the stable sort's. Bins of up to 256 keys are sorted by one
 //      warp, up to 512 by 64-thread CTAs, up to 1024 by 128-thread CTAs,
-//      larger ones by 512-thread CTAs
-//      (4096 keys in shared memory; beyond that, sorted 4096-key chunks
-//      merged pairwise in global memory). In shared memory each thread sorts
-//      8 values in registers, then sorted runs are merged (merge path);
+//      larger ones by 512-thread CTAs, 4096 keys in shared memory each; the
+//      chunks of a bin with more are sorted by a CTA each and then placed by
+//      one each: a key's position is the sum of its positions in every chunk.
+//      In shared memory each thread sorts 8 values in registers, then sorted
+//      runs are merged (merge path);
 //   5. write each sorted key and triangle, gathered by original index.
 //
 // Valid only when the bin order equals the signed key order (the camera
@@ -65,6 +66,7 @@ constexpr int kMediumCap = 512;     // keys per bin sorted by a 64-thread CTA
 constexpr int kSmallThreads = 128;
 constexpr int kSmallCap = 1024;     // keys per bin sorted by a 128-thread CTA
 constexpr int kTiers = 4;           // tiny, medium, small, large
+constexpr int kSizes = kTiers + 1;  // listed bins per tier, and listed chunks
 constexpr int kLargeThreads = 512;
 constexpr int kChunk = 4096;        // keys per shared-memory sort of a 512-thread CTA
 
@@ -90,13 +92,20 @@ __global__ void bin_count_kernel(const uint64_t* __restrict__ keys, int64_t Kcap
 // bins (delineate_tiles zero-fills its output). Non-empty bins are listed
 // for the sorting kernels, small and large ones apart.
 __global__ void bin_bounds_kernel(const int32_t* __restrict__ offsets, int64_t nbins, int64_t* __restrict__ bounds,
-                                  int2* __restrict__ lists, int32_t* __restrict__ list_sizes) {
+                                  int2* __restrict__ lists, int4* __restrict__ chunks,
+                                  int32_t* __restrict__ list_sizes) {
   for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nbins; b += (int64_t)gridDim.x * blockDim.x) {
     const int32_t s = offsets[b], e = offsets[b + 1];
     bounds[2 * b] = e > s ? s : 0;
     bounds[2 * b + 1] = e > s ? e : 0;
     if (e > s) {
       const int n = e - s;
+      if (n > kChunk) {  // at least 4097 keys: at most 2 K / 4096 chunks over all bins
+        const int many = (n + kChunk - 1) / kChunk;
+        const int first = atomicAdd(list_sizes + kTiers, many);
+        for (int c = 0; c < many; ++c) chunks[first + c] = make_int4(s, n, c, 0);
+        continue;
+      }
       const int which = n <= kTinyCap ? 0 : n <= kMediumCap ? 1 : n <= kSmallCap ? 2 : 3;
       lists[which * nbins + atomicAdd(list_sizes + which, 1)] = make_int2(s, n);
     }
@@ -232,7 +241,7 @@ __device__ __forceinline__ const uint64_t* block_merge_sort(const uint64_t* __re
 
 // 5. Sorted composites -> keys and triangles (gathered by original index),
 // four per thread in flight.
-template <int kCtaThreads, bool kSwizzled>
+template <int kCtaThreads>
 __device__ __forceinline__ void write_sorted(const uint64_t* sorted, int64_t n, int64_t start, uint64_t idx_mask,
                                              const uint64_t* __restrict__ keys_in,
                                              const int32_t* __restrict__ tri_in, uint64_t* __restrict__ keys_out,
@@ -243,7 +252,7 @@ __device__ __forceinline__ void write_sorted(const uint64_t* sorted, int64_t n, 
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
       const int64_t p = p0 + u * kCtaThreads;
-      idx[u] = p < n ? (int64_t)(sorted[kSwizzled ? swz((int)p) : p] & idx_mask) : -1;
+      idx[u] = p < n ? (int64_t)(sorted[swz((int)p)] & idx_mask) : -1;
     }
     uint64_t k[kUnroll];
     int32_t t[kUnroll];
@@ -278,7 +287,7 @@ __global__ void __launch_bounds__(32 * kTinyWarps)
   for (int l = blockIdx.x * kTinyWarps + warp; l < count; l += gridDim.x * kTinyWarps) {
     const int2 e = list[l];
     const uint64_t* sorted = block_merge_sort<32, true>(tmp + e.x, e.y, s[warp][0], s[warp][1], lane);
-    write_sorted<32, true>(sorted, e.y, e.x, idx_mask, keys_in, tri_in, keys_out, tri_out, lane);
+    write_sorted<32>(sorted, e.y, e.x, idx_mask, keys_in, tri_in, keys_out, tri_out, lane);
     __syncwarp();
   }
 }
@@ -298,78 +307,103 @@ __global__ void __launch_bounds__(kCtaThreads)
   for (int l = blockIdx.x; l < count; l += gridDim.x) {
     const int2 e = list[l];
     const uint64_t* sorted = block_merge_sort<kCtaThreads>(tmp + e.x, e.y, s, s2, threadIdx.x);
-    write_sorted<kCtaThreads, true>(sorted, e.y, e.x, idx_mask, keys_in, tri_in, keys_out, tri_out, threadIdx.x);
+    write_sorted<kCtaThreads>(sorted, e.y, e.x, idx_mask, keys_in, tri_in, keys_out, tri_out, threadIdx.x);
     __syncthreads();
   }
 }
 
-// Merges the sorted runs a = src[0, na) and b = src[na, na + nb) into
-// dst[0, na + nb); composites are distinct, so the order is unambiguous.
-// Each thread finds where its output range starts on the merge path, then
-// merges sequentially.
-__device__ __forceinline__ void merge_runs(const uint64_t* __restrict__ src, int64_t na, int64_t nb,
-                                           uint64_t* __restrict__ dst) {
-  const uint64_t* A = src;
-  const uint64_t* Bv = src + na;
-  const int64_t m = na + nb;
-  const int64_t per = (m + kLargeThreads - 1) / kLargeThreads;
-  const int64_t d0 = (int64_t)threadIdx.x * per;
-  if (d0 >= m) return;
-  const int64_t d1 = min(d0 + per, m);
-  // i = number of A elements among the first d0 outputs.
-  int64_t lo = max((int64_t)0, d0 - nb), hi = min(d0, na);
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if (A[mid] < Bv[d0 - mid - 1]) lo = mid + 1;
-    else hi = mid;
-  }
-  int64_t i = lo, j = d0 - lo;
-  for (int64_t d = d0; d < d1; ++d) {
-    if (j >= nb || (i < na && A[i] < Bv[j])) dst[d] = A[i++];
-    else dst[d] = Bv[j++];
-  }
-}
-
-// 4 + 5 for the listed bins of more than kSmallCap keys.
+// 4 + 5 for the listed bins of more than kSmallCap and at most kChunk keys, and
+// 4 for the listed chunks of larger bins (sorted in place).
 __global__ void __launch_bounds__(kLargeThreads)
-    bin_sort_large_kernel(uint64_t* __restrict__ tmp, uint64_t* __restrict__ alt, const int2* __restrict__ list,
+    bin_sort_large_kernel(uint64_t* __restrict__ tmp, const int2* __restrict__ list, const int4* __restrict__ chunks,
                           const int32_t* __restrict__ list_size, uint64_t idx_mask,
                           const uint64_t* __restrict__ keys_in, const int32_t* __restrict__ tri_in,
                           uint64_t* __restrict__ keys_out, int32_t* __restrict__ tri_out) {
   extern __shared__ uint64_t smem[];  // two buffers of kChunk entries
   uint64_t* s = smem;
   uint64_t* s2 = smem + kChunk;
-  const int count = *list_size;
+  const int count = list_size[0], chunk_count = list_size[1];
+  for (int l = blockIdx.x; l < chunk_count + count; l += gridDim.x) {  // chunks first: their bins take longest
+    if (l < chunk_count) {
+      const int4 e = chunks[l];
+      uint64_t* src = tmp + e.x + (int64_t)e.z * kChunk;
+      const int n = min(kChunk, e.y - e.z * kChunk);
+      const uint64_t* sorted = block_merge_sort<kLargeThreads>(src, n, s, s2, threadIdx.x);
+      for (int i = threadIdx.x; i < n; i += kLargeThreads) src[i] = sorted[swz(i)];
+    } else {
+      const int2 e = list[l - chunk_count];
+      const uint64_t* sorted = block_merge_sort<kLargeThreads>(tmp + e.x, e.y, s, s2, threadIdx.x);
+      write_sorted<kLargeThreads>(sorted, e.y, e.x, idx_mask, keys_in, tri_in, keys_out, tri_out, threadIdx.x);
+    }
+    __syncthreads();
+  }
+}
+
+// 4 + 5 for the bins of more than kChunk keys, whose chunks are sorted: a CTA
+// per chunk. A key's position in its bin is its position in its own chunk plus,
+// for every other chunk, the keys there that come before it (found in shared
+// memory; composites are distinct, so the order is unambiguous). The chunks of
+// a bin proceed side by side, where one CTA that sorted its chunks in turn and
+// merged them pairwise in global memory, 34 keys to a thread one after another,
+// made a 256^2 view (256 tiles, up to 17,000 keys in one) wait 160 us; the two
+// kernels now take 37.
+__global__ void __launch_bounds__(kLargeThreads)
+    bin_place_kernel(const uint64_t* __restrict__ tmp, const int4* __restrict__ chunks,
+                     const int32_t* __restrict__ chunk_count, uint64_t idx_mask,
+                     const uint64_t* __restrict__ keys_in, const int32_t* __restrict__ tri_in,
+                     uint64_t* __restrict__ keys_out, int32_t* __restrict__ tri_out) {
+  __shared__ uint64_t other[kChunk];
+  const int count = *chunk_count, t = threadIdx.x;
   for (int l = blockIdx.x; l < count; l += gridDim.x) {
-    const int2 e = list[l];
-    const int64_t start = e.x;
-    const int64_t n = e.y;
-    if (n <= kChunk) {
-      const uint64_t* sorted = block_merge_sort<kLargeThreads>(tmp + start, (int)n, s, s2, threadIdx.x);
-      write_sorted<kLargeThreads, true>(sorted, n, start, idx_mask, keys_in, tri_in, keys_out, tri_out, threadIdx.x);
-      __syncthreads();
-      continue;
-    }
-    uint64_t* src = tmp + start;
-    uint64_t* dst = alt + start;
-    for (int64_t c0 = 0; c0 < n; c0 += kChunk) {
-      const int len = (int)min((int64_t)kChunk, n - c0);
-      const uint64_t* sorted = block_merge_sort<kLargeThreads>(src + c0, len, s, s2, threadIdx.x);
-      for (int i = threadIdx.x; i < len; i += kLargeThreads) src[c0 + i] = sorted[swz(i)];
-      __syncthreads();
-    }
-    for (int64_t run = kChunk; run < n; run <<= 1) {
-      for (int64_t p0 = 0; p0 < n; p0 += 2 * run) {
-        const int64_t na = min(run, n - p0);
-        const int64_t nb = min(run, n - p0 - na);
-        merge_runs(src + p0, na, nb, dst + p0);
+    const int4 e = chunks[l];
+    const uint64_t* bin = tmp + e.x;
+    const int many = (e.y + kChunk - 1) / kChunk;
+    auto size_of = [&](int c) { return min(kChunk, e.y - c * kChunk); };
+    auto load = [&](int c, uint64_t (&v)[kPerThread]) {
+      const int n = c < many ? size_of(c) : 0;
+#pragma unroll
+      for (int u = 0; u < kPerThread; ++u) {
+        const int i = t + u * kLargeThreads;
+        v[u] = i < n ? __ldg(bin + (int64_t)c * kChunk + i) : ~0ull;
       }
+    };
+    uint64_t mine[kPerThread], next[kPerThread];
+    int place[kPerThread];
+    load(e.z, mine);
+#pragma unroll
+    for (int u = 0; u < kPerThread; ++u) place[u] = t + u * kLargeThreads;
+    int c = e.z == 0 ? 1 : 0;
+    load(c, next);
+    while (c < many) {
+      __syncthreads();  // the last chunk has been searched
+#pragma unroll
+      for (int u = 0; u < kPerThread; ++u) other[t + u * kLargeThreads] = next[u];  // padded with ~0
       __syncthreads();
-      uint64_t* t = src;
-      src = dst;
-      dst = t;
+      const int after = c + 1 == e.z ? c + 2 : c + 1;
+      load(after, next);  // on its way while this one is searched
+      int lo[kPerThread];
+#pragma unroll
+      for (int u = 0; u < kPerThread; ++u) lo[u] = 0;
+#pragma unroll 1
+      for (int step = kChunk / 2; step > 0; step >>= 1) {
+#pragma unroll
+        for (int u = 0; u < kPerThread; ++u)
+          if (other[lo[u] + step - 1] < mine[u]) lo[u] += step;
+      }
+      // kChunk - 1 keys have been counted at most: the last one is left.
+#pragma unroll
+      for (int u = 0; u < kPerThread; ++u) place[u] += lo[u] + (other[lo[u]] < mine[u] ? 1 : 0);
+      c = after;
     }
-    write_sorted<kLargeThreads, false>(src, n, start, idx_mask, keys_in, tri_in, keys_out, tri_out, threadIdx.x);
+    const int n = size_of(e.z);
+#pragma unroll
+    for (int u = 0; u < kPerThread; ++u) {
+      if (t + u * kLargeThreads < n) {
+        const int64_t from = (int64_t)(mine[u] & idx_mask);
+        keys_out[e.x + (int64_t)place[u]] = __ldg(keys_in + from);
+        tri_out[e.x + (int64_t)place[u]] = __ldg(tri_in + from);
+      }
+    }
     __syncthreads();
   }
 }
@@ -380,9 +414,9 @@ struct TileSortWorkspace {
   int32_t* counts;   // nbins + 1 (scanned in place into offsets)
   int32_t* cursors;  // nbins
   int2* lists;       // kTiers x nbins (start, count): tiny, medium, small and large non-empty bins
-  int32_t* list_sizes;  // kTiers
+  int32_t* list_sizes;  // kSizes
+  int4* chunks;      // (bin start, bin keys, chunk index): chunks of bins of more than kChunk keys
   uint64_t* tmp;     // K
-  uint64_t* alt;     // K
   void* scan_ws;
   size_t scan_bytes;
 };
@@ -397,9 +431,9 @@ size_t tile_sort_bytes(int64_t K, int64_t nbins, TileSortWorkspace* w, char* bas
   char* counts = take((size_t)(nbins + 1) * sizeof(int32_t));
   char* cursors = take((size_t)nbins * sizeof(int32_t));
   char* lists = take((size_t)kTiers * nbins * sizeof(int2));
-  char* list_sizes = take(kTiers * sizeof(int32_t));
+  char* list_sizes = take(kSizes * sizeof(int32_t));
+  char* chunks = take(((size_t)K / (kChunk / 2) + 1) * sizeof(int4));
   char* tmp = take((size_t)K * sizeof(uint64_t));
-  char* alt = take((size_t)K * sizeof(uint64_t));
   const size_t scan_bytes = mt_scan_workspace_bytes(nbins + 1);
   char* scan = take(scan_bytes);
   if (w) {
@@ -408,7 +442,7 @@ size_t tile_sort_bytes(int64_t K, int64_t nbins, TileSortWorkspace* w, char* bas
     w->lists = reinterpret_cast<int2*>(lists);
     w->list_sizes = reinterpret_cast<int32_t*>(list_sizes);
     w->tmp = reinterpret_cast<uint64_t*>(tmp);
-    w->alt = reinterpret_cast<uint64_t*>(alt);
+    w->chunks = reinterpret_cast<int4*>(chunks);
     w->scan_ws = scan;
     w->scan_bytes = scan_bytes;
   }
@@ -519,7 +553,7 @@ int mt_sort_keys_by_tile(const int64_t* keys, const int32_t* triangles, int64_t 
   const uint64_t idx_mask = (1ull << idx_bits) - 1ull;
   if (cudaMemsetAsync(w.counts, 0, (size_t)(nbins + 1) * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
   if (cudaMemsetAsync(w.cursors, 0, (size_t)nbins * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
-  if (cudaMemsetAsync(w.list_sizes, 0, kTiers * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
+  if (cudaMemsetAsync(w.list_sizes, 0, kSizes * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
   const uint64_t* k64 = reinterpret_cast<const uint64_t*>(keys);
   // A key outside every bin (never made by mt_generate_keys) is recorded in
   // the workspace status word; it is left out of the output.
@@ -529,7 +563,7 @@ int mt_sort_keys_by_tile(const int64_t* keys, const int32_t* triangles, int64_t 
   const int rc = mt_exclusive_scan_i32(w.counts, nbins + 1, w.scan_ws, w.scan_bytes, stream);
   if (rc != MT_OK) return rc;
   bin_bounds_kernel<<<grid_stride_blocks(nbins, kThreads), kThreads, 0, s>>>(w.counts, nbins, boundaries, w.lists,
-                                                                           w.list_sizes);
+                                                                           w.chunks, w.list_sizes);
   MT_CHECK_LAUNCH();
   bin_scatter_kernel<<<grid_stride_blocks(K, kThreads), kThreads, 0, s>>>(k64, K, num_keys, m, w.counts, w.cursors,
                                                                         idx_bits, low_mask_host, w.tmp);
@@ -544,11 +578,20 @@ int mt_sort_keys_by_tile(const int64_t* keys, const int32_t* triangles, int64_t 
   if (cudaEventRecord(fj.fork, s) != cudaSuccess) return MT_ERR_CUDA;
   for (int i = 0; i < 3; ++i)
     if (cudaStreamWaitEvent(fj.side[i], fj.fork, 0) != cudaSuccess) return MT_ERR_CUDA;
-  const unsigned large_ctas = (unsigned)(nbins < (int64_t)kSmCount * 2 ? nbins : (int64_t)kSmCount * 2);
+  const int64_t most_chunks = K / (kChunk / 2) + 1;
+  const int64_t large_items = nbins + most_chunks;
+  const unsigned large_ctas = (unsigned)(large_items < (int64_t)kSmCount * 2 ? large_items : (int64_t)kSmCount * 2);
   bin_sort_large_kernel<<<large_ctas, kLargeThreads, large_smem, fj.side[0]>>>(
-      w.tmp, w.alt, w.lists + 3 * nbins, w.list_sizes + 3, idx_mask, k64, triangles,
+      w.tmp, w.lists + 3 * nbins, w.chunks, w.list_sizes + 3, idx_mask, k64, triangles,
       reinterpret_cast<uint64_t*>(sorted_keys), sorted_triangles);
   MT_CHECK_LAUNCH();
+  if (K > kChunk) {
+    const unsigned place_ctas = (unsigned)(most_chunks < (int64_t)kSmCount * 2 ? most_chunks : (int64_t)kSmCount * 2);
+    bin_place_kernel<<<place_ctas, kLargeThreads, 0, fj.side[0]>>>(
+        w.tmp, w.chunks, w.list_sizes + kTiers, idx_mask, k64, triangles, reinterpret_cast<uint64_t*>(sorted_keys),
+        sorted_triangles);
+    MT_CHECK_LAUNCH();
+  }
   const unsigned tiny_ctas = (unsigned)(nbins < (int64_t)kSmCount * 5 ? nbins : (int64_t)kSmCount * 5);
   bin_sort_tiny_kernel<<<tiny_ctas, 32 * kTinyWarps, 0, s>>>(w.tmp, w.lists, w.list_sizes, idx_mask, k64, triangles,
                                                              reinterpret_cast<uint64_t*>(sorted_keys),
