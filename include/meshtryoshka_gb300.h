@@ -355,6 +355,17 @@ MT_API int mt_grid_sh_colors(const float* grid_spherical_harmonics, int32_t C, i
                              int32_t sh_degree, const float* camera_positions,
                              int32_t B, float* out_colors, mt_stream_t stream);
 
+/* The same, in the order of the grid's entries: vertex_offsets [S*G + 1] are
+ * the scanned counts that mt_create_triangle_vertices placed the vertices by
+ * (vertices of one grid entry's neighbourhood on every shell are evaluated
+ * together). NULL: in vertex order. */
+MT_API int mt_grid_sh_colors_by_entry(const float* grid_spherical_harmonics, int32_t C, int64_t G,
+                             const int32_t* vertex_sources, int64_t V,
+                             const int32_t* num_vertices, const int32_t* vertex_offsets,
+                             int32_t S, const float* vertices,
+                             int32_t sh_degree, const float* camera_positions,
+                             int32_t B, float* out_colors, mt_stream_t stream);
+
 /* Backward of mt_grid_sh_colors: grad_grid_sh [C,G,3] (every entry written)
  * from grad_colors [B,V,3] through the list of mt_build_vertex_grad_list.
  * The per-vertex SH gradient of mt_evaluate_spherical_harmonics_backward is

@@ -19,6 +19,8 @@
 // the grid through the per-grid-vertex contribution list, with the same bits
 // as the row path.
 
+#include <type_traits>
+
 #include "lookback.cuh"  // warp_inclusive_sum
 #include "mc_tables.h"
 #include "mt_common.cuh"
@@ -938,6 +940,19 @@ __global__ void entry_list_kernel(const float* __restrict__ gsdf, const int32_t*
 // sh_forward_kernel, so the same bits. Vertices at or past the live count are
 // not touched.
 // ---------------------------------------------------------------------------
+// A CTA takes kColourTile consecutive grid entries and deals their vertices, a
+// run for each shell, out to its threads, so that the grid's rows come from
+// memory once for all shells. In vertex order, shell after shell, they were
+// read again for each (7.3 GB at 352^3, 16 shells, instead of 1.5): 2.24 ms at
+// 512^3, 16 shells, 4 cameras, now 1.19. Where they stay in the L2 anyway
+// (kColourCached bytes) vertex order is as good: 55 us at 256^3, 8 shells
+// (81 MB of rows), where the tiles' search makes 59. Interpolating by
+// consecutive floats and turning them in shared memory, as the rows' kernel
+// does, spent more on partial batches than it saved: 1.50 ms and 77 us.
+constexpr int kColourTile = 256, kColourThreads = 128;
+constexpr int kColourShells = 32;  // more shells: vertex order
+constexpr int64_t kColourCached = (int64_t)100 << 20;
+
 template <int kCoeff>
 __device__ __forceinline__ void grid_sh_vertex(const float* __restrict__ gsh, int64_t G,
                                                const int32_t* __restrict__ sources, int64_t V,
@@ -956,17 +971,37 @@ __device__ __forceinline__ void grid_sh_vertex(const float* __restrict__ gsh, in
   sh_colors<kCoeff>(verts, V, coef, campos, B, v, out);
 }
 
-__global__ void grid_sh_colors_kernel(const float* __restrict__ gsh, int64_t G, const int32_t* __restrict__ sources,
-                                      int64_t V, const int32_t* __restrict__ count, const float* __restrict__ verts,
-                                      int n_coeff, const float* __restrict__ campos, int B, float* __restrict__ out) {
+template <int kCoeff>
+__global__ void __launch_bounds__(kColourThreads)
+    grid_sh_colors_kernel(const float* __restrict__ gsh, int64_t G, const int32_t* __restrict__ sources, int64_t V,
+                          const int32_t* __restrict__ count, const int32_t* __restrict__ voff, int S,
+                          const float* __restrict__ verts, const float* __restrict__ campos, int B,
+                          float* __restrict__ out) {
   const int64_t n = count ? min((int64_t)max(*count, 0), V) : V;
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-    switch (n_coeff) {
-      case 1: grid_sh_vertex<1>(gsh, G, sources, V, verts, campos, B, v, out); break;
-      case 4: grid_sh_vertex<4>(gsh, G, sources, V, verts, campos, B, v, out); break;
-      case 9: grid_sh_vertex<9>(gsh, G, sources, V, verts, campos, B, v, out); break;
-      default: grid_sh_vertex<16>(gsh, G, sources, V, verts, campos, B, v, out); break;
-    }
+  if (voff == nullptr) {  // vertex order: a CTA takes kColourThreads vertices
+    const int64_t v = blockIdx.x * (int64_t)kColourThreads + threadIdx.x;
+    if (v < n) grid_sh_vertex<kCoeff>(gsh, G, sources, V, verts, campos, B, v, out);
+    return;
+  }
+  __shared__ int ends[kColourShells];       // vertices of the tile up to and with shell s
+  __shared__ int32_t starts[kColourShells];  // shell s's first vertex of the tile
+  if (threadIdx.x < 32) {
+    const int64_t e0 = blockIdx.x * (int64_t)kColourTile, e1 = min(e0 + kColourTile, G);
+    const int s = threadIdx.x;
+    const int64_t first = s < S ? __ldg(voff + (int64_t)s * G + e0) : 0;
+    const int64_t last = s < S ? min((int64_t)__ldg(voff + (int64_t)s * G + e1), n) : 0;
+    ends[s] = warp_inclusive_sum((int)max(last - first, (int64_t)0));
+    starts[s] = (int32_t)first;
+  }
+  __syncthreads();
+  const int total = ends[kColourShells - 1];
+  for (int r = threadIdx.x; r < total; r += kColourThreads) {
+    int s = 0;  // the first shell that ends past r
+#pragma unroll
+    for (int step = kColourShells / 2; step > 0; step >>= 1)
+      if (ends[s + step - 1] <= r) s += step;
+    const int64_t v = starts[s] + (int64_t)(r - (s > 0 ? ends[s - 1] : 0));
+    grid_sh_vertex<kCoeff>(gsh, G, sources, V, verts, campos, B, v, out);
   }
 }
 
@@ -981,156 +1016,174 @@ __global__ void grid_sh_colors_kernel(const float* __restrict__ gsh, int64_t G, 
 // contiguous. In rounds of kShThreads entries, thread i forms entry i's
 // weighted SH gradient (all rows: the per-vertex d sh_v of sh_backward_kernel,
 // cameras in order, then weighted by the entry's (t, origin)) in shared
-// memory; then thread (row half h, grid vertex x) adds x's entries of the
-// round to its 8 rows in list order, carrying its sums across rounds. The
-// same sums in the same order as sh_backward_kernel + vertex_sh_gather_kernel.
+// memory, unless no camera sees the vertex (most of a large scene's: its
+// entry adds nothing); then thread (row half h, grid vertex x) adds x's entries
+// of the round to its 8 rows in list order. The sums stay in shared memory,
+// which leaves registers for six CTAs to an SM, and are written by consecutive
+// floats. The same sums in the same order as sh_backward_kernel +
+// vertex_sh_gather_kernel. Bound by the latency of the scattered reads (list
+// entry, then vertex, then colour): 2.60 ms at 512^3, 16 shells, 4 cameras with
+// the sums in registers (two CTAs' worth of threads) and every entry added,
+// now 1.92.
 constexpr int kShThreads = 128;
 constexpr int kShX = 64;
 constexpr int kShStride = 49;  // 48 values per entry; odd stride spreads rows over banks
+constexpr int kShCameras = 4;  // cameras whose gradients are loaded side by side
 
+// False (nothing written) when no camera passes a gradient to the vertex.
 template <bool kPacked>
-__device__ __forceinline__ void entry_sh_gradient(int2 e, int64_t V, const float* __restrict__ verts, int n_coeff,
+__device__ __forceinline__ bool entry_sh_gradient(int2 e, int64_t V, const float* __restrict__ verts, int n_coeff,
                                                   const float* __restrict__ campos, int B,
                                                   const float* __restrict__ colors,
                                                   const float* __restrict__ dcolors, float* __restrict__ out) {
   const int64_t vi = e.x & 0x7fffffff;
   const bool origin = e.x < 0;
   const float t = __int_as_float(e.y);
-  const float px = __ldg(verts + 3 * vi), py = __ldg(verts + 3 * vi + 1), pz = __ldg(verts + 3 * vi + 2);
   float d[16][3];
+  bool seen = false;
+  float px = 0.f, py = 0.f, pz = 0.f;
+  for (int b0 = 0; b0 < B; b0 += kShCameras) {
+    float g[kShCameras][3];
 #pragma unroll
-  for (int k = 0; k < 16; ++k) d[k][0] = d[k][1] = d[k][2] = 0.f;
-#pragma unroll 2
-  for (int b = 0; b < B; ++b) {
-    const int64_t o = (int64_t)b * V + vi;
-    float g[3];
-    colour_gradient<kPacked>(dcolors, o, g);
-    // Most (camera, vertex) pairs of a large scene are unseen: their colours
-    // are not read.
-    if (g[0] == 0.0f && g[1] == 0.0f && g[2] == 0.0f) continue;
-    bool any = false;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      g[c] = __ldg(colors + 3 * o + c) > 0.0f ? g[c] : 0.0f;
-      any |= g[c] != 0.0f;
+    for (int j = 0; j < kShCameras; ++j) {
+      g[j][0] = g[j][1] = g[j][2] = 0.0f;
+      if (b0 + j < B) colour_gradient<kPacked>(dcolors, (int64_t)(b0 + j) * V + vi, g[j]);
     }
-    if (!any) continue;
-    float dx, dy, dz;
-    view_dir_at(px, py, pz, campos + 3 * b, dx, dy, dz);
-    float basis[16];
-    sh_basis(dx, dy, dz, n_coeff, basis);
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      if (k < n_coeff) {
+    for (int j = 0; j < kShCameras; ++j) {
+      if (g[j][0] == 0.0f && g[j][1] == 0.0f && g[j][2] == 0.0f) continue;  // also every camera past B
+      const int64_t o = (int64_t)(b0 + j) * V + vi;
+      bool any = false;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) d[k][c] += basis[k] * g[c];
+      for (int c = 0; c < 3; ++c) {
+        g[j][c] = __ldg(colors + 3 * o + c) > 0.0f ? g[j][c] : 0.0f;
+        any |= g[j][c] != 0.0f;
+      }
+      if (!any) continue;
+      if (!seen) {
+        seen = true;
+        px = __ldg(verts + 3 * vi);
+        py = __ldg(verts + 3 * vi + 1);
+        pz = __ldg(verts + 3 * vi + 2);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) d[k][0] = d[k][1] = d[k][2] = 0.f;
+      }
+      float dx, dy, dz;
+      view_dir_at(px, py, pz, campos + 3 * (b0 + j), dx, dy, dz);
+      float basis[16];
+      sh_basis(dx, dy, dz, n_coeff, basis);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        if (k < n_coeff) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) d[k][c] += basis[k] * g[j][c];
+        }
       }
     }
   }
+  if (!seen) return false;
 #pragma unroll
   for (int k = 0; k < 16; ++k) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) out[3 * k + c] = weighted(d[k][c], t, origin);
   }
+  return true;
 }
 
 template <bool kPacked>
-__global__ void __launch_bounds__(kShThreads)
+__global__ void __launch_bounds__(kShThreads, 5)
     grid_sh_colors_backward_kernel(const int32_t* __restrict__ offsets, const int2* __restrict__ list, int64_t G,
                                    int64_t V, const float* __restrict__ verts, int C, int n_coeff,
                                    const float* __restrict__ campos, int B, const float* __restrict__ colors,
                                    const float* __restrict__ dcolors, float* __restrict__ gdsh) {
   __shared__ float s_grad[kShThreads * kShStride];
+  __shared__ float s_sum[kShX * kShStride];
+  __shared__ uint32_t s_seen[kShThreads / 32];
   const int tid = threadIdx.x;
   const int half = tid / kShX, xl = tid % kShX;  // rows 8*half .. 8*half+7 of grid vertex x0 + xl
-  for (int64_t x0 = (int64_t)blockIdx.x * kShX; x0 < G; x0 += (int64_t)gridDim.x * kShX) {
-    const int64_t x = x0 + xl;
-    const int32_t e_begin = __ldg(offsets + x0), e_end = __ldg(offsets + min(x0 + kShX, G));
-    const int32_t my_begin = x < G ? __ldg(offsets + x) : 0, my_end = x < G ? __ldg(offsets + x + 1) : 0;
-    float acc[8][3];
+  const int64_t x0 = (int64_t)blockIdx.x * kShX, x = x0 + xl;
+  const int32_t e_begin = __ldg(offsets + x0), e_end = __ldg(offsets + min(x0 + kShX, G));
+  const int32_t my_begin = x < G ? __ldg(offsets + x) : 0, my_end = x < G ? __ldg(offsets + x + 1) : 0;
+  float* sum = s_sum + xl * kShStride + 24 * half;
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) acc[kk][0] = acc[kk][1] = acc[kk][2] = 0.f;
-    for (int32_t base = e_begin; base < e_end; base += kShThreads) {
-      if (base + tid < e_end)
-        entry_sh_gradient<kPacked>(__ldg(list + base + tid), V, verts, n_coeff, campos, B, colors, dcolors,
-                                   s_grad + tid * kShStride);
-      __syncthreads();
-      const int32_t lo = max(my_begin, base), hi = min(my_end, base + kShThreads);
-      for (int32_t q = lo; q < hi; ++q) {
-        const float* src = s_grad + (q - base) * kShStride + 24 * half;
+  for (int j = 0; j < 24; ++j) sum[j] = 0.f;
+  for (int32_t base = e_begin; base < e_end; base += kShThreads) {
+    const bool seen = base + tid < e_end && entry_sh_gradient<kPacked>(__ldg(list + base + tid), V, verts, n_coeff, campos, B,
+                                                                       colors, dcolors, s_grad + tid * kShStride);
+    const uint32_t word = __ballot_sync(0xffffffffu, seen);
+    if ((tid & 31) == 0) s_seen[tid >> 5] = word;
+    __syncthreads();
+    const int32_t lo = max(my_begin, base) - base, hi = min(my_end, base + kShThreads) - base;
+    for (int32_t q = lo; q < hi; ++q) {
+      if (!((s_seen[q >> 5] >> (q & 31)) & 1u)) continue;
+      const float* src = s_grad + q * kShStride + 24 * half;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) acc[kk][c] += src[3 * kk + c];
-        }
-      }
-      __syncthreads();
+      for (int j = 0; j < 24; ++j) sum[j] += src[j];
     }
-    if (x < G) {
-#pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
-        const int k = 8 * half + kk;
-        if (k < C) {
-          float* dst = gdsh + ((int64_t)k * G + x) * 3;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) dst[c] = k < n_coeff ? acc[kk][c] : 0.f;
-        }
-      }
-    }
+    __syncthreads();
+  }
+  __syncthreads();
+  const int floats = 3 * (int)min((int64_t)kShX, G - x0);
+  for (int f = tid; f < floats; f += kShThreads) {
+    const int q = f / 3, c = f - 3 * q;
+    for (int k = 0; k < min(C, 16); ++k)
+      gdsh[(int64_t)k * 3 * G + 3 * x0 + f] = k < n_coeff ? s_sum[q * kShStride + 3 * k + c] : 0.f;
   }
 }
 
 // Two-pass form of the same backward (with scratch): pass 1, one thread per
 // live vertex v, forms d sh_v (cameras in order, as sh_backward_kernel) once
-// into a vertex-major array [V][16][3]; pass 2, one thread per (8-row half h,
-// grid vertex x), sums x's list entries of rows 8h .. 8h + 7 (96 contiguous
-// bytes per entry) weighted, in list order. The same bits as the one-pass
-// kernel, with each vertex's gradient formed once instead of once per entry.
+// into a vertex-major array [V][16][3], for the vertices that a camera passes a
+// gradient to (marked in `seen`; the others' rows are neither written nor
+// read: most of a large scene's); pass 2, one thread per (8-row half h, grid
+// vertex x), sums x's list entries of rows 8h .. 8h + 7 (96 contiguous bytes
+// per entry) weighted, in list order. The same bits as the one-pass kernel,
+// with each vertex's gradient formed once instead of once per entry. With
+// every row written and read, and the results stored by threads 24 B apart,
+// the two took 38 + 51 us at 256^3, 8 shells, 4 cameras and 0.92 + 1.16 ms at
+// 512^3, 16 shells; now 43 + 46 us and 0.66 + 0.60 ms.
 constexpr int kShGradThreads = 128;
 
 template <bool kPacked>
 __global__ void __launch_bounds__(kShGradThreads)
     vertex_sh_grad_kernel(const float* __restrict__ verts, int64_t V, const int32_t* __restrict__ count,
                           int n_coeff, const float* __restrict__ campos, int B, const float* __restrict__ colors,
-                          const float* __restrict__ dcolors, float4* __restrict__ out) {
+                          const float* __restrict__ dcolors, float4* __restrict__ out,
+                          uint8_t* __restrict__ seen) {
   // Each round, the CTA's kShGradThreads consecutive vertices form their
   // rows in shared memory, then write them as one contiguous block (full
   // 128-byte lines, where each thread's own 192-byte row would be written
   // 16 bytes at a time at a 192-byte stride).
   __shared__ float4 s_rows[kShGradThreads * 12];
+  __shared__ uint32_t s_seen[kShGradThreads / 32];
   const int64_t n = count ? min((int64_t)max(*count, 0), V) : V;
   for (int64_t v0 = (int64_t)blockIdx.x * kShGradThreads; v0 < n; v0 += (int64_t)gridDim.x * kShGradThreads) {
     const int64_t v = v0 + threadIdx.x;
+    bool any_camera = false;
     if (v < n) {
       const float px = __ldg(verts + 3 * v), py = __ldg(verts + 3 * v + 1), pz = __ldg(verts + 3 * v + 2);
       float d[16][3];
 #pragma unroll
       for (int k = 0; k < 16; ++k) d[k][0] = d[k][1] = d[k][2] = 0.f;
-      // Cameras two at a time: both cameras' colours and colour gradients
-      // are loaded together, then the cameras are added in order.
-      for (int b0 = 0; b0 < B; b0 += 2) {
-        float col[2][3], dcol[2][3];
+      for (int b0 = 0; b0 < B; b0 += kShCameras) {
+        float g[kShCameras][3];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const bool in = b0 + j < B;
-          const int64_t o = (int64_t)(b0 + j) * V + v;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            col[j][c] = in ? __ldg(colors + 3 * o + c) : 0.0f;
-            dcol[j][c] = 0.0f;
-          }
-          if (in) colour_gradient<kPacked>(dcolors, o, dcol[j]);
+        for (int j = 0; j < kShCameras; ++j) {
+          g[j][0] = g[j][1] = g[j][2] = 0.0f;
+          if (b0 + j < B) colour_gradient<kPacked>(dcolors, (int64_t)(b0 + j) * V + v, g[j]);
         }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          float g[3];
+        for (int j = 0; j < kShCameras; ++j) {
+          if (g[j][0] == 0.0f && g[j][1] == 0.0f && g[j][2] == 0.0f) continue;  // also every camera past B
+          const int64_t o = (int64_t)(b0 + j) * V + v;
           bool any = false;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            g[c] = col[j][c] > 0.0f ? dcol[j][c] : 0.0f;
-            any |= g[c] != 0.0f;
+            g[j][c] = __ldg(colors + 3 * o + c) > 0.0f ? g[j][c] : 0.0f;
+            any |= g[j][c] != 0.0f;
           }
-          if (!any) continue;  // also every camera past B (its g is zero)
+          if (!any) continue;
+          any_camera = true;
           float dx, dy, dz;
           view_dir_at(px, py, pz, campos + 3 * (b0 + j), dx, dy, dz);
           float basis[16];
@@ -1139,63 +1192,84 @@ __global__ void __launch_bounds__(kShGradThreads)
           for (int k = 0; k < 16; ++k) {
             if (k < n_coeff) {
 #pragma unroll
-              for (int c = 0; c < 3; ++c) d[k][c] += basis[k] * g[c];
+              for (int c = 0; c < 3; ++c) d[k][c] += basis[k] * g[j][c];
             }
           }
         }
       }
-      float4* row = s_rows + threadIdx.x * 12;
+      seen[v] = any_camera ? 1 : 0;
+      if (any_camera) {
+        float4* row = s_rows + threadIdx.x * 12;
 #pragma unroll
-      for (int q = 0; q < 12; ++q) {
-        const int j = 4 * q;
-        row[q] = make_float4(d[j / 3][j % 3], d[(j + 1) / 3][(j + 1) % 3], d[(j + 2) / 3][(j + 2) % 3],
-                             d[(j + 3) / 3][(j + 3) % 3]);
+        for (int q = 0; q < 12; ++q) {
+          const int j = 4 * q;
+          row[q] = make_float4(d[j / 3][j % 3], d[(j + 1) / 3][(j + 1) % 3], d[(j + 2) / 3][(j + 2) % 3],
+                               d[(j + 3) / 3][(j + 3) % 3]);
+        }
       }
     }
+    const uint32_t word = __ballot_sync(0xffffffffu, any_camera);
+    if ((threadIdx.x & 31) == 0) s_seen[threadIdx.x >> 5] = word;
     __syncthreads();
-    const int64_t rows = min((int64_t)kShGradThreads, n - v0);
-    for (int i = threadIdx.x; i < rows * 12; i += kShGradThreads) out[v0 * 12 + i] = s_rows[i];
-    __syncthreads();  // s_rows is written again by the next round
+    const int rows = (int)min((int64_t)kShGradThreads, n - v0);
+    for (int i = threadIdx.x; i < rows * 12; i += kShGradThreads) {
+      const int r = i / 12;
+      if ((s_seen[r >> 5] >> (r & 31)) & 1u) out[v0 * 12 + i] = s_rows[i];
+    }
+    __syncthreads();  // the shared rows are written again by the next round
   }
 }
 
-__global__ void grid_sh_gather_kernel(const int32_t* __restrict__ offsets, const int2* __restrict__ list, int64_t G,
-                                      const float4* __restrict__ dsh, int C, int n_coeff,
-                                      float* __restrict__ gdsh) {
-  const int64_t total = 2 * G;
-  for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < total; o += (int64_t)gridDim.x * blockDim.x) {
-    // Adjacent threads take the two halves of one grid vertex, so a vertex's
-    // 192-byte gradient row is read by neighbouring lanes together.
-    const int half = (int)(o & 1);
-    const int64_t x = o >> 1;
-    float acc[24];
+constexpr int kShGatherThreads = 256, kShGatherAhead = 4;
+
+__global__ void __launch_bounds__(kShGatherThreads)
+    grid_sh_gather_kernel(const int32_t* __restrict__ offsets, const int2* __restrict__ list, int64_t G,
+                          const float4* __restrict__ dsh, const uint8_t* __restrict__ seen, int C, int n_coeff,
+                          float* __restrict__ gdsh) {
+  // Adjacent threads take the two halves of one grid vertex, so a vertex's
+  // 192-byte gradient row is read by neighbouring lanes together; the CTA's
+  // sums are stored by consecutive floats.
+  constexpr int kX = kShGatherThreads / 2;
+  __shared__ float s_sum[kX * kShStride];
+  const int half = threadIdx.x & 1, xl = threadIdx.x >> 1;
+  const int64_t x0 = blockIdx.x * (int64_t)kX, x = x0 + xl;
+  float acc[24];
 #pragma unroll
-    for (int j = 0; j < 24; ++j) acc[j] = 0.f;
-    const int32_t end = __ldg(offsets + x + 1);
-    for (int32_t q = __ldg(offsets + x); q < end; ++q) {
-      const int2 e = __ldg(list + q);
-      const int64_t vi = e.x & 0x7fffffff;
-      const bool origin = e.x < 0;
-      const float t = __int_as_float(e.y);
-      const float4* src = dsh + vi * 12 + 6 * half;
+  for (int j = 0; j < 24; ++j) acc[j] = 0.f;
+  const int32_t end = x < G ? __ldg(offsets + x + 1) : 0;
+  for (int32_t q0 = x < G ? __ldg(offsets + x) : 0; q0 < end; q0 += kShGatherAhead) {
+    int2 e[kShGatherAhead];
+    bool use[kShGatherAhead];
+#pragma unroll
+    for (int j = 0; j < kShGatherAhead; ++j) e[j] = __ldg(list + min(q0 + j, end - 1));
+#pragma unroll
+    for (int j = 0; j < kShGatherAhead; ++j) use[j] = q0 + j < end && __ldg(seen + (e[j].x & 0x7fffffff)) != 0;
+#pragma unroll
+    for (int j = 0; j < kShGatherAhead; ++j) {
+      if (!use[j]) continue;
+      const bool origin = e[j].x < 0;
+      const float t = __int_as_float(e[j].y);
+      const float4* src = dsh + (int64_t)(e[j].x & 0x7fffffff) * 12 + 6 * half;
+      float4 val[6];
+#pragma unroll
+      for (int r = 0; r < 6; ++r) val[r] = __ldg(src + r);
 #pragma unroll
       for (int r = 0; r < 6; ++r) {
-        const float4 val = __ldg(src + r);
-        acc[4 * r + 0] += weighted(val.x, t, origin);
-        acc[4 * r + 1] += weighted(val.y, t, origin);
-        acc[4 * r + 2] += weighted(val.z, t, origin);
-        acc[4 * r + 3] += weighted(val.w, t, origin);
+        acc[4 * r + 0] += weighted(val[r].x, t, origin);
+        acc[4 * r + 1] += weighted(val[r].y, t, origin);
+        acc[4 * r + 2] += weighted(val[r].z, t, origin);
+        acc[4 * r + 3] += weighted(val[r].w, t, origin);
       }
     }
+  }
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      const int k = 8 * half + kk;
-      if (k < C) {
-        float* dst = gdsh + ((int64_t)k * G + x) * 3;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) dst[c] = k < n_coeff ? acc[3 * kk + c] : 0.f;
-      }
-    }
+  for (int j = 0; j < 24; ++j) s_sum[xl * kShStride + 24 * half + j] = acc[j];
+  __syncthreads();
+  const int floats = 3 * (int)min((int64_t)kX, G - x0);
+  for (int f = threadIdx.x; f < floats; f += kShGatherThreads) {
+    const int q = f / 3, c = f - 3 * q;
+    for (int k = 0; k < min(C, 16); ++k)
+      gdsh[(int64_t)k * 3 * G + 3 * x0 + f] = k < n_coeff ? s_sum[q * kShStride + 3 * k + c] : 0.f;
   }
 }
 
@@ -1551,16 +1625,20 @@ static int grid_sh_backward(const int32_t* list_offsets, const int32_t* list, in
   if (workspace && workspace_bytes >= mt_grid_sh_colors_backward_workspace_bytes(V) && Bn > 0) {
     float4* dsh = reinterpret_cast<float4*>(static_cast<char*>(workspace) + 256);
     MT_REQUIRE((reinterpret_cast<uintptr_t>(dsh) & 15) == 0);
-    vertex_sh_grad_kernel<kPacked><<<grid_stride_blocks(V, kShGradThreads), kShGradThreads, 0, st>>>(vertices, V, num_vertices, n, camera_positions,
-                                                                      Bn, out_colors, grad_colors, dsh);
+    uint8_t* seen = reinterpret_cast<uint8_t*>(dsh + 12 * V);
+    vertex_sh_grad_kernel<kPacked><<<grid_stride_blocks(V, kShGradThreads), kShGradThreads, 0, st>>>(
+        vertices, V, num_vertices, n, camera_positions, Bn, out_colors, grad_colors, dsh, seen);
     MT_CHECK_LAUNCH();
-    grid_sh_gather_kernel<<<grid_stride_blocks(2 * G, 256), 256, 0, st>>>(
-        list_offsets, reinterpret_cast<const int2*>(list), G, dsh, C, n, grad_grid_spherical_harmonics);
+    const int64_t blocks = (2 * G + kShGatherThreads - 1) / kShGatherThreads;
+    MT_REQUIRE(blocks < ((int64_t)1 << 31));
+    grid_sh_gather_kernel<<<(unsigned)blocks, kShGatherThreads, 0, st>>>(
+        list_offsets, reinterpret_cast<const int2*>(list), G, dsh, seen, C, n, grad_grid_spherical_harmonics);
     MT_CHECK_LAUNCH();
     return MT_OK;
   }
   const int64_t xblocks = (G + kShX - 1) / kShX;
-  grid_sh_colors_backward_kernel<kPacked><<<(unsigned)min(xblocks, (int64_t)152 * 32), kShThreads, 0, st>>>(
+  MT_REQUIRE(xblocks < ((int64_t)1 << 31));
+  grid_sh_colors_backward_kernel<kPacked><<<(unsigned)xblocks, kShThreads, 0, st>>>(
       list_offsets, reinterpret_cast<const int2*>(list), G, V, vertices, C, n, camera_positions, Bn, out_colors,
       grad_colors, grad_grid_spherical_harmonics);
   MT_CHECK_LAUNCH();
@@ -1886,22 +1964,45 @@ int mt_vertex_grads_from_list(const int32_t* list_offsets, const int32_t* list, 
   return MT_OK;
 }
 
-int mt_grid_sh_colors(const float* grid_spherical_harmonics, int32_t C, int64_t G, const int32_t* vertex_sources,
-                      int64_t V, const int32_t* num_vertices, const float* vertices, int32_t sh_degree,
-                      const float* camera_positions, int32_t B, float* out_colors, mt_stream_t stream) {
-  MT_REQUIRE(G >= 0 && V >= 0 && B >= 0 && sh_degree >= 0 && sh_degree <= 3);
+int mt_grid_sh_colors_by_entry(const float* grid_spherical_harmonics, int32_t C, int64_t G,
+                               const int32_t* vertex_sources, int64_t V, const int32_t* num_vertices,
+                               const int32_t* vertex_offsets, int32_t S, const float* vertices, int32_t sh_degree,
+                               const float* camera_positions, int32_t B, float* out_colors, mt_stream_t stream) {
+  MT_REQUIRE(G >= 0 && V >= 0 && B >= 0 && S >= 0 && sh_degree >= 0 && sh_degree <= 3);
   const int n = (sh_degree + 1) * (sh_degree + 1);
   MT_REQUIRE(C >= n);
   if (V == 0 || B == 0) return MT_OK;
   MT_REQUIRE(grid_spherical_harmonics && vertex_sources && vertices && camera_positions && out_colors);
-  grid_sh_colors_kernel<<<grid_stride_blocks(V, 256), 256, 0, as_stream(stream)>>>(
-      grid_spherical_harmonics, G, vertex_sources, V, num_vertices, vertices, n, camera_positions, B, out_colors);
+  const bool cached = 12 * G * n <= kColourCached;
+  const int32_t* offsets = S <= kColourShells && !cached ? vertex_offsets : nullptr;
+  const int64_t blocks = offsets ? (G + kColourTile - 1) / kColourTile : (V + kColourThreads - 1) / kColourThreads;
+  MT_REQUIRE(blocks < ((int64_t)1 << 31));
+  if (blocks == 0) return MT_OK;
+  auto launch = [&](auto coeff) {
+    grid_sh_colors_kernel<decltype(coeff)::value><<<(unsigned)blocks, kColourThreads, 0, as_stream(stream)>>>(
+        grid_spherical_harmonics, G, vertex_sources, V, num_vertices, offsets, S, vertices, camera_positions, B,
+        out_colors);
+  };
+  switch (n) {
+    case 1: launch(std::integral_constant<int, 1>{}); break;
+    case 4: launch(std::integral_constant<int, 4>{}); break;
+    case 9: launch(std::integral_constant<int, 9>{}); break;
+    default: launch(std::integral_constant<int, 16>{}); break;
+  }
   MT_CHECK_LAUNCH();
   return MT_OK;
 }
 
+int mt_grid_sh_colors(const float* grid_spherical_harmonics, int32_t C, int64_t G, const int32_t* vertex_sources,
+                      int64_t V, const int32_t* num_vertices, const float* vertices, int32_t sh_degree,
+                      const float* camera_positions, int32_t B, float* out_colors, mt_stream_t stream) {
+  return mt_grid_sh_colors_by_entry(grid_spherical_harmonics, C, G, vertex_sources, V, num_vertices, nullptr, 0,
+                                    vertices, sh_degree, camera_positions, B, out_colors, stream);
+}
+
 size_t mt_grid_sh_colors_backward_workspace_bytes(int64_t V) {
-  return 256 + (size_t)(V > 0 ? V : 0) * 48 * sizeof(float);
+  // The rows [V][16][3], then a byte per vertex.
+  return 256 + (size_t)(V > 0 ? V : 0) * (48 * sizeof(float) + 1);
 }
 
 int mt_grid_sh_colors_backward(const int32_t* list_offsets, const int32_t* list, int64_t G, int64_t V,

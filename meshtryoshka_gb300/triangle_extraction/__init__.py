@@ -452,12 +452,14 @@ def count_triangle_vertices(signed_distances: Tensor, lower_corners: Tensor, lev
     return counts
 
 
-# The grid SH backward forms each vertex's SH gradient once into scratch
-# (48 floats per vertex) and then gathers it per grid vertex; above this many
-# bytes of scratch (2.8 M vertices) it runs its one-pass form instead, which
-# forms a vertex's gradient once per list entry and needs no scratch (same
-# values): at the 512^3 / 16-shell scene the scratch would hold 3.5 GB.
-GRID_SH_BACKWARD_SCRATCH_LIMIT = 512 << 20
+# The grid SH backward forms each vertex's SH gradient once into scratch (193
+# bytes per vertex) and then gathers it per grid vertex; above this many bytes
+# of scratch (22 M vertices) it runs its one-pass form instead, which forms a
+# vertex's gradient once per list entry and needs no scratch (same values). At
+# the 512^3 / 16-shell scene (3.5 GB) the two passes take 1.26 ms, one 1.92.
+GRID_SH_BACKWARD_SCRATCH_LIMIT = 4 << 30
+# Scratch above this size is allocated for the call, not kept as workspace.
+_KEPT_SCRATCH = 512 << 20
 
 
 class DeferredSH:
@@ -473,6 +475,7 @@ class DeferredSH:
         self.grid_spherical_harmonics = grid_spherical_harmonics
         self.vertex_sources: Tensor | None = None  # [3, V] int32 (origin, axis corner, bits of t)
         self.num_vertices: Tensor | None = None  # device int32 live count (capacity mode) or None
+        self.vertex_offsets: Tensor | None = None  # [S * G + 1] int32, scanned counts per (shell, grid entry)
         self.list_offsets: Tensor | None = None  # [G + 1] int32
         self.contributions: Tensor | None = None  # [2V, 2] int32
 
@@ -507,8 +510,10 @@ class GridSHColors(torch.autograd.Function):
             campos = torch.empty((b, 3), dtype=torch.float32, device=device)
             nt.call("mt_camera_positions", nt.ptr(extrinsics), b, nt.ptr(campos), nt.stream(device))
             colors = torch.empty((b, v, 3), dtype=torch.float32, device=device)
-            nt.call("mt_grid_sh_colors", nt.ptr(gsh), c, g, nt.ptr(deferred.vertex_sources), v,
-                    nt.ptr(deferred.num_vertices), nt.ptr(vertices), int(sh_degree), nt.ptr(campos), b,
+            offsets = deferred.vertex_offsets
+            shells = (offsets.numel() - 1) // g if g > 0 else 0
+            nt.call("mt_grid_sh_colors_by_entry", nt.ptr(gsh), c, g, nt.ptr(deferred.vertex_sources), v,
+                    nt.ptr(deferred.num_vertices), nt.ptr(offsets), shells, nt.ptr(vertices), int(sh_degree), nt.ptr(campos), b,
                     nt.ptr(colors), nt.stream(device))
             ctx.save_for_backward(vertices, campos, colors)
             ctx.deferred = deferred
@@ -526,10 +531,13 @@ class GridSHColors(torch.autograd.Function):
             grad_gsh = torch.empty(ctx.gsh_shape, dtype=torch.float32, device=device)  # fully written
             v = vertices.shape[0]
             need = nt.library().mt_grid_sh_colors_backward_workspace_bytes(v)
-            if need <= GRID_SH_BACKWARD_SCRATCH_LIMIT:
-                ws_ptr, ws_bytes = nt.workspace(device).get(need)
-            else:
+            if need > GRID_SH_BACKWARD_SCRATCH_LIMIT:
                 ws_ptr, ws_bytes = None, 0  # the one-pass form: no scratch
+            elif need > _KEPT_SCRATCH:
+                scratch = torch.empty((need,), dtype=torch.uint8, device=device)
+                ws_ptr, ws_bytes = scratch.data_ptr(), need
+            else:
+                ws_ptr, ws_bytes = nt.workspace(device).get(need)
             rows, packed = nt.colour_gradient_rows(grad_colors)
             nt.call("mt_grid_sh_colors_packed_backward" if packed else "mt_grid_sh_colors_backward",
                     nt.ptr(d.list_offsets), nt.ptr(d.contributions), g, v, nt.ptr(vertices), c, ctx.sh_degree,
@@ -603,6 +611,7 @@ class CreateTriangleVertices(torch.autograd.Function):
                         nt.ptr(level_sets), s, nt.ptr(vertex_offsets), v, nt.ptr(inverse), nt.ptr(offsets),
                         nt.ptr(contributions), ws_ptr, ws_bytes, nt.stream(device))
                 deferred.vertex_sources = sources
+                deferred.vertex_offsets = vertex_offsets
                 deferred.num_vertices = (vertex_offsets[-1:].view(()) if capacity is not None else None)
                 deferred.list_offsets = offsets
                 deferred.contributions = contributions
