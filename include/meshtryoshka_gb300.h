@@ -564,8 +564,11 @@ MT_API int mt_generate_keys(const float* depth, int64_t V, const int32_t* faces,
  * K are dropped. *out_num_keys (device int64) receives the live key count,
  * which may exceed K. xy must be 8-byte aligned. workspace (16-byte
  * aligned): at least mt_bound_and_generate_keys_workspace_bytes(B * F) bytes
- * (about 20 bytes per item; it holds each item's tile rectangle and key depth
- * between the kernels). */
+ * (about 22 bytes per item; it holds the tile rectangle and key depth of the
+ * items that touch a tile between the kernels).
+ * mt_bound_keys and mt_write_bounded_keys are its two halves, for callers that
+ * read the count (*out_num_keys) back and size the keys by it: the workspace
+ * carries the records from one to the other. */
 MT_API size_t mt_bound_and_generate_keys_workspace_bytes(int64_t items);
 MT_API int mt_bound_and_generate_keys(
     const float* xy, const float* depth, int64_t V, const int32_t* faces,
@@ -575,6 +578,17 @@ MT_API int mt_bound_and_generate_keys(
     const int32_t* layout, int64_t K, int64_t* out_keys, int32_t* out_triangles,
     int64_t* out_num_keys, void* workspace, size_t workspace_bytes,
     mt_stream_t stream);
+MT_API int mt_bound_keys(
+    const float* xy, const float* depth, int64_t V, const int32_t* faces,
+    int64_t F, const int32_t* num_faces, int32_t B, int32_t tile_h,
+    int32_t tile_w, int32_t rows, int32_t cols, const int64_t* cameras,
+    float near_plane, int64_t* out_num_keys, void* workspace,
+    size_t workspace_bytes, mt_stream_t stream);
+MT_API int mt_write_bounded_keys(
+    int64_t F, const int32_t* shell_face_boundaries, int32_t S, int32_t B,
+    int32_t cols, const int64_t* cameras, const int32_t* layout, int64_t K,
+    int64_t* out_keys, int32_t* out_triangles, void* workspace,
+    size_t workspace_bytes, mt_stream_t stream);
 
 /* triangle_rasterization/delineate_tiles.slang:14-58 (+ the zero fill of
  * delineate_tiles.py:40, done here). out_boundaries [B, shell_dim,

@@ -99,6 +99,8 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
         I32,
         [P, P, I64, P, I64, P, P, I32, I32, I32, I32, I32, I32, P, c_float, P, I64, P, P, P, P, c_size_t, P],
     ),
+    "mt_bound_keys": (I32, [P, P, I64, P, I64, P, I32, I32, I32, I32, I32, P, c_float, P, P, c_size_t, P]),
+    "mt_write_bounded_keys": (I32, [I64, P, I32, I32, I32, P, P, I64, P, P, P, c_size_t, P]),
     "mt_delineate_tiles": (I32, [P, I64, P, P, I32, I32, I32, I64, P, P]),
     "mt_sort_keys_by_tile_supported": (I32, [P, I32, I32, I64]),
     "mt_sort_keys_by_tile_workspace_bytes": (c_size_t, [I64, I64]),
@@ -179,6 +181,7 @@ KERNELS_PER_CALL = {
     "mt_intersect_and_composite_forward": 4,  # warp masks, tile-order histogram and scatter, composite
     "mt_sort_keys_by_tile": 9,  # count, scan, tile ranges, scatter, tiny / medium / small / large bin sorts, placing
     "mt_bound_and_generate_keys": 3,  # rectangles + chunk counts, chunk scan, keys
+    "mt_bound_keys": 2,
     "mt_build_vertex_grad_list": 4,  # corner inverse, count, scan, fill
     "mt_grid_sh_colors_backward": 2,  # per-vertex SH gradients, per-grid-vertex sums
     "mt_grid_sh_colors_packed_backward": 2,

@@ -298,28 +298,34 @@ __device__ __forceinline__ uint32_t face_shell(const int32_t* __restrict__ sfb, 
 }
 
 // ---------------------------------------------------------------------------
-// Tile bounds, key offsets and keys for calls with a key capacity (nothing is
-// read back). The keys and their order equal bound_kernel followed by an
-// inclusive scan of the counts and keys_kernel: item i = (camera, face) in
-// row-major order writes its keys at the sum of the counts of items < i.
+// Tile bounds, key offsets and keys of a render. The keys and their order equal
+// bound_kernel followed by an inclusive scan of the counts and keys_kernel:
+// item i = (camera, face) in row-major order writes its keys at the sum of the
+// counts of items < i.
 //
 // The B*F items are split into chunks of kFusedItems x kFusedThreads items,
 // one CTA each, striped (item j * kFusedThreads + tid of the chunk) so that a
 // warp's loads are adjacent. Three launches, no CTA waits on another:
-//   chunk_bounds_kernel  each item's tile rectangle (int4) and key depth into
-//                        workspace records, and each chunk's key count;
-//   chunk_scan_kernel    one CTA: exclusive scan of the chunk counts, and the
-//                        total key count;
+//   chunk_bounds_kernel  the tile rectangle (int4) and key depth of the items
+//                        that touch a tile, in item order at the start of the
+//                        chunk's records, with their places in the chunk; and
+//                        the chunk's item and key counts;
+//   chunk_scan_kernel    one CTA: exclusive scan of the chunks' key counts, and
+//                        the total (many chunks: the library's scan);
 //   chunk_keys_kernel    reads its chunk's records back (coalesced), scans
-//                        them and writes the keys load-balanced.
+//                        them and writes the keys.
+// Most items touch no tile (back faces, faces outside the image), and a record
+// for each of them was most of both kernels' traffic: 1003 and 769 us at 512^3,
+// 16 shells, 4 cameras (96 M live faces x cameras), now 975 and 245.
 // ---------------------------------------------------------------------------
 constexpr int kFusedThreads = 256;
 constexpr int kFusedItems = 4;
 constexpr int kFusedSubTile = kFusedThreads * kFusedItems;
 constexpr int kChunkScanThreads = 1024;
-// Workspace: [0,256) status word (unused here), chunk counts (int64 per
-// chunk), the rectangle records (int4 per item), the key depths (float per
-// item); each region starts on a 256-byte boundary.
+// Workspace: [0,256) status word (unused here), the chunks' key counts (int64
+// each) and item counts (int32 each), the rectangle records (int4 per item),
+// the key depths (float per item) and the places (uint16 per item); each region
+// starts on a 256-byte boundary.
 constexpr size_t kFusedHeader = 256;
 
 __host__ __device__ inline size_t round256(size_t x) { return (x + 255) / 256 * 256; }
@@ -334,8 +340,12 @@ struct FusedArgs {
   int B, tile_h, tile_w, rows, cols;
   const int64_t* cameras;
   float near;
-  int64_t chunk;  // items per chunk (a multiple of kFusedSubTile)
 };
+
+// The int32 count of bound_kernel, widened as the scan widens it.
+__device__ __forceinline__ int64_t tile_count(const TileBounds& t) {
+  return (int64_t)((t.r1 - t.r0) * (t.c1 - t.c0));
+}
 
 // Bounds (and key depth) of this thread's kFusedItems items of the sub-tile
 // starting at item `first`, loads of all items issued together.
@@ -344,7 +354,8 @@ __device__ __forceinline__ void subtile_bounds(const FusedArgs& a, int64_t first
                                                TileBounds (&t)[kFusedItems], float (&mean)[kFusedItems]) {
   {
     const int64_t i0 = first + threadIdx.x;
-    int b = (int)(i0 / a.F);
+    // In 32 bits where the items allow: a 64-bit division takes 100 instructions.
+    int b = (end >> 32) == 0 ? (int)((uint32_t)i0 / (uint32_t)a.F) : (int)(i0 / a.F);
     int64_t f = i0 - (int64_t)b * a.F;
 #pragma unroll
     for (int j = 0; j < kFusedItems; ++j) {
@@ -365,6 +376,8 @@ __device__ __forceinline__ void subtile_bounds(const FusedArgs& a, int64_t first
 #pragma unroll
     for (int c = 0; c < 3; ++c) corner[j][c] = ok ? __ldg(a.faces + 3 * face[j] + c) : -1;
   }
+  // Depths beside the positions: read only for faces with a rectangle, they
+  // would wait for the positions (1051 us instead of 1002 at 512^3).
   float2 p[kFusedItems][3];
   float d[kFusedItems][3];
   bool ok[kFusedItems];
@@ -392,11 +405,6 @@ __device__ __forceinline__ void subtile_bounds(const FusedArgs& a, int64_t first
   }
 }
 
-// The int32 count of bound_kernel, widened as the scan widens it.
-__device__ __forceinline__ int64_t tile_count(const TileBounds& t) {
-  return (int64_t)((t.r1 - t.r0) * (t.c1 - t.c0));
-}
-
 template <typename T>
 __device__ __forceinline__ T block_sum(T x, T* s_warp) {
   x = warp_sum(x);
@@ -408,36 +416,65 @@ __device__ __forceinline__ T block_sum(T x, T* s_warp) {
   return total;
 }
 
-__global__ void __launch_bounds__(kFusedThreads, 3)
-    chunk_bounds_kernel(FusedArgs a, int4* __restrict__ rect, float* __restrict__ key_depth,
-                        int64_t* __restrict__ chunk_counts) {
-  __shared__ int64_t s_warp[kFusedThreads / 32];
+struct ChunkRecords {
+  int64_t* keys;    // per chunk: key count, then (scanned) its first key; and one more
+  int32_t* items;   // per chunk: records
+  int4* rect;       // per record (a chunk's start at its first item)
+  float* depth;
+  uint16_t* place;  // item's place in its chunk
+  void* scan;       // the key counts' scan
+  size_t scan_bytes;
+};
+
+__global__ void __launch_bounds__(kFusedThreads, 3) chunk_bounds_kernel(FusedArgs a, ChunkRecords rec) {
+  constexpr int kWarps = kFusedThreads / 32;
+  __shared__ int64_t s_warp[kWarps];
+  __shared__ int s_live[kFusedItems * kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t items = (int64_t)a.B * a.F;
-  const int64_t first = blockIdx.x * a.chunk, end = min(first + a.chunk, items);
+  const int64_t first = blockIdx.x * (int64_t)kFusedSubTile, end = min(first + kFusedSubTile, items);
   const int64_t live = a.num_faces ? min((int64_t)max(*a.num_faces, 0), a.F) : a.F;
+  int cam[kFusedItems];
+  int64_t face[kFusedItems];
+  TileBounds t[kFusedItems];
+  float mean[kFusedItems];
+  subtile_bounds(a, first, end, live, cam, face, t, mean);
   int64_t sum = 0;
-  for (int64_t sub = first; sub < end; sub += kFusedSubTile) {
-    int cam[kFusedItems];
-    int64_t face[kFusedItems];
-    TileBounds t[kFusedItems];
-    float mean[kFusedItems];
-    subtile_bounds(a, sub, end, live, cam, face, t, mean);
+  uint32_t touching[kFusedItems];
 #pragma unroll
-    for (int j = 0; j < kFusedItems; ++j) {
-      const int64_t i = sub + (int64_t)j * kFusedThreads + threadIdx.x;
-      if (i < end) {
-        rect[i] = make_int4(t[j].r0, t[j].c0, t[j].r1, t[j].c1);
-        key_depth[i] = mean[j];
-      }
-      sum += tile_count(t[j]);
+  for (int j = 0; j < kFusedItems; ++j) {
+    const int64_t count = tile_count(t[j]);
+    sum += count;
+    touching[j] = __ballot_sync(0xffffffffu, count != 0);
+    if (lane == 0) s_live[j * kWarps + warp] = __popc(touching[j]);
+  }
+  const int64_t total = block_sum(sum, s_warp);  // its barrier also publishes s_live
+  // The counts of all (item row, warp) pairs, one to a lane, scanned in every warp.
+  static_assert(kFusedItems * kWarps == 32, "a lane to a pair");
+  const int mine = s_live[lane], upto = warp_inclusive_sum(mine);
+  const int all = __shfl_sync(0xffffffffu, upto, 31);
+#pragma unroll
+  for (int j = 0; j < kFusedItems; ++j) {
+    const int before = __shfl_sync(0xffffffffu, upto - mine, j * kWarps + warp) + __popc(touching[j] & lanemask_lt());
+    if ((touching[j] >> lane) & 1u) {
+      rec.rect[first + before] = make_int4(t[j].r0, t[j].c0, t[j].r1, t[j].c1);
+      rec.depth[first + before] = mean[j];
+      rec.place[first + before] = (uint16_t)(j * kFusedThreads + threadIdx.x);
     }
   }
-  const int64_t total = block_sum(sum, s_warp);
-  if (threadIdx.x == 0) chunk_counts[blockIdx.x] = total;
+  if (threadIdx.x == 0) {
+    rec.keys[blockIdx.x] = total;
+    rec.items[blockIdx.x] = all;
+    if (blockIdx.x == 0) rec.keys[gridDim.x] = 0;  // becomes the total
+  }
 }
 
 // Exclusive scan of the chunk counts in place (one CTA); *out_count = total.
 // Rounds of kChunkScanThreads x 4 counts, each thread's four loaded together.
+// For few chunks: beyond kOneCtaChunks the library's scan over many CTAs takes
+// over (512^3's 117,000 chunks were 29 rounds here, 117 us).
+constexpr int64_t kOneCtaChunks = 16 * kChunkScanThreads;
+
 __global__ void __launch_bounds__(kChunkScanThreads)
     chunk_scan_kernel(int64_t* __restrict__ counts, int64_t chunks, int64_t* __restrict__ out_count) {
   constexpr int kPer = 4;
@@ -474,62 +511,50 @@ __global__ void __launch_bounds__(kChunkScanThreads)
   if (tid == 0) *out_count = running;
 }
 
-// Each thread writes the keys of its own items (in row-major tile order, at
-// the item's exclusive offset: the chunk's offset + the CTA scan of the
-// counts), as keys_kernel does, from the records instead of gathers.
+// Each thread writes the keys of its records (in row-major tile order, at the
+// item's exclusive offset: the chunk's offset + the CTA scan of the counts), as
+// keys_kernel does.
 __global__ void __launch_bounds__(kFusedThreads)
-    chunk_keys_kernel(FusedArgs a, const int4* __restrict__ rect, const float* __restrict__ key_depth,
-                      const int64_t* __restrict__ chunk_offsets, const int32_t* __restrict__ sfb, int S,
-                      KeyLayout L, int64_t K, uint64_t* __restrict__ out_keys, int32_t* __restrict__ out_tri) {
-  __shared__ int64_t s_warp[kFusedItems][kFusedThreads / 32];
+    chunk_keys_kernel(FusedArgs a, ChunkRecords rec, const int32_t* __restrict__ sfb, int S, KeyLayout L, int64_t K,
+                      uint64_t* __restrict__ out_keys, int32_t* __restrict__ out_tri) {
+  constexpr int kWarps = kFusedThreads / 32;
+  __shared__ int64_t s_warp[2][kWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t items = (int64_t)a.B * a.F;
-  const int64_t sub = (int64_t)blockIdx.x * kFusedSubTile;
-  const int64_t end = min(sub + kFusedSubTile, items);
-  TileBounds t[kFusedItems];
-  float kd[kFusedItems];
+  const int many = rec.items[blockIdx.x];
+  const int64_t first = blockIdx.x * (int64_t)kFusedSubTile;
+  const int first_cam = (int)(first / a.F);
+  const int64_t first_face = first - (int64_t)first_cam * a.F;
+  int64_t base = rec.keys[blockIdx.x];
+  int turn = 0;
+  for (int p0 = 0; p0 < many; p0 += kFusedThreads, turn ^= 1) {
+    const int64_t i = first + p0 + tid;
+    const bool in = p0 + tid < many;
+    const int4 r4 = in ? __ldcs(rec.rect + i) : make_int4(0, 0, 0, 0);
+    const float depth = in ? __ldcs(rec.depth + i) : 0.0f;
+    const int place = in ? (int)__ldcs(rec.place + i) : 0;
+    const TileBounds tb{r4.x, r4.y, r4.z, r4.w};
+    const int64_t count = tile_count(tb);
+    const int64_t inc = warp_inclusive_sum(count);
+    if (lane == 31) s_warp[turn][warp] = inc;
+    __syncthreads();
+    int64_t below = 0, all = 0;
 #pragma unroll
-  for (int j = 0; j < kFusedItems; ++j) {
-    const int64_t i = sub + (int64_t)j * kFusedThreads + tid;
-    const int4 r = i < end ? __ldcs(rect + i) : make_int4(0, 0, 0, 0);
-    kd[j] = i < end ? __ldcs(key_depth + i) : 0.0f;
-    t[j] = TileBounds{r.x, r.y, r.z, r.w};
-  }
-  int64_t inc[kFusedItems];
-#pragma unroll
-  for (int j = 0; j < kFusedItems; ++j) {
-    inc[j] = warp_inclusive_sum(tile_count(t[j]));
-    if (lane == 31) s_warp[j][warp] = inc[j];
-  }
-  __syncthreads();
-  int64_t base = chunk_offsets[blockIdx.x];
-#pragma unroll
-  for (int j = 0; j < kFusedItems; ++j) {
-    int64_t below = 0, row = 0;
-#pragma unroll
-    for (int w = 0; w < kFusedThreads / 32; ++w) {
-      const int64_t x = s_warp[j][w];
-      row += x;
+    for (int w = 0; w < kWarps; ++w) {
+      const int64_t x = s_warp[turn][w];
+      all += x;
       below += (w < warp) ? x : 0;
     }
-    inc[j] += base + below;  // inclusive offset of item j
-    base += row;
-  }
-  int b;
-  int64_t f;
-  {
-    const int64_t i0 = sub + tid;
-    b = (int)(i0 / a.F);
-    f = i0 - (int64_t)b * a.F;
-  }
-#pragma unroll
-  for (int j = 0; j < kFusedItems; ++j) {
-    const TileBounds& tb = t[j];
     if (tb.r1 > tb.r0 && tb.c1 > tb.c0) {
-      int64_t k = inc[j] - tile_count(tb);
+      int64_t k = base + below + inc - count;
+      int b = first_cam;
+      int64_t f = first_face + place;
+      while (f >= a.F) {
+        f -= a.F;
+        ++b;
+      }
       const uint64_t fixed = (((uint64_t)b & field_mask(L.cam_len)) << L.cam_off) |
                              (((uint64_t)face_shell(sfb, S, f) & field_mask(L.shell_len)) << L.shell_off) |
-                             ((uint64_t)__float_as_uint(kd[j]) << L.depth_off);
+                             ((uint64_t)__float_as_uint(depth) << L.depth_off);
       const int width = a.cameras ? (int)a.cameras[6 * b + 1] : a.cols;
       for (int r = tb.r0; r < tb.r1 && k < K; ++r) {
         for (int c = tb.c0; c < tb.c1; ++c) {
@@ -541,11 +566,7 @@ __global__ void __launch_bounds__(kFusedThreads)
         }
       }
     }
-    f += kFusedThreads;
-    while (f >= a.F) {
-      f -= a.F;
-      ++b;
-    }
+    base += all;
   }
 }
 
@@ -694,10 +715,89 @@ int mt_generate_keys(const float* depth, int64_t V, const int32_t* faces, int64_
 
 static int64_t fused_chunks(int64_t items) { return (items + kFusedSubTile - 1) / kFusedSubTile; }
 
+static size_t chunk_records(int64_t items, char* base, ChunkRecords* rec) {
+  const int64_t chunks = fused_chunks(items);
+  size_t off = kFusedHeader;
+  auto take = [&](size_t bytes) {
+    char* p = base ? base + off : nullptr;
+    off += round256(bytes);
+    return p;
+  };
+  char* keys = take((size_t)(chunks + 1) * sizeof(int64_t));
+  char* counts = take((size_t)chunks * sizeof(int32_t));
+  char* rect = take((size_t)items * sizeof(int4));
+  char* depth = take((size_t)items * sizeof(float));
+  char* place = take((size_t)items * sizeof(uint16_t));
+  const size_t scan_bytes = mt_scan_workspace_bytes(chunks + 1);
+  char* scan = take(scan_bytes);
+  if (rec)
+    *rec = ChunkRecords{reinterpret_cast<int64_t*>(keys), reinterpret_cast<int32_t*>(counts),
+                        reinterpret_cast<int4*>(rect), reinterpret_cast<float*>(depth),
+                        reinterpret_cast<uint16_t*>(place), scan, scan_bytes};
+  return off;
+}
+
 size_t mt_bound_and_generate_keys_workspace_bytes(int64_t items) {
-  if (items < 0) items = 0;
-  return kFusedHeader + round256((size_t)fused_chunks(items) * sizeof(int64_t)) +
-         round256((size_t)items * sizeof(int4)) + (size_t)items * sizeof(float);
+  return chunk_records(items < 0 ? 0 : items, nullptr, nullptr);
+}
+
+int mt_bound_keys(const float* xy, const float* depth, int64_t V, const int32_t* faces, int64_t F,
+                  const int32_t* num_faces, int32_t B, int32_t tile_h, int32_t tile_w, int32_t rows, int32_t cols,
+                  const int64_t* cameras, float near_plane, int64_t* out_num_keys, void* workspace,
+                  size_t workspace_bytes, mt_stream_t stream) {
+  MT_REQUIRE(V >= 0 && F >= 0 && B >= 0 && tile_h > 0 && tile_w > 0 && rows >= 0 && cols >= 0);
+  MT_REQUIRE(out_num_keys);
+  const cudaStream_t s = as_stream(stream);
+  const int64_t items = (int64_t)B * F;
+  if (items == 0)
+    return cudaMemsetAsync(out_num_keys, 0, sizeof(int64_t), s) == cudaSuccess ? MT_OK : MT_ERR_CUDA;
+  MT_REQUIRE(xy && depth && faces && workspace);
+  MT_REQUIRE((reinterpret_cast<uintptr_t>(xy) & 7) == 0);  // positions are read as float2
+  MT_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0);
+  if (workspace_bytes < mt_bound_and_generate_keys_workspace_bytes(items)) return MT_ERR_WORKSPACE_TOO_SMALL;
+  const int64_t chunks = fused_chunks(items);
+  MT_REQUIRE(chunks < (int64_t)0x7fffffff);
+  ChunkRecords rec;
+  chunk_records(items, static_cast<char*>(workspace), &rec);
+  const FusedArgs a{xy, depth, V, faces, F, num_faces, B, tile_h, tile_w, rows, cols, cameras, near_plane};
+  chunk_bounds_kernel<<<(unsigned)chunks, kFusedThreads, 0, s>>>(a, rec);
+  MT_CHECK_LAUNCH();
+  if (chunks > kOneCtaChunks) {
+    const int rc = mt_exclusive_scan_i64(rec.keys, chunks + 1, rec.scan, rec.scan_bytes, stream);
+    if (rc != MT_OK) return rc;
+    if (cudaMemcpyAsync(out_num_keys, rec.keys + chunks, sizeof(int64_t), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+      return MT_ERR_CUDA;
+    return MT_OK;
+  }
+  chunk_scan_kernel<<<1, kChunkScanThreads, 0, s>>>(rec.keys, chunks, out_num_keys);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
+}
+
+int mt_write_bounded_keys(int64_t F, const int32_t* shell_face_boundaries, int32_t S, int32_t B, int32_t cols,
+                          const int64_t* cameras, const int32_t* layout, int64_t K, int64_t* out_keys,
+                          int32_t* out_triangles, void* workspace, size_t workspace_bytes, mt_stream_t stream) {
+  MT_REQUIRE(F >= 0 && B >= 0 && S >= 0 && K >= 0 && cols >= 0 && layout);
+  KeyLayout L{layout[0], layout[1], layout[2], layout[3], layout[4], layout[5], layout[6]};
+  MT_REQUIRE(layout_ok(L));
+  const int64_t items = (int64_t)B * F;
+  if (items == 0 || K == 0) return MT_OK;
+  MT_REQUIRE(out_keys && out_triangles && workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0);
+  MT_REQUIRE(S == 0 || shell_face_boundaries);
+  if (workspace_bytes < mt_bound_and_generate_keys_workspace_bytes(items)) return MT_ERR_WORKSPACE_TOO_SMALL;
+  const int64_t chunks = fused_chunks(items);
+  MT_REQUIRE(chunks < (int64_t)0x7fffffff);
+  ChunkRecords rec;
+  chunk_records(items, static_cast<char*>(workspace), &rec);
+  FusedArgs a{};
+  a.F = F;
+  a.B = B;
+  a.cols = cols;
+  a.cameras = cameras;
+  chunk_keys_kernel<<<(unsigned)chunks, kFusedThreads, 0, as_stream(stream)>>>(
+      a, rec, shell_face_boundaries, S, L, K, reinterpret_cast<uint64_t*>(out_keys), out_triangles);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
 }
 
 int mt_bound_and_generate_keys(const float* xy, const float* depth, int64_t V, const int32_t* faces, int64_t F,
@@ -707,36 +807,14 @@ int mt_bound_and_generate_keys(const float* xy, const float* depth, int64_t V, c
                                int32_t* out_triangles, int64_t* out_num_keys, void* workspace, size_t workspace_bytes,
                                mt_stream_t stream) {
   MT_REQUIRE(V >= 0 && F >= 0 && B >= 0 && S >= 0 && K >= 0 && layout);
-  MT_REQUIRE(tile_h > 0 && tile_w > 0 && rows >= 0 && cols >= 0);
   KeyLayout L{layout[0], layout[1], layout[2], layout[3], layout[4], layout[5], layout[6]};
   MT_REQUIRE(layout_ok(L));
-  MT_REQUIRE(out_num_keys);
-  const cudaStream_t s = as_stream(stream);
-  const int64_t items = (int64_t)B * F;
-  if (items == 0)
-    return cudaMemsetAsync(out_num_keys, 0, sizeof(int64_t), s) == cudaSuccess ? MT_OK : MT_ERR_CUDA;
-  MT_REQUIRE(xy && depth && faces && workspace);
-  MT_REQUIRE((reinterpret_cast<uintptr_t>(xy) & 7) == 0);  // positions are read as float2
-  MT_REQUIRE(K == 0 || (out_keys && out_triangles));
-  MT_REQUIRE(S == 0 || shell_face_boundaries);
-  if (workspace_bytes < mt_bound_and_generate_keys_workspace_bytes(items)) return MT_ERR_WORKSPACE_TOO_SMALL;
-  const int64_t chunks = fused_chunks(items);
-  MT_REQUIRE(chunks < (int64_t)0x7fffffff);
-  FusedArgs a{xy, depth, V, faces, F, num_faces, B, tile_h, tile_w, rows, cols, cameras, near_plane, kFusedSubTile};
-  MT_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0);
-  char* base = static_cast<char*>(workspace);
-  int64_t* counts = reinterpret_cast<int64_t*>(base + kFusedHeader);
-  int4* rect = reinterpret_cast<int4*>(base + kFusedHeader + round256((size_t)chunks * sizeof(int64_t)));
-  float* key_depth = reinterpret_cast<float*>(reinterpret_cast<char*>(rect) + round256((size_t)items * sizeof(int4)));
-  chunk_bounds_kernel<<<(unsigned)chunks, kFusedThreads, 0, s>>>(a, rect, key_depth, counts);
-  MT_CHECK_LAUNCH();
-  chunk_scan_kernel<<<1, kChunkScanThreads, 0, s>>>(counts, chunks, out_num_keys);
-  MT_CHECK_LAUNCH();
-  chunk_keys_kernel<<<(unsigned)chunks, kFusedThreads, 0, s>>>(a, rect, key_depth, counts, shell_face_boundaries, S,
-                                                               L, K, reinterpret_cast<uint64_t*>(out_keys),
-                                                               out_triangles);
-  MT_CHECK_LAUNCH();
-  return MT_OK;
+  MT_REQUIRE((int64_t)B * F == 0 || ((K == 0 || (out_keys && out_triangles)) && (S == 0 || shell_face_boundaries)));
+  const int rc = mt_bound_keys(xy, depth, V, faces, F, num_faces, B, tile_h, tile_w, rows, cols, cameras, near_plane,
+                               out_num_keys, workspace, workspace_bytes, stream);
+  if (rc != MT_OK) return rc;
+  return mt_write_bounded_keys(F, shell_face_boundaries, S, B, cols, cameras, layout, K, out_keys, out_triangles,
+                               workspace, workspace_bytes, stream);
 }
 
 int mt_delineate_tiles(const int64_t* sorted_keys, int64_t K, const int64_t* num_keys, const int32_t* layout,

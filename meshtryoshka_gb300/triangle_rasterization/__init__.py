@@ -376,14 +376,36 @@ def bound_and_generate_keys(vertices: Tensor, depths: Tensor, faces: Tensor, she
 
 def _keys(positions, depths, faces, shell_face_boundaries, grid, near_plane, num_faces, key_defines,
           key_capacity) -> PairedKeys:
-    """Keys of a render call: one fused kernel when the call has a key
-    capacity, else the reference's bound_triangles -> generate_keys chain."""
+    """Keys of a render call, equal to the chain bound_triangles ->
+    generate_keys without its per-item bounds and offsets; without a key
+    capacity the key count is read back between the two halves."""
     if key_capacity is not None:
         return bound_and_generate_keys(positions, depths, faces, shell_face_boundaries, grid, near_plane,
                                        key_defines, key_capacity, num_faces)
-    bounds = bound_triangles(positions, depths, faces, grid, near_plane, num_faces)
-    return generate_keys(depths, faces, shell_face_boundaries, bounds.tile_minima, bounds.tile_maxima,
-                         bounds.num_tiles_overlapped, grid, key_defines)
+    with annotate("bound_and_generate_keys"):
+        assert near_plane >= 0
+        vertices, depths, faces, sfb = _f32(positions), _f32(depths), _i32(faces), _i32(shell_face_boundaries)
+        device = nt.require_cuda(vertices, depths, faces)
+        c, v, _ = vertices.shape
+        f = faces.shape[0]
+        rows, cols = grid.grid_shape
+        nf = _i32(num_faces) if num_faces is not None else None
+        table = _camera_table(grid, device)
+        _check_key_budget(grid, key_defines)
+        layout = _layout(key_defines)
+        need = int(nt.library().mt_bound_and_generate_keys_workspace_bytes(c * f))
+        # Not the library workspace: other calls may come between the halves.
+        records = torch.empty((need,), dtype=torch.uint8, device=device)
+        count = torch.empty((), dtype=torch.int64, device=device)
+        nt.call("mt_bound_keys", nt.ptr(vertices), nt.ptr(depths), v, nt.ptr(faces), f, nt.ptr(nf), c,
+                grid.tile_shape[0], grid.tile_shape[1], rows, cols, nt.ptr(table), float(near_plane), count.data_ptr(),
+                records.data_ptr(), need, nt.stream(device))
+        num_keys = int(count.item())
+        keys = torch.empty(num_keys, dtype=torch.int64, device=device)
+        tri = torch.empty(num_keys, dtype=torch.int32, device=device)
+        nt.call("mt_write_bounded_keys", f, nt.ptr(sfb), sfb.shape[0], c, cols, nt.ptr(table), layout, num_keys,
+                nt.ptr(keys), nt.ptr(tri), records.data_ptr(), need, nt.stream(device))
+        return PairedKeys(keys, tri, None)
 
 
 @annotate("sort_keys")
@@ -976,10 +998,8 @@ def rasterize(vertices, faces, shell_face_boundaries, extrinsics, intrinsics, im
     key_defines = create_key_defines(("camera", num_camera_bits), ("shell", num_shell_bits),
                                      ("tile", num_tile_bits), ("depth", 32))
     positions, depths = project_vertices(vertices, extrinsics, intrinsics)
-    bounds = bound_triangles(positions, depths, faces, grid, near_plane)
-    paired = generate_keys(depths, faces, shell_face_boundaries, bounds.tile_minima, bounds.tile_maxima,
-                           bounds.num_tiles_overlapped, grid, key_defines)
-    del bounds, depths
+    paired = _keys(positions, depths, faces, shell_face_boundaries, grid, near_plane, None, key_defines, None)
+    del depths
     paired, tile_boundaries = _sort_and_delineate(paired, grid, key_defines, True)
     return intersect(positions, faces, paired.triangle_indices, tile_boundaries, grid, key_defines)
 
