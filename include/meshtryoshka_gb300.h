@@ -127,6 +127,10 @@ MT_API int64_t mt_exclusive_scan_i32_static_max_elements(void);
 MT_API int mt_compute_vertex_occupancy(const int32_t* occupancy, int32_t I, int32_t J,
                                 int32_t KP, int32_t* vertex_occupancy,
                                 int32_t* vertex_counts, mt_stream_t stream);
+/* With mt_count_occupancy's voxel_counts (unless NULL) in the same pass. */
+MT_API int mt_count_grid(const int32_t* occupancy, int32_t I, int32_t J, int32_t KP,
+                         int32_t* vertex_occupancy, int32_t* vertex_counts,
+                         int32_t* voxel_counts, mt_stream_t stream);
 
 /* triangle_extraction/count_occupancy.slang:3-20 (+ count_occupancy.py:30).
  * voxel_counts: (I+1)(J+1)(KP+1)+1 entries; popcount of occupied words,

@@ -522,7 +522,7 @@ int mt_upscale_occupancy(const int32_t* occupancy, const int32_t* mask, int32_t 
              (uint64_t)(KP2 + 1) * 32ull * (uint64_t)KP * 32ull <= 0xffffffffull);
   MT_REQUIRE(occupancy && out);
   const int64_t total = (int64_t)I2 * J2 * KP2;
-  upscale_occupancy_kernel<<<grid_stride_blocks(total, kThreads), kThreads, 0, as_stream(stream)>>>(
+  upscale_occupancy_kernel<<<grid_stride_blocks(total, kThreads, 128), kThreads, 0, as_stream(stream)>>>(
       occupancy, mask, (uint32_t)I, (uint32_t)J, (uint32_t)KP, (uint32_t)I2, (uint32_t)J2, (uint32_t)KP2, out);
   MT_CHECK_LAUNCH();
   return MT_OK;

@@ -206,13 +206,18 @@ def extract_voxels(occupancy: Tensor) -> Voxels:
     occupancy = _i32(occupancy, "occupancy")
     i, j, kp = occupancy.shape
     logging.debug(f"Extracting voxels for grid with shape ({i}, {j}, {kp * 32}).")
-    vertex_occupancy, vertex_counts = compute_vertex_occupancy(occupancy)
-    voxel_counts = count_occupancy(occupancy)
+    # compute_vertex_occupancy and count_occupancy in one pass.
+    device = nt.require_cuda(occupancy)
+    shape = (i + 1, j + 1, kp + 1)
+    kw = dict(dtype=torch.int32, device=device)
+    vertex_occupancy = torch.empty(shape, **kw)
+    vertex_counts, voxel_counts = (torch.empty((vertex_occupancy.numel() + 1,), **kw) for _ in range(2))
+    nt.call("mt_count_grid", nt.ptr(occupancy), i, j, kp, vertex_occupancy.data_ptr(), vertex_counts.data_ptr(),
+            voxel_counts.data_ptr(), nt.stream(device))
     compute_exclusive_cumsum(vertex_counts)
     compute_exclusive_cumsum(voxel_counts)
     totals = torch.stack((vertex_counts[-1], voxel_counts[-1])).cpu()
     num_vertices, num_voxels = int(totals[0]), int(totals[1])
-    shape = vertex_occupancy.shape
     return create_voxels(
         occupancy,
         voxel_counts[:-1].view(shape),
