@@ -1356,23 +1356,34 @@ __global__ void count_faces_kernel(const float* __restrict__ sdf, const int32_t*
 // Writes only faces below F and searches only vertices below V (the
 // buffers' capacities); with consistent offsets neither bound is reached.
 //
-// Work is dealt by face slot: a warp reads 32 consecutive (shell, voxel)
-// items (shell-major, the order of the slot offsets) in one coalesced load;
-// their slots are contiguous, so lane r takes the r-th slot of the span (its
-// item by a shuffle search over the warp's running edge counts) and every
-// lane resolves one edge: full lanes, and consecutive lanes write
-// consecutive face corners. The case tables sit in shared memory, as lanes
-// read different cases.
-__global__ void __launch_bounds__(256)
+// Work is dealt by face slot: a CTA reads kFaceItems consecutive (shell,
+// voxel) items (shell-major, the order of the slot offsets), marks each slot of
+// theirs with its item in shared memory (at most 15 to an item; they are
+// contiguous) and gives the slots to its threads in turn: full lanes, and
+// consecutive lanes write consecutive face corners. An entry's up to three
+// vertices' types are read side by side. The case tables sit in shared memory,
+// as lanes read different cases. Dealt by warps of 32 items (38 slots, two
+// rounds of lanes for them; the item by a search over shuffles, the types one
+// after another, a 64-bit division by three) 401 us at 512^3, 8 shells
+// (15 M faces), 870 at 16 shells and 24 M, 43 at 256^3; now 409, 829 and 36: what
+// is left is the chain neighbour -> offsets -> types of scattered reads.
+constexpr int kFaceItems = 256;
+
+__global__ void __launch_bounds__(kFaceItems)
     create_faces_kernel(const int32_t* __restrict__ neighbors, const int32_t* __restrict__ indices, int64_t Nv,
                         int64_t G, int64_t V, const int32_t* __restrict__ voff, const uint8_t* __restrict__ types,
                         const uint8_t* __restrict__ codes, int S, const int32_t* __restrict__ foff, int64_t F,
                         int32_t* __restrict__ faces, int32_t* __restrict__ voxel_indices) {
+  constexpr int kWarps = kFaceItems / 32;
   __shared__ uint64_t s_edges[256];
   __shared__ uint8_t s_count[256];
   __shared__ int8_t s_owner[12];
   __shared__ uint8_t s_axis[12];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
+  __shared__ uint8_t s_code[kFaceItems];
+  __shared__ int s_first[kFaceItems];   // an item's first slot in the CTA's
+  __shared__ int s_warp[kWarps];
+  __shared__ uint8_t s_item[kFaceItems * 16];  // item of each slot
+  for (int i = threadIdx.x; i < 256; i += kFaceItems) {
     s_edges[i] = c_mc_edges[i];
     s_count[i] = c_mc_count[i];
   }
@@ -1380,63 +1391,59 @@ __global__ void __launch_bounds__(256)
     s_owner[threadIdx.x] = c_mc_owner[threadIdx.x];
     s_axis[threadIdx.x] = c_mc_axis[threadIdx.x];
   }
-  __syncthreads();
   const int64_t total = (int64_t)S * Nv;
-  const int lane = threadIdx.x & 31;
-  const int64_t first_warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = first_warp * 32; base < total; base += warps * 32) {
-    const int64_t mine = base + lane;
-    const uint32_t code = mine < total ? (uint32_t)codes[mine] : 0u;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t step = (int64_t)gridDim.x * kFaceItems;
+  int64_t base = blockIdx.x * (int64_t)kFaceItems;
+  uint32_t next = base + threadIdx.x < total ? (uint32_t)codes[base + threadIdx.x] : 0u;
+  __syncthreads();
+  for (; base < total; base += step) {
+    const uint32_t code = next;
+    const int64_t ahead = base + step + threadIdx.x;
+    next = ahead < total ? (uint32_t)codes[ahead] : 0u;
     const int n = s_count[code];
-    int incl = n;  // inclusive scan of the edge counts over the warp
+    const int incl = warp_inclusive_sum(n);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();  // also: the last step's slots are done
+    int before = incl - n, span = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += u;
+    for (int w = 0; w < kWarps; ++w) {
+      before += w < warp ? s_warp[w] : 0;
+      span += s_warp[w];
     }
-    const int span = __shfl_sync(0xffffffffu, incl, 31);
+    s_code[threadIdx.x] = (uint8_t)code;
+    s_first[threadIdx.x] = before;
+    for (int k = 0; k < n; ++k) s_item[before + k] = (uint8_t)threadIdx.x;
+    __syncthreads();
     if (span == 0) continue;
     const int64_t first_slot = __ldg(foff + base);
-    const int64_t s_base = base / Nv;  // shell of the warp's first item (one division per warp step)
-    for (int start = 0; start < span; start += 32) {
-      const int r = start + lane;
-      int src = 0;  // item holding slot r: smallest src with incl[src] > r
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int u = __shfl_sync(0xffffffffu, incl, src + step - 1);
-        if (u <= r) src += step;
-      }
-      const uint32_t c = __shfl_sync(0xffffffffu, code, src);
-      const int before = __shfl_sync(0xffffffffu, incl - n, src);
-      if (r >= span) continue;
-      const int e = r - before;
-      const int64_t item = base + src;
-      int s = (int)s_base;
-      int64_t v = item - s_base * Nv;
-      while (v >= Nv) {  // at most ceil(32 / Nv) steps
+    const int64_t first_shell = base / Nv;
+    const int64_t first_voxel = base - first_shell * Nv;
+    for (int r = threadIdx.x; r < span; r += kFaceItems) {
+      const int item = s_item[r];
+      int64_t v = first_voxel + item;
+      int64_t row = first_shell * G;  // of the shell's vertex offsets
+      while (v >= Nv) {  // at most kFaceItems / Nv steps
         v -= Nv;
-        ++s;
+        row += G;
       }
-      const int eid = (int)((s_edges[c] >> (4 * e)) & 15u);
+      const int eid = (int)((s_edges[s_code[item]] >> (4 * (r - s_first[item]))) & 15u);
       const int owner = s_owner[eid];
-      const uint8_t axis = s_axis[eid];
+      const uint32_t axis = s_axis[eid];
       const int64_t nb = (owner < 0) ? v : (int64_t)__ldg(neighbors + (int64_t)owner * Nv + v);
-      const int64_t vo = (int64_t)s * G + nb;
-      const int32_t vstart = __ldg(voff + vo);
-      const int32_t count = __ldg(voff + vo + 1) - vstart;
-      int32_t target = -1;
-      for (int q = 0; q < count; ++q) {
-        if ((int64_t)vstart + q >= V) break;
-        if (types[vstart + q] == axis) {
-          target = vstart + q;
-          break;
-        }
-      }
+      const int32_t vstart = __ldg(voff + row + nb);
+      const int32_t count = __ldg(voff + row + nb + 1) - vstart;
+      // The entry's first vertex of the edge's axis (there is one); vertices
+      // past the capacity were not written.
+      uint32_t type[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        type[q] = q < count && (int64_t)vstart + q < V ? (uint32_t)__ldg(types + vstart + q) : 255u;
+      const int32_t target = type[0] == axis ? vstart : type[1] == axis ? vstart + 1 : type[2] == axis ? vstart + 2 : -1;
       const int64_t slot = first_slot + r;
-      const int64_t tri = slot / 3;
+      const int64_t tri = (slot >> 32) == 0 ? (int64_t)((uint32_t)slot / 3u) : slot / 3;
       if (tri >= F) continue;
-      const int corner = 2 - (int)(slot % 3);
+      const int corner = 2 - (int)(slot - 3 * tri);
       faces[tri * 3 + corner] = target;
       if (corner == 0) voxel_indices[tri] = __ldg(indices + v);
     }
