@@ -453,8 +453,27 @@ __device__ __forceinline__ uint32_t key_mask(const CompositeArgs& a, int warps, 
 // Keys past num_keys (a device value; all K when NULL) get no mask: no tile
 // range reaches them. Each thread takes two keys and issues their dependent
 // loads (key and triangle, face, projected corners) side by side.
+//
+// Runs before the launch's other kernels, so it also clears their counters
+// (`clear`): a fill of a few bytes costs a launch of its own.
+struct ClearedCounters {
+  unsigned long long* work;  // work items claimed
+  unsigned long long* hits;  // hit-bit batches reserved, or NULL
+  int32_t* order;            // tile order's header (kOrderHeader words), or NULL
+};
+constexpr int kOrderBuckets = 256;
+constexpr int kOrderHeader = 2 * kOrderBuckets;
+
 __global__ void warp_mask_kernel(CompositeArgs a, int64_t K_capacity, const int64_t* __restrict__ num_keys,
-                                 uint32_t* __restrict__ masks) {
+                                 uint32_t* __restrict__ masks, ClearedCounters clear) {
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+      *clear.work = 0;
+      if (clear.hits) *clear.hits = 0;
+    }
+    if (clear.order)
+      for (int i = threadIdx.x; i < kOrderHeader; i += blockDim.x) clear.order[i] = 0;
+  }
   const int warps = (a.tile_h * a.tile_w + 31) / 32;
   const int64_t K = num_keys ? min(max(*num_keys, (int64_t)0), K_capacity) : K_capacity;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -922,9 +941,6 @@ __device__ __forceinline__ int64_t next_item(unsigned long long* counter, int la
 // Buffer (int32): [0, 256) bucket sizes, [256, 512) bucket cursors, then one
 // global tile index per tile.
 // ---------------------------------------------------------------------------
-constexpr int kOrderBuckets = 256;
-constexpr int kOrderHeader = 2 * kOrderBuckets;
-
 __device__ __forceinline__ int order_bucket(const CompositeArgs& a, int64_t gt) {
   int64_t bi = gt;  // index of the tile's range in `bounds`
   if (a.cameras != nullptr) {
@@ -1994,15 +2010,18 @@ int mt_intersect_and_composite_forward(const float* xy, const float* colors, con
   HitStore hs;
   rc = make_hit_store(a, hit_bits, hit_bits_bytes, hs);
   if (rc != MT_OK) return rc;
-  if (hs.next && cudaMemsetAsync(hs.next, 0, 8, s) != cudaSuccess) return MT_ERR_CUDA;
+  MT_REQUIRE(tile_order == nullptr || tile_order_bytes >= mt_composite_tile_order_bytes(a.total_tiles));
   if (K > 0) {
-    warp_mask_kernel<<<grid_stride_blocks(K, 256), 256, 0, s>>>(a, K, num_keys, warp_masks);
+    const ClearedCounters clear{reinterpret_cast<unsigned long long*>(work_counter), hs.next, tile_order};
+    warp_mask_kernel<<<grid_stride_blocks(K, 256), 256, 0, s>>>(a, K, num_keys, warp_masks, clear);
     MT_CHECK_LAUNCH();
+  } else if ((hs.next && cudaMemsetAsync(hs.next, 0, 8, s) != cudaSuccess) ||
+             cudaMemsetAsync(work_counter, 0, sizeof(uint64_t), s) != cudaSuccess ||
+             (tile_order &&
+              cudaMemsetAsync(tile_order, 0, kOrderHeader * sizeof(int32_t), s) != cudaSuccess)) {
+    return MT_ERR_CUDA;
   }
-  if (cudaMemsetAsync(work_counter, 0, sizeof(uint64_t), s) != cudaSuccess) return MT_ERR_CUDA;
   if (tile_order) {
-    MT_REQUIRE(tile_order_bytes >= mt_composite_tile_order_bytes(a.total_tiles));
-    if (cudaMemsetAsync(tile_order, 0, kOrderHeader * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
     const unsigned blocks = grid_stride_blocks(a.total_tiles, 256, 1);
     order_histogram_kernel<<<blocks, 256, 0, s>>>(a, tile_order);
     MT_CHECK_LAUNCH();

@@ -419,6 +419,7 @@ struct TileSortWorkspace {
   uint64_t* tmp;     // K
   void* scan_ws;
   size_t scan_bytes;
+  size_t cleared;    // bytes from `counts` that start at zero
 };
 
 size_t tile_sort_bytes(int64_t K, int64_t nbins, TileSortWorkspace* w, char* base) {
@@ -428,10 +429,12 @@ size_t tile_sort_bytes(int64_t K, int64_t nbins, TileSortWorkspace* w, char* bas
     off += align256(bytes);
     return p;
   };
-  char* counts = take((size_t)(nbins + 1) * sizeof(int32_t));
-  char* cursors = take((size_t)nbins * sizeof(int32_t));
+  // Cleared by one fill: counts, cursors and list sizes are adjacent.
+  const size_t cleared = (size_t)(2 * nbins + 1 + kSizes) * sizeof(int32_t);
+  char* counts = take(cleared);
+  char* cursors = counts ? counts + (size_t)(nbins + 1) * sizeof(int32_t) : nullptr;
+  char* list_sizes = counts ? cursors + (size_t)nbins * sizeof(int32_t) : nullptr;
   char* lists = take((size_t)kTiers * nbins * sizeof(int2));
-  char* list_sizes = take(kSizes * sizeof(int32_t));
   char* chunks = take(((size_t)K / (kChunk / 2) + 1) * sizeof(int4));
   char* tmp = take((size_t)K * sizeof(uint64_t));
   const size_t scan_bytes = mt_scan_workspace_bytes(nbins + 1);
@@ -445,6 +448,7 @@ size_t tile_sort_bytes(int64_t K, int64_t nbins, TileSortWorkspace* w, char* bas
     w->chunks = reinterpret_cast<int4*>(chunks);
     w->scan_ws = scan;
     w->scan_bytes = scan_bytes;
+    w->cleared = cleared;
   }
   return off;
 }
@@ -539,7 +543,9 @@ int mt_sort_keys_by_tile(const int64_t* keys, const int32_t* triangles, int64_t 
   cudaStream_t s = as_stream(stream);
   if (nbins > 0) {
     MT_REQUIRE(boundaries);
-    if (cudaMemsetAsync(boundaries, 0, (size_t)nbins * 2 * sizeof(int64_t), s) != cudaSuccess) return MT_ERR_CUDA;
+    // With keys, bin_bounds_kernel writes every range.
+    if (K == 0 && cudaMemsetAsync(boundaries, 0, (size_t)nbins * 2 * sizeof(int64_t), s) != cudaSuccess)
+      return MT_ERR_CUDA;
   }
   if (K == 0 || nbins == 0) return MT_OK;
   MT_REQUIRE(keys && triangles && sorted_keys && sorted_triangles && workspace);
@@ -551,9 +557,7 @@ int mt_sort_keys_by_tile(const int64_t* keys, const int32_t* triangles, int64_t 
   const int idx_bits = K > 1 ? bit_length((uint64_t)(K - 1)) : 1;
   const uint64_t low_mask_host = (1ull << low_bits) - 1ull;
   const uint64_t idx_mask = (1ull << idx_bits) - 1ull;
-  if (cudaMemsetAsync(w.counts, 0, (size_t)(nbins + 1) * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
-  if (cudaMemsetAsync(w.cursors, 0, (size_t)nbins * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
-  if (cudaMemsetAsync(w.list_sizes, 0, kSizes * sizeof(int32_t), s) != cudaSuccess) return MT_ERR_CUDA;
+  if (cudaMemsetAsync(w.counts, 0, w.cleared, s) != cudaSuccess) return MT_ERR_CUDA;
   const uint64_t* k64 = reinterpret_cast<const uint64_t*>(keys);
   // A key outside every bin (never made by mt_generate_keys) is recorded in
   // the workspace status word; it is left out of the output.
