@@ -556,7 +556,8 @@ int mt_intersect(const float* xy, int64_t V, const int32_t* faces, const int32_t
   const size_t smem = intersect_smem(bs);
   auto launch = [&](auto kernel_c) -> int {
     constexpr auto kKernel = decltype(kernel_c)::value;
-    if (set_smem<kKernel>(smem) != MT_OK) return MT_ERR_CUDA;
+    // The list ranges' static shared memory counts towards the same limit.
+    if (set_smem<kKernel>(smem + 1024) != MT_OK) return MT_ERR_CUDA;
     // As many CTAs as fit on the device at once.
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kKernel, bs, smem) != cudaSuccess) return MT_ERR_CUDA;

@@ -10,12 +10,14 @@ import torch
 from meshtryoshka_gb300 import subdivision
 from meshtryoshka_gb300 import triangle_extraction as te
 
+from oracle import oracle
+
 from . import semantics
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("c", [1, 4, 5, 9, 16])
+@pytest.mark.parametrize("c", [1, 4, 5, 9, 16, 18, 33])
 @pytest.mark.parametrize("density,tol,more", [(0.01, 1e-6, 0), (0.2, 0.08, 0), (1.0, 0.08, 7)])
 def test_canonical_rows_in_place(cuda_device, c, density, tol, more):
     rng = np.random.default_rng(c)
@@ -35,6 +37,26 @@ def test_canonical_rows_in_place(cuda_device, c, density, tol, more):
     assert got.signed_distances.numel() > 0
     for a, b in zip(got, want):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+@pytest.mark.parametrize("c", [1, 5, 16, 18])
+def test_infinities_and_nan_stay_where_they_are(cuda_device, c):
+    """Absent corners add nothing, not even a zero times an infinity."""
+    rng = np.random.default_rng(c)
+    occ = semantics.pack(rng.random((7, 9, 64)) < 0.3)
+    vox = oracle.extract_voxels(occ)
+    v = vox.vertices.shape[0]
+    sdf = rng.normal(size=v).astype(np.float32)
+    sh = rng.normal(size=(c, v, 3)).astype(np.float32)
+    for value in (np.inf, -np.inf, np.nan, 3e38):
+        sh.reshape(-1)[rng.integers(0, sh.size, 40)] = value
+    everything = np.full_like(occ, -1)
+    with np.errstate(all="ignore"):
+        want = oracle.upscale_parameters(sdf, sh, occ, everything, (12, 11, 96))
+    got = te.upscale_parameters(*(torch.from_numpy(x).to(cuda_device) for x in (sdf, sh, occ, everything)), (12, 11, 96))
+    np.testing.assert_array_equal(got.signed_distances.cpu().numpy(), want[0])
+    np.testing.assert_array_equal(got.spherical_harmonics.cpu().numpy(), want[1])
+    assert np.isfinite(want[1]).any() and not np.isfinite(want[1]).all()
 
 
 def test_too_few_rows_are_refused(cuda_device):

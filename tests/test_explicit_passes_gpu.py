@@ -17,7 +17,7 @@ from .test_rasterization_gpu import _adversarial_triangles
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("tile", [(16, 16), (8, 4), (10, 10), (1, 33), (32, 32)])
+@pytest.mark.parametrize("tile", [(16, 16), (8, 4), (10, 10), (1, 33), (20, 29), (32, 32)])
 @pytest.mark.parametrize("kind", ["mixed", "fine", "large"])
 def test_first_hits_match_oracle(cuda_device, tile, kind):
     rng = np.random.default_rng(sum(tile))
