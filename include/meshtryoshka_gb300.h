@@ -239,6 +239,13 @@ MT_API int mt_iota_i32(int64_t n, int32_t* values, mt_stream_t stream);
 MT_API int mt_index_sorted_runs(const int64_t* sorted_keys, const int32_t* order,
                          int64_t n, int32_t* out, mt_stream_t stream);
 
+/* out[v] = the index of the first key equal to keys[v] (index_vertices.py:6-51
+ * after its keys), by a hash table in workspace (16-byte aligned, at least
+ * mt_index_keys_workspace_bytes(n) bytes). n < 2^31. */
+MT_API size_t mt_index_keys_workspace_bytes(int64_t n);
+MT_API int mt_index_keys(const int64_t* keys, int64_t n, int32_t* out, void* workspace,
+                         size_t workspace_bytes, mt_stream_t stream);
+
 /* ------------------------------------------------------------------------
  * Per-step marching cubes (triangle_extraction/__init__.py:75-157
  * tessellate_voxels). G = voxels + subvoxels, Nv = voxels, S = level sets,

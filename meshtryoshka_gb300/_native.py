@@ -57,6 +57,8 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_pack_point_keys": (I32, [P, I64, I32, P, P, P]),
     "mt_iota_i32": (I32, [I64, P, P]),
     "mt_index_sorted_runs": (I32, [P, P, I64, P, P]),
+    "mt_index_keys_workspace_bytes": (c_size_t, [I64]),
+    "mt_index_keys": (I32, [P, I64, P, P, c_size_t, P]),
     "mt_count_triangle_vertices": (I32, [P, P, I64, P, I32, P, P]),
     "mt_create_triangle_vertices": (
         I32,
@@ -183,6 +185,7 @@ KERNELS_PER_CALL = {
     "mt_sort_keys_by_tile": 9,  # count, scan, tile ranges, scatter, tiny / medium / small / large bin sorts, placing
     "mt_bound_and_generate_keys": 3,  # rectangles + chunk counts, chunk scan, keys
     "mt_bound_keys": 2,
+    "mt_index_keys": 2,  # claim, look up
     "mt_build_vertex_grad_list": 4,  # corner inverse, count, scan, fill
     "mt_grid_sh_colors_backward": 2,  # per-vertex SH gradients, per-grid-vertex sums
     "mt_grid_sh_colors_packed_backward": 2,

@@ -496,6 +496,67 @@ __global__ void run_heads_kernel(const int64_t* __restrict__ sorted_keys, const 
   }
 }
 
+// ---------------------------------------------------------------------------
+// First index of every key by an open-addressing table (linear probing, at most
+// half full, so a probe meets its key or an empty slot): each key claims a slot
+// and the slot keeps its least index; then every key looks its slot up. The
+// same result as the stable sort followed by run heads, which moves every key
+// eight times: 114 us for 424,000 points, this 30. Bound by the latency of
+// the table's scattered reads and atomics.
+//
+// Table: [slots] keys, then [slots + 1] indices, all bits set where empty; the
+// last index stands for the key whose bits are all set.
+// ---------------------------------------------------------------------------
+constexpr unsigned long long kEmptyKey = ~0ull;
+
+// MurmurHash3's 64-bit finalizer (Appleby).
+__device__ __forceinline__ uint64_t mix_key(uint64_t x) {
+  x ^= x >> 33;
+  x *= 0xff51afd7ed558ccdull;
+  x ^= x >> 33;
+  x *= 0xc4ceb9fe1a85ec53ull;
+  return x ^ (x >> 33);
+}
+
+__global__ void claim_keys_kernel(const int64_t* __restrict__ keys, int64_t n, unsigned long long* table,
+                                  uint32_t* first, uint64_t mask) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long key = (unsigned long long)__ldg(keys + v);
+    uint64_t slot = mask + 1;
+    if (key != kEmptyKey) {
+      slot = mix_key(key) & mask;
+      for (uint64_t probes = 0; probes <= mask; ++probes, slot = (slot + 1) & mask) {
+        // Read first: a key that many points share is claimed by few.
+        unsigned long long there = *(volatile unsigned long long*)(table + slot);
+        if (there == kEmptyKey) there = atomicCAS(table + slot, kEmptyKey, key);
+        if (there == kEmptyKey || there == key) break;
+      }
+    }
+    if (*(volatile uint32_t*)(first + slot) > (uint32_t)v) atomicMin(first + slot, (uint32_t)v);
+  }
+}
+
+__global__ void look_up_keys_kernel(const int64_t* __restrict__ keys, int64_t n,
+                                    const unsigned long long* __restrict__ table, const uint32_t* __restrict__ first,
+                                    uint64_t mask, int32_t* __restrict__ out) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long key = (unsigned long long)__ldg(keys + v);
+    uint64_t slot = mask + 1;
+    if (key != kEmptyKey) {
+      slot = mix_key(key) & mask;
+      for (uint64_t probes = 0; probes <= mask; ++probes, slot = (slot + 1) & mask)
+        if (__ldg(table + slot) == key) break;
+    }
+    out[v] = (int32_t)__ldg(first + slot);
+  }
+}
+
+int64_t key_slots(int64_t n) {
+  int64_t slots = 64;
+  while (slots < 2 * n) slots <<= 1;
+  return slots;
+}
+
 }  // namespace
 }  // namespace mt
 
@@ -624,6 +685,30 @@ int mt_iota_i32(int64_t n, int32_t* values, mt_stream_t stream) {
   if (n == 0) return MT_OK;
   MT_REQUIRE(values);
   iota_kernel<<<grid_stride_blocks(n, kThreads), kThreads, 0, as_stream(stream)>>>(n, values);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
+}
+
+size_t mt_index_keys_workspace_bytes(int64_t n) {
+  if (n <= 0) return 0;
+  return (size_t)key_slots(n) * 12 + 16;
+}
+
+int mt_index_keys(const int64_t* keys, int64_t n, int32_t* out, void* workspace, size_t workspace_bytes,
+                  mt_stream_t stream) {
+  MT_REQUIRE(n >= 0 && n <= 0x7fffffff);
+  if (n == 0) return MT_OK;
+  MT_REQUIRE(keys && out && workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0);
+  const size_t bytes = mt_index_keys_workspace_bytes(n);
+  if (workspace_bytes < bytes) return MT_ERR_WORKSPACE_TOO_SMALL;
+  const int64_t slots = key_slots(n);
+  unsigned long long* table = static_cast<unsigned long long*>(workspace);
+  uint32_t* first = reinterpret_cast<uint32_t*>(table + slots);
+  const cudaStream_t s = as_stream(stream);
+  if (cudaMemsetAsync(workspace, 0xff, bytes, s) != cudaSuccess) return MT_ERR_CUDA;
+  claim_keys_kernel<<<grid_stride_blocks(n, kThreads, 32), kThreads, 0, s>>>(keys, n, table, first, slots - 1);
+  MT_CHECK_LAUNCH();
+  look_up_keys_kernel<<<grid_stride_blocks(n, kThreads, 32), kThreads, 0, s>>>(keys, n, table, first, slots - 1, out);
   MT_CHECK_LAUNCH();
   return MT_OK;
 }

@@ -376,18 +376,14 @@ def get_occupancy_mesh(occupancy: Tensor, colors: Tensor) -> Mesh:
     return Mesh(vertices, triangle_colors)
 
 
-def _index_pairs(keys: Tensor, values: Tensor) -> Tensor:
-    """Stable sort of (key, original index), then every index mapped to the
-    first original index of its run of equal keys."""
+def _first_equal(keys: Tensor) -> Tensor:
+    """Every index mapped to the first index of an equal key."""
     device = keys.device
     n = keys.numel()
-    sorted_keys = torch.empty_like(keys)
-    order = torch.empty_like(values)
     out = torch.empty((n,), dtype=torch.int32, device=device)
-    ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_sort_pairs_workspace_bytes(n))
-    nt.call("mt_sort_pairs_i64_i32", keys.data_ptr(), values.data_ptr(), sorted_keys.data_ptr(), order.data_ptr(), n,
-            None, 0, 64, ws_ptr, ws_bytes, nt.stream(device))
-    nt.call("mt_index_sorted_runs", sorted_keys.data_ptr(), order.data_ptr(), n, out.data_ptr(), nt.stream(device))
+    need = int(nt.library().mt_index_keys_workspace_bytes(n))
+    table = torch.empty((need,), dtype=torch.uint8, device=device)
+    nt.call("mt_index_keys", keys.data_ptr(), n, out.data_ptr(), table.data_ptr(), need, nt.stream(device))
     return out
 
 
@@ -403,9 +399,7 @@ def index_keys(keys: Tensor) -> Tensor:
         return torch.empty((0,), dtype=torch.int32, device=device)
     if n > 2**31 - 1:
         raise ValueError("index_keys handles at most 2^31 - 1 keys")
-    values = torch.empty((n,), dtype=torch.int32, device=device)
-    nt.call("mt_iota_i32", n, values.data_ptr(), nt.stream(device))
-    return _index_pairs(keys, values)
+    return _first_equal(keys)
 
 
 def index_vertices(points: Tensor, tol: float = 1e-5) -> Tensor:
@@ -434,7 +428,7 @@ def index_vertices(points: Tensor, tol: float = 1e-5) -> Tensor:
     values = torch.empty((v,), dtype=torch.int32, device=device)
     nt.call("mt_pack_point_keys", quantized.data_ptr(), v, bits, keys.data_ptr(), values.data_ptr(),
             nt.stream(device))
-    return _index_pairs(keys, values)
+    return _first_equal(keys)
 
 
 # ---------------------------------------------------------------------------
