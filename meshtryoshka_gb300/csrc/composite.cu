@@ -704,12 +704,14 @@ __device__ __forceinline__ uint32_t edge_span(const TriGeom& g, const CullBox& b
   if (!box.rows) return kFullSpan;
   const RowEdges q = row_edges(g, bx, 7.0f);
   uint32_t span = 0u;
+  // Its own rows only: the lanes' triangles lie in different rows of the block,
+  // and a loop over the block's rows ran all four for every batch.
+  const int r0 = max((int)ceilf(fmaxf(box.y0 - by, -1.0f)), 0);
+  const int r1 = min((int)floorf(fminf(box.y1 - by, 4.0f)), 3);
 #pragma unroll 1  // rolled: the unrolled rows cost more in instruction-cache misses than they save
-  for (int r = 0; r < 4; ++r) {
-    const float y = by + (float)r;
-    if (!(y >= box.y0 && y <= box.y1)) continue;
+  for (int r = r0; r <= r1; ++r) {
     float xl, xu;
-    if (!row_columns(q, box, g.thr, y, xl, xu)) continue;
+    if (!row_columns(q, box, g.thr, by + (float)r, xl, xu)) continue;
     const int c0 = max((int)ceilf(fmaxf(xl - bx, -1.0f)), 0);
     const int c1 = min((int)floorf(fminf(xu - bx, 8.0f)), 7);
     if (c0 <= c1) span |= ((uint32_t)c0 | ((uint32_t)(c1 - c0 + 1) << 3)) << (8 * r);
