@@ -136,19 +136,13 @@ class Capacities:
         return Capacities(grow(stats["V"]), grow(stats["F"]), grow(stats["K"]))
 
 
-_AFFINE: dict = {}
-
-
 def uncontract_stand_in(vertices: Tensor) -> Tensor:
     """2 v - 1, the linear stand-in for the trainer's uncontract(), as one
-    elementwise kernel (-1 + v * 2: v * 2 is exact, so the value is that of
-    2.0 * v - 1.0)."""
-    key = str(vertices.device)
-    consts = _AFFINE.get(key)
-    if consts is None:
-        consts = (torch.tensor(-1.0, device=vertices.device), torch.tensor(2.0, device=vertices.device))
-        _AFFINE[key] = consts
-    return torch.addcmul(consts[0], vertices, consts[1])
+    elementwise kernel (-1 - (-2) v: the product is exact, so the value is that
+    of 2.0 * v - 1.0; with scalars it takes wide loads, where constants held
+    on the device made it a broadcast, 135 us instead of 58 for 18 M
+    vertices)."""
+    return torch.rsub(vertices, -1.0, alpha=-2.0)
 
 
 def forward_counted(w: Workload, caps: Capacities, gradient_mode: str | None = None,
