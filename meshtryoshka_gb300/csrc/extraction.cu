@@ -419,6 +419,23 @@ __device__ __forceinline__ float lerp_ref(float a, float b, float t) {
 // vertex from its two corners. Consecutive threads write consecutive
 // vertices of one row, so the [C, V, 3] output is written coalesced.
 // ---------------------------------------------------------------------------
+constexpr int kShellsPerChunk = 21;
+
+__device__ __forceinline__ uint64_t crossing_bits(const Corners4& c, const float* __restrict__ level_sets, int s0,
+                                                  int s1) {
+  uint64_t bits = 0;
+  for (int s = s0; s < s1; ++s) bits |= (uint64_t)crossing_mask(c, __ldg(level_sets + s)) << (3 * (s - s0));
+  return bits;
+}
+
+// One thread per entry: the crossings of its three edges with all shells (up
+// to kShellsPerChunk at a time) as a bit each, then a turn per shell. Where
+// vertices are few (1.4 to an entry at 512^3, 8 shells) a lane takes its own
+// shells: 206 us, with the warp's lanes taking every shell that one of them
+// crosses 284. Where they are many (2.2 at 16 shells) the lanes take them
+// together, to write neighbouring vertices: 535 us, each its own 656. A loop over
+// every (axis, shell) pair took 332 and 612, and 25 us at 256^3, 8 shells, now 15.
+template <bool kTogether>
 __global__ void create_vertices_kernel(const float* __restrict__ gv, const float* __restrict__ gsdf,
                                        const int32_t* __restrict__ lower, int64_t G,
                                        const float* __restrict__ level_sets, int S,
@@ -427,34 +444,47 @@ __global__ void create_vertices_kernel(const float* __restrict__ gv, const float
                                        int32_t* __restrict__ sources) {
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < G; g += (int64_t)gridDim.x * blockDim.x) {
     const Corners4 c = load_corners(gsdf, lower, G, g);
-    const int32_t i0 = __ldg(lower + g);
-    uint32_t any = 0;
-    for (int s = 0; s < S; ++s) any |= crossing_mask(c, __ldg(level_sets + s));
-    if (any == 0) continue;
-    const float v0x = __ldg(gv + 3 * (int64_t)i0), v0y = __ldg(gv + 3 * (int64_t)i0 + 1),
-                v0z = __ldg(gv + 3 * (int64_t)i0 + 2);
-    for (int a = 0; a < 3; ++a) {
-      if (!((any >> a) & 1u)) continue;
-      const int32_t i1 = c.idx[a];
-      const float d1 = c.d[a];
-      const float v1x = __ldg(gv + 3 * (int64_t)i1), v1y = __ldg(gv + 3 * (int64_t)i1 + 1),
-                  v1z = __ldg(gv + 3 * (int64_t)i1 + 2);
-      const uint32_t below_a = (1u << a) - 1u;
-      for (int s = 0; s < S; ++s) {
-        const float iso = __ldg(level_sets + s);
-        const uint32_t m = crossing_mask(c, iso);
-        if (!((m >> a) & 1u)) continue;
-        const int64_t vi = (int64_t)__ldg(voff + (int64_t)s * G + g) + __popc(m & below_a);
-        if (vi >= V) continue;  // beyond the caller's capacity (reported by the caller's count check)
-        const float t = mc_weight(c.d0, d1, iso);
-        out_v[3 * vi + 0] = lerp_ref(v0x, v1x, t);
-        out_v[3 * vi + 1] = lerp_ref(v0y, v1y, t);
-        out_v[3 * vi + 2] = lerp_ref(v0z, v1z, t);
-        out_sdf[vi] = lerp_ref(c.d0, d1, t);
-        out_type[vi] = (uint8_t)a;
-        sources[vi] = i0;
-        sources[V + vi] = i1;
-        sources[2 * V + vi] = __float_as_int(t);
+    for (int s0 = 0; s0 < S; s0 += kShellsPerChunk) {
+      const uint64_t crossings = crossing_bits(c, level_sets, s0, min(S, s0 + kShellsPerChunk));
+      // Shells that the entry crosses, or with kTogether some lane of the warp
+      // (bit 3 s).
+      uint64_t shells = (crossings | (crossings >> 1) | (crossings >> 2)) & 0x1249249249249249ull;
+      if constexpr (kTogether) {
+        const unsigned warp = __activemask();
+        shells = (uint64_t)__reduce_or_sync(warp, (uint32_t)(shells >> 32)) << 32 |
+                 __reduce_or_sync(warp, (uint32_t)shells);
+      }
+      if (shells == 0) continue;
+      const int32_t i0 = __ldg(lower + g);
+      float v0x = 0.f, v0y = 0.f, v0z = 0.f;
+      if (crossings != 0) {
+        v0x = __ldg(gv + 3 * (int64_t)i0);
+        v0y = __ldg(gv + 3 * (int64_t)i0 + 1);
+        v0z = __ldg(gv + 3 * (int64_t)i0 + 2);
+      }
+      for (; shells; shells &= shells - 1) {
+        const int at = __ffsll((long long)shells) - 1, sl = at / 3;
+        uint32_t m = (uint32_t)(crossings >> at) & 7u;
+        if (m == 0) continue;
+        int64_t vi = (int64_t)__ldg(voff + (int64_t)(s0 + sl) * G + g);
+        const float iso = __ldg(level_sets + s0 + sl);
+        for (; m; m &= m - 1, ++vi) {
+          if (vi >= V) break;  // beyond the caller's capacity (reported by the caller's count check)
+          const int a = __ffs(m) - 1;
+          const int32_t i1 = a == 0 ? c.idx[0] : a == 1 ? c.idx[1] : c.idx[2];
+          const float d1 = a == 0 ? c.d[0] : a == 1 ? c.d[1] : c.d[2];
+          const float v1x = __ldg(gv + 3 * (int64_t)i1), v1y = __ldg(gv + 3 * (int64_t)i1 + 1),
+                      v1z = __ldg(gv + 3 * (int64_t)i1 + 2);
+          const float t = mc_weight(c.d0, d1, iso);
+          out_v[3 * vi + 0] = lerp_ref(v0x, v1x, t);
+          out_v[3 * vi + 1] = lerp_ref(v0y, v1y, t);
+          out_v[3 * vi + 2] = lerp_ref(v0z, v1z, t);
+          out_sdf[vi] = lerp_ref(c.d0, d1, t);
+          out_type[vi] = (uint8_t)a;
+          sources[vi] = i0;
+          sources[V + vi] = i1;
+          sources[2 * V + vi] = __float_as_int(t);
+        }
       }
     }
   }
@@ -621,15 +651,6 @@ __global__ void invert_corners_kernel(const int32_t* __restrict__ lower, int64_t
     if (zero1) zero1[e] = 0u;
   }
   if (zero0 && blockIdx.x == 0 && threadIdx.x == 0) zero0[G] = 0;
-}
-
-constexpr int kShellsPerChunk = 21;
-
-__device__ __forceinline__ uint64_t crossing_bits(const Corners4& c, const float* __restrict__ level_sets, int s0,
-                                                  int s1) {
-  uint64_t bits = 0;
-  for (int s = s0; s < s1; ++s) bits |= (uint64_t)crossing_mask(c, __ldg(level_sets + s)) << (3 * (s - s0));
-  return bits;
 }
 
 // One contribution list of grid vertex x for the shells of one chunk: the
@@ -1774,9 +1795,13 @@ int mt_create_triangle_vertices(const float* grid_vertices, const float* grid_si
   if (G == 0 || S == 0 || V == 0) return MT_OK;
   MT_REQUIRE(grid_vertices && grid_signed_distances && lower_corners && level_sets && vertex_offsets && vertices &&
              signed_distances && vertex_types && vertex_sources);
-  create_vertices_kernel<<<grid_stride_blocks(G, 128), 128, 0, as_stream(stream)>>>(
-      grid_vertices, grid_signed_distances, lower_corners, G, level_sets, S, vertex_offsets, V, vertices,
-      signed_distances, vertex_types, vertex_sources);
+  auto launch = [&](auto together) {
+    create_vertices_kernel<decltype(together)::value><<<grid_stride_blocks(G, 128), 128, 0, as_stream(stream)>>>(
+        grid_vertices, grid_signed_distances, lower_corners, G, level_sets, S, vertex_offsets, V, vertices,
+        signed_distances, vertex_types, vertex_sources);
+  };
+  if (V > 2 * G) launch(std::true_type{});
+  else launch(std::false_type{});
   MT_CHECK_LAUNCH();
   if (spherical_harmonics == nullptr) return MT_OK;  // rows left to mt_grid_sh_colors
   MT_REQUIRE(grid_spherical_harmonics);
