@@ -895,7 +895,7 @@ __global__ void vertex_grads_from_list_kernel(const int32_t* __restrict__ offset
 // r of x's segment word; pass 2 writes the segment at x's scanned offset plus
 // the lengths of x's earlier segments. Each entry loads its own corners once
 // (a pass per grid vertex loads four entries' corners for each: 318 + 411 us
-// at 512^3, 8 shells; this 205 + 290).
+// at 512^3, 8 shells; this 126 + 221, a turn per crossed shell).
 // Counts and segment words start at zero (cleared by invert_corners_kernel).
 // ---------------------------------------------------------------------------
 template <bool kFill>
@@ -907,6 +907,8 @@ __global__ void entry_list_kernel(const float* __restrict__ gsdf, const int32_t*
     const Corners4 c = load_corners(gsdf, lower, G, e);
     const uint64_t bits = crossing_bits(c, level_sets, 0, S);
     if (bits == 0) continue;
+    // The shells that the entry crosses (bit 3 s), a turn each.
+    const uint64_t shells = (bits | (bits >> 1) | (bits >> 2)) & 0x1249249249249249ull;
     int64_t x[4];
     x[0] = __ldg(lower + e);
 #pragma unroll
@@ -917,9 +919,9 @@ __global__ void entry_list_kernel(const float* __restrict__ gsdf, const int32_t*
     if (!(owns[0] || owns[1] || owns[2] || owns[3])) continue;
     if (!kFill) {
       int n[4] = {0, 0, 0, 0};
-      for (int s = 0; s < S; ++s) {
-        const uint32_t m = (uint32_t)(bits >> (3 * s)) & 7u;
-        if (m == 0) continue;
+      for (uint64_t left = shells; left; left &= left - 1) {
+        const int at = __ffsll((long long)left) - 1, s = at / 3;
+        const uint32_t m = (uint32_t)(bits >> at) & 7u;
         const int64_t base = __ldg(voff + (int64_t)s * G + e);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
@@ -950,9 +952,9 @@ __global__ void entry_list_kernel(const float* __restrict__ gsdf, const int32_t*
           pos[r] = (int64_t)__ldg(counts + x[r]) + earlier;  // counts = scanned offsets here
         }
       }
-      for (int s = 0; s < S; ++s) {
-        const uint32_t m = (uint32_t)(bits >> (3 * s)) & 7u;
-        if (m == 0) continue;
+      for (uint64_t left = shells; left; left &= left - 1) {
+        const int at = __ffsll((long long)left) - 1, s = at / 3;
+        const uint32_t m = (uint32_t)(bits >> at) & 7u;
         const float iso = __ldg(level_sets + s);
         const int64_t base = __ldg(voff + (int64_t)s * G + e);
 #pragma unroll
