@@ -70,6 +70,12 @@ MT_API size_t mt_scan_workspace_bytes(int64_t n);
 MT_API int mt_exclusive_scan_i32(int32_t* data, int64_t n, void* workspace,
                           size_t workspace_bytes, mt_stream_t stream);
 
+/* out[0..n] (n + 1 entries, 16-byte aligned) <- exclusive prefix sum of n bytes
+ * (4-byte aligned), or with set_bits of the numbers of their set bits; out[n]
+ * is the total. workspace: mt_scan_workspace_bytes(n + 1) bytes. */
+MT_API int mt_exclusive_scan_bytes(const uint8_t* bytes, int64_t n, int32_t set_bits, int32_t* out,
+                                   void* workspace, size_t workspace_bytes, mt_stream_t stream);
+
 /* data[0..n) <- exclusive prefix sum of data[0..n), in place (int64). */
 MT_API int mt_exclusive_scan_i64(int64_t* data, int64_t n, void* workspace,
                           size_t workspace_bytes, mt_stream_t stream);
@@ -259,6 +265,14 @@ MT_API int mt_count_triangle_vertices(const float* signed_distances,
                                const float* level_sets, int32_t S,
                                int32_t* counts, mt_stream_t stream);
 
+/* The edges counted there: crossings[S*G], bit a of a byte = the entry's edge
+ * along axis a crosses the level set. mt_exclusive_scan_bytes with set_bits
+ * gives the scanned counts. */
+MT_API int mt_count_triangle_crossings(const float* signed_distances,
+                                       const int32_t* lower_corners, int64_t G,
+                                       const float* level_sets, int32_t S,
+                                       uint8_t* crossings, mt_stream_t stream);
+
 /* triangle_extraction/create_triangle_vertices.slang:145-199 (forward).
  * vertex_offsets: exclusive scan of the counts above (S*G+1 entries).
  * grid_sh [C,G,3]; outputs vertices [V,3], signed_distances [V],
@@ -439,6 +453,14 @@ MT_API int mt_count_triangle_faces(const float* signed_distances,
                             int32_t* face_counts, uint8_t* cell_codes,
                             mt_stream_t stream);
 
+/* The same with a byte to a count, [S*Nv], for mt_exclusive_scan_bytes. */
+MT_API int mt_count_triangle_faces_bytes(const float* signed_distances,
+                                         const int32_t* lower_corners, int64_t G,
+                                         const int32_t* upper_corners, int64_t Nv,
+                                         const float* level_sets, int32_t S,
+                                         uint8_t* face_counts, uint8_t* cell_codes,
+                                         mt_stream_t stream);
+
 /* The shell boundaries of triangle_extraction/__init__.py:145-146 from the
  * two scanned count arrays (vertex_offsets: S*G + 1 entries, face_offsets:
  * S*Nv + 1): vertex_boundaries[s] = vertex_offsets[(s + 1) G],
@@ -472,6 +494,16 @@ MT_API int mt_create_triangle_faces(const int32_t* neighbors, const int32_t* ind
                              const int32_t* face_offsets, int64_t F,
                              int32_t* faces, int32_t* voxel_indices,
                              mt_stream_t stream);
+
+/* The same from mt_count_triangle_crossings' bytes, for vertices that
+ * mt_create_triangle_vertices placed by their scan: an entry's vertex of an
+ * axis is the one after its crossings of earlier axes. V: the vertices that
+ * were written; no face names one at or past it. */
+MT_API int mt_create_triangle_faces_by_crossings(
+    const int32_t* neighbors, const int32_t* indices, int64_t Nv, int64_t G,
+    int64_t V, const int32_t* vertex_offsets, const uint8_t* crossings,
+    const uint8_t* cell_codes, int32_t S, const int32_t* face_offsets,
+    int64_t F, int32_t* faces, int32_t* voxel_indices, mt_stream_t stream);
 
 
 /* ------------------------------------------------------------------------

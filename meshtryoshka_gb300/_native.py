@@ -33,6 +33,7 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_version": (I32, []),
     "mt_scan_workspace_bytes": (c_size_t, [I64]),
     "mt_exclusive_scan_i32": (I32, [P, I64, P, c_size_t, P]),
+    "mt_exclusive_scan_bytes": (I32, [P, I64, I32, P, P, c_size_t, P]),
     "mt_exclusive_scan_i64": (I32, [P, I64, P, c_size_t, P]),
     "mt_inclusive_scan_i32_to_i64": (I32, [P, P, I64, P, c_size_t, P]),
     "mt_exclusive_scan_i32_static": (I32, [P, I64, P]),
@@ -60,6 +61,7 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_index_keys_workspace_bytes": (c_size_t, [I64]),
     "mt_index_keys": (I32, [P, I64, P, P, c_size_t, P]),
     "mt_count_triangle_vertices": (I32, [P, P, I64, P, I32, P, P]),
+    "mt_count_triangle_crossings": (I32, [P, P, I64, P, I32, P, P]),
     "mt_create_triangle_vertices": (
         I32,
         [P, P, P, I32, P, I64, P, I32, P, I64, P, P, P, P, P, P, P],
@@ -71,8 +73,13 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     ),
     "mt_create_triangle_vertices_backward_workspace_bytes": (c_size_t, [I64, I64]),
     "mt_count_triangle_faces": (I32, [P, P, I64, P, I64, P, I32, P, P, P]),
+    "mt_count_triangle_faces_bytes": (I32, [P, P, I64, P, I64, P, I32, P, P, P]),
     "mt_compute_sdf_regularizers": (I32, [P, P, P, I64, P, I64, I32, I32, I32, P, P, P, P]),
     "mt_compute_sdf_regularizers_backward": (I32, [P, P, P, I64, P, I64, I32, I32, I32, P, P, P, P, P]),
+    "mt_create_triangle_faces_by_crossings": (
+        I32,
+        [P, P, I64, I64, I64, P, P, P, I32, P, I64, P, P, P],
+    ),
     "mt_create_triangle_faces": (
         I32,
         [P, P, I64, I64, I64, P, P, P, I32, P, I64, P, P, P],

@@ -373,6 +373,15 @@ __device__ __forceinline__ Corners4 load_corners(const float* __restrict__ sdf, 
   return c;
 }
 
+// Bit a of the result: edge `a` of entry g crosses level set `iso`. The same
+// predicate sizes the outputs (count) and places vertices (create), so the
+// writes always stay inside the counted range.
+__device__ __forceinline__ uint32_t crossing_mask(const Corners4& c, float iso) {
+  const bool b0 = c.d0 < iso;
+  return (uint32_t)(b0 != (c.d[0] < iso)) | ((uint32_t)(b0 != (c.d[1] < iso)) << 1) |
+         ((uint32_t)(b0 != (c.d[2] < iso)) << 2);
+}
+
 __global__ void count_vertices_kernel(const float* __restrict__ sdf, const int32_t* __restrict__ lower, int64_t G,
                                       const float* __restrict__ level_sets, int S, int32_t* __restrict__ counts) {
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < G; g += (int64_t)gridDim.x * blockDim.x) {
@@ -386,13 +395,14 @@ __global__ void count_vertices_kernel(const float* __restrict__ sdf, const int32
   if (blockIdx.x == 0 && threadIdx.x == 0) counts[(int64_t)S * G] = 0;
 }
 
-// Bit a of the result: edge `a` of entry g crosses level set `iso`. The same
-// predicate sizes the outputs (count) and places vertices (create), so the
-// writes always stay inside the counted range.
-__device__ __forceinline__ uint32_t crossing_mask(const Corners4& c, float iso) {
-  const bool b0 = c.d0 < iso;
-  return (uint32_t)(b0 != (c.d[0] < iso)) | ((uint32_t)(b0 != (c.d[1] < iso)) << 1) |
-         ((uint32_t)(b0 != (c.d[2] < iso)) << 2);
+// The crossings themselves, a byte each, for the scan that takes their numbers
+// and the faces, which then find an edge's vertex without the types.
+__global__ void count_crossings_kernel(const float* __restrict__ sdf, const int32_t* __restrict__ lower, int64_t G,
+                                       const float* __restrict__ level_sets, int S, uint8_t* __restrict__ crossings) {
+  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < G; g += (int64_t)gridDim.x * blockDim.x) {
+    const Corners4 c = load_corners(sdf, lower, G, g);
+    for (int s = 0; s < S; ++s) crossings[(int64_t)s * G + g] = (uint8_t)crossing_mask(c, __ldg(level_sets + s));
+  }
 }
 
 // create_triangle_vertices.slang:87-96: t is detached; positions / SH / sdf
@@ -1352,9 +1362,11 @@ __device__ __forceinline__ void load_cube(const float* __restrict__ sdf, const i
   cube[7] = __ldg(sdf + __ldg(upper + Nv + v));
 }
 
+// Count: int32_t (with the closing zero), or uint8_t for mt_exclusive_scan_bytes.
+template <typename Count>
 __global__ void count_faces_kernel(const float* __restrict__ sdf, const int32_t* __restrict__ lower, int64_t G,
                                    const int32_t* __restrict__ upper, int64_t Nv,
-                                   const float* __restrict__ level_sets, int S, int32_t* __restrict__ counts,
+                                   const float* __restrict__ level_sets, int S, Count* __restrict__ counts,
                                    uint8_t* __restrict__ codes) {
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < Nv; v += (int64_t)gridDim.x * blockDim.x) {
     float cube[8];
@@ -1368,7 +1380,7 @@ __global__ void count_faces_kernel(const float* __restrict__ sdf, const int32_t*
       counts[(int64_t)s * Nv + v] = c_mc_count[code];
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) counts[(int64_t)S * Nv] = 0;
+  if (sizeof(Count) == 4 && blockIdx.x == 0 && threadIdx.x == 0) counts[(int64_t)S * Nv] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1379,36 +1391,38 @@ __global__ void count_faces_kernel(const float* __restrict__ sdf, const int32_t*
 // Writes only faces below F and searches only vertices below V (the
 // buffers' capacities); with consistent offsets neither bound is reached.
 //
-// Work is dealt by face slot: a CTA reads kFaceItems consecutive (shell,
-// voxel) items (shell-major, the order of the slot offsets), marks each slot of
-// theirs with its item in shared memory (at most 15 to an item; they are
-// contiguous) and gives the slots to its threads in turn: full lanes, and
-// consecutive lanes write consecutive face corners. An entry's up to three
-// vertices' types are read side by side. The case tables sit in shared memory,
-// as lanes read different cases. Dealt by warps of 32 items (38 slots, two
-// rounds of lanes for them; the item by a search over shuffles, the types one
-// after another, a 64-bit division by three) 401 us at 512^3, 8 shells
-// (15 M faces), 870 at 16 shells and 24 M, 43 at 256^3; now 409, 829 and 36: what
-// is left is the chain neighbour -> offsets -> types of scattered reads.
-constexpr int kFaceItems = 256;
+// Work is dealt by triangle: a CTA reads kPer consecutive (shell, voxel) items
+// (shell-major, the order of the slot offsets) for each of its threads, marks
+// each of their triangles with its item in shared memory (at most 5 to an item;
+// their slots are contiguous) and gives the triangles to its threads in turn,
+// which have all of an item's look-ups once for three edges and the loads of the
+// three side by side. Types are read where a caller has no crossings (an entry's
+// up to three side by side). Bound by its instructions: dealt by slots, with a
+// look-up of item, table and 64-bit addresses for each, 822 us at 512^3,
+// 16 shells (24 M faces), 382 at 8 shells, 35 at 256^3, 8 shells; now 418, 203
+// and 17 (with 4, 2 and 1 items to a thread 457, 570 and 626 at 16 shells). Grids
+// that do not give every SM two CTAs of 8 items to a thread take one item to a
+// thread: a 64^3 sphere's shell 5 us, with 8 items 9.
+constexpr int kFaceThreads = 256;
 
-__global__ void __launch_bounds__(kFaceItems)
+template <bool kCrossings, int kPer>
+__global__ void __launch_bounds__(kFaceThreads)
     create_faces_kernel(const int32_t* __restrict__ neighbors, const int32_t* __restrict__ indices, int64_t Nv,
                         int64_t G, int64_t V, const int32_t* __restrict__ voff, const uint8_t* __restrict__ types,
                         const uint8_t* __restrict__ codes, int S, const int32_t* __restrict__ foff, int64_t F,
                         int32_t* __restrict__ faces, int32_t* __restrict__ voxel_indices) {
-  constexpr int kWarps = kFaceItems / 32;
+  constexpr int kWarps = kFaceThreads / 32, kItems = kFaceThreads * kPer;
   __shared__ uint64_t s_edges[256];
-  __shared__ uint8_t s_count[256];
+  __shared__ uint8_t s_count[256];  // triangles
   __shared__ int8_t s_owner[12];
   __shared__ uint8_t s_axis[12];
-  __shared__ uint8_t s_code[kFaceItems];
-  __shared__ int s_first[kFaceItems];   // an item's first slot in the CTA's
   __shared__ int s_warp[kWarps];
-  __shared__ uint8_t s_item[kFaceItems * 16];  // item of each slot
-  for (int i = threadIdx.x; i < 256; i += kFaceItems) {
+  __shared__ uint8_t s_code[kItems];
+  __shared__ uint16_t s_first[kItems];     // an item's first triangle in the CTA's
+  __shared__ uint16_t s_item[kItems * 5];  // item of each triangle
+  for (int i = threadIdx.x; i < 256; i += kFaceThreads) {
     s_edges[i] = c_mc_edges[i];
-    s_count[i] = c_mc_count[i];
+    s_count[i] = c_mc_count[i] / 3;
   }
   if (threadIdx.x < 12) {
     s_owner[threadIdx.x] = c_mc_owner[threadIdx.x];
@@ -1416,61 +1430,121 @@ __global__ void __launch_bounds__(kFaceItems)
   }
   const int64_t total = (int64_t)S * Nv;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t step = (int64_t)gridDim.x * kFaceItems;
-  int64_t base = blockIdx.x * (int64_t)kFaceItems;
-  uint32_t next = base + threadIdx.x < total ? (uint32_t)codes[base + threadIdx.x] : 0u;
+  const int64_t step = (int64_t)gridDim.x * kItems;
+  const int64_t step_shells = step / Nv, step_voxels = step - step_shells * Nv;
+  int64_t base = blockIdx.x * (int64_t)kItems;
+  int64_t first_shell = base / Nv, first_voxel = base - first_shell * Nv;
+  const int own = threadIdx.x * kPer;  // the thread's items are own .. own + kPer - 1
+  uint32_t next[kPer];
+  auto read = [&](int64_t from) {
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) next[k] = from + own + k < total ? (uint32_t)__ldg(codes + from + own + k) : 0u;
+  };
+  read(base);
+  int32_t next_slot = base < total ? __ldg(foff + base) : 0;
   __syncthreads();
   for (; base < total; base += step) {
-    const uint32_t code = next;
-    const int64_t ahead = base + step + threadIdx.x;
-    next = ahead < total ? (uint32_t)codes[ahead] : 0u;
-    const int n = s_count[code];
+    uint32_t code[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) code[k] = next[k];
+    const int64_t first_tri = next_slot / 3;
+    read(base + step);
+    next_slot = base + step < total ? __ldg(foff + base + step) : 0;
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) n += s_count[code[k]];
     const int incl = warp_inclusive_sum(n);
     if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();  // also: the last step's slots are done
+    __syncthreads();  // also: the last step's triangles are done
     int before = incl - n, span = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
       before += w < warp ? s_warp[w] : 0;
       span += s_warp[w];
     }
-    s_code[threadIdx.x] = (uint8_t)code;
-    s_first[threadIdx.x] = before;
-    for (int k = 0; k < n; ++k) s_item[before + k] = (uint8_t)threadIdx.x;
+    if (n > 0) {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const int many = s_count[code[k]];
+        s_code[own + k] = (uint8_t)code[k];
+        s_first[own + k] = (uint16_t)before;
+        for (int j = 0; j < many; ++j) s_item[before++] = (uint16_t)(own + k);
+      }
+    }
     __syncthreads();
-    if (span == 0) continue;
-    const int64_t first_slot = __ldg(foff + base);
-    const int64_t first_shell = base / Nv;
-    const int64_t first_voxel = base - first_shell * Nv;
-    for (int r = threadIdx.x; r < span; r += kFaceItems) {
-      const int item = s_item[r];
+    for (int q = threadIdx.x; q < span; q += kFaceThreads) {
+      const int item = s_item[q];
       int64_t v = first_voxel + item;
       int64_t row = first_shell * G;  // of the shell's vertex offsets
-      while (v >= Nv) {  // at most kFaceItems / Nv steps
+      while (v >= Nv) {  // at most kItems / Nv steps
         v -= Nv;
         row += G;
       }
-      const int eid = (int)((s_edges[s_code[item]] >> (4 * (r - s_first[item]))) & 15u);
-      const int owner = s_owner[eid];
-      const uint32_t axis = s_axis[eid];
-      const int64_t nb = (owner < 0) ? v : (int64_t)__ldg(neighbors + (int64_t)owner * Nv + v);
-      const int32_t vstart = __ldg(voff + row + nb);
-      const int32_t count = __ldg(voff + row + nb + 1) - vstart;
-      // The entry's first vertex of the edge's axis (there is one); vertices
-      // past the capacity were not written.
-      uint32_t type[3];
+      const uint32_t edges = (uint32_t)(s_edges[s_code[item]] >> (12 * (q - s_first[item])));
+      int64_t at[3];  // each edge's entry, in the shell's row
+      uint32_t axis[3], m[3];
+      int32_t start[3];
 #pragma unroll
-      for (int q = 0; q < 3; ++q)
-        type[q] = q < count && (int64_t)vstart + q < V ? (uint32_t)__ldg(types + vstart + q) : 255u;
-      const int32_t target = type[0] == axis ? vstart : type[1] == axis ? vstart + 1 : type[2] == axis ? vstart + 2 : -1;
-      const int64_t slot = first_slot + r;
-      const int64_t tri = (slot >> 32) == 0 ? (int64_t)((uint32_t)slot / 3u) : slot / 3;
-      if (tri >= F) continue;
-      const int corner = 2 - (int)(slot - 3 * tri);
-      faces[tri * 3 + corner] = target;
-      if (corner == 0) voxel_indices[tri] = __ldg(indices + v);
+      for (int e = 0; e < 3; ++e) {
+        const int eid = (int)((edges >> (4 * e)) & 15u);
+        const int owner = s_owner[eid];
+        axis[e] = s_axis[eid];
+        at[e] = row + ((owner < 0) ? v : (int64_t)__ldg(neighbors + (int64_t)owner * Nv + v));
+      }
+      const int32_t voxel = __ldg(indices + v);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        start[e] = __ldg(voff + at[e]);
+        if constexpr (kCrossings) m[e] = (uint32_t)__ldg(types + at[e]);
+      }
+      const int64_t tri = first_tri + q;
+      if ((uint64_t)tri >= (uint64_t)F) continue;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        // The entry's vertex of the edge's axis (there is one); vertices past
+        // the capacity were not written.
+        int32_t target = -1;
+        if constexpr (kCrossings) {
+          const int32_t found = start[e] + __popc(m[e] & ((1u << axis[e]) - 1u));
+          if (((m[e] >> axis[e]) & 1u) && found < V) target = found;
+        } else {
+          const int32_t count = __ldg(voff + at[e] + 1) - start[e];
+          uint32_t type[3];
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            type[i] = i < count && (int64_t)start[e] + i < V ? (uint32_t)__ldg(types + start[e] + i) : 255u;
+#pragma unroll
+          for (int i = 2; i >= 0; --i)
+            if (type[i] == axis[e]) target = start[e] + i;
+        }
+        faces[tri * 3 + 2 - e] = target;
+      }
+      voxel_indices[tri] = voxel;
+    }
+    first_shell += step_shells;
+    first_voxel += step_voxels;
+    if (first_voxel >= Nv) {
+      first_voxel -= Nv;
+      ++first_shell;
     }
   }
+}
+
+template <bool kCrossings>
+int launch_create_faces(const int32_t* neighbors, const int32_t* indices, int64_t Nv, int64_t G, int64_t V,
+                        const int32_t* voff, const uint8_t* types, const uint8_t* codes, int S, const int32_t* foff,
+                        int64_t F, int32_t* faces, int32_t* voxel_indices, cudaStream_t stream) {
+  const int64_t total = (int64_t)S * Nv;
+  auto launch = [&](auto per) {
+    constexpr int kPer = decltype(per)::value;
+    const int64_t tiles = (total + kFaceThreads * kPer - 1) / (kFaceThreads * kPer);
+    create_faces_kernel<kCrossings, kPer><<<grid_stride_blocks(tiles, 1), kFaceThreads, 0, stream>>>(
+        neighbors, indices, Nv, G, V, voff, types, codes, S, foff, F, faces, voxel_indices);
+  };
+  if (total >= (int64_t)2 * kSmCount * 8 * kFaceThreads) launch(std::integral_constant<int, 8>{});
+  else launch(std::integral_constant<int, 1>{});
+  MT_CHECK_LAUNCH();
+  return MT_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1770,6 +1844,17 @@ int mt_count_triangle_vertices(const float* signed_distances, const int32_t* low
   return MT_OK;
 }
 
+int mt_count_triangle_crossings(const float* signed_distances, const int32_t* lower_corners, int64_t G,
+                                const float* level_sets, int32_t S, uint8_t* crossings, mt_stream_t stream) {
+  MT_REQUIRE(G >= 0 && S >= 0);
+  if (G == 0 || S == 0) return MT_OK;
+  MT_REQUIRE(signed_distances && lower_corners && level_sets && crossings);
+  count_crossings_kernel<<<grid_stride_blocks(G, 256), 256, 0, as_stream(stream)>>>(signed_distances, lower_corners,
+                                                                                   G, level_sets, S, crossings);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
+}
+
 int mt_create_triangle_vertices_live_t_backward(const float* grid_vertices, const float* grid_signed_distances,
                                                 const float* grid_spherical_harmonics, int32_t C, int64_t G,
                                                 const int32_t* vertex_sources, int64_t V, const int32_t* num_vertices,
@@ -1895,6 +1980,18 @@ int mt_count_triangle_faces(const float* signed_distances, const int32_t* lower_
   return MT_OK;
 }
 
+int mt_count_triangle_faces_bytes(const float* signed_distances, const int32_t* lower_corners, int64_t G,
+                                  const int32_t* upper_corners, int64_t Nv, const float* level_sets, int32_t S,
+                                  uint8_t* face_counts, uint8_t* cell_codes, mt_stream_t stream) {
+  MT_REQUIRE(G >= 0 && Nv >= 0 && S >= 0);
+  if (Nv == 0 || S == 0) return MT_OK;
+  MT_REQUIRE(signed_distances && lower_corners && upper_corners && level_sets && face_counts && cell_codes);
+  count_faces_kernel<<<grid_stride_blocks(Nv, 256), 256, 0, as_stream(stream)>>>(
+      signed_distances, lower_corners, G, upper_corners, Nv, level_sets, S, face_counts, cell_codes);
+  MT_CHECK_LAUNCH();
+  return MT_OK;
+}
+
 int mt_create_triangle_faces(const int32_t* neighbors, const int32_t* indices, int64_t Nv, int64_t G, int64_t V,
                              const int32_t* vertex_offsets, const uint8_t* vertex_types, const uint8_t* cell_codes,
                              int32_t S, const int32_t* face_offsets, int64_t F, int32_t* faces,
@@ -1903,11 +2000,20 @@ int mt_create_triangle_faces(const int32_t* neighbors, const int32_t* indices, i
   if (Nv == 0 || S == 0 || F == 0) return MT_OK;
   MT_REQUIRE(neighbors && indices && vertex_offsets && vertex_types && cell_codes && face_offsets && faces &&
              voxel_indices);
-  create_faces_kernel<<<grid_stride_blocks((int64_t)S * Nv, 256), 256, 0, as_stream(stream)>>>(
-      neighbors, indices, Nv, G, V, vertex_offsets, vertex_types, cell_codes, S, face_offsets, F, faces,
-      voxel_indices);
-  MT_CHECK_LAUNCH();
-  return MT_OK;
+  return launch_create_faces<false>(neighbors, indices, Nv, G, V, vertex_offsets, vertex_types, cell_codes, S, face_offsets,
+                                    F, faces, voxel_indices, as_stream(stream));
+}
+
+int mt_create_triangle_faces_by_crossings(const int32_t* neighbors, const int32_t* indices, int64_t Nv, int64_t G,
+                                          int64_t V, const int32_t* vertex_offsets, const uint8_t* crossings,
+                                          const uint8_t* cell_codes, int32_t S, const int32_t* face_offsets, int64_t F,
+                                          int32_t* faces, int32_t* voxel_indices, mt_stream_t stream) {
+  MT_REQUIRE(Nv >= 0 && G >= 0 && V >= 0 && S >= 0 && F >= 0);
+  if (Nv == 0 || S == 0 || F == 0) return MT_OK;
+  MT_REQUIRE(neighbors && indices && vertex_offsets && crossings && cell_codes && face_offsets && faces &&
+             voxel_indices);
+  return launch_create_faces<true>(neighbors, indices, Nv, G, V, vertex_offsets, crossings, cell_codes, S, face_offsets,
+                                    F, faces, voxel_indices, as_stream(stream));
 }
 
 int mt_compute_sdf_regularizers(const float* grid_signed_distances, const int32_t* voxel_neighbors,

@@ -43,6 +43,80 @@ constexpr int scan_items() {
 // The smallest tile of any scan here: workspaces are sized by it.
 constexpr int kScanTileMin = kScanThreads * 24;
 
+// Exclusive scan of n bytes (kBits: of their numbers of set bits) into n + 1
+// int32. The tiles and the order of the sums are scan_kernel's; a round is the
+// 4 bytes of a lane, whose results are one 16-byte store. Counts that fit a byte
+// are a quarter of the bytes to write and to read: 53 M vertex counts of 8
+// shells at 512^3 took 111 us to scan in place as int32, this takes 71.
+template <bool kBits>
+__global__ void __launch_bounds__(kScanThreads)
+    scan_bytes_kernel(const uint8_t* in, int32_t* out, int64_t n, uint32_t* counter, uint64_t* desc, int* status) {
+  constexpr int kItems = scan_items<int32_t>(), R = kItems / 4, kWarps = kScanThreads / 32;
+  __shared__ uint32_t s_tile;
+  __shared__ int32_t s_warp[kWarps];
+  __shared__ int32_t s_prefix;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) s_tile = atomicAdd(counter, 1u);
+  __syncthreads();
+  const int64_t tile = s_tile;
+  const int64_t seg = tile * (kScanThreads * kItems) + (int64_t)warp * (32 * kItems);
+  const bool full = seg + 32 * kItems <= n;
+  uint32_t x[R];  // 4 bytes each
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t first = seg + (int64_t)(32 * r + lane) * 4;
+    if (full) {
+      x[r] = __ldcs(reinterpret_cast<const uint32_t*>(in + first));
+    } else {
+      x[r] = 0;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) x[r] |= first + v < n ? (uint32_t)in[first + v] << (8 * v) : 0u;
+    }
+  }
+  auto value = [](uint32_t word, int v) -> int32_t {
+    const uint32_t byte = (word >> (8 * v)) & 0xffu;
+    return kBits ? __popc(byte) : (int32_t)byte;
+  };
+  int32_t lane_excl[R];
+  int32_t warp_total = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int32_t mine = kBits ? __popc(x[r]) : (int32_t)__dp4a(x[r], 0x01010101u, 0u);
+    const int32_t inc = warp_inclusive_sum(mine);
+    lane_excl[r] = inc - mine + warp_total;
+    warp_total += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  if (lane == 0) s_warp[warp] = warp_total;
+  __syncthreads();
+  if (warp == 0) {
+    const int32_t w = lane < kWarps ? s_warp[lane] : 0;
+    const int32_t wi = warp_inclusive_sum(w);
+    if (lane < kWarps) s_warp[lane] = wi - w;
+    const int32_t block_total = __shfl_sync(0xffffffffu, wi, kWarps - 1);
+    const int32_t prefix = lookback_prefix<int32_t>(desc, tile, block_total, status);
+    if (lane == 0) s_prefix = prefix;
+  }
+  __syncthreads();
+  const int32_t offset = s_prefix + s_warp[warp];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t first = seg + (int64_t)(32 * r + lane) * 4;
+    int4 y;
+    y.x = lane_excl[r] + offset;
+    y.y = y.x + value(x[r], 0);
+    y.z = y.y + value(x[r], 1);
+    y.w = y.z + value(x[r], 2);
+    if (full) {
+      __stcs(reinterpret_cast<int4*>(out + first), y);
+    } else {
+      if (first <= n) out[first] = y.x;
+      if (first + 1 <= n) out[first + 1] = y.y;
+      if (first + 2 <= n) out[first + 2] = y.z;
+      if (first + 3 <= n) out[first + 3] = y.w;
+    }
+  }
+}
+
 template <typename TI, typename TO, bool kInclusive, bool kVector>
 __global__ void __launch_bounds__(kScanThreads)
     scan_kernel(const TI* in, TO* out, int64_t n, uint32_t* counter, uint64_t* desc, int* status) {
@@ -151,6 +225,24 @@ int launch_scan(const TI* in, TO* out, int64_t n, void* ws, size_t ws_bytes, cud
   return MT_OK;
 }
 
+int launch_scan_bytes(const uint8_t* in, int64_t n, bool bits, int32_t* out, void* ws, size_t ws_bytes,
+                      cudaStream_t stream) {
+  MT_REQUIRE(n >= 0 && out != nullptr && ws != nullptr && (n == 0 || in != nullptr));
+  MT_REQUIRE((reinterpret_cast<uintptr_t>(in) & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
+  constexpr int64_t kTile = (int64_t)kScanThreads * scan_items<int32_t>();
+  const int64_t tiles = n / kTile + 1;  // n + 1 results
+  MT_REQUIRE(tiles < (int64_t)0x7fffffff);
+  if (ws_bytes < mt_scan_workspace_bytes(n + 1)) return MT_ERR_WORKSPACE_TOO_SMALL;
+  char* base = static_cast<char*>(ws);
+  if (cudaMemsetAsync(base + 4, 0, kScanHeader - 4 + (size_t)tiles * 8, stream) != cudaSuccess) return MT_ERR_CUDA;
+  uint32_t* counter = reinterpret_cast<uint32_t*>(base + 4);
+  uint64_t* desc = reinterpret_cast<uint64_t*>(base + kScanHeader);
+  auto* kernel = bits ? scan_bytes_kernel<true> : scan_bytes_kernel<false>;
+  kernel<<<(unsigned)tiles, kScanThreads, 0, stream>>>(in, out, n, counter, desc, reinterpret_cast<int*>(base));
+  MT_CHECK_LAUNCH();
+  return MT_OK;
+}
+
 // One warp looks back from tile 1 over a descriptor array whose tile 0 never
 // publishes: the wait gives up after `spin_limit` polls, records
 // MT_ERR_DEVICE_TIMEOUT in the status word and treats the missing tile as an
@@ -178,6 +270,11 @@ size_t mt_scan_workspace_bytes(int64_t n) {
 
 int mt_exclusive_scan_i32(int32_t* data, int64_t n, void* ws, size_t ws_bytes, mt_stream_t stream) {
   return mt::launch_scan<int32_t, int32_t, false>(data, data, n, ws, ws_bytes, mt::as_stream(stream));
+}
+
+int mt_exclusive_scan_bytes(const uint8_t* bytes, int64_t n, int32_t set_bits, int32_t* out, void* ws, size_t ws_bytes,
+                            mt_stream_t stream) {
+  return mt::launch_scan_bytes(bytes, n, set_bits != 0, out, ws, ws_bytes, mt::as_stream(stream));
 }
 
 int mt_exclusive_scan_i64(int64_t* data, int64_t n, void* ws, size_t ws_bytes, mt_stream_t stream) {

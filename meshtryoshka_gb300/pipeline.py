@@ -267,14 +267,14 @@ def step_bytes(stats: dict) -> dict[str, float]:
     G, Nv, V, F, C, S, B, P, K, T = (stats[k] for k in ("G", "Nv", "V", "F", "C", "S", "B", "P", "K", "T"))
     return {
         # tessellation
-        "count_vertices": G * (16 + 16) + 4 * S * G,
-        "scans": 8 * S * G + 8 * S * Nv,
+        "count_vertices": G * (16 + 16) + S * G,
+        "scans": 5 * S * G + 5 * S * Nv,
         # per entry: 4 corner ids, 4 SDFs, 4 positions, its offsets; per
         # vertex: position, SDF, type, source record (origin, corner, t)
         "create_vertices": G * (16 + 4 * (4 + 12) + 4 * S) + V * (12 + 4 + 1 + 12),
         # corner inverse, per-entry list counts, their scan, list fill
         "contribution_list": G * (16 + 16) + G * (16 + 4) + 8 * G + G * 16 + 16 * V,
-        "count_faces": Nv * (32 + 32) + 5 * S * Nv,
+        "count_faces": Nv * (32 + 32) + 2 * S * Nv,
         "create_faces": Nv * (28 + 4 + S) + 8 * S * Nv + 16 * F,
         # render front end
         "uncontract": 24 * V,

@@ -451,6 +451,34 @@ def count_triangle_vertices(signed_distances: Tensor, lower_corners: Tensor, lev
     return counts
 
 
+def _scan_bytes(counts: Tensor, set_bits: bool) -> Tensor:
+    """Exclusive scan (n + 1 int32) of n bytes, or of their set bits."""
+    device = counts.device
+    n = counts.numel()
+    out = torch.empty((n + 1,), dtype=torch.int32, device=device)
+    ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_scan_workspace_bytes(n + 1))
+    nt.call("mt_exclusive_scan_bytes", nt.ptr(counts), n, int(set_bits), out.data_ptr(), ws_ptr, ws_bytes,
+            nt.stream(device))
+    return out
+
+
+def _vertex_offsets(signed_distances: Tensor, lower_corners: Tensor, level_sets: Tensor) -> tuple[Tensor, Tensor]:
+    """count_triangle_vertices and its scan, by a byte per (level set, entry)
+    that holds the crossings; those too, for the faces."""
+    with annotate("count_triangle_vertices"):
+        signed_distances = _f32(signed_distances, "signed_distances")
+        lower_corners = _i32(lower_corners, "lower_corners")
+        level_sets = _f32(level_sets, "level_sets")
+        device = nt.require_cuda(signed_distances, lower_corners, level_sets)
+        (s,) = level_sets.shape
+        _, g = lower_corners.shape
+        crossings = torch.empty((s * g,), dtype=torch.uint8, device=device)
+        nt.call("mt_count_triangle_crossings", nt.ptr(signed_distances), nt.ptr(lower_corners), g, nt.ptr(level_sets),
+                s, nt.ptr(crossings), nt.stream(device))
+    with annotate("compute_exclusive_cumsum"):
+        return _scan_bytes(crossings, True), crossings
+
+
 # The grid SH backward forms each vertex's SH gradient once into scratch (193
 # bytes per vertex) and then gathers it per grid vertex; above this many bytes
 # of scratch (22 M vertices) it runs its one-pass form instead, which forms a
@@ -736,6 +764,25 @@ def count_triangle_faces(
     return CountTriangleFacesResult(counts, codes)
 
 
+def _face_offsets(signed_distances: Tensor, lower_corners: Tensor, upper_corners: Tensor,
+                  level_sets: Tensor) -> tuple[Tensor, Tensor]:
+    """count_triangle_faces and its scan, by counts of a byte."""
+    with annotate("count_triangle_faces"):
+        signed_distances = _f32(signed_distances, "signed_distances")
+        lower_corners = _i32(lower_corners, "lower_corners")
+        upper_corners = _i32(upper_corners, "upper_corners")
+        level_sets = _f32(level_sets, "level_sets")
+        device = nt.require_cuda(signed_distances, lower_corners, upper_corners, level_sets)
+        _, nv = upper_corners.shape
+        _, g = lower_corners.shape
+        (s,) = level_sets.shape
+        codes, counts = (torch.empty((s, nv), dtype=torch.uint8, device=device) for _ in range(2))
+        nt.call("mt_count_triangle_faces_bytes", nt.ptr(signed_distances), nt.ptr(lower_corners), g,
+                nt.ptr(upper_corners), nv, nt.ptr(level_sets), s, nt.ptr(counts), nt.ptr(codes), nt.stream(device))
+    with annotate("compute_exclusive_cumsum"):
+        return _scan_bytes(counts, False), codes
+
+
 class CreateTriangleFacesResult(NamedTuple):
     faces: Tensor
     voxel_indices: Tensor | None
@@ -756,6 +803,15 @@ def create_triangle_faces(
 ) -> CreateTriangleFacesResult:
     """``capacity`` (optional) sizes the outputs to a fixed row count; faces
     past it are not written and nothing is read back."""
+    return _create_triangle_faces("mt_create_triangle_faces", signed_distances, neighbors, indices, vertex_offsets,
+                                  triangle_vertex_types, triangle_vertex_types.shape[0], voxel_cell_codes, level_sets,
+                                  face_offsets, num_faces, capacity)
+
+
+def _create_triangle_faces(entry, signed_distances, neighbors, indices, vertex_offsets, types, num_vertices,
+                           voxel_cell_codes, level_sets, face_offsets, num_faces, capacity):
+    """``types``: the vertices' types, or for mt_create_triangle_faces_by_crossings
+    the entries' crossings."""
     device = nt.require_cuda(signed_distances, neighbors, indices, vertex_offsets, face_offsets)
     _, nv = neighbors.shape
     (s,) = level_sets.shape
@@ -768,10 +824,10 @@ def create_triangle_faces(
     voxel_indices = torch.empty((f,), dtype=torch.int32, device=device)
     neighbors, indices = _i32(neighbors, "neighbors"), _i32(indices, "indices")
     vertex_offsets, face_offsets = _i32(vertex_offsets, "vertex_offsets"), _i32(face_offsets, "face_offsets")
-    types, codes = triangle_vertex_types.contiguous(), voxel_cell_codes.contiguous()
+    types, codes = types.contiguous(), voxel_cell_codes.contiguous()
     nt.call(
-        "mt_create_triangle_faces",
-        nt.ptr(neighbors), nt.ptr(indices), nv, g, types.shape[0], nt.ptr(vertex_offsets), nt.ptr(types),
+        entry,
+        nt.ptr(neighbors), nt.ptr(indices), nv, g, num_vertices, nt.ptr(vertex_offsets), nt.ptr(types),
         nt.ptr(codes), s,
         nt.ptr(face_offsets), f, nt.ptr(faces), nt.ptr(voxel_indices), nt.stream(device),
     )
@@ -928,11 +984,8 @@ def _tessellate(signed_distances, vertices, spherical_harmonics, neighbors, lowe
     _, nv = upper_corners.shape
 
     with torch.no_grad():
-        vertex_offsets = count_triangle_vertices(signed_distances, lower_corners, level_sets)
-        compute_exclusive_cumsum(vertex_offsets)
-        face_offsets, voxel_cell_codes = count_triangle_faces(signed_distances, lower_corners, upper_corners,
-                                                              level_sets)
-        compute_exclusive_cumsum(face_offsets)
+        vertex_offsets, crossings = _vertex_offsets(signed_distances, lower_corners, level_sets)
+        face_offsets, voxel_cell_codes = _face_offsets(signed_distances, lower_corners, upper_corners, level_sets)
         if capacity is None:
             # One device->host read for both totals and the scans' status word.
             ws = nt.workspace(device)
@@ -947,7 +1000,7 @@ def _tessellate(signed_distances, vertices, spherical_harmonics, neighbors, lowe
             counts = TessellationCounts(vertex_offsets[-1], torch.empty((), dtype=torch.int32, device=device))
 
     deferred = DeferredSH(spherical_harmonics) if defer_sh else None
-    triangle_vertices, triangle_sdf, triangle_sh, triangle_types = create_triangle_vertices(
+    triangle_vertices, triangle_sdf, triangle_sh, _ = create_triangle_vertices(
         vertices, signed_distances, spherical_harmonics, lower_corners, level_sets, vertex_offsets,
         num_vertices if capacity is None else None, None if capacity is None else num_vertices, deferred,
         t_gradient=t_gradient,
@@ -956,10 +1009,12 @@ def _tessellate(signed_distances, vertices, spherical_harmonics, neighbors, lowe
         triangle_sh = deferred
 
     with torch.no_grad():
-        faces, voxel_indices = create_triangle_faces(
-            signed_distances, neighbors, indices, vertex_offsets, triangle_types, voxel_cell_codes, level_sets,
-            face_offsets, num_faces if capacity is None else None, None if capacity is None else num_faces,
-        )
+        with annotate("create_triangle_faces"):
+            faces, voxel_indices = _create_triangle_faces(
+                "mt_create_triangle_faces_by_crossings", signed_distances, neighbors, indices, vertex_offsets, crossings,
+                triangle_vertices.shape[0], voxel_cell_codes, level_sets, face_offsets,
+                num_faces if capacity is None else None, None if capacity is None else num_faces,
+            )
         # vertex_offsets[1:].view(S, -1)[:, -1] and face_offsets[...] // 3 (and
         # the counted face total) in one launch.
         vertex_boundaries = torch.empty((num_level_sets,), dtype=torch.int32, device=device)
