@@ -461,7 +461,7 @@ def run_ours(args, rank, world, local):
         "mt_intersect_and_composite_forward": ("composite_fwd", "warp_masks"),
         "mt_sort_keys_by_tile": ("tile_sort",),
         "mt_bound_and_generate_keys": ("keys",),
-        "mt_grid_sh_colors_by_entry": ("grid_sh_colors",),
+        "mt_grid_sh_colors_of_seen": ("grid_sh_colors",),
         "mt_create_triangle_faces_by_crossings": ("create_faces",),
     }
     totals = {k: sum(v) for k, v in per_call.items()}

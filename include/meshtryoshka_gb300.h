@@ -391,6 +391,20 @@ MT_API int mt_grid_sh_colors_by_entry(const float* grid_spherical_harmonics, int
                              int32_t sh_degree, const float* camera_positions,
                              int32_t B, float* out_colors, mt_stream_t stream);
 
+/* The same for the vertices with a byte set in seen [V] (NULL: all); the others'
+ * colours are not written. mt_mark_seen_vertices sets the bytes of the vertices
+ * of the keys' triangles (num_keys: NULL or the device live count) and clears
+ * the rest. */
+MT_API int mt_grid_sh_colors_of_seen(const float* grid_spherical_harmonics, int32_t C, int64_t G,
+                             const int32_t* vertex_sources, int64_t V,
+                             const int32_t* num_vertices, const int32_t* vertex_offsets,
+                             int32_t S, const float* vertices,
+                             int32_t sh_degree, const float* camera_positions,
+                             int32_t B, const uint8_t* seen, float* out_colors, mt_stream_t stream);
+MT_API int mt_mark_seen_vertices(const int32_t* triangles, int64_t K, const int64_t* num_keys,
+                                 const int32_t* faces, int64_t F, int64_t V, uint8_t* seen,
+                                 mt_stream_t stream);
+
 /* Backward of mt_grid_sh_colors: grad_grid_sh [C,G,3] (every entry written)
  * from grad_colors [B,V,3] through the list of mt_build_vertex_grad_list.
  * The per-vertex SH gradient of mt_evaluate_spherical_harmonics_backward is

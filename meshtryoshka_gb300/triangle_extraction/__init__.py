@@ -489,6 +489,16 @@ GRID_SH_BACKWARD_SCRATCH_LIMIT = 4 << 30
 _KEPT_SCRATCH = 512 << 20
 
 
+# Renders form the colours of only the vertices that some key's triangle names,
+# where there are fewer keys than faces (so that some faces have none; both are
+# sizes that the host knows) and the grid's SH rows are more than this many bytes
+# (below, they stay in the L2 and every colour takes 50 us). At 512^3, 16 shells,
+# with 4 cameras inside the scene (0.7 keys to a face) the marks take 79 us and
+# the colours 590 instead of 1190; one camera outside a 480^3 scene 849 -> 845 us
+# a step, but two (1.1 keys to a face) would lose: 1304 -> 1317.
+SEEN_COLOURS_BYTES = 100 << 20
+
+
 class DeferredSH:
     """Per-vertex SH coefficients that are never formed (not in the
     reference): stands where ``Triangles.spherical_harmonics`` holds the
@@ -512,9 +522,26 @@ class DeferredSH:
         v = self.vertex_sources.shape[1] if self.vertex_sources is not None else 0
         return (c, v, 3)
 
-    def evaluate(self, vertices: Tensor, extrinsics: Tensor, sh_degree: int) -> Tensor:
-        """evaluate_spherical_harmonics(vertices, rows, extrinsics, sh_degree)."""
-        return GridSHColors.apply(self.grid_spherical_harmonics, vertices, extrinsics, sh_degree, self)
+    def evaluate(self, vertices: Tensor, extrinsics: Tensor, sh_degree: int, seen: Tensor | None = None) -> Tensor:
+        """evaluate_spherical_harmonics(vertices, rows, extrinsics, sh_degree).
+        ``seen`` (uint8 [vertex]): only the colours of vertices whose byte is
+        set are formed; the others' must not be read."""
+        return GridSHColors.apply(self.grid_spherical_harmonics, vertices, extrinsics, sh_degree, self, seen)
+
+    def seen_vertices(self, triangles: Tensor, num_keys: Tensor | None, faces: Tensor,
+                      sh_degree: int) -> Tensor | None:
+        """The vertices that the keys' triangles name, for ``evaluate``; None
+        where every colour is as well formed."""
+        if triangles.numel() > faces.shape[0] or 12 * self.grid_spherical_harmonics.shape[1] * (sh_degree + 1) ** 2 <= SEEN_COLOURS_BYTES:
+            return None
+        with annotate("seen_vertices"):
+            device = nt.require_cuda(triangles, faces)
+            v = self.vertex_sources.shape[1]
+            seen = torch.empty((v,), dtype=torch.uint8, device=device)
+            triangles, faces = _i32(triangles, "triangles"), _i32(faces, "faces")
+            nt.call("mt_mark_seen_vertices", nt.ptr(triangles), triangles.numel(), nt.ptr(num_keys), nt.ptr(faces),
+                    faces.shape[0], v, nt.ptr(seen), nt.stream(device))
+            return seen
 
 
 class GridSHColors(torch.autograd.Function):
@@ -523,7 +550,7 @@ class GridSHColors(torch.autograd.Function):
     the gradient goes straight to the grid SH."""
 
     @staticmethod
-    def forward(ctx, grid_spherical_harmonics, vertices, extrinsics, sh_degree, deferred):
+    def forward(ctx, grid_spherical_harmonics, vertices, extrinsics, sh_degree, deferred, seen=None):
         with annotate("grid_sh_colors_forward"):
             gsh = _f32(grid_spherical_harmonics, "grid_spherical_harmonics")
             vertices = _f32(vertices, "vertices")
@@ -539,9 +566,9 @@ class GridSHColors(torch.autograd.Function):
             colors = torch.empty((b, v, 3), dtype=torch.float32, device=device)
             offsets = deferred.vertex_offsets
             shells = (offsets.numel() - 1) // g if g > 0 else 0
-            nt.call("mt_grid_sh_colors_by_entry", nt.ptr(gsh), c, g, nt.ptr(deferred.vertex_sources), v,
-                    nt.ptr(deferred.num_vertices), nt.ptr(offsets), shells, nt.ptr(vertices), int(sh_degree), nt.ptr(campos), b,
-                    nt.ptr(colors), nt.stream(device))
+            nt.call("mt_grid_sh_colors_of_seen", nt.ptr(gsh), c, g, nt.ptr(deferred.vertex_sources), v,
+                    nt.ptr(deferred.num_vertices), nt.ptr(offsets), shells, nt.ptr(vertices), int(sh_degree),
+                    nt.ptr(campos), b, nt.ptr(seen), nt.ptr(colors), nt.stream(device))
             ctx.save_for_backward(vertices, campos, colors)
             ctx.deferred = deferred
             ctx.gsh_shape = gsh.shape
@@ -570,7 +597,7 @@ class GridSHColors(torch.autograd.Function):
                     nt.ptr(d.list_offsets), nt.ptr(d.contributions), g, v, nt.ptr(vertices), c, ctx.sh_degree,
                     nt.ptr(campos), campos.shape[0], nt.ptr(colors), rows.data_ptr() or None, nt.ptr(grad_gsh), nt.ptr(d.num_vertices), ws_ptr, ws_bytes,
                     nt.stream(device))
-            return grad_gsh, None, None, None, None
+            return grad_gsh, None, None, None, None, None
 
 
 class CreateTriangleVerticesResult(NamedTuple):

@@ -551,6 +551,20 @@ def evaluate_spherical_harmonics(vertices: Tensor, spherical_harmonics: Tensor, 
     return EvaluateSphericalHarmonics.apply(vertices, spherical_harmonics, extrinsics, sh_degree)
 
 
+def _seen_vertices(spherical_harmonics, paired: PairedKeys, faces: Tensor, sh_degree: int) -> Tensor | None:
+    """Of a deferred SH, the vertices of the keys' triangles (before the sort)."""
+    if isinstance(spherical_harmonics, Tensor) or not hasattr(spherical_harmonics, "seen_vertices"):
+        return None
+    return spherical_harmonics.seen_vertices(paired.triangle_indices, paired.count, faces, sh_degree)
+
+
+def _colors(vertices: Tensor, spherical_harmonics, extrinsics: Tensor, sh_degree: int, seen: Tensor | None) -> Tensor:
+    """evaluate_spherical_harmonics of the vertices that ``seen`` marks (None: all)."""
+    if seen is None:
+        return evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
+    return spherical_harmonics.evaluate(vertices, extrinsics, sh_degree, seen)
+
+
 # ---------------------------------------------------------------------------
 # Fused compositing (intersect_and_composite.py:24-175)
 # ---------------------------------------------------------------------------
@@ -1066,8 +1080,9 @@ def render_fused(extrinsics, intrinsics, image_shape, vertices, faces, shell_fac
                    key_capacity)
     del depths
     LAST_RENDER_STATS.update(num_keys=paired.num_keys, num_tiles=grid.num_tiles_per_image, key_count=paired.count)
+    seen = _seen_vertices(spherical_harmonics, paired, faces, sh_degree)
     paired, tile_boundaries = _sort_and_delineate(paired, grid, key_defines, False)
-    colors = evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
+    colors = _colors(vertices, spherical_harmonics, extrinsics, sh_degree, seen)
     t = tile_boundaries.shape[2]
     images = IntersectAndComposite.apply(positions, colors, signed_distances, faces, sharpness, paired.keys,
                                          paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid,
@@ -1117,8 +1132,9 @@ def render_cameras(extrinsics, intrinsics, image_shapes, vertices, faces, shell_
                    key_capacity)
     del depths
     LAST_RENDER_STATS.update(num_keys=paired.num_keys, num_tiles=grid.camera_tiles, key_count=paired.count)
+    seen = _seen_vertices(spherical_harmonics, paired, faces, sh_degree)
     paired, tile_boundaries = _sort_and_delineate(paired, grid, key_defines, False)
-    colors = evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
+    colors = _colors(vertices, spherical_harmonics, extrinsics, sh_degree, seen)
     t = tile_boundaries.shape[2]
     raw = IntersectAndComposite.apply(positions, colors, signed_distances, faces, sharpness, paired.keys,
                                       paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
@@ -1167,8 +1183,9 @@ def render_fused_loss(extrinsics, intrinsics, image_shape, vertices, faces, shel
                    key_capacity)
     del depths
     LAST_RENDER_STATS.update(num_keys=paired.num_keys, num_tiles=grid.camera_tiles, key_count=paired.count)
+    seen = _seen_vertices(spherical_harmonics, paired, faces, sh_degree)
     paired, tile_boundaries = _sort_and_delineate(paired, grid, key_defines, False)
-    colors = evaluate_spherical_harmonics(vertices, spherical_harmonics, extrinsics, sh_degree)
+    colors = _colors(vertices, spherical_harmonics, extrinsics, sh_degree, seen)
     t = tile_boundaries.shape[2]
     return IntersectCompositeLoss.apply(positions, colors, signed_distances, faces, sharpness, paired.keys,
                                         paired.triangle_indices, tile_boundaries.view(b, t, 2), s, grid, key_defines,
