@@ -905,7 +905,8 @@ __global__ void vertex_grads_from_list_kernel(const int32_t* __restrict__ offset
 // r of x's segment word; pass 2 writes the segment at x's scanned offset plus
 // the lengths of x's earlier segments. Each entry loads its own corners once
 // (a pass per grid vertex loads four entries' corners for each: 318 + 411 us
-// at 512^3, 8 shells; this 126 + 221, a turn per crossed shell).
+// at 512^3, 8 shells; this 105 + 221, a turn per crossed shell; the count, which
+// is its set bits where no vertex is past the capacity, 126 by turns).
 // Counts and segment words start at zero (cleared by invert_corners_kernel).
 // ---------------------------------------------------------------------------
 template <bool kFill>
@@ -913,6 +914,7 @@ __global__ void entry_list_kernel(const float* __restrict__ gsdf, const int32_t*
                                   const float* __restrict__ level_sets, int S, const int32_t* __restrict__ voff,
                                   const int32_t* __restrict__ inverse, int64_t V, int32_t* __restrict__ counts,
                                   uint32_t* __restrict__ segments, int2* __restrict__ list) {
+  const bool fit = (int64_t)__ldg(voff + (int64_t)S * G) <= V;  // no vertex past the capacity
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < G; e += (int64_t)gridDim.x * blockDim.x) {
     const Corners4 c = load_corners(gsdf, lower, G, e);
     const uint64_t bits = crossing_bits(c, level_sets, 0, S);
@@ -928,8 +930,10 @@ __global__ void entry_list_kernel(const float* __restrict__ gsdf, const int32_t*
     for (int r = 0; r < 4; ++r) owns[r] = x[r] >= 0 && x[r] < G && __ldg(inverse + r * G + x[r]) == (int32_t)e;
     if (!(owns[0] || owns[1] || owns[2] || owns[3])) continue;
     if (!kFill) {
-      int n[4] = {0, 0, 0, 0};
-      for (uint64_t left = shells; left; left &= left - 1) {
+      int n[4] = {__popcll(bits), __popcll(bits & 0x1249249249249249ull), __popcll(bits & 0x2492492492492492ull),
+                  __popcll(bits & 0x4924924924924924ull)};
+      if (!fit) n[0] = n[1] = n[2] = n[3] = 0;
+      for (uint64_t left = fit ? 0ull : shells; left; left &= left - 1) {
         const int at = __ffsll((long long)left) - 1, s = at / 3;
         const uint32_t m = (uint32_t)(bits >> at) & 7u;
         const int64_t base = __ldg(voff + (int64_t)s * G + e);
