@@ -51,30 +51,58 @@ __global__ void camera_positions_kernel(const float* __restrict__ ext, int B, fl
 // ---------------------------------------------------------------------------
 // project_vertices.slang:51-92. cam = W2C [v, 1]; xy = (K cam).xy / cam.z.
 // ---------------------------------------------------------------------------
-__global__ void project_kernel(const float* __restrict__ verts, int64_t V, const float* __restrict__ ext,
-                               const float* __restrict__ intr, int B, float* __restrict__ out_xy,
-                               float* __restrict__ out_depth) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
-    const float x = verts[3 * v], y = verts[3 * v + 1], z = verts[3 * v + 2];
-    for (int b = 0; b < B; ++b) {
-      const float* E = ext + 16 * b;
-      const float* K = intr + 9 * b;
-      // mul(W2C, float4(v, 1)) and mul(K, cam.xyz): row sums left to right.
-      float cam[3];
+// A CTA takes kEach vertices for each of its threads, so that a camera's 21
+// values are read once for them (they were a quarter of the instructions).
+// kPair: out_xy is 8-byte aligned. 14.7 M vertices and 4 cameras: 300 us with
+// one vertex to a thread and two stores of a position, now 233 (the writes alone
+// 130); 505,000 vertices 16, now 9.
+constexpr int kProjectThreads = 256;
+
+template <int kEach, bool kPair>
+__global__ void __launch_bounds__(kProjectThreads)
+    project_kernel(const float* __restrict__ verts, int64_t V, const float* __restrict__ ext,
+                   const float* __restrict__ intr, int B, float* __restrict__ out_xy, float* __restrict__ out_depth) {
+  for (int64_t base = blockIdx.x * (int64_t)(kEach * kProjectThreads) + threadIdx.x; base < V;
+       base += (int64_t)gridDim.x * (kEach * kProjectThreads)) {
+    float x[kEach], y[kEach], z[kEach];
 #pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        const float* row = E + 4 * r;
-        cam[r] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(row[0], x), __fmul_rn(row[1], y)), __fmul_rn(row[2], z)),
-                           __fmul_rn(row[3], 1.0f));
+    for (int j = 0; j < kEach; ++j) {
+      const int64_t v = min(base + j * kProjectThreads, V - 1);
+      x[j] = __ldg(verts + 3 * v);
+      y[j] = __ldg(verts + 3 * v + 1);
+      z[j] = __ldg(verts + 3 * v + 2);
+    }
+    for (int b = 0; b < B; ++b) {
+      float E[12], K[6];
+#pragma unroll
+      for (int i = 0; i < 12; ++i) E[i] = __ldg(ext + 16 * b + i);
+#pragma unroll
+      for (int i = 0; i < 6; ++i) K[i] = __ldg(intr + 9 * b + i);
+#pragma unroll
+      for (int j = 0; j < kEach; ++j) {
+        const int64_t v = base + j * kProjectThreads;
+        if (v >= V) break;
+        // mul(W2C, float4(v, 1)) and mul(K, cam.xyz): row sums left to right.
+        float cam[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+          cam[r] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(E[4 * r], x[j]), __fmul_rn(E[4 * r + 1], y[j])),
+                                       __fmul_rn(E[4 * r + 2], z[j])),
+                             __fmul_rn(E[4 * r + 3], 1.0f));
+        const float kx =
+            __fadd_rn(__fadd_rn(__fmul_rn(K[0], cam[0]), __fmul_rn(K[1], cam[1])), __fmul_rn(K[2], cam[2]));
+        const float ky =
+            __fadd_rn(__fadd_rn(__fmul_rn(K[3], cam[0]), __fmul_rn(K[4], cam[1])), __fmul_rn(K[5], cam[2]));
+        const int64_t o = (int64_t)b * V + v;
+        const float px = __fdiv_rn(kx, cam[2]), py = __fdiv_rn(ky, cam[2]);
+        if constexpr (kPair) {
+          reinterpret_cast<float2*>(out_xy)[o] = make_float2(px, py);
+        } else {
+          out_xy[2 * o] = px;
+          out_xy[2 * o + 1] = py;
+        }
+        out_depth[o] = cam[2];
       }
-      const float kx =
-          __fadd_rn(__fadd_rn(__fmul_rn(K[0], cam[0]), __fmul_rn(K[1], cam[1])), __fmul_rn(K[2], cam[2]));
-      const float ky =
-          __fadd_rn(__fadd_rn(__fmul_rn(K[3], cam[0]), __fmul_rn(K[4], cam[1])), __fmul_rn(K[5], cam[2]));
-      const int64_t o = (int64_t)b * V + v;
-      out_xy[2 * o] = __fdiv_rn(kx, cam[2]);
-      out_xy[2 * o + 1] = __fdiv_rn(ky, cam[2]);
-      out_depth[o] = cam[2];
     }
   }
 }
@@ -647,8 +675,19 @@ int mt_project_vertices(const float* vertices, int64_t V, const float* extrinsic
   MT_REQUIRE(V >= 0 && B >= 0);
   if (V == 0 || B == 0) return MT_OK;
   MT_REQUIRE(vertices && extrinsics && intrinsics && out_xy && out_depth);
-  project_kernel<<<grid_stride_blocks(V, 256), 256, 0, as_stream(stream)>>>(vertices, V, extrinsics, intrinsics, B,
-                                                                           out_xy, out_depth);
+  auto launch = [&](auto each, auto pair) {
+    constexpr int kEach = decltype(each)::value;
+    project_kernel<kEach, decltype(pair)::value>
+        <<<grid_stride_blocks(V, kEach * kProjectThreads), kProjectThreads, 0, as_stream(stream)>>>(
+            vertices, V, extrinsics, intrinsics, B, out_xy, out_depth);
+  };
+  // Four vertices to a thread where that leaves every SM two CTAs.
+  const bool four = V >= (int64_t)2 * kSmCount * 4 * kProjectThreads;
+  const bool pair = (reinterpret_cast<uintptr_t>(out_xy) & 7) == 0;
+  if (four && pair) launch(std::integral_constant<int, 4>{}, std::true_type{});
+  else if (four) launch(std::integral_constant<int, 4>{}, std::false_type{});
+  else if (pair) launch(std::integral_constant<int, 1>{}, std::true_type{});
+  else launch(std::integral_constant<int, 1>{}, std::false_type{});
   MT_CHECK_LAUNCH();
   return MT_OK;
 }
