@@ -914,7 +914,8 @@ __global__ void entry_list_kernel(const float* __restrict__ gsdf, const int32_t*
                                   const float* __restrict__ level_sets, int S, const int32_t* __restrict__ voff,
                                   const int32_t* __restrict__ inverse, int64_t V, int32_t* __restrict__ counts,
                                   uint32_t* __restrict__ segments, int2* __restrict__ list) {
-  const bool fit = (int64_t)__ldg(voff + (int64_t)S * G) <= V;  // no vertex past the capacity
+  // No vertex past the capacity. Without level sets a caller may have no offsets.
+  const bool fit = S == 0 || (int64_t)__ldg(voff + (int64_t)S * G) <= V;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < G; e += (int64_t)gridDim.x * blockDim.x) {
     const Corners4 c = load_corners(gsdf, lower, G, e);
     const uint64_t bits = crossing_bits(c, level_sets, 0, S);
