@@ -820,8 +820,9 @@ MT_API int mt_ssaa_loss(const float* raw, int32_t B, int32_t H, int32_t W, int32
  * __init__.py:274-287) from the compositing output: per output pixel, the
  * mean of rgb + T * background over its ssaa x ssaa sub-pixels, clipped to
  * [0,1]. raw: every camera's [4, h*ssaa, w*ssaa] back to back (so
- * [B,4,H,W] for cameras of one size); shapes: host [B,2], (h, w) of each
- * output image; images: host array of B device pointers, each [3,h,w]. */
+ * [B,4,H,W] for cameras of one size; NULL when no image has a pixel); shapes:
+ * host [B,2], (h, w) of each output image; images: host array of B device
+ * pointers, each [3,h,w] (NULL for one without pixels). */
 MT_API int mt_finish_images(const float* raw, int32_t B, const int32_t* shapes, int32_t ssaa,
                             const float* background, float* const* images, mt_stream_t stream);
 

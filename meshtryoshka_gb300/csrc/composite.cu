@@ -1863,6 +1863,13 @@ int for_finish_batches(int32_t B, float* const* images, const int32_t* shapes, i
   return MT_OK;
 }
 
+// Whether no camera's image has a pixel (its buffers may then be NULL).
+bool no_pixels(int32_t B, const int32_t* shapes) {
+  for (int32_t b = 0; b < B; ++b)
+    if (shapes[2 * b] > 0 && shapes[2 * b + 1] > 0) return false;
+  return true;
+}
+
 int check_args(const CompositeArgs& a) {
   if (a.B < 0 || a.S < 1 || a.rows < 0 || a.cols < 0 || a.tile_h < 1 || a.tile_w < 1 || a.H < 0 || a.W < 0)
     return MT_ERR_INVALID_ARGUMENT;
@@ -2188,7 +2195,8 @@ int mt_finish_images(const float* raw, int32_t B, const int32_t* shapes, int32_t
                      float* const* images, mt_stream_t stream) {
   MT_REQUIRE(B >= 0 && ssaa >= 1);
   if (B == 0) return MT_OK;
-  MT_REQUIRE(raw && shapes && background && images);
+  MT_REQUIRE(shapes && background && images);
+  MT_REQUIRE(raw || no_pixels(B, shapes));
   const bool even = (reinterpret_cast<uintptr_t>(raw) & 7) == 0;
   return for_finish_batches(B, images, shapes, ssaa, even, [&](auto kind, const FinishBatch& batch, unsigned ctas) {
     finish_images_kernel<decltype(kind)::value><<<ctas, kFinishThreads, 0, as_stream(stream)>>>(raw, batch, ssaa,
@@ -2201,7 +2209,8 @@ int mt_finish_images_backward(const float* raw, int32_t B, const int32_t* shapes
                               mt_stream_t stream) {
   MT_REQUIRE(B >= 0 && ssaa >= 1);
   if (B == 0) return MT_OK;
-  MT_REQUIRE(raw && shapes && background && grad_images && grad_raw);
+  MT_REQUIRE(shapes && background && grad_images);
+  MT_REQUIRE((raw && grad_raw) || no_pixels(B, shapes));
   const bool even = ((reinterpret_cast<uintptr_t>(raw) | reinterpret_cast<uintptr_t>(grad_raw)) & 7) == 0;
   float* const* grads = const_cast<float* const*>(grad_images);
   return for_finish_batches(B, grads, shapes, ssaa, even, [&](auto kind, const FinishBatch& batch, unsigned ctas) {

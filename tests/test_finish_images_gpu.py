@@ -97,3 +97,30 @@ def test_other_backgrounds_take_tensor_operations(cuda_device):
         assert tr._finishable(raw, plain.clone().requires_grad_(True))
     with torch.autograd.forward_ad.dual_level():
         assert not tr._finishable(raw, torch.autograd.forward_ad.make_dual(plain, torch.ones_like(plain)))
+
+
+@pytest.mark.parametrize("ssaa", [1, 2])
+@pytest.mark.parametrize("shape", [(0, 24), (16, 0), (0, 0)])
+def test_images_without_pixels(cuda_device, shape, ssaa):
+    """Empty images and zero gradients, from cameras of one size and of several."""
+    d = cuda_device
+    vertices = torch.tensor([[-1.0, -1, 0], [1, -1, 0], [0, 1, 0]], device=d)
+    faces = torch.tensor([[0, 1, 2]], dtype=torch.int32, device=d)
+    extrinsics = torch.eye(4, device=d).repeat(2, 1, 1)
+    extrinsics[:, 2, 3] = 3.0
+    intrinsics = torch.tensor([[10.0, 0, 5], [0, 10, 5], [0, 0, 1]], device=d).repeat(2, 1, 1)
+    sdf = torch.zeros(3, device=d, requires_grad=True)
+    sh = torch.ones(1, 3, 3, device=d, requires_grad=True)
+    args = (vertices, faces, torch.tensor([1], dtype=torch.int32, device=d), sdf, sh, 0, 40.0,
+            torch.tensor(BACKGROUND, device=d))
+    image = tr.render_fused(extrinsics, intrinsics, shape, *args, ssaa=ssaa)
+    assert image.shape == (2, 3, *shape)
+    grads = torch.autograd.grad(image.sum(), (sdf, sh))
+    assert [g.shape for g in grads] == [(3,), (1, 3, 3)] and not any(g.any() for g in grads)
+    if ssaa == 1:
+        images = tr.render_cameras(extrinsics, intrinsics, [shape, (0, 7)], *args)
+        assert [x.shape for x in images] == [(3, *shape), (3, 0, 7)]
+        grads = torch.autograd.grad(sum(x.sum() for x in images), (sdf, sh))
+        assert not any(g.any() for g in grads)
+        images = tr.render_cameras(extrinsics, intrinsics, [shape, (9, 7)], *args)
+        assert [x.shape for x in images] == [(3, *shape), (3, 9, 7)]
