@@ -508,6 +508,25 @@ class _PackedGradients:
                 nt.stream(self.rows.device))
         return self.rows[..., :3] if in_place else colors, sdf
 
+    def split_like(self, colors: Tensor, sdf: Tensor, in_place: bool) -> tuple[Tensor, Tensor]:
+        """``split`` in the shapes of the kernel's inputs, which it reads flat:
+        signed distances may be a column, and both longer than the vertices."""
+        b, v, _ = self.rows.shape
+        grad_colors, grad_sdf = self.split(in_place and colors.shape == (b, v, 3))
+        return _flat_like(grad_colors, colors), _flat_like(grad_sdf, sdf)
+
+
+def _flat_like(grad: Tensor, like: Tensor) -> Tensor:
+    """``grad`` in the shape of ``like``, element by element; zeros past its end."""
+    if grad.shape == like.shape:
+        return grad
+    if grad.numel() == like.numel():
+        return grad.view(like.shape)
+    out = torch.zeros_like(like)
+    n = min(grad.numel(), like.numel())
+    out.view(-1)[:n] = grad.view(-1)[:n]
+    return out
+
 
 class EvaluateSphericalHarmonics(torch.autograd.Function):
     @staticmethod
@@ -681,7 +700,7 @@ class IntersectAndComposite(torch.autograd.Function):
                     int(mode == "exact"), nt.ptr(ctx.hits), _numel(ctx.hits),
                     nt.ptr(staging), _numel(staging), nt.ptr(ctx.order), _numel(ctx.order), grid.cta_threads,
                     nt.stream(device))
-            grad_colors, grad_sdf = packed.split(packed_colour_gradient)
+            grad_colors, grad_sdf = packed.split_like(colors, sdf, packed_colour_gradient)
             return (None, grad_colors, grad_sdf, None, grad_sharp if sharp_is_tensor else None, None, None, None,
                     None, None, None, None, None, None)
 
@@ -768,7 +787,7 @@ class IntersectCompositeLoss(torch.autograd.Function):
                     nt.ptr(packed.rows), nt.ptr(grad_sharp), int(mode == "exact"),
                     nt.ptr(ctx.hits), _numel(ctx.hits), nt.ptr(staging), _numel(staging), nt.ptr(ctx.order),
                     _numel(ctx.order), grid.cta_threads, nt.stream(device))
-            grad_colors, grad_sdf = packed.split(packed_colour_gradient)
+            grad_colors, grad_sdf = packed.split_like(colors, sdf, packed_colour_gradient)
             return (None, grad_colors, grad_sdf, None, grad_sharp if sharp_is_tensor else None, None, None, None,
                     None, None, None, None, None, None, None, None, None)
 
@@ -966,7 +985,7 @@ class ShadeShells(torch.autograd.Function):
             if background is None or any(ctx.needs_input_grad):
                 out_colors, out_t = torch.empty((b * h * w, 3), **kw), torch.empty((b * h * w,), **kw)
             nt.call("mt_shade_shells", nt.ptr(uv), nt.ptr(index), b, s, h, w, nt.ptr(faces), nt.ptr(sdf),
-                    nt.ptr(colors), sdf.shape[0], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
+                    nt.ptr(colors), colors.shape[1], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
                     nt.ptr(out_t), nt.ptr(image), nt.stream(device))
             ctx.save_for_backward(uv, index, faces, sdf, colors, sharp, background, out_colors, out_t)
             ctx.meta = (gradient_mode or _GRADIENT_MODE, torch.is_tensor(sharpness), packed_colour_gradient)
@@ -981,14 +1000,14 @@ class ShadeShells(torch.autograd.Function):
             device = sdf.device
             b, s, h, w = index.shape
             gsharp = torch.zeros_like(sharp)
-            packed = _PackedGradients(b, sdf.shape[0], device)
+            packed = _PackedGradients(b, colors.shape[1], device)
             go = grad_out.contiguous() if grad_out is not None else None
             gt = grad_t.contiguous() if grad_t is not None else None
             nt.call("mt_shade_shells_backward", nt.ptr(uv), nt.ptr(index), b, s, h, w, nt.ptr(faces), nt.ptr(sdf),
-                    nt.ptr(colors), sdf.shape[0], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
+                    nt.ptr(colors), colors.shape[1], nt.ptr(sharp), nt.ptr(background), nt.ptr(out_colors),
                     nt.ptr(out_t), nt.ptr(go), nt.ptr(gt), nt.ptr(packed.rows), nt.ptr(gsharp),
                     int(mode == "exact"), nt.stream(device))
-            gcol, gsdf = packed.split(packed_colour_gradient)
+            gcol, gsdf = packed.split_like(colors, sdf, packed_colour_gradient)
             return None, None, None, gsdf, gcol, gsharp if sharp_is_tensor else None, None, None, None
 
 

@@ -92,3 +92,41 @@ def test_stage_and_render_gradients(cuda_device, mode, tile):
     want = torch.autograd.grad((chained[:, :3] + chained[:, 3:] * background[:, None, None]).clip(0, 1), (sdf, sh), gi)
     for a, x in zip(got, want):
         _close(a, x)
+
+
+@pytest.mark.parametrize("call", ["fused", "explicit", "cameras", "loss"])
+@pytest.mark.parametrize("shape", ["column", "longer"])
+def test_gradients_have_the_inputs_shapes(cuda_device, call, shape):
+    """Signed distances as a column, or in a buffer longer than the vertices."""
+    sc = make_scene(n=32, sh_degree=1, image_shape=(48, 40))
+    d = cuda_device
+    ext, intr, vertices, faces, sfb, sh, background = (
+        torch.from_numpy(np.ascontiguousarray(x)).to(d)
+        for x in (sc.extrinsics, sc.intrinsics, sc.vertices, sc.faces, sc.face_boundaries, sc.sh, sc.background))
+    plain = torch.from_numpy(sc.sdf).to(d)
+    other = plain[:, None] if shape == "column" else torch.cat((plain, plain.new_full((37,), 5.0)))
+    target = torch.zeros((1, 3, *sc.image_shape), device=d)
+
+    def gradients(sdf):
+        sdf, rows = sdf.clone().requires_grad_(True), sh.clone().requires_grad_(True)
+        mesh = (vertices, faces, sfb, sdf, rows, sc.sh_degree, 40.0, background)
+        if call == "loss":
+            loss = tr.render_fused_loss(ext, intr, sc.image_shape, *mesh, target)
+        elif call == "cameras":
+            loss = sum((x ** 2).mean() for x in tr.render_cameras(ext, intr, [sc.image_shape], *mesh))
+        else:
+            loss = (tr.render(ext, intr, sc.image_shape, *mesh, mode=call) ** 2).mean()
+        return torch.autograd.grad(loss, (sdf, rows))
+
+    want, want_sh = gradients(plain)
+    got, got_sh = gradients(other)
+    assert got.shape == other.shape
+    _close(got.view(-1)[:len(plain)], want)
+    _close(got_sh, want_sh)
+    assert not got.view(-1)[len(plain):].any()
+
+
+def test_gradient_of_longer_colours(cuda_device):
+    grad = torch.randn((1, 5, 3), device=cuda_device)
+    assert torch.equal(tr._flat_like(grad, torch.empty((1, 7, 3), device=cuda_device))[:, :5], grad)
+    assert tr._flat_like(grad, grad) is grad
