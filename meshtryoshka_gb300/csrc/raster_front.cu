@@ -333,13 +333,15 @@ __device__ __forceinline__ uint32_t face_shell(const int32_t* __restrict__ sfb, 
 //
 // The B*F items are split into chunks of kFusedItems x kFusedThreads items,
 // one CTA each, striped (item j * kFusedThreads + tid of the chunk) so that a
-// warp's loads are adjacent. Three launches, no CTA waits on another:
+// warp's loads are adjacent. Three launches (four for many chunks), no CTA
+// waits on another:
 //   chunk_bounds_kernel  the tile rectangle (int4) and key depth of the items
 //                        that touch a tile, in item order at the start of the
 //                        chunk's records, with their places in the chunk; and
 //                        the chunk's item and key counts;
-//   chunk_scan_kernel    one CTA: exclusive scan of the chunks' key counts, and
-//                        the total (many chunks: the library's scan);
+//   chunk_scan_kernel    exclusive scan of the chunks' key counts, and the
+//                        total: one CTA, or for many chunks one to each group
+//                        of them and then one over the groups' totals;
 //   chunk_keys_kernel    reads its chunk's records back (coalesced), scans
 //                        them and writes the keys.
 // Most items touch no tile (back faces, faces outside the image), and a record
@@ -350,10 +352,10 @@ constexpr int kFusedThreads = 256;
 constexpr int kFusedItems = 4;
 constexpr int kFusedSubTile = kFusedThreads * kFusedItems;
 constexpr int kChunkScanThreads = 1024;
-// Workspace: [0,256) status word (unused here), the chunks' key counts (int64
-// each) and item counts (int32 each), the rectangle records (int4 per item),
-// the key depths (float per item) and the places (uint16 per item); each region
-// starts on a 256-byte boundary.
+// Workspace: [0,256) status word (unused here: nothing waits), the chunks' key
+// counts (int64 each) and item counts (int32 each), the groups' totals (int64
+// each), the rectangle records (int4 per item), the key depths (float per item)
+// and the places (uint16 per item); each region starts on a 256-byte boundary.
 constexpr size_t kFusedHeader = 256;
 
 __host__ __device__ inline size_t round256(size_t x) { return (x + 255) / 256 * 256; }
@@ -445,13 +447,12 @@ __device__ __forceinline__ T block_sum(T x, T* s_warp) {
 }
 
 struct ChunkRecords {
-  int64_t* keys;    // per chunk: key count, then (scanned) its first key; and one more
+  int64_t* keys;    // per chunk: key count, then (scanned) its first key, of its group where there are groups
   int32_t* items;   // per chunk: records
+  int64_t* groups;  // per kScanGroup chunks: key count, then (scanned) its first key; NULL: one group
   int4* rect;       // per record (a chunk's start at its first item)
   float* depth;
   uint16_t* place;  // item's place in its chunk
-  void* scan;       // the key counts' scan
-  size_t scan_bytes;
 };
 
 __global__ void __launch_bounds__(kFusedThreads, 3) chunk_bounds_kernel(FusedArgs a, ChunkRecords rec) {
@@ -493,27 +494,29 @@ __global__ void __launch_bounds__(kFusedThreads, 3) chunk_bounds_kernel(FusedArg
   if (threadIdx.x == 0) {
     rec.keys[blockIdx.x] = total;
     rec.items[blockIdx.x] = all;
-    if (blockIdx.x == 0) rec.keys[gridDim.x] = 0;  // becomes the total
   }
 }
 
-// Exclusive scan of the chunk counts in place (one CTA); *out_count = total.
-// Rounds of kChunkScanThreads x 4 counts, each thread's four loaded together.
-// For few chunks: beyond kOneCtaChunks the library's scan over many CTAs takes
-// over (512^3's 117,000 chunks were 29 rounds here, 117 us).
-constexpr int64_t kOneCtaChunks = 16 * kChunkScanThreads;
+// Exclusive scans in place, a CTA to each `group` consecutive counts; totals[CTA]
+// = its sum. Rounds of kScanGroup counts, each thread's four loaded together.
+// Up to kOneCtaChunks chunks are one group; of more, every round gets a CTA of
+// its own and the totals a second launch (512^3's 117,000 chunks in 29 rounds of
+// one CTA took 117 us).
+constexpr int kScanGroup = 4 * kChunkScanThreads;
+constexpr int64_t kOneCtaChunks = 4 * kScanGroup;
 
 __global__ void __launch_bounds__(kChunkScanThreads)
-    chunk_scan_kernel(int64_t* __restrict__ counts, int64_t chunks, int64_t* __restrict__ out_count) {
-  constexpr int kPer = 4;
+    chunk_scan_kernel(int64_t* __restrict__ counts, int64_t chunks, int64_t group, int64_t* __restrict__ totals) {
+  constexpr int kPer = kScanGroup / kChunkScanThreads;
   __shared__ int64_t s_warp[kChunkScanThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t begin = blockIdx.x * group, end = min(begin + group, chunks);
   int64_t running = 0;
-  for (int64_t base = 0; base < chunks; base += (int64_t)kChunkScanThreads * kPer) {
+  for (int64_t base = begin; base < end; base += kScanGroup) {
     const int64_t c0 = base + (int64_t)tid * kPer;
     int64_t x[kPer];
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) x[k] = c0 + k < chunks ? counts[c0 + k] : 0;
+    for (int k = 0; k < kPer; ++k) x[k] = c0 + k < end ? counts[c0 + k] : 0;
     int64_t mine = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) mine += x[k];
@@ -530,13 +533,13 @@ __global__ void __launch_bounds__(kChunkScanThreads)
     int64_t run = running + below + inc - mine;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-      if (c0 + k < chunks) counts[c0 + k] = run;
+      if (c0 + k < end) counts[c0 + k] = run;
       run += x[k];
     }
     running += all;
     __syncthreads();
   }
-  if (tid == 0) *out_count = running;
+  if (tid == 0) totals[blockIdx.x] = running;
 }
 
 // Each thread writes the keys of its records (in row-major tile order, at the
@@ -552,7 +555,7 @@ __global__ void __launch_bounds__(kFusedThreads)
   const int64_t first = blockIdx.x * (int64_t)kFusedSubTile;
   const int first_cam = (int)(first / a.F);
   const int64_t first_face = first - (int64_t)first_cam * a.F;
-  int64_t base = rec.keys[blockIdx.x];
+  int64_t base = rec.keys[blockIdx.x] + (rec.groups ? rec.groups[blockIdx.x / kScanGroup] : 0);
   int turn = 0;
   for (int p0 = 0; p0 < many; p0 += kFusedThreads, turn ^= 1) {
     const int64_t i = first + p0 + tid;
@@ -756,23 +759,26 @@ static int64_t fused_chunks(int64_t items) { return (items + kFusedSubTile - 1) 
 
 static size_t chunk_records(int64_t items, char* base, ChunkRecords* rec) {
   const int64_t chunks = fused_chunks(items);
+  const int64_t groups = chunks > kOneCtaChunks ? (chunks + kScanGroup - 1) / kScanGroup : 0;
   size_t off = kFusedHeader;
   auto take = [&](size_t bytes) {
     char* p = base ? base + off : nullptr;
     off += round256(bytes);
     return p;
   };
-  char* keys = take((size_t)(chunks + 1) * sizeof(int64_t));
+  char* keys = take((size_t)chunks * sizeof(int64_t));
   char* counts = take((size_t)chunks * sizeof(int32_t));
+  char* totals = take((size_t)groups * sizeof(int64_t));
   char* rect = take((size_t)items * sizeof(int4));
   char* depth = take((size_t)items * sizeof(float));
   char* place = take((size_t)items * sizeof(uint16_t));
-  const size_t scan_bytes = mt_scan_workspace_bytes(chunks + 1);
-  char* scan = take(scan_bytes);
   if (rec)
-    *rec = ChunkRecords{reinterpret_cast<int64_t*>(keys), reinterpret_cast<int32_t*>(counts),
-                        reinterpret_cast<int4*>(rect), reinterpret_cast<float*>(depth),
-                        reinterpret_cast<uint16_t*>(place), scan, scan_bytes};
+    *rec = ChunkRecords{reinterpret_cast<int64_t*>(keys),
+                        reinterpret_cast<int32_t*>(counts),
+                        groups ? reinterpret_cast<int64_t*>(totals) : nullptr,
+                        reinterpret_cast<int4*>(rect),
+                        reinterpret_cast<float*>(depth),
+                        reinterpret_cast<uint16_t*>(place)};
   return off;
 }
 
@@ -801,14 +807,15 @@ int mt_bound_keys(const float* xy, const float* depth, int64_t V, const int32_t*
   const FusedArgs a{xy, depth, V, faces, F, num_faces, B, tile_h, tile_w, rows, cols, cameras, near_plane};
   chunk_bounds_kernel<<<(unsigned)chunks, kFusedThreads, 0, s>>>(a, rec);
   MT_CHECK_LAUNCH();
-  if (chunks > kOneCtaChunks) {
-    const int rc = mt_exclusive_scan_i64(rec.keys, chunks + 1, rec.scan, rec.scan_bytes, stream);
-    if (rc != MT_OK) return rc;
-    if (cudaMemcpyAsync(out_num_keys, rec.keys + chunks, sizeof(int64_t), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-      return MT_ERR_CUDA;
-    return MT_OK;
+  int64_t* counts = rec.keys;
+  int64_t many = chunks;
+  if (rec.groups) {
+    many = (chunks + kScanGroup - 1) / kScanGroup;
+    chunk_scan_kernel<<<(unsigned)many, kChunkScanThreads, 0, s>>>(rec.keys, chunks, kScanGroup, rec.groups);
+    MT_CHECK_LAUNCH();
+    counts = rec.groups;
   }
-  chunk_scan_kernel<<<1, kChunkScanThreads, 0, s>>>(rec.keys, chunks, out_num_keys);
+  chunk_scan_kernel<<<1, kChunkScanThreads, 0, s>>>(counts, many, many, out_num_keys);
   MT_CHECK_LAUNCH();
   return MT_OK;
 }

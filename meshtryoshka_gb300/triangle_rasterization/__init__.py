@@ -370,8 +370,13 @@ def bound_and_generate_keys(vertices: Tensor, depths: Tensor, faces: Tensor, she
     nt.call("mt_bound_and_generate_keys", nt.ptr(vertices), nt.ptr(depths), v, nt.ptr(faces), f, nt.ptr(nf),
             nt.ptr(sfb), sfb.shape[0], c, grid.tile_shape[0], grid.tile_shape[1], rows, cols,
             nt.ptr(_camera_table(grid, device)), float(near_plane), _layout(key_defines), num_keys, nt.ptr(keys),
-            nt.ptr(tri), live.data_ptr(), ws_ptr, ws_bytes, nt.stream(device))
+            nt.ptr(tri), live.data_ptr(), ws_ptr, ws_bytes, nt.stream(device),
+            launches=3 + (c * f > _ONE_SCAN_ITEMS))
     return PairedKeys(keys, tri, live)
+
+
+# (camera, face) items whose chunk counts one CTA scans; more take one launch more.
+_ONE_SCAN_ITEMS = 1 << 24
 
 
 def _keys(positions, depths, faces, shell_face_boundaries, grid, near_plane, num_faces, key_defines,
@@ -399,7 +404,7 @@ def _keys(positions, depths, faces, shell_face_boundaries, grid, near_plane, num
         count = torch.empty((), dtype=torch.int64, device=device)
         nt.call("mt_bound_keys", nt.ptr(vertices), nt.ptr(depths), v, nt.ptr(faces), f, nt.ptr(nf), c,
                 grid.tile_shape[0], grid.tile_shape[1], rows, cols, nt.ptr(table), float(near_plane), count.data_ptr(),
-                records.data_ptr(), need, nt.stream(device))
+                records.data_ptr(), need, nt.stream(device), launches=2 + (c * f > _ONE_SCAN_ITEMS))
         num_keys = int(count.item())
         keys = torch.empty(num_keys, dtype=torch.int64, device=device)
         tri = torch.empty(num_keys, dtype=torch.int32, device=device)

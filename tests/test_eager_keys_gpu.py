@@ -41,3 +41,30 @@ def test_equal_the_chain(cuda_device, b, f, spread, ragged):
         want = tr.generate_keys(t[1], t[2], t[3], rect.tile_minima, rect.tile_maxima, rect.num_tiles_overlapped, grid, kd)
         assert torch.equal(got.keys, want.keys)
         assert torch.equal(got.triangle_indices, want.triangle_indices)
+
+
+@pytest.mark.parametrize("b,f", [(1, 1 << 24), (1, (1 << 24) + 1), (3, 5_600_017), (2, (5 << 22) // 2 + 1024)])
+def test_many_chunks(cuda_device, b, f):
+    """Counts scanned by one CTA at most, and by one to each group of chunks: at
+    the line between them, a group's edge and within one. Also by capacity."""
+    d = cuda_device
+    rng = torch.Generator(d).manual_seed(f)
+    v, h, w = 4096, 64, 96
+    xy = torch.rand((b, v, 2), generator=rng, device=d) * 40 * w
+    depth = torch.rand((b, v), generator=rng, device=d) + 0.5
+    first = torch.randint(0, v - 2, (f, 1), generator=rng, device=d, dtype=torch.int32)
+    faces = (first + torch.arange(3, dtype=torch.int32, device=d)).contiguous()
+    xy[:, 1::2] = xy[:, ::2] + torch.rand((b, v // 2, 2), generator=rng, device=d) * 9
+    faces[f // 2:, 1:] = faces[f // 2:, 1:].flip(1)
+    bounds = torch.tensor([f // 3, f // 2, f], dtype=torch.int32, device=d)
+    grid = tr.TileGrid((16, 8), (h, w), b, 3)
+    kd = tr.create_key_defines(("camera", 7), ("tile", 19), ("depth", 32), ("shell", 6))
+    rect = tr.bound_triangles(xy, depth, faces, grid, 0.2)
+    want = tr.generate_keys(depth, faces, bounds, rect.tile_minima, rect.tile_maxima, rect.num_tiles_overlapped, grid, kd)
+    assert want.keys.numel() > 0
+    got = tr._keys(xy, depth, faces, bounds, grid, 0.2, None, kd, None)
+    assert torch.equal(got.keys, want.keys) and torch.equal(got.triangle_indices, want.triangle_indices)
+    n = want.keys.numel() - 1  # one key too few
+    got = tr._keys(xy, depth, faces, bounds, grid, 0.2, None, kd, n)
+    assert int(got.count) == n + 1
+    assert torch.equal(got.keys, want.keys[:n]) and torch.equal(got.triangle_indices, want.triangle_indices[:n])

@@ -97,3 +97,10 @@ def test_compositing_buffer_sizes_without_gpu():
     assert lib.mt_composite_tile_order_bytes(0) == 512 * 4
     assert lib.mt_composite_staging_bytes(4, 1000) == 128 + 32 * 4 * 1000
     assert lib.mt_composite_staging_bytes(0, 1000) == 0
+
+
+def test_no_wait_of_the_key_kernels_goes_unreported():
+    """A look-back scan reports a wait that gave up through its workspace's status
+    word; the key kernels, whose workspace nobody reads one from, wait on nothing."""
+    source = (ROOT / "meshtryoshka_gb300" / "csrc" / "raster_front.cu").read_text()
+    assert not re.findall(r"mt_exclusive_scan_\w+\(|mt_inclusive_scan_\w+\(|lookback_prefix", source)
