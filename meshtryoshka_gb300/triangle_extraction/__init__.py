@@ -485,8 +485,16 @@ def _vertex_offsets(signed_distances: Tensor, lower_corners: Tensor, level_sets:
 # vertex's gradient once per list entry and needs no scratch (same values). At
 # the 512^3 / 16-shell scene (3.5 GB) the two passes take 1.26 ms, one 1.92.
 GRID_SH_BACKWARD_SCRATCH_LIMIT = 4 << 30
-# Scratch above this size is allocated for the call, not kept as workspace.
+# Scratch above this size is allocated for the call, not kept as workspace, and
+# the one-pass form runs where the device has no room for it.
 _KEPT_SCRATCH = 512 << 20
+
+
+def _scratch(nbytes: int, device) -> Tensor | None:
+    try:
+        return torch.empty((nbytes,), dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 # Renders form the colours of only the vertices that some key's triangle names,
@@ -585,11 +593,10 @@ class GridSHColors(torch.autograd.Function):
             grad_gsh = torch.empty(ctx.gsh_shape, dtype=torch.float32, device=device)  # fully written
             v = vertices.shape[0]
             need = nt.library().mt_grid_sh_colors_backward_workspace_bytes(v)
-            if need > GRID_SH_BACKWARD_SCRATCH_LIMIT:
-                ws_ptr, ws_bytes = None, 0  # the one-pass form: no scratch
-            elif need > _KEPT_SCRATCH:
-                scratch = torch.empty((need,), dtype=torch.uint8, device=device)
-                ws_ptr, ws_bytes = scratch.data_ptr(), need
+            if need > _KEPT_SCRATCH or need > GRID_SH_BACKWARD_SCRATCH_LIMIT:
+                scratch = _scratch(need, device) if need <= GRID_SH_BACKWARD_SCRATCH_LIMIT else None
+                # None: the one-pass form.
+                ws_ptr, ws_bytes = (None, 0) if scratch is None else (scratch.data_ptr(), need)
             else:
                 ws_ptr, ws_bytes = nt.workspace(device).get(need)
             rows, packed = nt.colour_gradient_rows(grad_colors)

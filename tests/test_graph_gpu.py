@@ -16,6 +16,7 @@ from __future__ import annotations
 import pytest
 import torch
 
+from meshtryoshka_gb300 import _native as nt
 from meshtryoshka_gb300 import graph, pipeline
 from meshtryoshka_gb300 import triangle_extraction as te
 from meshtryoshka_gb300 import triangle_rasterization as tr
@@ -222,3 +223,51 @@ def test_captured_step_input_set_with_other_cameras(cuda_device):
     assert abs(loss1 - loss_e) <= LOSS_RTOL * abs(loss_e)
     _close(g_sdf, gsdf_e)
     _close(g_sh, gsh_e)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_grid_sh_backward_on_a_full_device(cuda_device, monkeypatch, captured):
+    """Where the two-pass form's scratch cannot be allocated, the one-pass form
+    gives the same bits; also inside a capture."""
+    stream = torch.cuda.Stream()  # the capture's, and autograd's: the leaves' too
+    with torch.cuda.stream(stream):
+        w = pipeline.build_workload("small", cuda_device)
+        with torch.no_grad():
+            _, stats = pipeline.forward(w)
+        caps = pipeline.Capacities.around(stats)
+        gsh = w.grid_sh.detach().clone().requires_grad_(True)
+
+        def gradient():
+            tri, counts = te.tessellate_voxels_counted(
+                w.grid_sdf.detach(), w.voxels.vertices, gsh, w.voxels.neighbors, w.voxels.lower_corners,
+                w.voxels.upper_corners, w.voxels.indices, w.level_sets, caps.vertices, caps.faces, defer_sh=True)
+            verts = pipeline.uncontract_stand_in(tri.vertices.detach())
+            colors = tr.evaluate_spherical_harmonics(verts, tri.spherical_harmonics, w.extrinsics, w.sh_degree)
+            live = torch.arange(colors.shape[1], device=cuda_device) < counts.num_vertices
+            return torch.autograd.grad((colors * live[:, None]).sum(), gsh)[0]
+
+        want = gradient()
+        assert float(want.abs().max()) > 0
+
+        monkeypatch.setattr(te, "_KEPT_SCRATCH", 0)  # allocated for the call, as the largest scenes' is
+        empty, refused = torch.empty, []
+        need = int(nt.library().mt_grid_sh_colors_backward_workspace_bytes(caps.vertices))
+
+        def full(*args, **kwargs):
+            if args == ((need,),):
+                refused.append(args)
+                raise torch.OutOfMemoryError("no room")
+            return empty(*args, **kwargs)
+
+        monkeypatch.setattr(torch, "empty", full)
+        torch.cuda.synchronize()
+        if captured:
+            capture = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(capture, stream=stream):
+                got = gradient()
+            capture.replay()
+        else:
+            got = gradient()
+        torch.cuda.synchronize()
+        assert refused
+        torch.testing.assert_close(got, want, rtol=0, atol=0)
