@@ -341,7 +341,7 @@ __device__ __forceinline__ uint32_t face_shell(const int32_t* __restrict__ sfb, 
 //                        the chunk's item and key counts;
 //   chunk_scan_kernel    exclusive scan of the chunks' key counts, and the
 //                        total: one CTA, or for many chunks one to each group
-//                        of them and then one over the groups' totals;
+//                        of them, after chunk_group_kernel has summed each;
 //   chunk_keys_kernel    reads its chunk's records back (coalesced), scans
 //                        them and writes the keys.
 // Most items touch no tile (back faces, faces outside the image), and a record
@@ -447,9 +447,9 @@ __device__ __forceinline__ T block_sum(T x, T* s_warp) {
 }
 
 struct ChunkRecords {
-  int64_t* keys;    // per chunk: key count, then (scanned) its first key, of its group where there are groups
+  int64_t* keys;    // per chunk: key count, then (scanned) its first key
   int32_t* items;   // per chunk: records
-  int64_t* groups;  // per kScanGroup chunks: key count, then (scanned) its first key; NULL: one group
+  int64_t* groups;  // per kScanGroup chunks: key count; NULL: one group
   int4* rect;       // per record (a chunk's start at its first item)
   float* depth;
   uint16_t* place;  // item's place in its chunk
@@ -497,21 +497,51 @@ __global__ void __launch_bounds__(kFusedThreads, 3) chunk_bounds_kernel(FusedArg
   }
 }
 
-// Exclusive scans in place, a CTA to each `group` consecutive counts; totals[CTA]
-// = its sum. Rounds of kScanGroup counts, each thread's four loaded together.
-// Up to kOneCtaChunks chunks are one group; of more, every round gets a CTA of
-// its own and the totals a second launch (512^3's 117,000 chunks in 29 rounds of
-// one CTA took 117 us).
-constexpr int kScanGroup = 4 * kChunkScanThreads;
+// Exclusive scan of the chunk counts in place, a CTA to each `group` consecutive
+// ones; *out_count = total. Rounds of kScanGroup counts, each thread's four
+// loaded together. Up to kOneCtaChunks chunks are one group (512^3's 117,000 in
+// 29 rounds of one CTA took 117 us); of more, every kScanGroup are one, whose
+// sum is known (`totals`), and each CTA adds up those of the groups before it.
+constexpr int kScanPer = 4, kScanGroup = kScanPer * kChunkScanThreads;
 constexpr int64_t kOneCtaChunks = 4 * kScanGroup;
 
+// Sum of x over the CTA's kChunkScanThreads threads.
+__device__ __forceinline__ int64_t scan_block_sum(int64_t x, int64_t* s_warp) {
+  x = warp_sum(x);
+  if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = x;
+  __syncthreads();
+  int64_t total = 0;
+#pragma unroll
+  for (int w = 0; w < kChunkScanThreads / 32; ++w) total += s_warp[w];
+  __syncthreads();
+  return total;
+}
+
 __global__ void __launch_bounds__(kChunkScanThreads)
-    chunk_scan_kernel(int64_t* __restrict__ counts, int64_t chunks, int64_t group, int64_t* __restrict__ totals) {
-  constexpr int kPer = kScanGroup / kChunkScanThreads;
+    chunk_group_kernel(const int64_t* __restrict__ counts, int64_t chunks, int64_t* __restrict__ totals) {
+  __shared__ int64_t s_warp[kChunkScanThreads / 32];
+  int64_t mine = 0;
+#pragma unroll
+  for (int k = 0; k < kScanPer; ++k) {
+    const int64_t c = blockIdx.x * (int64_t)kScanGroup + k * kChunkScanThreads + threadIdx.x;
+    mine += c < chunks ? counts[c] : 0;
+  }
+  const int64_t total = scan_block_sum(mine, s_warp);
+  if (threadIdx.x == 0) totals[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kChunkScanThreads)
+    chunk_scan_kernel(int64_t* __restrict__ counts, int64_t chunks, int64_t group,
+                      const int64_t* __restrict__ totals, int64_t* __restrict__ out_count) {
+  constexpr int kPer = kScanPer;
   __shared__ int64_t s_warp[kChunkScanThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t begin = blockIdx.x * group, end = min(begin + group, chunks);
   int64_t running = 0;
+  if (totals) {
+    for (int64_t g = tid; g < blockIdx.x; g += kChunkScanThreads) running += totals[g];
+    running = scan_block_sum(running, s_warp);
+  }
   for (int64_t base = begin; base < end; base += kScanGroup) {
     const int64_t c0 = base + (int64_t)tid * kPer;
     int64_t x[kPer];
@@ -539,7 +569,7 @@ __global__ void __launch_bounds__(kChunkScanThreads)
     running += all;
     __syncthreads();
   }
-  if (tid == 0) totals[blockIdx.x] = running;
+  if (tid == 0 && blockIdx.x == gridDim.x - 1) *out_count = running;
 }
 
 // Each thread writes the keys of its records (in row-major tile order, at the
@@ -555,7 +585,7 @@ __global__ void __launch_bounds__(kFusedThreads)
   const int64_t first = blockIdx.x * (int64_t)kFusedSubTile;
   const int first_cam = (int)(first / a.F);
   const int64_t first_face = first - (int64_t)first_cam * a.F;
-  int64_t base = rec.keys[blockIdx.x] + (rec.groups ? rec.groups[blockIdx.x / kScanGroup] : 0);
+  int64_t base = rec.keys[blockIdx.x];
   int turn = 0;
   for (int p0 = 0; p0 < many; p0 += kFusedThreads, turn ^= 1) {
     const int64_t i = first + p0 + tid;
@@ -807,15 +837,13 @@ int mt_bound_keys(const float* xy, const float* depth, int64_t V, const int32_t*
   const FusedArgs a{xy, depth, V, faces, F, num_faces, B, tile_h, tile_w, rows, cols, cameras, near_plane};
   chunk_bounds_kernel<<<(unsigned)chunks, kFusedThreads, 0, s>>>(a, rec);
   MT_CHECK_LAUNCH();
-  int64_t* counts = rec.keys;
-  int64_t many = chunks;
+  const int64_t group = rec.groups ? kScanGroup : chunks;
+  const unsigned groups = (unsigned)((chunks + group - 1) / group);
   if (rec.groups) {
-    many = (chunks + kScanGroup - 1) / kScanGroup;
-    chunk_scan_kernel<<<(unsigned)many, kChunkScanThreads, 0, s>>>(rec.keys, chunks, kScanGroup, rec.groups);
+    chunk_group_kernel<<<groups, kChunkScanThreads, 0, s>>>(rec.keys, chunks, rec.groups);
     MT_CHECK_LAUNCH();
-    counts = rec.groups;
   }
-  chunk_scan_kernel<<<1, kChunkScanThreads, 0, s>>>(counts, many, many, out_num_keys);
+  chunk_scan_kernel<<<groups, kChunkScanThreads, 0, s>>>(rec.keys, chunks, group, rec.groups, out_num_keys);
   MT_CHECK_LAUNCH();
   return MT_OK;
 }
