@@ -30,9 +30,10 @@
 // store's capacity lasts; the backward re-walks the same way, reads those
 // bits instead of testing again (gathering only the triangles some pixel
 // hits), re-solves each hit's barycentrics and applies the suffix trick of
-// the reference. Batches past the capacity are tested again. A hit's gradient
-// goes to its triangle's three vertices in global memory: colour and signed
-// distance of a (camera, vertex) side by side, one 16-byte reduction each.
+// the reference. Batches past the capacity are tested again. Hits' gradients
+// go to their triangles' three vertices in global memory, summed first over the
+// warp's lanes that hold hits of one triangle: colour and signed distance of a
+// (camera, vertex) side by side, one 16-byte reduction each.
 // Two routings:
 //   reference (exact_adjoint = 0): the deferred gradient of the previous
 //     (outer) hit is scattered to the previous triangle's vertices with the
@@ -1200,30 +1201,59 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps)
   }
 }
 
-// Adds a hit's gradient to its triangle's vertices. (Sums per triangle in
-// shared memory, flushed when its batch retired, cost more than they saved:
-// shared-memory float additions are loops of compare-and-swap, and a triangle
-// of a fine mesh has two to four hits in a warp. Five million hits: 60 to 80 us
-// as 16-byte reductions, 40 to 170 us in shared memory and 150 to 200 us as
-// scalar ones. Backward kernel of the 256^3 step: 195 us with the sums, now
-// 118; of the 512^3 step 2.20 ms, now 1.06.)
-__device__ __forceinline__ void scatter(const CompositeArgs& a, const CompositeGrads& gr, int cam, int3 vid, float u,
-                                        float v, float w, const float (&drgb)[3], float dsdf) {
+// Adds a hit's gradient to its triangle's vertices, as one 16-byte reduction for
+// each (colour and signed distance). The lanes here that hold hits of one
+// triangle (`at` names it) are summed first, along the chain of their lanes in a
+// logarithm of steps, and the lowest of them adds the sums: a vertex of large
+// triangles gets one rounded addition for a warp's hits, not up to 32 (two
+// shells of triangles of 600 px at 1024^2: largest relative error 2e-6 to 5e-6,
+// 2e-5 with every hit added by itself). The sums cost the kernel 115 to 122 us
+// in the 256^3 step and 1.06 to 1.16 ms in the 512^3 step, whose triangles have
+// one to four hits in a warp. (Per triangle in shared memory, over a batch, they
+// cost more: shared-memory float additions are loops of compare-and-swap; 195 us
+// and 2.20 ms.)
+__device__ __forceinline__ void scatter(const CompositeArgs& a, const CompositeGrads& gr, int cam, int lane, int at,
+                                        int3 vid, float u, float v, float w, const float (&drgb)[3], float dsdf) {
   if (drgb[0] == 0.f && drgb[1] == 0.f && drgb[2] == 0.f && dsdf == 0.f) return;
-  const int id[3] = {vid.x, vid.y, vid.z};
+  const uint32_t live = __activemask();
+  const uint32_t group = __match_any_sync(live, at);
   const float wt[3] = {u, v, w};
+  float g[3][4];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) g[q][c] = wt[q] * drgb[c];
+    g[q][3] = wt[q] * dsdf;
+  }
+  const uint32_t above = group & (0xfffffffeu << lane);
+  int next = above ? __ffs(above) - 1 : 32;  // the next lane whose sum is not in this one's
+  while (__any_sync(live, next < 32)) {
+    const bool more = next < 32;
+    const int from = more ? next : lane;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float x = __shfl_sync(live, g[q][c], from);
+        if (more) g[q][c] += x;
+      }
+    const int after = __shfl_sync(live, next, from);
+    next = more ? after : 32;
+  }
+  if (lane != __ffs(group) - 1) return;
+  const int id[3] = {vid.x, vid.y, vid.z};
   if (gr.packed) {
     float4* rows = gr.packed + (int64_t)cam * a.V;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) red_add(rows + id[q], wt[q] * drgb[0], wt[q] * drgb[1], wt[q] * drgb[2], wt[q] * dsdf);
+    for (int q = 0; q < 3; ++q) red_add(rows + id[q], g[q][0], g[q][1], g[q][2], g[q][3]);
     return;
   }
   float* gc = gr.grad_colors + (int64_t)cam * a.V * 3;
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) atomicAdd(gc + 3 * (int64_t)id[q] + c, wt[q] * drgb[c]);
-    atomicAdd(gr.grad_sdf + id[q], wt[q] * dsdf);
+    for (int c = 0; c < 3; ++c) atomicAdd(gc + 3 * (int64_t)id[q] + c, g[q][c]);
+    atomicAdd(gr.grad_sdf + id[q], g[q][3]);
   }
 }
 
@@ -1291,6 +1321,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
   float dp_rgb[3] = {0.f, 0.f, 0.f};
   float dp_sdf = 0.f;
   int3 prev_vid = make_int3(0, 0, 0);
+  int prev_at = 0;  // the previous hit's triangle: its place in the warp's walk
   float pu = 0.f, pv = 0.f, pw = 0.f;
 
   const int64_t start = a.bounds[2 * ((int64_t)cam * T + px.tile)];
@@ -1427,12 +1458,13 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
         if (last_shell != -1) {
           dp_sdf += d_oc * ko * s;
           const float su = gr.exact ? pu : u, sv = gr.exact ? pv : v, sw = gr.exact ? pw : w;
-          scatter(a, gr, cam, prev_vid, su, sv, sw, dp_rgb, dp_sdf);
+          scatter(a, gr, cam, lane, prev_at, prev_vid, su, sv, sw, dp_rgb, dp_sdf);
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) dp_rgb[c] = d_color[c];
         dp_sdf = d_ic * ki * s;
         prev_vid = ws.vids[i];
+        prev_at = kBatch * batch + i;
         pu = u;
         pv = v;
         pw = w;
@@ -1463,7 +1495,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
     }
   }
   // The last hit's deferred gradient, with its own weights.
-  if (px.in_image && last_shell != -1) scatter(a, gr, cam, prev_vid, pu, pv, pw, dp_rgb, dp_sdf);
+  if (px.in_image && last_shell != -1) scatter(a, gr, cam, lane, prev_at, prev_vid, pu, pv, pw, dp_rgb, dp_sdf);
 
   // Sharpness gradient: one atomic per warp.
   float x = px.in_image ? d_sharp : 0.f;

@@ -130,3 +130,75 @@ def test_gradient_of_longer_colours(cuda_device):
     grad = torch.randn((1, 5, 3), device=cuda_device)
     assert torch.equal(tr._flat_like(grad, torch.empty((1, 7, 3), device=cuda_device))[:, :5], grad)
     assert tr._flat_like(grad, grad) is grad
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (8, 8), (12, 20)])
+def test_sums_over_large_triangles(cuda_device, tile):
+    """Colour gradients of two shells of eight triangles that fill the image,
+    against 64 bits.
+
+    A warp's hits of a triangle are one addition to its vertices. n additions of
+    like terms in some order, each rounded to nearest, miss the sum S by about
+    sqrt(n / 3) 0.41 2^-24 S (the partial sums grow evenly to S): four of these
+    for n, the warp blocks (8x4 pixels) of the triangles around a vertex and a
+    quarter more for those that a triangle covers in part, and 16 units for a
+    term's own roundings, which all terms may share. Added one by one, 32 times
+    as many additions miss it by six times as much."""
+    d, size = cuda_device, 1024
+    at = torch.linspace(-8, size + 8, 3, device=d)
+    xy = torch.stack(torch.meshgrid(at, at, indexing="xy"), -1).reshape(-1, 2)
+    xy[4] += torch.tensor([37.0, -21.0], device=d)  # the vertex inside
+    first = torch.tensor([0, 1, 3, 4], dtype=torch.int32, device=d)[:, None]
+    corners = torch.tensor([[0, 3, 1], [1, 3, 4]], dtype=torch.int32, device=d)
+    one = (first + corners.view(1, -1)).view(-1, 3)
+    v, shells = xy.shape[0], 2
+    faces = torch.cat((one, one + v))
+    levels, sharpness = (0.01, -0.01), 40.0
+    sdf = torch.tensor(levels, device=d).repeat_interleave(v)
+    positions = xy.repeat(shells, 1)[None].contiguous()
+    depths = torch.tensor([1.0, 2.0], device=d).repeat_interleave(v)[None].contiguous()
+    grid = tr.TileGrid(tile, (size, size), 1, shells)
+    kd = tr.create_key_defines(("camera", 6), ("tile", 20), ("depth", 32), ("shell", 6))
+    ends = torch.tensor([8, 16], dtype=torch.int32, device=d)
+    rect = tr.bound_triangles(positions, depths, faces, grid, 0.2)
+    if not rect.num_tiles_overlapped.any():  # seen from behind
+        faces = faces.flip(1).contiguous()
+        rect = tr.bound_triangles(positions, depths, faces, grid, 0.2)
+    keys = tr.sort_keys(tr.generate_keys(depths, faces, ends, rect.tile_minima, rect.tile_maxima,
+                                         rect.num_tiles_overlapped, grid, kd))
+    ranges = tr.delineate_tiles(keys, grid, kd, False).view(1, -1, 2)
+    rng = torch.Generator(d).manual_seed(1)
+    colors = torch.rand((1, shells * v, 3), generator=rng, device=d).requires_grad_(True)
+    upstream = torch.rand((1, 4, size, size), generator=rng, device=d) + 0.5
+    upstream[:, 3] = 0
+    raw = tr.intersect_and_composite(positions, colors, sdf, faces, sharpness, keys.keys, keys.triangle_indices, ranges,
+                                     shells, grid, kd, "exact")
+    (got,) = torch.autograd.grad(raw, colors, upstream)
+
+    pixels = torch.arange(size, device=d, dtype=torch.float64) + 0.5
+    points = torch.stack(torch.meshgrid(pixels, pixels, indexing="xy"), -1).view(-1, 2)
+    terms = upstream[0, :3].double().permute(1, 2, 0).reshape(-1, 3)
+    sums = torch.zeros((v, 3), dtype=torch.float64, device=d)
+    blocks = torch.zeros(v, dtype=torch.float64, device=d)
+    free = torch.ones(len(points), dtype=torch.bool, device=d)
+
+    def cross(p, q, r):
+        return (q - p)[0] * (r - p)[..., 1] - (q - p)[1] * (r - p)[..., 0]
+
+    for corner in one.tolist():
+        p = xy[corner].double()
+        area = cross(p[0], p[1], p[2])
+        weights = torch.stack([cross(p[(q + 1) % 3], p[(q + 2) % 3], points) for q in range(3)], -1) / area
+        inside = (weights >= 0).all(-1) & free  # weights agree where two triangles meet
+        free &= ~inside
+        sums[corner] += (weights[inside][..., None] * terms[inside][:, None]).sum(0)
+        blocks[corner] += abs(area) / 2 / 32 * 1.25
+    assert not free.any()
+    outer, light = 1.0, 1.0
+    for shell, level in enumerate(levels):
+        inner = 1.0 / (1.0 + np.exp(-float(np.float32(level)) * sharpness))
+        alpha = min(max((outer - inner + 1e-5) / (outer + 1e-5), 0.0), 1.0)
+        want = light * alpha * sums
+        light, outer = light * (1.0 - alpha), inner
+        bound = (4 * 0.41 * (blocks / 3).sqrt() + 16)[:, None] * 2.0**-24 * want.abs()
+        assert float(((got[0, shell * v:(shell + 1) * v] - want).abs() / bound).max()) <= 1.0
