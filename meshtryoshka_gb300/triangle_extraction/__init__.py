@@ -317,10 +317,12 @@ def _upscale_parameters(old_signed_distances, old_spherical_harmonics, old_occup
     num_sh, num_old, _ = old_spherical_harmonics.shape
     sh_rows = num_old
     if canonical is not None:
-        # A canonical duplicate's index is below the vertex count.
+        # A canonical duplicate's index is below the vertex count; with fewer rows
+        # than vertices the largest is looked up.
         num_old = canonical.shape[0]
-        if min(sh_rows, old_signed_distances.shape[0]) < num_old:
-            raise IndexError("old_signed_distances and old_spherical_harmonics have fewer rows than vertices")
+        rows = min(sh_rows, old_signed_distances.shape[0])
+        if rows < num_old and int(canonical.max()) >= rows:
+            raise IndexError("old_signed_distances and old_spherical_harmonics lack the row of a canonical vertex")
     elif old_signed_distances.shape[0] != num_old:
         raise ValueError("old_signed_distances and old_spherical_harmonics disagree on the vertex count")
 

@@ -65,3 +65,21 @@ def test_too_few_rows_are_refused(cuda_device):
     sh = torch.zeros((1, vox.num_vertices, 3), device=cuda_device)
     with pytest.raises(IndexError):
         subdivision.subdivide(vox, sh.new_zeros(vox.num_vertices - 1), sh, occ, vox.indices, (6, 8, 64))
+
+
+def test_rows_past_the_last_canonical_vertex_are_not_needed(cuda_device):
+    """With a tolerance that merges the last vertices into earlier ones."""
+    rng = np.random.default_rng(0)
+    occ = torch.from_numpy(semantics.pack(np.ones((3, 4, 32), bool))).to(cuda_device)
+    vox = te.extract_voxels(occ)
+    tol = 0.9
+    rows = int(te.index_vertices(vox.vertices, tol).max()) + 1
+    assert rows < vox.num_vertices
+    sdf = torch.from_numpy(rng.normal(size=vox.num_vertices).astype(np.float32)).to(cuda_device)
+    sh = torch.from_numpy(rng.normal(size=(4, vox.num_vertices, 3)).astype(np.float32)).to(cuda_device)
+    want = subdivision.subdivide(vox, sdf, sh, occ, vox.indices, (6, 8, 64), tol=tol)
+    got = subdivision.subdivide(vox, sdf[:rows], sh[:, :rows], occ, vox.indices, (6, 8, 64), tol=tol)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    with pytest.raises(IndexError):
+        subdivision.subdivide(vox, sdf[:rows - 1], sh, occ, vox.indices, (6, 8, 64), tol=tol)
