@@ -148,7 +148,8 @@ __global__ void __launch_bounds__(kThreads, kThreads <= 256 ? 4 : 1)
           if (first != kNone) {
             float u, v, w;
             hit_test(sf[first].g, fx, fy, u, v, w);
-            reinterpret_cast<float2*>(out_uv)[o] = make_float2(u, v);
+            out_uv[2 * o] = u;
+            out_uv[2 * o + 1] = v;
             out_index[o] = sf[first].face;
             active = false;
             best[tid] = -1;
@@ -158,7 +159,8 @@ __global__ void __launch_bounds__(kThreads, kThreads <= 256 ? 4 : 1)
       __syncthreads();  // the next list's chunks overwrite the shared ones
     }
     if (active) {
-      reinterpret_cast<float2*>(out_uv)[o] = make_float2(0.f, 0.f);
+      out_uv[2 * o] = 0.f;
+      out_uv[2 * o + 1] = 0.f;
       out_index[o] = -1;
     }
   }
@@ -550,7 +552,6 @@ int mt_intersect(const float* xy, int64_t V, const int32_t* faces, const int32_t
   const int64_t blocks = (int64_t)B * S * rows * cols;
   if (blocks == 0 || H == 0 || W == 0) return MT_OK;
   MT_REQUIRE(xy && faces && tile_boundaries && out_uv && out_index);
-  MT_REQUIRE((reinterpret_cast<uintptr_t>(out_uv) & 7) == 0);
   MT_REQUIRE(blocks < ((int64_t)1 << 31));
   const int bs = tile_h * tile_w;
   const size_t smem = intersect_smem(bs);

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from meshtryoshka_gb300 import _native as nt
+from meshtryoshka_gb300 import triangle_rasterization as tr
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,32 @@ def test_no_level_sets_and_no_offsets(cuda_device, g):
                 None, None, 0, inverse.data_ptr(), None, grads[0].data_ptr(), grads[1].data_ptr(), workspace,
                 need if workspace else 0, nt.stream(cuda_device))
         assert not any(x.any() for x in grads)
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (9, 7), (20, 29)])
+def test_first_hits_into_an_unaligned_buffer(cuda_device, tile):
+    """out_uv at a 4-byte boundary: hits, misses and tiles without triangles."""
+    d, (h, w) = cuda_device, (45, 70)
+    rng = torch.Generator(d).manual_seed(3)
+    f = 40
+    xy = torch.rand((1, f, 1, 2), generator=rng, device=d) * 40 + torch.rand((1, f, 3, 2), generator=rng, device=d) * 9
+    xy = xy.view(1, 3 * f, 2).contiguous()
+    depths = torch.rand((1, 3 * f), generator=rng, device=d) + 1
+    faces = torch.arange(3 * f, dtype=torch.int32, device=d).view(f, 3)
+    faces = torch.cat((faces, faces.flip(1))).contiguous()  # one of the two faces the camera
+    ends = torch.tensor([f, 2 * f], dtype=torch.int32, device=d)
+    grid = tr.TileGrid(tile, (h, w), 1, 2)
+    kd = tr.create_key_defines(("camera", 6), ("shell", 6), ("tile", 20), ("depth", 32))
+    rect = tr.bound_triangles(xy, depths, faces, grid, 0.2)
+    keys = tr.sort_keys(tr.generate_keys(depths, faces, ends, rect.tile_minima, rect.tile_maxima,
+                                         rect.num_tiles_overlapped, grid, kd))
+    ranges = tr.delineate_tiles(keys, grid, kd, True).contiguous()
+    want = tr.intersect(xy, faces, keys.triangle_indices, ranges, grid, kd)
+    assert 0 < int((want.index >= 0).sum()) < want.index.numel()
+    rows, cols = grid.grid_shape
+    uv = torch.full((want.uv.numel() + 1,), 7.0, device=d)
+    index = torch.empty_like(want.index)
+    nt.call("mt_intersect", xy.data_ptr(), xy.shape[1], faces.data_ptr(), keys.triangle_indices.data_ptr(),
+            ranges.data_ptr(), 1, 2, rows, cols, *tile, h, w, uv.data_ptr() + 4, index.data_ptr(), nt.stream(d))
+    assert torch.equal(uv[1:].view(want.uv.shape), want.uv) and torch.equal(index, want.index)
+    assert float(uv[0]) == 7.0
