@@ -277,12 +277,19 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return t.data_ptr() if t.numel() > 0 else None
 
 
+def _stream_of(index: int) -> int:
+    return torch.cuda.current_stream(index).cuda_stream
+
+
+# The handle from the runtime's own table, where this PyTorch has that call: a
+# torch.cuda.Stream object costs 5 us on a Grace core, and every entry point
+# needs the handle.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _stream_of)
+
+
 def stream(device: torch.device) -> int:
-    """Handle of the current stream (asked of the runtime's own table: a
-    torch.cuda.Stream object costs 5 us on a Grace core, and every entry point
-    needs the handle)."""
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    return torch._C._cuda_getCurrentRawStream(index)
+    """Handle of the current stream."""
+    return _raw_stream(device.index if device.index is not None else torch.cuda.current_device())
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:
@@ -343,7 +350,7 @@ _workspaces: dict[tuple[int, int], Workspace] = {}
 
 def workspace(device: torch.device) -> Workspace:
     index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (index, torch._C._cuda_getCurrentRawStream(index))
+    key = (index, _raw_stream(index))
     ws = _workspaces.get(key)
     if ws is None:
         ws = Workspace(device)

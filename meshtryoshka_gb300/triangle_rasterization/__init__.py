@@ -856,12 +856,13 @@ class FinishImages(torch.autograd.Function):
 
 def _finishable(raw: Tensor, background: Tensor) -> bool:
     """Whether the finishing kernels take this background: a plain float32
-    [3] on the render's device that no gradient or tangent is asked of.
+    [3] on the render's device that no gradient or tangent is asked of (where
+    PyTorch does not say whether tangents are, that counts as yes).
     Everything else goes through tensor operations."""
     return (type(background) in (Tensor, torch.nn.Parameter) and background.device == raw.device
             and background.dtype == torch.float32 and background.shape == (3,) and background.is_contiguous()
             and not (background.requires_grad and torch.is_grad_enabled())
-            and torch.autograd.forward_ad._current_level < 0)
+            and getattr(torch.autograd.forward_ad, "_current_level", 0) < 0)
 
 
 # ---------------------------------------------------------------------------

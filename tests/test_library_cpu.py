@@ -104,3 +104,20 @@ def test_no_wait_of_the_key_kernels_goes_unreported():
     word; the key kernels, whose workspace nobody reads one from, wait on nothing."""
     source = (ROOT / "meshtryoshka_gb300" / "csrc" / "raster_front.cu").read_text()
     assert not re.findall(r"mt_exclusive_scan_\w+\(|mt_inclusive_scan_\w+\(|lookback_prefix", source)
+
+
+def test_without_pytorchs_private_names():
+    """The stream handle and the choice of the finishing kernels do without them."""
+    import subprocess
+    import sys
+
+    code = """
+import types, torch
+del torch._C._cuda_getCurrentRawStream, torch.autograd.forward_ad._current_level
+from meshtryoshka_gb300 import _native as nt
+from meshtryoshka_gb300 import triangle_rasterization as tr
+torch.cuda.current_stream = lambda index: types.SimpleNamespace(cuda_stream=7 + index)
+assert nt.stream(torch.device("cuda:1")) == 8
+assert not tr._finishable(torch.zeros(4), torch.zeros(3))
+"""
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True, timeout=300)
