@@ -2,8 +2,11 @@
 
 from __future__ import annotations
 
+from contextlib import contextmanager
+
 import torch
 
+from meshtryoshka_gb300 import record
 from meshtryoshka_gb300.record import annotate
 
 
@@ -30,3 +33,28 @@ def test_an_exception_passes_through():
             raise KeyError("inside")
     except KeyError as e:
         assert e.args == ("inside",)
+
+
+def test_the_cheap_form_unless_a_profiler_runs(monkeypatch):
+    opened = []
+
+    def form(kind):
+        @contextmanager
+        def opens(name):
+            opened.append((kind, name))
+            yield
+
+        return opens
+
+    monkeypatch.setattr(record, "record_function", form("dispatched"))
+    monkeypatch.setattr(record, "_Fast", form("fast"))
+    assert _sum(1) == 2
+    with annotate("block"):
+        pass
+    assert opened == [("fast", "annotated_sum"), ("fast", "block")]
+    opened.clear()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]):
+        assert _sum(1) == 2
+        with annotate("block"):
+            pass
+    assert opened == [("dispatched", "annotated_sum"), ("dispatched", "block")]

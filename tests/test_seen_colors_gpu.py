@@ -54,3 +54,47 @@ def test_same_loss_and_gradients(cuda_device, monkeypatch, shift):
     for x, y in ((d0, d1), (h0, h1)):  # the atomic sums' order
         assert bool(torch.isfinite(y).all())
         assert float((x - y).abs().max()) <= 1e-4 * max(float(x.abs().max()), 1e-12)
+
+
+@pytest.mark.parametrize("call", ["fused", "cameras", "loss"])
+def test_unseen_colours_are_not_read(cuda_device, monkeypatch, call):
+    """NaN in the place of every colour that was not formed changes nothing."""
+    w = pipeline.build_workload("small", cuda_device)
+    d, b = cuda_device, w.extrinsics.shape[0]
+    h, wd = w.image_shape
+    extrinsics = w.extrinsics.clone()
+    extrinsics[:, 0, 3] += 0.6  # a part of the scene outside the image
+    rows = torch.randn((16, w.voxels.num_vertices, 3), generator=torch.Generator().manual_seed(0)).to(d) * 0.3
+    target = torch.rand((b, 3, h, wd), generator=torch.Generator().manual_seed(1)).to(d)
+    poisoned = []
+
+    def evaluate(self, vertices, extrinsics, sh_degree, seen=None):
+        colors = inner(self, vertices, extrinsics, sh_degree, seen)
+        if seen is not None:
+            colors.data[:, seen == 0] = float("nan")
+            poisoned.append(int((seen == 0).sum()))
+        return colors
+
+    inner = te.DeferredSH.evaluate
+    monkeypatch.setattr(te.DeferredSH, "evaluate", evaluate)
+    results = []
+    for limit in (1 << 40, -1):
+        monkeypatch.setattr(te, "SEEN_COLOURS_BYTES", limit)
+        sdf, sh = w.grid_sdf.detach().clone().requires_grad_(True), rows.clone().requires_grad_(True)
+        tri = te.tessellate_voxels(sdf, w.voxels.vertices, sh, w.voxels.neighbors, w.voxels.lower_corners,
+                                   w.voxels.upper_corners, w.voxels.indices, w.level_sets, defer_sh=True)
+        mesh = (pipeline.uncontract_stand_in(tri.vertices), tri.faces, tri.face_boundaries, tri.signed_distances,
+                tri.spherical_harmonics, 3, 40.0, torch.zeros(3, device=d))
+        if call == "loss":
+            loss = tr.render_fused_loss(extrinsics, w.intrinsics, (h, wd), *mesh, target)
+        elif call == "cameras":
+            images = tr.render_cameras(extrinsics, w.intrinsics, [(h, wd)] * b, *mesh)
+            loss = ((torch.stack(images) - target) ** 2).mean()
+        else:
+            loss = ((tr.render_fused(extrinsics, w.intrinsics, (h, wd), *mesh) - target) ** 2).mean()
+        loss.backward()
+        results.append((loss.detach(), sdf.grad, sh.grad))
+    assert len(poisoned) == 1 and poisoned[0] > 0
+    for x, y in zip(*results):  # the atomic sums' order
+        assert bool(torch.isfinite(y).all())
+        assert float((x - y).abs().max()) <= 1e-4 * max(float(x.abs().max()), 1e-12)
