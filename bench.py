@@ -454,6 +454,10 @@ def run_ours(args, rank, world, local):
 
     # Roofline of the dominant entry point (largest share of device time).
     peak, peak_kind = measured_peaks()
+    sizes = pipeline.key_sizes(w)
+    stats["touching"] = sizes["touching"]
+    if "mt_mark_seen_vertices" in per_call:
+        stats["seen"] = sizes["named"]
     bytes_by_stage = pipeline.step_bytes(stats)
     # Library entry point -> the step_bytes stages its kernels cover.
     stages_of = {
@@ -462,6 +466,8 @@ def run_ours(args, rank, world, local):
         "mt_sort_keys_by_tile": ("tile_sort",),
         "mt_bound_and_generate_keys": ("keys",),
         "mt_grid_sh_colors_of_seen": ("grid_sh_colors",),
+        "mt_mark_seen_vertices": ("seen_marks",),
+        "mt_unpack_gradients": ("unpack_gradients",),
         "mt_create_triangle_faces_by_crossings": ("create_faces",),
     }
     totals = {k: sum(v) for k, v in per_call.items()}

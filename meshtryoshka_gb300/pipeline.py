@@ -19,6 +19,7 @@ from . import _native as nt
 from . import synthetic
 from . import triangle_extraction as te
 from . import triangle_rasterization as tr
+from .record import recording
 
 
 @dataclass
@@ -257,14 +258,35 @@ def reference_algorithm_bytes(stats: dict) -> dict[str, float]:
     }
 
 
+def key_sizes(w: Workload) -> dict[str, int]:
+    """What ``step_bytes`` counts besides ``forward``'s sizes: ``touching``, the
+    (camera, face) pairs that have a key, and ``named``, the vertices of faces
+    that have one."""
+    store: dict = {}
+    with torch.no_grad(), recording(store):
+        _, stats = forward(w)
+    face = store["sorted_triangles"].long()
+    camera = (store["sorted_keys"] >> 58) & 63  # the key's upper six bits
+    return {
+        "touching": int(torch.unique(camera * max(stats["F"], 1) + face).numel()),
+        "named": int(torch.unique(store["faces"][torch.unique(face)]).numel()),
+    }
+
+
 def step_bytes(stats: dict) -> dict[str, float]:
     """Compulsory traffic of the kernels the captured training step runs
     (``graph.CapturedTrainingStep``: deferred SH, the contribution list, the
     capacity-mode keys, the tile-bucketed sort, warp masks, the compositing
     kernels with the MSE epilogue), from the measured sizes. Each input read
     once, each output written once, gathers counted once per consumer;
-    scratch that only speeds a kernel up (stored hit bits) is not counted."""
+    scratch that only speeds a kernel up (stored hit bits) is not counted.
+    ``touching`` (of ``key_sizes``; as many as can be where it is missing): the
+    (camera, face) pairs that get a record. ``seen``: the marked vertices where
+    only their colours are formed."""
     G, Nv, V, F, C, S, B, P, K, T = (stats[k] for k in ("G", "Nv", "V", "F", "C", "S", "B", "P", "K", "T"))
+    records = stats.get("touching", min(B * F, K))
+    marked = "seen" in stats
+    U = stats.get("seen", V)
     return {
         # tessellation
         "count_vertices": G * (16 + 16) + S * G,
@@ -279,17 +301,19 @@ def step_bytes(stats: dict) -> dict[str, float]:
         # render front end
         "uncontract": 24 * V,
         "project": 12 * V + 12 * B * V,
-        "grid_sh_colors": V * (12 + 12) + 2 * 12 * C * V + 12 * B * V,
-        "keys": B * F * (12 + 36 + 20) + B * F * 20 + 12 * K,
+        "seen_marks": 4 * K + 12 * min(records, F) + V if marked else 0,
+        "grid_sh_colors": U * (12 + 12) + 2 * 12 * C * U + 12 * B * U + (V if marked else 0),
+        "keys": B * F * (12 + 36) + 2 * 22 * records + 12 * K,
         "tile_sort": 60 * K + 16 * B * T,
         "warp_masks": K * (8 + 4 + 12 + 24) + 4 * K,
         # compositing with the MSE epilogue (target read, output written)
         "composite_fwd": K * 96 + 16 * P + 12 * P,
-        "gradient_zero_fill": 12 * B * V + 4 * V,
+        "gradient_zero_fill": 16 * B * V,
         "composite_bwd": K * 96 + 16 * P + 12 * P + 16 * V * B,
+        "unpack_gradients": 16 * B * V + 4 * V,
         # grid SH gradient: per-vertex SH gradient once, then per grid vertex
         # the weighted sum over its list entries
-        "grid_sh_bwd": 12 * B * V + 24 * V + 12 * C * V + 16 * V + 2 * 12 * C * V + 12 * C * G,
+        "grid_sh_bwd": 16 * B * V + 24 * U + 12 * C * U + 16 * V + 2 * 12 * C * U + 12 * C * G,
         "grid_sdf_bwd": 16 * V + 4 * V + 16 * G,
     }
 
