@@ -233,7 +233,7 @@ MT_API int mt_quantize_points(const float* points, int64_t V, float inv_tol,
                        mt_stream_t stream);
 
 /* index_vertices.py:23-25: keys[v] = (x << 2 shift) | (y << shift) | z,
- * values[v] = v. */
+ * values[v] = v (unless NULL). */
 MT_API int mt_pack_point_keys(const int64_t* quantized, int64_t V, int32_t shift,
                        int64_t* keys, int32_t* values, mt_stream_t stream);
 
@@ -380,21 +380,13 @@ MT_API int mt_grid_sh_colors(const float* grid_spherical_harmonics, int32_t C, i
                              int32_t sh_degree, const float* camera_positions,
                              int32_t B, float* out_colors, mt_stream_t stream);
 
-/* The same, in the order of the grid's entries: vertex_offsets [S*G + 1] are
- * the scanned counts that mt_create_triangle_vertices placed the vertices by
- * (vertices of one grid entry's neighbourhood on every shell are evaluated
- * together). NULL: in vertex order. */
-MT_API int mt_grid_sh_colors_by_entry(const float* grid_spherical_harmonics, int32_t C, int64_t G,
-                             const int32_t* vertex_sources, int64_t V,
-                             const int32_t* num_vertices, const int32_t* vertex_offsets,
-                             int32_t S, const float* vertices,
-                             int32_t sh_degree, const float* camera_positions,
-                             int32_t B, float* out_colors, mt_stream_t stream);
-
 /* The same for the vertices with a byte set in seen [V] (NULL: all); the others'
- * colours are not written. mt_mark_seen_vertices sets the bytes of the vertices
- * of the keys' triangles (num_keys: NULL or the device live count) and clears
- * the rest. */
+ * colours are not written. vertex_offsets [S*G + 1] are the scanned counts that
+ * mt_create_triangle_vertices placed the vertices by: with them, the vertices of
+ * one grid entry's neighbourhood on every shell are evaluated together (NULL: in
+ * vertex order). mt_mark_seen_vertices sets the bytes of the vertices of the
+ * keys' triangles (num_keys: NULL or the device live count) and clears the
+ * rest. */
 MT_API int mt_grid_sh_colors_of_seen(const float* grid_spherical_harmonics, int32_t C, int64_t G,
                              const int32_t* vertex_sources, int64_t V,
                              const int32_t* num_vertices, const int32_t* vertex_offsets,

@@ -90,7 +90,6 @@ _SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "mt_build_vertex_grad_list": (I32, [P, P, I64, P, I32, P, I64, P, P, P, P, c_size_t, P]),
     "mt_vertex_grads_from_list": (I32, [P, P, I64, P, P, P, P, P]),
     "mt_grid_sh_colors": (I32, [P, I32, I64, P, I64, P, P, I32, P, I32, P, P]),
-    "mt_grid_sh_colors_by_entry": (I32, [P, I32, I64, P, I64, P, P, I32, P, I32, P, I32, P, P]),
     "mt_grid_sh_colors_of_seen": (I32, [P, I32, I64, P, I64, P, P, I32, P, I32, P, I32, P, P, P]),
     "mt_mark_seen_vertices": (I32, [P, I64, P, P, I64, I64, P, P]),
     "mt_grid_sh_colors_backward_workspace_bytes": (c_size_t, [I64]),

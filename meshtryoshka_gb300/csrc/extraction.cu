@@ -2185,14 +2185,6 @@ int mt_grid_sh_colors_of_seen(const float* grid_spherical_harmonics, int32_t C, 
   return MT_OK;
 }
 
-int mt_grid_sh_colors_by_entry(const float* grid_spherical_harmonics, int32_t C, int64_t G,
-                               const int32_t* vertex_sources, int64_t V, const int32_t* num_vertices,
-                               const int32_t* vertex_offsets, int32_t S, const float* vertices, int32_t sh_degree,
-                               const float* camera_positions, int32_t B, float* out_colors, mt_stream_t stream) {
-  return mt_grid_sh_colors_of_seen(grid_spherical_harmonics, C, G, vertex_sources, V, num_vertices, vertex_offsets, S,
-                                   vertices, sh_degree, camera_positions, B, nullptr, out_colors, stream);
-}
-
 int mt_mark_seen_vertices(const int32_t* triangles, int64_t K, const int64_t* num_keys, const int32_t* faces,
                           int64_t F, int64_t V, uint8_t* seen, mt_stream_t stream) {
   MT_REQUIRE(K >= 0 && F >= 0 && V >= 0);
@@ -2210,8 +2202,8 @@ int mt_mark_seen_vertices(const int32_t* triangles, int64_t K, const int64_t* nu
 int mt_grid_sh_colors(const float* grid_spherical_harmonics, int32_t C, int64_t G, const int32_t* vertex_sources,
                       int64_t V, const int32_t* num_vertices, const float* vertices, int32_t sh_degree,
                       const float* camera_positions, int32_t B, float* out_colors, mt_stream_t stream) {
-  return mt_grid_sh_colors_by_entry(grid_spherical_harmonics, C, G, vertex_sources, V, num_vertices, nullptr, 0,
-                                    vertices, sh_degree, camera_positions, B, out_colors, stream);
+  return mt_grid_sh_colors_of_seen(grid_spherical_harmonics, C, G, vertex_sources, V, num_vertices, nullptr, 0,
+                                   vertices, sh_degree, camera_positions, B, nullptr, out_colors, stream);
 }
 
 size_t mt_grid_sh_colors_backward_workspace_bytes(int64_t V) {

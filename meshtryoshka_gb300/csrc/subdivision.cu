@@ -458,13 +458,13 @@ __global__ void quantize_points_kernel(const float* __restrict__ points, int64_t
 }
 
 // keys = (x << 2 shift) | (y << shift) | z with two's complement shifts,
-// values = 0 .. V-1.
+// values = 0 .. V-1 (unless NULL).
 __global__ void pack_point_keys_kernel(const int64_t* __restrict__ q, int64_t V, int shift,
                                        int64_t* __restrict__ keys, int32_t* __restrict__ values) {
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t x = (uint64_t)q[3 * v + 0], y = (uint64_t)q[3 * v + 1], z = (uint64_t)q[3 * v + 2];
     keys[v] = (int64_t)((x << (2 * shift)) | (y << shift) | z);
-    values[v] = (int32_t)v;
+    if (values) values[v] = (int32_t)v;
   }
 }
 
@@ -673,7 +673,7 @@ int mt_pack_point_keys(const int64_t* quantized, int64_t V, int32_t shift, int64
                        mt_stream_t stream) {
   MT_REQUIRE(V >= 0 && V <= 0x7fffffffll && shift >= 0 && shift <= 21);
   if (V == 0) return MT_OK;
-  MT_REQUIRE(quantized && keys && values);
+  MT_REQUIRE(quantized && keys);
   pack_point_keys_kernel<<<grid_stride_blocks(V, kThreads), kThreads, 0, as_stream(stream)>>>(quantized, V, shift,
                                                                                             keys, values);
   MT_CHECK_LAUNCH();

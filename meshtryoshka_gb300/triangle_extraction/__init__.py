@@ -427,9 +427,7 @@ def index_vertices(points: Tensor, tol: float = 1e-5) -> Tensor:
     if bits * 3 > 63:
         raise RuntimeError(f"need {bits*3} bits, exceed 63 bits total")
     keys = torch.empty((v,), dtype=torch.int64, device=device)
-    values = torch.empty((v,), dtype=torch.int32, device=device)
-    nt.call("mt_pack_point_keys", quantized.data_ptr(), v, bits, keys.data_ptr(), values.data_ptr(),
-            nt.stream(device))
+    nt.call("mt_pack_point_keys", quantized.data_ptr(), v, bits, keys.data_ptr(), None, nt.stream(device))
     return _first_equal(keys)
 
 

@@ -68,3 +68,26 @@ def test_first_hits_into_an_unaligned_buffer(cuda_device, tile):
             ranges.data_ptr(), 1, 2, rows, cols, *tile, h, w, uv.data_ptr() + 4, index.data_ptr(), nt.stream(d))
     assert torch.equal(uv[1:].view(want.uv.shape), want.uv) and torch.equal(index, want.index)
     assert float(uv[0]) == 7.0
+
+
+@pytest.mark.parametrize("n", [1, 64, 5003])
+def test_first_equal_keys_by_sorting(cuda_device, n):
+    """Point keys and their numbers, a stable sort and its runs' heads give what
+    the hash table gives; the numbers may be left out."""
+    d = cuda_device
+    rng = torch.Generator(d).manual_seed(n)
+    quantized = torch.randint(-4, 5, (n, 3), generator=rng, device=d)
+    keys, same = (torch.empty((n,), dtype=torch.int64, device=d) for _ in range(2))
+    numbers, iota, order, got, want = (torch.empty((n,), dtype=torch.int32, device=d) for _ in range(5))
+    nt.call("mt_pack_point_keys", quantized.data_ptr(), n, 4, keys.data_ptr(), numbers.data_ptr(), nt.stream(d))
+    nt.call("mt_pack_point_keys", quantized.data_ptr(), n, 4, same.data_ptr(), None, nt.stream(d))
+    nt.call("mt_iota_i32", n, iota.data_ptr(), nt.stream(d))
+    assert torch.equal(same, keys) and torch.equal(iota, numbers)
+    scratch, need = nt.workspace(d).get(nt.library().mt_sort_pairs_workspace_bytes(n))
+    nt.call("mt_sort_pairs_i64_i32", keys.data_ptr(), iota.data_ptr(), same.data_ptr(), order.data_ptr(), n, None, 0,
+            64, scratch, need, nt.stream(d))
+    nt.call("mt_index_sorted_runs", same.data_ptr(), order.data_ptr(), n, got.data_ptr(), nt.stream(d))
+    need = int(nt.library().mt_index_keys_workspace_bytes(n))
+    table = torch.empty((need,), dtype=torch.uint8, device=d)
+    nt.call("mt_index_keys", keys.data_ptr(), n, want.data_ptr(), table.data_ptr(), need, nt.stream(d))
+    assert torch.equal(got, want)
