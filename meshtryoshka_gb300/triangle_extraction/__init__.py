@@ -516,11 +516,13 @@ class DeferredSH:
     with ``defer_sh``: the vertices' source records and the per-grid-vertex
     contribution list that both backward passes use."""
 
+    # Without them (an object saved before there were any), vertex order.
+    vertex_offsets: Tensor | None = None  # [S * G + 1] int32, scanned counts per (shell, grid entry)
+
     def __init__(self, grid_spherical_harmonics: Tensor):
         self.grid_spherical_harmonics = grid_spherical_harmonics
         self.vertex_sources: Tensor | None = None  # [3, V] int32 (origin, axis corner, bits of t)
         self.num_vertices: Tensor | None = None  # device int32 live count (capacity mode) or None
-        self.vertex_offsets: Tensor | None = None  # [S * G + 1] int32, scanned counts per (shell, grid entry)
         self.list_offsets: Tensor | None = None  # [G + 1] int32
         self.contributions: Tensor | None = None  # [2V, 2] int32
 
@@ -573,7 +575,7 @@ class GridSHColors(torch.autograd.Function):
             nt.call("mt_camera_positions", nt.ptr(extrinsics), b, nt.ptr(campos), nt.stream(device))
             colors = torch.empty((b, v, 3), dtype=torch.float32, device=device)
             offsets = deferred.vertex_offsets
-            shells = (offsets.numel() - 1) // g if g > 0 else 0
+            shells = (offsets.numel() - 1) // g if offsets is not None and g > 0 else 0
             nt.call("mt_grid_sh_colors_of_seen", nt.ptr(gsh), c, g, nt.ptr(deferred.vertex_sources), v,
                     nt.ptr(deferred.num_vertices), nt.ptr(offsets), shells, nt.ptr(vertices), int(sh_degree),
                     nt.ptr(campos), b, nt.ptr(seen), nt.ptr(colors), nt.stream(device))

@@ -271,3 +271,21 @@ def test_grid_sh_backward_on_a_full_device(cuda_device, monkeypatch, captured):
         torch.cuda.synchronize()
         assert refused
         torch.testing.assert_close(got, want, rtol=0, atol=0)
+
+
+def test_deferred_rows_without_offsets(cuda_device):
+    """A DeferredSH without the vertices' offsets (saved by an earlier version)
+    gives the same colours and gradients."""
+    w = pipeline.build_workload("small", cuda_device)
+    gsh = w.grid_sh.detach().clone().requires_grad_(True)
+    tri = te.tessellate_voxels(w.grid_sdf.detach(), w.voxels.vertices, gsh, w.voxels.neighbors,
+                               w.voxels.lower_corners, w.voxels.upper_corners, w.voxels.indices, w.level_sets,
+                               defer_sh=True)
+    results = []
+    for offsets in (True, False):
+        if not offsets:
+            del tri.spherical_harmonics.vertex_offsets
+        colors = tr.evaluate_spherical_harmonics(tri.vertices.detach(), tri.spherical_harmonics, w.extrinsics, w.sh_degree)
+        results.append((colors, *torch.autograd.grad(colors.sum(), gsh)))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
