@@ -315,10 +315,15 @@ class Workspace:
 
     Byte 0 holds the library's device status word, zeroed on allocation.
     Calls that use a workspace are stream-ordered, so one workspace per device
-    is shared by all calls on that device's current stream.
+    is shared by all calls on that device's current stream. An entry point
+    enqueues several kernels that hand their scratch on, without the
+    interpreter's lock: ``lock`` is held from asking for the scratch until they
+    are all enqueued (``call_with_workspace``), so that another thread's on the
+    same stream come before or after them, and its growth of the buffer too.
     """
 
     def __init__(self, device: torch.device):
+        self.lock = threading.RLock()
         self.device = device
         self.buffer = torch.zeros(0, dtype=torch.uint8, device=device)
 
@@ -352,15 +357,28 @@ def workspace(device: torch.device) -> Workspace:
     key = (index, _raw_stream(index))
     ws = _workspaces.get(key)
     if ws is None:
-        ws = Workspace(device)
-        _workspaces[key] = ws
+        with _lock:  # one for the stream, also when threads ask first together
+            ws = _workspaces.get(key)
+            if ws is None:
+                ws = Workspace(device)
+                _workspaces[key] = ws
     return ws
+
+
+def call_with_workspace(name: str, nbytes: int, device: torch.device, *args, launches: int | None = None) -> None:
+    """``call(name, *args, workspace, its size, stream)`` with at least
+    ``nbytes`` of the current stream's workspace."""
+    ws = workspace(device)
+    with ws.lock:
+        pointer, size = ws.get(nbytes)
+        call(name, *args, pointer, size, stream(device), launches=launches)
 
 
 __all__ = [
     "library",
     "library_path",
     "call",
+    "call_with_workspace",
     "ptr",
     "stream",
     "require_cuda",

@@ -105,8 +105,7 @@ def compute_exclusive_cumsum(x: Tensor) -> None:
     n = x.numel()
     if n == 0:
         return
-    ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_scan_workspace_bytes(n))
-    nt.call("mt_exclusive_scan_i32", x.data_ptr(), n, ws_ptr, ws_bytes, nt.stream(device))
+    nt.call_with_workspace("mt_exclusive_scan_i32", nt.library().mt_scan_workspace_bytes(n), device, x.data_ptr(), n)
 
 
 # ---------------------------------------------------------------------------
@@ -456,9 +455,8 @@ def _scan_bytes(counts: Tensor, set_bits: bool) -> Tensor:
     device = counts.device
     n = counts.numel()
     out = torch.empty((n + 1,), dtype=torch.int32, device=device)
-    ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_scan_workspace_bytes(n + 1))
-    nt.call("mt_exclusive_scan_bytes", nt.ptr(counts), n, int(set_bits), out.data_ptr(), ws_ptr, ws_bytes,
-            nt.stream(device))
+    nt.call_with_workspace("mt_exclusive_scan_bytes", nt.library().mt_scan_workspace_bytes(n + 1), device,
+                           nt.ptr(counts), n, int(set_bits), out.data_ptr())
     return out
 
 
@@ -595,17 +593,18 @@ class GridSHColors(torch.autograd.Function):
             grad_gsh = torch.empty(ctx.gsh_shape, dtype=torch.float32, device=device)  # fully written
             v = vertices.shape[0]
             need = nt.library().mt_grid_sh_colors_backward_workspace_bytes(v)
+            rows, packed = nt.colour_gradient_rows(grad_colors)
+            entry = "mt_grid_sh_colors_packed_backward" if packed else "mt_grid_sh_colors_backward"
+            args = (nt.ptr(d.list_offsets), nt.ptr(d.contributions), g, v, nt.ptr(vertices), c, ctx.sh_degree,
+                    nt.ptr(campos), campos.shape[0], nt.ptr(colors), rows.data_ptr() or None, nt.ptr(grad_gsh),
+                    nt.ptr(d.num_vertices))
             if need > _KEPT_SCRATCH or need > GRID_SH_BACKWARD_SCRATCH_LIMIT:
                 scratch = _scratch(need, device) if need <= GRID_SH_BACKWARD_SCRATCH_LIMIT else None
                 # None: the one-pass form.
-                ws_ptr, ws_bytes = (None, 0) if scratch is None else (scratch.data_ptr(), need)
+                nt.call(entry, *args, *((None, 0) if scratch is None else (scratch.data_ptr(), need)),
+                        nt.stream(device))
             else:
-                ws_ptr, ws_bytes = nt.workspace(device).get(need)
-            rows, packed = nt.colour_gradient_rows(grad_colors)
-            nt.call("mt_grid_sh_colors_packed_backward" if packed else "mt_grid_sh_colors_backward",
-                    nt.ptr(d.list_offsets), nt.ptr(d.contributions), g, v, nt.ptr(vertices), c, ctx.sh_degree,
-                    nt.ptr(campos), campos.shape[0], nt.ptr(colors), rows.data_ptr() or None, nt.ptr(grad_gsh), nt.ptr(d.num_vertices), ws_ptr, ws_bytes,
-                    nt.stream(device))
+                nt.call_with_workspace(entry, need, device, *args)
             return grad_gsh, None, None, None, None, None
 
 
@@ -669,10 +668,10 @@ class CreateTriangleVertices(torch.autograd.Function):
                 inverse = torch.empty((4, g), dtype=torch.int32, device=device)
                 offsets = torch.empty((g + 1,), dtype=torch.int32, device=device)
                 contributions = torch.empty((2 * v, 2), dtype=torch.int32, device=device)
-                ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_build_vertex_grad_list_workspace_bytes(g))
-                nt.call("mt_build_vertex_grad_list", nt.ptr(grid_signed_distances), nt.ptr(voxel_lower_corners), g,
-                        nt.ptr(level_sets), s, nt.ptr(vertex_offsets), v, nt.ptr(inverse), nt.ptr(offsets),
-                        nt.ptr(contributions), ws_ptr, ws_bytes, nt.stream(device))
+                nt.call_with_workspace(
+                    "mt_build_vertex_grad_list", nt.library().mt_build_vertex_grad_list_workspace_bytes(g), device,
+                    nt.ptr(grid_signed_distances), nt.ptr(voxel_lower_corners), g, nt.ptr(level_sets), s,
+                    nt.ptr(vertex_offsets), v, nt.ptr(inverse), nt.ptr(offsets), nt.ptr(contributions))
                 deferred.vertex_sources = sources
                 deferred.vertex_offsets = vertex_offsets
                 deferred.num_vertices = (vertex_offsets[-1:].view(()) if capacity is not None else None)
@@ -721,14 +720,12 @@ class CreateTriangleVertices(torch.autograd.Function):
             gs = grad_spherical_harmonics.contiguous() if grad_spherical_harmonics is not None else None
             if ctx.live_t is not None:
                 gd = None  # with t live, the vertex SDF is the level set: no gradient reaches the corners
-            ws_ptr, ws_bytes = nt.workspace(device).get(
-                nt.library().mt_create_triangle_vertices_backward_workspace_bytes(g, v))
-            nt.call(
+            nt.call_with_workspace(
                 "mt_create_triangle_vertices_backward",
+                nt.library().mt_create_triangle_vertices_backward_workspace_bytes(g, v), device,
                 nt.ptr(grid_signed_distances), c, nt.ptr(lower_corners), g, nt.ptr(level_sets), s,
                 nt.ptr(vertex_offsets), nt.ptr(gv), nt.ptr(gd), nt.ptr(gs), v, nt.ptr(inverse),
-                nt.ptr(grad_grid_vertices), nt.ptr(grad_grid_sdf), nt.ptr(grad_grid_sh), ws_ptr, ws_bytes,
-                nt.stream(device),
+                nt.ptr(grad_grid_vertices), nt.ptr(grad_grid_sdf), nt.ptr(grad_grid_sh),
             )
             if ctx.live_t is not None:
                 grid_vertices, grid_sh, sources, counted = ctx.live_t

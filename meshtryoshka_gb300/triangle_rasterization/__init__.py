@@ -326,9 +326,8 @@ def generate_keys(depths: Tensor, faces: Tensor, shell_face_boundaries: Tensor, 
     n = counts.numel()
     offsets = torch.empty((n,), dtype=torch.int64, device=device)
     if n > 0:
-        ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_scan_workspace_bytes(n))
-        nt.call("mt_inclusive_scan_i32_to_i64", counts.data_ptr(), offsets.data_ptr(), n, ws_ptr, ws_bytes,
-                nt.stream(device))
+        nt.call_with_workspace("mt_inclusive_scan_i32_to_i64", nt.library().mt_scan_workspace_bytes(n), device,
+                               counts.data_ptr(), offsets.data_ptr(), n)
     live = None
     if capacity is not None:
         num_keys = int(capacity)
@@ -366,12 +365,12 @@ def bound_and_generate_keys(vertices: Tensor, depths: Tensor, faces: Tensor, she
     live = torch.empty((), dtype=torch.int64, device=device)
     rows, cols = grid.grid_shape
     nf = _i32(num_faces) if num_faces is not None else None
-    ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_bound_and_generate_keys_workspace_bytes(c * f))
-    nt.call("mt_bound_and_generate_keys", nt.ptr(vertices), nt.ptr(depths), v, nt.ptr(faces), f, nt.ptr(nf),
-            nt.ptr(sfb), sfb.shape[0], c, grid.tile_shape[0], grid.tile_shape[1], rows, cols,
-            nt.ptr(_camera_table(grid, device)), float(near_plane), _layout(key_defines), num_keys, nt.ptr(keys),
-            nt.ptr(tri), live.data_ptr(), ws_ptr, ws_bytes, nt.stream(device),
-            launches=3 + (c * f > _ONE_SCAN_ITEMS))
+    nt.call_with_workspace(
+        "mt_bound_and_generate_keys", nt.library().mt_bound_and_generate_keys_workspace_bytes(c * f), device,
+        nt.ptr(vertices), nt.ptr(depths), v, nt.ptr(faces), f, nt.ptr(nf), nt.ptr(sfb), sfb.shape[0], c,
+        grid.tile_shape[0], grid.tile_shape[1], rows, cols, nt.ptr(_camera_table(grid, device)), float(near_plane),
+        _layout(key_defines), num_keys, nt.ptr(keys), nt.ptr(tri), live.data_ptr(),
+        launches=3 + (c * f > _ONE_SCAN_ITEMS))
     return PairedKeys(keys, tri, live)
 
 
@@ -426,9 +425,9 @@ def sort_keys(paired_keys: PairedKeys, grid: TileGrid | None = None) -> PairedKe
     if n == 0:
         return PairedKeys(out_keys, out_tri, live)
     device = nt.require_cuda(keys, tri)
-    ws_ptr, ws_bytes = nt.workspace(device).get(nt.library().mt_sort_pairs_workspace_bytes(n))
-    nt.call("mt_sort_pairs_i64_i32", keys.data_ptr(), tri.data_ptr(), out_keys.data_ptr(), out_tri.data_ptr(), n,
-            nt.ptr(live), 0, 64, ws_ptr, ws_bytes, nt.stream(device))
+    nt.call_with_workspace("mt_sort_pairs_i64_i32", nt.library().mt_sort_pairs_workspace_bytes(n), device,
+                           keys.data_ptr(), tri.data_ptr(), out_keys.data_ptr(), out_tri.data_ptr(), n, nt.ptr(live),
+                           0, 64)
     return PairedKeys(out_keys, out_tri, live)
 
 
@@ -473,10 +472,9 @@ def _sort_and_delineate(paired_keys: PairedKeys, grid: TileGrid, key_defines,
     out_keys = torch.empty_like(keys)
     out_tri = torch.empty_like(tri)
     bounds = torch.empty((b, sd, t, 2), dtype=torch.int64, device=device)
-    ws_ptr, ws_bytes = nt.workspace(device).get(lib.mt_sort_keys_by_tile_workspace_bytes(n, b * sd * t))
-    nt.call("mt_sort_keys_by_tile", keys.data_ptr(), tri.data_ptr(), n, nt.ptr(paired_keys.count), layout,
-            int(separate_shells), b, sd, t, out_keys.data_ptr(), out_tri.data_ptr(), bounds.data_ptr(), ws_ptr,
-            ws_bytes, nt.stream(device))
+    nt.call_with_workspace("mt_sort_keys_by_tile", lib.mt_sort_keys_by_tile_workspace_bytes(n, b * sd * t), device,
+                           keys.data_ptr(), tri.data_ptr(), n, nt.ptr(paired_keys.count), layout,
+                           int(separate_shells), b, sd, t, out_keys.data_ptr(), out_tri.data_ptr(), bounds.data_ptr())
     note(sorted_keys=out_keys, sorted_triangles=out_tri, tile_boundaries=bounds, key_count=paired_keys.count)
     return PairedKeys(out_keys, out_tri, paired_keys.count), bounds
 

@@ -121,3 +121,45 @@ assert nt.stream(torch.device("cuda:1")) == 8
 assert not tr._finishable(torch.zeros(4), torch.zeros(3))
 """
     subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True, timeout=300)
+
+
+def test_threads_take_turns_at_a_streams_workspace(monkeypatch):
+    """Entry points with scratch are enqueued whole, one thread's after another's:
+    no thread grows or hands out the buffer while another's call is under way."""
+    import threading
+    import time
+
+    import torch
+
+    from meshtryoshka_gb300 import _native as nt
+
+    ws = nt.Workspace(torch.device("cpu"))
+    under_way, most, seen = [], [], []
+
+    def call(name, *args, launches=None):
+        pointer, size, stream = args[-3:]
+        under_way.append(name)
+        most.append(len(under_way))
+        time.sleep(0.002)  # the interpreter's lock is released, as in the library
+        seen.append(pointer == ws.buffer.data_ptr() and size == ws.buffer.numel() and stream == 7)
+        under_way.remove(name)
+
+    monkeypatch.setattr(nt, "workspace", lambda device: ws)
+    monkeypatch.setattr(nt, "stream", lambda device: 7)
+    monkeypatch.setattr(nt, "call", call)
+
+    def work(i):
+        for k in range(5):
+            nt.call_with_workspace(f"entry {i}", 10_000 * (i + 1) * (k + 1), ws.device, i, k)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(most) == 20 and max(most) == 1 and all(seen)
+
+
+def test_scratch_is_asked_for_under_its_lock():
+    for path in (ROOT / "meshtryoshka_gb300").rglob("*.py"):
+        assert not re.findall(r"workspace\([\w.]*\)\.get\(", path.read_text()), path
