@@ -758,8 +758,8 @@ MT_API int mt_intersect_and_composite_backward(
 
 /* The same into packed_gradients [B,V,4] (+=, 16-byte aligned): a (camera,
  * vertex)'s colour gradient and the camera's part of its signed distance's,
- * one 16-byte reduction for a vertex of a triangle that a warp hits where the
- * separate tensors take four of 4 bytes. */
+ * one 16-byte reduction per vertex for a hit, or for a warp's hits of a large
+ * triangle, where the separate tensors take four of 4 bytes. */
 MT_API int mt_intersect_and_composite_packed_backward(
     const float* xy, const float* colors, const float* signed_distances, int64_t V,
     const int32_t* faces, const float* sharpness, const int64_t* sorted_keys,

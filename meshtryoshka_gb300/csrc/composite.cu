@@ -31,8 +31,8 @@
 // bits instead of testing again (gathering only the triangles some pixel
 // hits), re-solves each hit's barycentrics and applies the suffix trick of
 // the reference. Batches past the capacity are tested again. Hits' gradients
-// go to their triangles' three vertices in global memory, summed first over the
-// warp's lanes that hold hits of one triangle: colour and signed distance of a
+// go to their triangles' three vertices in global memory, summed first where many
+// of the warp's lanes hold hits of one triangle: colour and signed distance of a
 // (camera, vertex) side by side, one 16-byte reduction each.
 // Two routings:
 //   reference (exact_adjoint = 0): the deferred gradient of the previous
@@ -1202,20 +1202,29 @@ __global__ void __launch_bounds__(32 * kWarps, 32 / kWarps)
 }
 
 // Adds a hit's gradient to its triangle's vertices, as one 16-byte reduction for
-// each (colour and signed distance). The lanes here that hold hits of one
-// triangle (`at` names it) are summed first, along the chain of their lanes in a
-// logarithm of steps, and the lowest of them adds the sums: a vertex of large
-// triangles gets one rounded addition for a warp's hits, not up to 32 (two
-// shells of triangles of 600 px at 1024^2: largest relative error 2e-6 to 5e-6,
-// 2e-5 with every hit added by itself). The sums cost the kernel 115 to 122 us
-// in the 256^3 step and 1.06 to 1.16 ms in the 512^3 step, whose triangles have
-// one to four hits in a warp. (Per triangle in shared memory, over a batch, they
-// cost more: shared-memory float additions are loops of compare-and-swap; 195 us
-// and 2.20 ms.)
-__device__ __forceinline__ void scatter(const CompositeArgs& a, const CompositeGrads& gr, int cam, int lane, int at,
-                                        int3 vid, float u, float v, float w, const float (&drgb)[3], float dsdf) {
-  if (drgb[0] == 0.f && drgb[1] == 0.f && drgb[2] == 0.f && dsdf == 0.f) return;
-  const uint32_t live = __activemask();
+// each (colour and signed distance). Where kTogether lanes or more hold hits of
+// one triangle here (`at` names it), they are summed first, along the chain of
+// their lanes in a logarithm of steps, and the lowest of them adds the sums: a
+// vertex of large triangles gets one rounded addition for a warp's hits, not up
+// to 32. Colour gradients of two shells against 64 bits (relative, root mean
+// square): cells of 512 px at 1024^2 1.7e-6 (every hit added by itself 1e-5), of
+// 32 px at 512^2 2.0e-7 (7.4e-7), of 8 px 1.2e-7 (2.1e-7). From two lanes on
+// another tenth to sixth of the error goes, at much the same time; but a fine mesh's
+// sums, one to four hits to a warp, then stray as far from the oracle's
+// hit-by-hit ones as its tests allow (entries that nearly cancel, 1e-4). The
+// kernel takes 118 us in the 256^3 step (single hits 115), 1.08 ms in the 512^3
+// step (1.06). (Per triangle in shared memory, over a batch, 195 us and 2.20 ms:
+// shared-memory float additions are loops of compare-and-swap.)
+constexpr int kTogether = 6;
+
+__device__ __forceinline__ bool any_gradient(const float (&drgb)[3], float dsdf) {
+  return drgb[0] != 0.f || drgb[1] != 0.f || drgb[2] != 0.f || dsdf != 0.f;
+}
+
+// `live`: the lanes that are here together.
+__device__ __forceinline__ void scatter(const CompositeArgs& a, const CompositeGrads& gr, int cam, int lane,
+                                        uint32_t live, int at, int3 vid, float u, float v, float w,
+                                        const float (&drgb)[3], float dsdf) {
   const uint32_t group = __match_any_sync(live, at);
   const float wt[3] = {u, v, w};
   float g[3][4];
@@ -1225,22 +1234,25 @@ __device__ __forceinline__ void scatter(const CompositeArgs& a, const CompositeG
     for (int c = 0; c < 3; ++c) g[q][c] = wt[q] * drgb[c];
     g[q][3] = wt[q] * dsdf;
   }
-  const uint32_t above = group & (0xfffffffeu << lane);
-  int next = above ? __ffs(above) - 1 : 32;  // the next lane whose sum is not in this one's
-  while (__any_sync(live, next < 32)) {
-    const bool more = next < 32;
-    const int from = more ? next : lane;
+  const bool together = __popc(group) >= kTogether;
+  if (__any_sync(live, together)) {
+    const uint32_t above = together ? group & (0xfffffffeu << lane) : 0u;
+    int next = above ? __ffs(above) - 1 : 32;  // the next lane whose sum is not in this one's
+    while (__any_sync(live, next < 32)) {
+      const bool more = next < 32;
+      const int from = more ? next : lane;
 #pragma unroll
-    for (int q = 0; q < 3; ++q)
+      for (int q = 0; q < 3; ++q)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float x = __shfl_sync(live, g[q][c], from);
-        if (more) g[q][c] += x;
-      }
-    const int after = __shfl_sync(live, next, from);
-    next = more ? after : 32;
+        for (int c = 0; c < 4; ++c) {
+          const float x = __shfl_sync(live, g[q][c], from);
+          if (more) g[q][c] += x;
+        }
+      const int after = __shfl_sync(live, next, from);
+      next = more ? after : 32;
+    }
+    if (together && lane != __ffs(group) - 1) return;
   }
-  if (lane != __ffs(group) - 1) return;
   const int id[3] = {vid.x, vid.y, vid.z};
   if (gr.packed) {
     float4* rows = gr.packed + (int64_t)cam * a.V;
@@ -1407,14 +1419,20 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
       pop(walk, nb);
     }
     if (!stored && active) hits = batch_hits(ws.geo, nb, px.fx, px.fy, last_shell, ws.saved, lane);
-    if (active) {
-      int n = 0;
-      while (hits) {
-        const int i = __ffs(hits) - 1;
+    // Rounds of a hit to each lane, whose lanes add their gradients together.
+    if (!active) hits = 0u;
+    for (int n = 0;;) {
+      int i = -1, k = 0;
+      while (i < 0 && hits) {
+        const int at = __ffs(hits) - 1;
         hits &= hits - 1;
-        const int k = n++;
+        k = n++;
+        if (ws.geo[at].shell > last_shell) i = at;
+      }
+      const uint32_t round = __ballot_sync(0xffffffffu, i >= 0);
+      if (round == 0u) break;
+      if (i >= 0) {
         const TriGeom& g = ws.geo[i];
-        if (g.shell <= last_shell) continue;
         float u, v, w;
         if (stored)
           hit_test(g, px.fx, px.fy, u, v, w);  // a hit: the solve gives the forward's (u, v, w)
@@ -1455,10 +1473,12 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
         const float ko = outer_cdf * outer_cdf * e_out;
         d_sharp += d_ic * ki * sdf_in + d_oc * ko * outer_sdf;
 
-        if (last_shell != -1) {
-          dp_sdf += d_oc * ko * s;
+        if (last_shell != -1) dp_sdf += d_oc * ko * s;
+        const bool add = last_shell != -1 && any_gradient(dp_rgb, dp_sdf);
+        const uint32_t live = __ballot_sync(round, add);
+        if (add) {
           const float su = gr.exact ? pu : u, sv = gr.exact ? pv : v, sw = gr.exact ? pw : w;
-          scatter(a, gr, cam, lane, prev_at, prev_vid, su, sv, sw, dp_rgb, dp_sdf);
+          scatter(a, gr, cam, lane, live, prev_at, prev_vid, su, sv, sw, dp_rgb, dp_sdf);
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) dp_rgb[c] = d_color[c];
@@ -1476,7 +1496,7 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
         last_shell = g.shell;
         if (last_shell == a.S - 1) {
           active = false;
-          break;
+          hits = 0u;
         }
       }
     }
@@ -1495,7 +1515,9 @@ __device__ __forceinline__ bool backward_item(const CompositeArgs& a, const uint
     }
   }
   // The last hit's deferred gradient, with its own weights.
-  if (px.in_image && last_shell != -1) scatter(a, gr, cam, lane, prev_at, prev_vid, pu, pv, pw, dp_rgb, dp_sdf);
+  const bool add = px.in_image && last_shell != -1 && any_gradient(dp_rgb, dp_sdf);
+  const uint32_t live = __ballot_sync(0xffffffffu, add);
+  if (add) scatter(a, gr, cam, lane, live, prev_at, prev_vid, pu, pv, pw, dp_rgb, dp_sdf);
 
   // Sharpness gradient: one atomic per warp.
   float x = px.in_image ? d_sharp : 0.f;

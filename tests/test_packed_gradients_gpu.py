@@ -138,7 +138,8 @@ def test_hits_of_a_warp_are_summed_first(cuda_device, monkeypatch, tile):
     2^24, where floats lie 2 apart: a hit's own contribution (below 1) would leave
     a row as it is, the sum over a warp's block of 8x4 pixels does not. Every
     addition rounds by at most 1, so a row misses 2^24 and its sum by at most the
-    number of (block, triangle) pairs around its vertex."""
+    additions to it: one for every block and triangle around its vertex with six
+    pixels or more in common, else one for each pixel."""
     d, size, start = cuda_device, 512, 2.0**24
     inner_init = tr._PackedGradients.__init__
 
@@ -178,7 +179,7 @@ def test_hits_of_a_warp_are_summed_first(cuda_device, monkeypatch, tile):
 
     pixels = torch.arange(size, device=d, dtype=torch.float64) + 0.5
     points = torch.stack(torch.meshgrid(pixels, pixels, indexing="xy"), -1).view(-1, 2)
-    sums, blocks = (torch.zeros(v, dtype=torch.float64, device=d) for _ in range(2))
+    sums, additions = (torch.zeros(v, dtype=torch.float64, device=d) for _ in range(2))
     free = torch.ones(len(points), dtype=torch.bool, device=d)
 
     def cross(p, q, r):
@@ -188,8 +189,9 @@ def test_hits_of_a_warp_are_summed_first(cuda_device, monkeypatch, tile):
         p = xy[corner].double()
         weights = torch.stack([cross(p[(q + 1) % 3], p[(q + 2) % 3], points) for q in range(3)], -1)
         weights /= cross(p[0], p[1], p[2])
-        touched = (weights >= -1e-3).all(-1)  # and pixels that rounding may give to this side
-        blocks[corner] += touched.view(size // 4, 4, size // 8, 8).any(3).any(1).sum()
+        # Pixels of the blocks that are the triangle's, and that rounding may make so.
+        sure, most = ((weights >= x).all(-1).view(size // 4, 4, size // 8, 8).sum((1, 3)) for x in (1e-3, -1e-3))
+        additions[corner] += torch.where(sure >= 6, most.clamp(max=1), most).sum()
         inside = (weights >= 0).all(-1) & free  # weights agree where two triangles meet
         free &= ~inside
         sums[corner] += weights[inside].sum(0)
@@ -199,7 +201,7 @@ def test_hits_of_a_warp_are_summed_first(cuda_device, monkeypatch, tile):
         inner = 1.0 / (1.0 + np.exp(-float(np.float32(level)) * sharpness))
         alpha = min(max((outer - inner + 1e-5) / (outer + 1e-5), 0.0), 1.0)
         want = 2.0 * light * alpha * sums
-        assert 2.0 * light * alpha < 1.0 and float((want / blocks).min()) > 1.5  # the test tells the two apart
+        assert 2.0 * light * alpha < 1.0 and float((want / additions).min()) > 1.5  # the test tells the two apart
         light, outer = light * (1.0 - alpha), inner
         off = (got[0, shell * v:(shell + 1) * v].double() - start - want[:, None]).abs()
-        assert float((off / blocks[:, None]).max()) <= 1.0
+        assert float((off / additions[:, None]).max()) <= 1.0
