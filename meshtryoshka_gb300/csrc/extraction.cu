@@ -2010,8 +2010,9 @@ int mt_count_triangle_faces_bytes(const float* signed_distances, const int32_t* 
                                   const int32_t* upper_corners, int64_t Nv, const float* level_sets, int32_t S,
                                   uint8_t* face_counts, uint8_t* cell_codes, mt_stream_t stream) {
   MT_REQUIRE(G >= 0 && Nv >= 0 && S >= 0);
+  MT_REQUIRE(Nv == 0 || (signed_distances && lower_corners && upper_corners && cell_codes));
   if (Nv == 0 || S == 0) return MT_OK;
-  MT_REQUIRE(signed_distances && lower_corners && upper_corners && level_sets && face_counts && cell_codes);
+  MT_REQUIRE(level_sets && face_counts);
   count_faces_kernel<<<grid_stride_blocks(Nv, 256), 256, 0, as_stream(stream)>>>(
       signed_distances, lower_corners, G, upper_corners, Nv, level_sets, S, face_counts, cell_codes);
   MT_CHECK_LAUNCH();

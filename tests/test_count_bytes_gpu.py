@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 import torch
 
+from meshtryoshka_gb300 import pipeline
 from meshtryoshka_gb300 import triangle_extraction as te
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +56,13 @@ def test_offsets_and_faces(cuda_device, side, shells, nans):
         live = min(faces, f)
         assert torch.equal(got.faces[:live], want.faces[:live])
         assert torch.equal(got.voxel_indices[:live], want.voxel_indices[:live])
+
+
+@pytest.mark.parametrize("counted", [False, True])
+def test_no_level_sets_are_refused(cuda_device, counted):
+    w = pipeline.build_workload("small", cuda_device)
+    v = w.voxels
+    args = (w.grid_sdf.detach(), v.vertices, w.grid_sh.detach(), v.neighbors, v.lower_corners, v.upper_corners,
+            v.indices, w.level_sets[:0])
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        te.tessellate_voxels_counted(*args, 10, 10) if counted else te.tessellate_voxels(*args)
